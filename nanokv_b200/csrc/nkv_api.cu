@@ -265,6 +265,14 @@ int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
               "decode_rows: %d rows requested from %d tokens", n, hist->tokens);
   NKV_REQUIRE(decoder_dtype == NKV_F32 || decoder_dtype == NKV_BF16, NKV_ERR_INVALID,
               "decode_rows: decoder dtype");
+  auto aligned = [](const void* pointer) { return (reinterpret_cast<uintptr_t>(pointer) & 15) == 0; };
+  // bf16 operators and rows: the tensor-core kernel (same two roundings); fp32 operators, other result
+  // types and shapes it does not tile: the CUDA-core kernel
+  if (decoder_dtype == NKV_BF16 && out_dtype == NKV_BF16 && !simt_forced() && hist->tokens > 0 &&
+      tc_decode_supported(*hist, J) && aligned(decoder) && aligned(mean) && aligned(out)) {
+    DecodeTensor t{hist, decoder, mean, rows_index, out, J, 0, nullptr, nullptr};
+    return tc_decode(&t, 1, n, J, J, false, true, nullptr, sm_count(), static_cast<cudaStream_t>(stream));
+  }
   return simt_decode_rows(*hist, rows_index, n, decoder, decoder_dtype, mean, J, out, out_dtype,
                           static_cast<cudaStream_t>(stream));
 }

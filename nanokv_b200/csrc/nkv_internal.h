@@ -72,6 +72,22 @@ int tc_attn_codec(const void* q, int64_t q_stride_token, int64_t q_stride_head, 
 int tc_prepare_decoder(const void* w_bf16, int64_t rows, int rank, void* out_bf16, cudaStream_t stream);
 bool tc_attn_supported(int dk, int dv, int rank);
 int tc_wait_expiry_selftest(int kind, long long budget_cycles, int32_t* status_word, cudaStream_t stream);
+// One tensor of a row decode: element (row, head, column) of the result goes to
+// out[row * row_stride + head * head_stride + column]
+struct DecodeTensor {
+  const nkv_history* hist;
+  const void* decoder;       // bf16 [J, rank]
+  const float* bias;         // f32 [J]
+  const int32_t* rows;       // listed rows, or NULL
+  void* out;
+  int64_t row_stride, head_stride;
+  const nkv_rope* rope;      // or NULL
+  const nkv_camera* camera;  // or NULL
+};
+bool tc_decode_supported(const nkv_history& h, int J);
+int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool w_perm, bool round_bias,
+              int32_t* status, int sms, cudaStream_t stream);
+int sm_count();
 bool tc_project_supported(int J, int r);
 bool tc_project_quant_supported(int J, int r, int group);
 int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,

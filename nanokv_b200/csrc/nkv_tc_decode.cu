@@ -1,0 +1,526 @@
+// Rows of a compressed history rebuilt on tcgen05 tensor cores, one or two tensors per launch:
+//   row[t] = bf16(bf16(latent[t] decoder^T + bias) + centre[t]),  latent[t] = bf16(code * scale),
+// plus the positional restore (rotation, camera transform) where the caller asks for it.
+//
+// The product is [n tokens x rank] x [J x rank]^T.  A cluster of two CTAs owns a tile of 256 tokens
+// (128 per CTA) and computes 256 columns of J at a time with cta_group::2 MMAs: the tile's codes are
+// expanded ONCE into bf16 latents that stay in shared memory for all of its columns (160 KB at rank
+// 640), and only decoder rows are streamed (TMA, each CTA of a pair loads half of the 256 rows, so a
+// pair reads every decoder byte once per 256 tokens: 64 bytes per clock and SM at the full MMA rate;
+// one CTA on its own would need 128, which the L2 does not deliver to 148 SMs).  Two accumulators of
+// 256 columns in TMEM: the epilogue of a tile runs under the MMAs of the next one.
+//
+// Work is the list of (tensor, 256-token tile, 256-column tile) in that order; every cluster takes a
+// contiguous run of equal length, so the last wave is never emptier than one tile and a run expands
+// two or three token tiles.  No wait crosses clusters.
+//
+// Bound: the decoder stream from L2 into three 16 KB stages (all that 160 KB of latents leave at rank
+// 640).  28,080 rows x 5,120 columns at rank 640, K and V (two calls): 0.545 ms = 675 TFLOP/s; the
+// CUDA-core kernel that served bf16 operators before took 17.9 ms.
+//
+// Warps 0-7: expansion and epilogue (warp w serves TMEM lanes 32 (w & 3) .. and column half w >> 2),
+// warp 8 lane 0: TMA, warp 9 of the even CTA: MMA.
+#include "nkv_internal.h"
+#include "nkv_tc.cuh"
+#include "nkv_tc_dequant.cuh"
+
+namespace nkv {
+namespace {
+
+using namespace tc;
+
+constexpr int TM = 128;                     // tokens per CTA (256 per cluster)
+constexpr int TN = 256;                     // columns per accumulator
+constexpr int COMPUTE_WARPS = 8;
+constexpr int THREADS = COMPUTE_WARPS * 32 + 64;
+constexpr int CHUNK_BYTES = TM * 128;       // [128 rows x 64 bf16], 128-byte swizzle
+constexpr int MAX_CHUNKS = 10;              // rank <= 640
+constexpr int MAX_STAGES = 8;
+constexpr int META = 1024;
+constexpr int SCRATCH = COMPUTE_WARPS * 2048;
+constexpr size_t SMEM_LIMIT = 232448;
+
+enum Bar { FULL = 0, FREE = 8, A_FULL = 16, ACC_FULL = 26, ACC_FREE = 28, NUM_BARS = 30 };
+
+struct Tensor {
+  nkv_history h;
+  const float* bias;
+  const int32_t* rows;        // listed rows, or NULL: rows 0 .. n
+  uint16_t* out;              // element (row, head, column): row * row_stride + head * head_stride + column
+  long long row_stride, head_stride;
+  nkv_rope rope;              // cos_sin == NULL: none
+  nkv_camera cam;             // matrices == NULL: none
+};
+
+struct Params {
+  Tensor t[2];
+  int tensors, n, J, D, nchunks, ngroups, group, w_perm, round_bias, nstages;
+  int m_tiles, n_tiles, total;
+  int32_t* status;
+};
+
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y,
+                                                 uint32_t bar_cluster_addr) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar_cluster_addr)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot_in_smem, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                   smem_u32(slot_in_smem)), "r"(columns) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns)
+               : "memory");
+}
+// D[256 x N over the pair] (+)= A B^T; each CTA holds its 128 rows of A and half of B's rows
+__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                              uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
+      : "memory");
+}
+// one arrival on the barrier at this offset in both CTAs of the pair once the MMAs issued so far are done
+__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+      " [%0], %1;" ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+
+// a run of column tiles of one token tile
+struct Run { int tensor, m, nt0, count; };
+__device__ __forceinline__ Run run_at(const Params& p, int w, int w_end) {
+  Run r;
+  const int seg = w / p.n_tiles;
+  r.nt0 = w - seg * p.n_tiles;
+  r.count = min(p.n_tiles - r.nt0, w_end - w);
+  r.tensor = seg / p.m_tiles;
+  r.m = seg - r.tensor * p.m_tiles;
+  return r;
+}
+
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code) ? 1 : 0) != 0;
+}
+
+template <bool POS>
+__global__ void __launch_bounds__(THREADS, 1)
+decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_constant__ CUtensorMap map_1,
+                   const __grid_constant__ Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + NUM_BARS * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + NUM_BARS * 8 + 4);
+  uint8_t* a_tiles = smem + META;
+  uint8_t* b_tiles = a_tiles + p.nchunks * CHUNK_BYTES;
+  uint8_t* scratch = b_tiles + p.nstages * CHUNK_BYTES;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t cta = cluster_ctarank();
+  const int clusters = gridDim.x >> 1, cluster = blockIdx.x >> 1;
+  const int w_begin = static_cast<int>(static_cast<long long>(p.total) * cluster / clusters);
+  const int w_end = static_cast<int>(static_cast<long long>(p.total) * (cluster + 1) / clusters);
+  const int nst = p.nstages, nchunks = p.nchunks;
+
+  if (tid == 0) {
+    for (int s = 0; s < MAX_STAGES; ++s) {
+      mbar_init(&bars[FULL + s], 1);
+      mbar_init(&bars[FREE + s], 1);
+    }
+    for (int c = 0; c < MAX_CHUNKS; ++c) mbar_init(&bars[A_FULL + c], 2 * COMPUTE_WARPS);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&bars[ACC_FULL + b], 1);
+      mbar_init(&bars[ACC_FREE + b], 2 * COMPUTE_WARPS);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  if (warp == 9) tmem_alloc_pair(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();      // the peer's barriers exist before anyone arrives on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 8) {
+    // ---------------------------------------------------------------- TMA: decoder rows
+    if (lane == 0) {
+      prefetch_tensormap(&map_0);
+      if (p.tensors > 1) prefetch_tensormap(&map_1);
+      bool ok = true;
+      int it = 0;
+      for (int w = w_begin; w < w_end && ok;) {
+        const Run r = run_at(p, w, w_end);
+        const CUtensorMap* map = r.tensor ? &map_1 : &map_0;
+        for (int k = 0; k < r.count && ok; ++k) {
+          const int y = (r.nt0 + k) * TN + static_cast<int>(cta) * TM;
+          for (int c = 0; c < nchunks; ++c, ++it) {
+            const int s = it % nst, u = it / nst;
+            if (u >= 1) ok = mbar_wait_cluster(&bars[FREE + s], (u - 1) & 1, abort_flag, 700 + s);
+            if (!ok) break;
+            // both halves land on the even CTA's barrier, whose MMA warp reads them
+            if (cta == 0) mbar_arrive_expect_tx(&bars[FULL + s], 2 * CHUNK_BYTES);
+            tma_load_2d_pair(b_tiles + s * CHUNK_BYTES, map, c * 64, y, map_to_cta(smem_u32(&bars[FULL + s]), 0));
+          }
+        }
+        w += r.count;
+      }
+      if (!ok) {   // let copies already in flight land before the CTA goes away
+        const long long start = clock64();
+        while (clock64() - start < (1ll << 21)) {}
+      }
+    }
+    __syncwarp();
+  } else if (warp == 9) {
+    if (cta == 0) {
+      // -------------------------------------------------------------- MMA issuer of the pair
+      const bool leader = elect_one();
+      const uint32_t idesc = make_idesc_bf16(2 * TM, TN);
+      const uint32_t a_base = smem_u32(a_tiles), b_base = smem_u32(b_tiles);
+      bool ok = true;
+      int it = 0, tile = 0, seg = 0;
+      for (int w = w_begin; w < w_end && ok; ++seg) {
+        const Run r = run_at(p, w, w_end);
+        for (int k = 0; k < r.count && ok; ++k, ++tile) {
+          const int b = tile & 1, use = tile >> 1;
+          if (use >= 1) ok = wait_all(&bars[ACC_FREE + b], (use - 1) & 1, abort_flag, 710 + b);
+          const uint32_t acc = tmem_base + b * TN;
+          for (int c = 0; c < nchunks && ok; ++c, ++it) {
+            const int s = it % nst, u = it / nst;
+            if (k == 0) ok = wait_all(&bars[A_FULL + c], seg & 1, abort_flag, 720 + c);
+            ok = ok && wait_all(&bars[FULL + s], u & 1, abort_flag, 730 + s);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t a_desc = make_smem_desc_sw128(a_base + c * CHUNK_BYTES);
+            const uint64_t b_desc = make_smem_desc_sw128(b_base + s * CHUNK_BYTES);
+            if (leader) {
+              mma_bf16_pair(acc, a_desc, b_desc, idesc, c > 0);
+              mma_bf16_pair(acc, a_desc + 2, b_desc + 2, idesc, true);
+              mma_bf16_pair(acc, a_desc + 4, b_desc + 4, idesc, true);
+              mma_bf16_pair(acc, a_desc + 6, b_desc + 6, idesc, true);
+              mma_commit_pair(&bars[FREE + s]);
+            }
+            __syncwarp();
+          }
+          if (ok && leader) mma_commit_pair(&bars[ACC_FULL + b]);
+          __syncwarp();
+        }
+        w += r.count;
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ expansion and epilogue
+    const int row = tid & 127, wg = tid >> 7, wrow0 = 32 * (warp & 3);
+    const uint32_t lane_sel = static_cast<uint32_t>(wrow0) << 16;
+    uint8_t* stage = scratch + warp * 2048;
+    bool ok = true;
+    int tile = 0;                       // tiles whose epilogue is done or pending, in order
+    auto arrive_even = [&](uint64_t* bar) {   // one arrival per warp on the even CTA's barrier
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(bar), 0));
+    };
+    // this lane's token of a run (its row of the tile): history row, or -1 past the end of the list
+    auto token_of = [&](const Run& r) {
+      const int m = (r.m * 2 + static_cast<int>(cta)) * TM + row;
+      if (m >= p.n) return -1;
+      const Tensor& t = p.t[r.tensor];
+      const int tok = t.rows != nullptr ? __ldg(t.rows + m) : m;
+      return tok < 0 || tok >= t.h.tokens ? -1 : tok;
+    };
+    auto expand = [&](const Run& r, int tok) {
+      const nkv_history& h = p.t[r.tensor].h;
+      const uint8_t* codes = h.codes + static_cast<size_t>(tok < 0 ? 0 : tok) * (h.rank >> 1) + wg * 16;
+      const uint16_t* scales = static_cast<const uint16_t*>(h.scales) + static_cast<size_t>(tok < 0 ? 0 : tok) * p.ngroups;
+      // half of the codes in flight at a time: 16 bytes of five chunks
+#pragma unroll
+      for (int half = 0; half < MAX_CHUNKS / 5; ++half) {
+        uint4 code[5];
+        uint16_t sbits[5];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          const int c = half * 5 + i;
+          code[i] = make_uint4(0, 0, 0, 0);
+          sbits[i] = 0;
+          if (c < nchunks && tok >= 0) {
+            code[i] = __ldg(reinterpret_cast<const uint4*>(codes + c * 32));
+            sbits[i] = __ldg(scales + (p.ngroups == 1 ? 0 : (c * 64 + wg * 32) / p.group));
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          const int c = half * 5 + i;
+          if (c < nchunks) {
+            const uint32_t words[4] = {code[i].x, code[i].y, code[i].z, code[i].w};
+            uint8_t* dst = a_tiles + c * CHUNK_BYTES;
+            const uint32_t pair = static_cast<uint32_t>(sbits[i]) * 0x00010001u;
+            const __nv_bfloat162 scale2 = *reinterpret_cast<const __nv_bfloat162*>(&pair);
+            const float sc = scale_to_float(sbits[i], h.scale_dtype);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              uint4 v;
+              if (h.scale_dtype == NKV_BF16) v = p.w_perm ? dequant8_bf16_perm(words[k], scale2) : dequant8_bf16(words[k], scale2);
+              else v = p.w_perm ? dequant8_perm(words[k], sc) : dequant8(words[k], sc);
+              *reinterpret_cast<uint4*>(dst + sw128_offset(row, wg * 32 + k * 8)) = v;
+            }
+            fence_proxy_async_all();       // the pair's MMAs read this through the async proxy
+            arrive_even(&bars[A_FULL + c]);
+          }
+        }
+      }
+    };
+    // columns [n0 + 128 wg, +128) of this warp's 32 rows, 32 columns at a time
+    auto epilogue = [&](const Run& r, int nt, int tok, int crow) {
+      const Tensor& t = p.t[r.tensor];
+      const int b = tile & 1, use = tile >> 1;
+      const int m0 = (r.m * 2 + static_cast<int>(cta)) * TM + wrow0;
+      const int rounds = min(4, max(0, (p.J - nt * TN - wg * 128) / 32));
+      // centre rows: 4 lanes read the 16-byte pieces of one row, 8 rows per load instruction; all
+      // rounds are requested ahead of the accumulator wait
+      int crow_of[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) crow_of[i] = __shfl_sync(0xffffffffu, tok < 0 ? -1 : crow, i * 8 + lane / 4);
+      uint4 cen_all[4][4];
+#pragma unroll
+      for (int sub = 0; sub < 4; ++sub) {
+        const uint16_t* cbase = static_cast<const uint16_t*>(t.h.centers) + nt * TN + wg * 128 + sub * 32 + (lane & 3) * 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          cen_all[sub][i] = make_uint4(0, 0, 0, 0);
+          if (sub < rounds && crow_of[i] >= 0)
+            cen_all[sub][i] = __ldg(reinterpret_cast<const uint4*>(cbase + static_cast<size_t>(crow_of[i]) * t.h.center_width));
+        }
+      }
+      // positional restore: this token's table rows
+      const bool rotate = POS && t.rope.cos_sin != nullptr;
+      int coord_t = 0, coord_h = 0, coord_w = 0;
+      const int band_a = t.rope.table_half - 2 * (t.rope.table_half / 3);
+      const int band_b = band_a + t.rope.table_half / 3;
+      if (rotate) {
+        const int pos = tok >= 0 ? max(__ldg(t.rope.positions + tok), 0) : 0;
+        const int last = t.rope.table_rows - 1;
+        if (t.rope.frame_seqlen == 0) {
+          coord_t = coord_h = coord_w = min(pos, last);
+        } else {
+          const int frame = pos / t.rope.frame_seqlen, spatial = pos - frame * t.rope.frame_seqlen;
+          const int prow = spatial / t.rope.width;
+          coord_t = min(frame, last);
+          coord_h = min(prow, last);
+          coord_w = min(spatial - prow * t.rope.width, last);
+        }
+      }
+      const bool transform = POS && t.cam.matrices != nullptr;
+      const float* cam_frame = nullptr;
+      if (transform)
+        cam_frame = t.cam.matrices + static_cast<size_t>(min(max(tok, 0) / t.cam.tokens_per_frame, t.cam.frames - 1)) * 64;
+
+      ok = wait_all(&bars[ACC_FULL + b], use & 1, abort_flag, 740 + b);
+      if (!ok) return;
+      tc_fence_after();
+#pragma unroll
+      for (int sub = 0; sub < 4; ++sub) {
+        if (sub >= rounds) break;
+        const int col0 = nt * TN + wg * 128 + sub * 32;
+        uint32_t acc_raw[32];
+        tmem_ld32_issue(tmem_base + lane_sel + b * TN + wg * 128 + sub * 32, acc_raw);
+        float bias[32];
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 b4 = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j));
+          bias[j] = b4.x; bias[j + 1] = b4.y; bias[j + 2] = b4.z; bias[j + 3] = b4.w;
+        }
+        if (p.round_bias) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) bias[j] = round_to_bf16(bias[j]);
+        }
+        uint4 cen[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int rloc = i * 8 + lane / 4, piece = lane & 3;
+          *reinterpret_cast<uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4)) = cen_all[sub][i];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          cen[j] = *reinterpret_cast<const uint4*>(stage + lane * 64 + ((j ^ (lane & 3)) << 4));
+        __syncwarp();
+        tmem_ld32_wait(acc_raw);
+        const int head = col0 / p.D, dcol = col0 - head * p.D;
+        uint32_t packed[16];
+#pragma unroll
+        for (int j4 = 0; j4 < 4; ++j4) {
+          const uint32_t cwords[4] = {cen[j4].x, cen[j4].y, cen[j4].z, cen[j4].w};
+          float block[8];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const int j = j4 * 8 + w * 2;
+            // two bf16 roundings: of (product + bias), then of (+ centre); the packed addition of two
+            // bf16 numbers rounds their exact sum once
+            const uint32_t first = pack_bf16x2(__uint_as_float(acc_raw[j]) + bias[j], __uint_as_float(acc_raw[j + 1]) + bias[j + 1]);
+            const __nv_bfloat162 sum = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&first),
+                                               *reinterpret_cast<const __nv_bfloat162*>(&cwords[w]));
+            packed[j4 * 4 + w] = *reinterpret_cast<const uint32_t*>(&sum);
+            if (POS) {
+              float x0 = __uint_as_float(packed[j4 * 4 + w] << 16), x1 = __uint_as_float(packed[j4 * 4 + w] & 0xFFFF0000u);
+              if (rotate) {   // the pair (x0, x1) of the rebuilt bf16 key is one complex number
+                const int local = dcol / 2 + j4 * 4 + w;
+                const int pg = t.rope.pair_index ? __ldg(t.rope.pair_index + head * (p.D / 2) + local) : local;
+                const int coord = pg < band_a ? coord_t : (pg < band_b ? coord_h : coord_w);
+                const float2 cs = __ldg(reinterpret_cast<const float2*>(t.rope.cos_sin) + static_cast<size_t>(coord) * t.rope.table_half + pg);
+                const float k0 = x0, k1 = x1;
+                x0 = fmaf(k0, cs.x, -(k1 * cs.y));
+                x1 = fmaf(k0, cs.y, k1 * cs.x);
+                packed[j4 * 4 + w] = pack_bf16x2(x0, x1);
+              }
+              block[2 * w] = x0;
+              block[2 * w + 1] = x1;
+            }
+          }
+          if (POS && transform) {   // the four two-element slots of the block, mixed by the frame's matrix
+            const int which = __ldg(t.cam.cam_index + head * (p.D / 8) + dcol / 8 + j4) & 3;
+            const float4* m = reinterpret_cast<const float4*>(cam_frame + which * 16);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) block[k] = round_to_bf16(block[k]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 mi = __ldg(m + i);
+              const float c0 = round_to_bf16(mi.x), c1 = round_to_bf16(mi.y);
+              const float c2 = round_to_bf16(mi.z), c3 = round_to_bf16(mi.w);
+              const float y0 = fmaf(c3, block[6], fmaf(c2, block[4], fmaf(c1, block[2], c0 * block[0])));
+              const float y1 = fmaf(c3, block[7], fmaf(c2, block[5], fmaf(c1, block[3], c0 * block[1])));
+              packed[j4 * 4 + i] = pack_bf16x2(y0, y1);
+            }
+          }
+        }
+        // through the warp's staging area, so that a store instruction writes whole 64-byte row pieces
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<uint4*>(stage + lane * 64 + ((j ^ (lane & 3)) << 4)) =
+              make_uint4(packed[j * 4], packed[j * 4 + 1], packed[j * 4 + 2], packed[j * 4 + 3]);
+        __syncwarp();
+        uint16_t* dst = t.out + head * t.head_stride + dcol + (lane & 3) * 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int rloc = i * 8 + lane / 4, piece = lane & 3;
+          const uint4 v = *reinterpret_cast<const uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4));
+          if (crow_of[i] >= 0) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(m0 + rloc) * t.row_stride) = v;
+        }
+        __syncwarp();
+      }
+      tc_fence_before();
+      arrive_even(&bars[ACC_FREE + b]);
+      ++tile;
+    };
+
+    Run prev{};
+    int prev_tok = -1, prev_crow = 0;
+    bool pending = false;      // the last column tile of the previous run awaits its epilogue
+    for (int w = w_begin; w < w_end && ok;) {
+      const Run r = run_at(p, w, w_end);
+      const int tok = token_of(r);
+      const int crow = tok < 0 ? 0 : center_row_of(p.t[r.tensor].h, tok);
+      // the latents in shared memory are free once the previous run's last tile is complete; the new
+      // ones go in before that tile's epilogue, so that the MMAs of this run start under it
+      if (pending) ok = wait_all(&bars[ACC_FULL + (tile & 1)], (tile >> 1) & 1, abort_flag, 750);
+      if (!ok) break;
+      expand(r, tok);
+      if (pending) epilogue(prev, prev.nt0 + prev.count - 1, prev_tok, prev_crow);
+      for (int k = 0; k + 1 < r.count && ok; ++k) epilogue(r, r.nt0 + k, tok, crow);
+      prev = r;
+      prev_tok = tok;
+      prev_crow = crow;
+      pending = true;
+      w += r.count;
+    }
+    if (ok && pending) epilogue(prev, prev.nt0 + prev.count - 1, prev_tok, prev_crow);
+  }
+  tc_fence_before();
+  __syncthreads();
+  // neither CTA leaves while the other may still arrive on its barriers or read its operands
+  cluster_sync_all();
+  if (warp == 9) tmem_dealloc_pair(tmem_base, 512);
+  if (tid == 0 && *abort_flag && p.status) atomicCAS(p.status, 0, *abort_flag);
+}
+
+size_t smem_bytes(int nchunks, int stages) {
+  return 1024 + META + static_cast<size_t>(nchunks + stages) * CHUNK_BYTES + SCRATCH;
+}
+
+}  // namespace
+
+bool tc_decode_supported(const nkv_history& h, int J) {
+  return h.rank % 64 == 0 && h.rank <= 64 * MAX_CHUNKS && J % 64 == 0 && h.center_width % 8 == 0 &&
+         (h.group == 32 || h.group % 64 == 0) && h.rank % h.group == 0 &&
+         ((reinterpret_cast<uintptr_t>(h.codes) | reinterpret_cast<uintptr_t>(h.centers)) & 15) == 0;
+}
+
+int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool w_perm, bool round_bias,
+              int32_t* status, int sms, cudaStream_t stream) {
+  if (n == 0) return NKV_OK;
+  Params p{};
+  CUtensorMap maps[2];
+  bool positional = false;
+  for (int i = 0; i < count; ++i) {
+    const DecodeTensor& src = tensors[i];
+    Tensor& t = p.t[i];
+    t.h = *src.hist;
+    t.bias = src.bias;
+    t.rows = src.rows;
+    t.out = static_cast<uint16_t*>(src.out);
+    t.row_stride = src.row_stride;
+    t.head_stride = src.head_stride;
+    if (src.rope != nullptr) { t.rope = *src.rope; positional = true; }
+    if (src.camera != nullptr) { t.cam = *src.camera; positional = true; }
+    uint64_t dims[2] = {static_cast<uint64_t>(t.h.rank), static_cast<uint64_t>(J)};
+    uint64_t strides[1] = {static_cast<uint64_t>(t.h.rank) * 2};
+    uint32_t box[2] = {64, TM};
+    int rc = encode_tensor_map(&maps[i], 2, src.decoder, 2, dims, strides, box, 128);
+    if (rc != NKV_OK) return rc;
+  }
+  if (count == 1) maps[1] = maps[0];
+  const nkv_history& h = p.t[0].h;
+  p.tensors = count;
+  p.n = n; p.J = J; p.D = D;
+  p.nchunks = h.rank / 64;
+  p.group = h.group;
+  p.ngroups = h.rank / h.group;
+  p.w_perm = w_perm ? 1 : 0;
+  p.round_bias = round_bias ? 1 : 0;
+  p.nstages = MAX_STAGES;
+  while (p.nstages > 2 && smem_bytes(p.nchunks, p.nstages) > SMEM_LIMIT) --p.nstages;
+  const size_t smem = smem_bytes(p.nchunks, p.nstages);
+  p.m_tiles = ceil_div(n, 2 * TM);
+  p.n_tiles = ceil_div(J, TN);
+  p.total = count * p.m_tiles * p.n_tiles;
+  p.status = status;
+  const int pairs = p.total < sms / 2 ? p.total : sms / 2;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(2 * pairs);
+  config.blockDim = dim3(THREADS);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  auto kernel = positional ? decode_gemm_kernel<true> : decode_gemm_kernel<false>;
+  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  NKV_CUDA(cudaLaunchKernelEx(&config, kernel, maps[0], maps[1], p));
+  return NKV_OK;
+}
+
+}  // namespace nkv

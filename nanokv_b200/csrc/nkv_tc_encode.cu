@@ -427,12 +427,8 @@ bool tc_project_supported(int J, int r) {
          smem_bytes(nacc, nb, 0) <= 232448;
 }
 
-// Tokens per CTA (<= TM): the MMA always spans TM rows, but the operand build, the loads and the
-// epilogue scale with the rows a CTA owns, so the token tiles are sized to fill whole rounds of the
-// SMs instead of leaving the last round mostly empty (12,480 tokens: 147 CTAs of 85 rows instead
-// of 98 of 128).  Not below 64 rows: every CTA streams the whole B operand from L2.
-int pick_rows(int S, int column_parts) {
-  // SM count of the current device, cached per device ordinal
+// SM count of the current device, cached per device ordinal
+int sm_count() {
   static std::atomic<int> cached[64];
   int device = 0, sms = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) device = -1;
@@ -443,6 +439,15 @@ int pick_rows(int S, int column_parts) {
       sms = 148;
     if (device >= 0) cached[device].store(sms, std::memory_order_relaxed);
   }
+  return sms;
+}
+
+// Tokens per CTA (<= TM): the MMA always spans TM rows, but the operand build, the loads and the
+// epilogue scale with the rows a CTA owns, so the token tiles are sized to fill whole rounds of the
+// SMs instead of leaving the last round mostly empty (12,480 tokens: 147 CTAs of 85 rows instead
+// of 98 of 128).  Not below 64 rows: every CTA streams the whole B operand from L2.
+int pick_rows(int S, int column_parts) {
+  const int sms = sm_count();
   const long long units = static_cast<long long>(ceil_div(S, TM)) * column_parts;
   const long long waves = (units + sms - 1) / sms;
   const long long tiles = waves * sms / column_parts;
