@@ -369,6 +369,26 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
                        float scale, void* out, float* lse, int32_t* status_word, int splits,
                        void* workspace, size_t workspace_bytes, void* stream);
 
+/*
+ * The read of nkv_attn_codec_pos with K and V rows rebuilt in `workspace` a batch of heads at a time
+ * (at most 512 MB of rows, at least one head) and then attended: two kernels per batch, same
+ * arithmetic, and no state shared between launches.  It is the faster form wherever its workspace is
+ * affordable; nkv_attn_codec_pos stays for callers that hand out no such memory and for ranks above
+ * 640.  `splits`: upper bound of the history splits, 0: the library's choice.
+ * nkv_attn_codec_rows_workspace_bytes is 0 where this form does not apply (fp32, rank above 640,
+ * head widths other than 64 and 128).
+ */
+size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, int dv, int tokens,
+                                           int rank, int group, int splits);
+int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
+                        int Q, int heads, int dk, int dv,
+                        const nkv_history* hist_k, const nkv_history* hist_v,
+                        const void* wk, const float* bias_k, const void* wv, const float* bias_v,
+                        int weight_order,
+                        const nkv_rope* rope, const nkv_camera* camera_k, const nkv_camera* camera_v,
+                        float scale, void* out, float* lse, int32_t* status_word, int splits,
+                        void* workspace, size_t workspace_bytes, void* stream);
+
 /* The camera transform applied to explicit rows x [S, heads, d] (reduced queries with P^T,
  * attention outputs with P): out [S, heads, d] contiguous, same dtype. */
 int nkv_camera_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head, int S,
@@ -395,6 +415,19 @@ int nkv_attention_lse(const void* q, const void* k, const void* v, int dtype,
                       int64_t kv_stride_token, int64_t kv_stride_head,
                       int Q, int N, int heads, int d, int dv, float scale,
                       void* out, float* lse, void* stream);
+
+/*
+ * The same on the tensor cores, for bf16 rows with d == dv in {64, 128}, N > 0, 16-byte aligned rows
+ * and strides in multiples of 8 elements.  status_word as for nkv_attn_codec.  workspace:
+ * nkv_attention_lse_workspace_bytes bytes for history splits, or NULL (one split).
+ */
+size_t nkv_attention_lse_workspace_bytes(int Q, int heads, int d, int N);
+int nkv_attention_lse_bf16(const void* q, const void* k, const void* v,
+                           int64_t q_stride_token, int64_t q_stride_head,
+                           int64_t kv_stride_token, int64_t kv_stride_head,
+                           int Q, int N, int heads, int d, int dv, float scale,
+                           void* out, float* lse, int32_t* status_word,
+                           void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * P-way log-sum-exp merge of attention partials: lse = logsumexp_p lse_p,

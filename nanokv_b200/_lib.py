@@ -84,6 +84,12 @@ SIGNATURES = {
                                    c_void_p, c_void_p, c_int, POINTER(Rope), POINTER(Camera), POINTER(Camera),
                                    c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_size_t,
                                    c_void_p]),
+    "nkv_attn_codec_rows_workspace_bytes": (c_size_t, [c_int] * 9),
+    "nkv_attn_codec_rows": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int, c_int, c_int, c_int,
+                                    POINTER(History), POINTER(History), c_void_p, c_void_p,
+                                    c_void_p, c_void_p, c_int, POINTER(Rope), POINTER(Camera), POINTER(Camera),
+                                    c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_size_t,
+                                    c_void_p]),
     "nkv_decoder_prepare": (c_int, [c_void_p, c_int64, c_int, c_void_p, c_void_p]),
     "nkv_camera_rows": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int, c_int, c_int, POINTER(Camera),
                                 c_void_p, c_void_p]),
@@ -92,6 +98,10 @@ SIGNATURES = {
     "nkv_attention_lse": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_int64,
                                   c_int64, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                   c_void_p, c_void_p]),
+    "nkv_attention_lse_workspace_bytes": (c_size_t, [c_int] * 4),
+    "nkv_attention_lse_bf16": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
+                                       c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p,
+                                       c_void_p, c_void_p, c_size_t, c_void_p]),
     "nkv_lse_merge": (c_int, [POINTER(c_void_p), POINTER(c_void_p), c_int, c_int64, c_int, c_int,
                               c_void_p, c_void_p, c_void_p]),
     "nkv_history_moments_workspace_bytes": (c_size_t, [c_int, c_int]),

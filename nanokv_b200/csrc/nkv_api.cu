@@ -346,13 +346,9 @@ int nkv_attn_codec_rope(const void* q, int dtype, int64_t q_stride_token, int64_
                             out, lse, status_word, splits, workspace, workspace_bytes, stream);
 }
 
-int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
-                       int Q, int heads, int dk, int dv, const nkv_history* hist_k,
-                       const nkv_history* hist_v, const void* wk, const float* bias_k,
-                       const void* wv, const float* bias_v, int weight_order, const nkv_rope* rope,
-                       const nkv_camera* camera_k, const nkv_camera* camera_v, float scale,
-                       void* out, float* lse, int32_t* status_word, int splits, void* workspace,
-                       size_t workspace_bytes, void* stream) {
+static int check_read(int dtype, int Q, int heads, int dk, int dv, const nkv_history* hist_k,
+                      const nkv_history* hist_v, int weight_order, const nkv_rope* rope,
+                      const nkv_camera* camera_k, const nkv_camera* camera_v) {
   int rc = check_history(hist_k, "K");
   if (rc != NKV_OK) return rc;
   rc = check_history(hist_v, "V");
@@ -362,10 +358,6 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
               NKV_ERR_INVALID, "K and V histories differ in tokens / rank / group / scale dtype");
   NKV_REQUIRE(dtype == NKV_F32 || dtype == NKV_BF16, NKV_ERR_INVALID, "attn_codec: dtype");
   NKV_REQUIRE(Q >= 0 && heads >= 0, NKV_ERR_INVALID, "attn_codec: Q=%d heads=%d", Q, heads);
-  NKV_REQUIRE(splits >= 1 && splits <= 16, NKV_ERR_INVALID, "attn_codec: splits=%d (1..16)", splits);
-  NKV_REQUIRE(workspace_bytes >= nkv_attn_codec_workspace_bytes(Q, heads, dv, splits),
-              NKV_ERR_INVALID, "attn_codec: workspace of %zu bytes is too small for %d splits",
-              workspace_bytes, splits);
   const bool prepared = weight_order == NKV_WEIGHTS_KERNEL_ORDER;
   NKV_REQUIRE(weight_order == NKV_WEIGHTS_NATURAL || prepared, NKV_ERR_INVALID,
               "attn_codec: weight_order=%d", weight_order);
@@ -384,6 +376,23 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
     rc = check_camera(camera_v, dv);
     if (rc != NKV_OK) return rc;
   }
+  return NKV_OK;
+}
+
+int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
+                       int Q, int heads, int dk, int dv, const nkv_history* hist_k,
+                       const nkv_history* hist_v, const void* wk, const float* bias_k,
+                       const void* wv, const float* bias_v, int weight_order, const nkv_rope* rope,
+                       const nkv_camera* camera_k, const nkv_camera* camera_v, float scale,
+                       void* out, float* lse, int32_t* status_word, int splits, void* workspace,
+                       size_t workspace_bytes, void* stream) {
+  int rc = check_read(dtype, Q, heads, dk, dv, hist_k, hist_v, weight_order, rope, camera_k, camera_v);
+  if (rc != NKV_OK) return rc;
+  NKV_REQUIRE(splits >= 1 && splits <= 16, NKV_ERR_INVALID, "attn_codec: splits=%d (1..16)", splits);
+  NKV_REQUIRE(workspace_bytes >= nkv_attn_codec_workspace_bytes(Q, heads, dv, splits),
+              NKV_ERR_INVALID, "attn_codec: workspace of %zu bytes is too small for %d splits",
+              workspace_bytes, splits);
+  const bool prepared = weight_order == NKV_WEIGHTS_KERNEL_ORDER;
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == NKV_BF16 && !simt_forced())
     return tc_attn_codec(q, q_stride_token, q_stride_head, Q, heads, dk, dv, hist_k, hist_v, wk,
@@ -392,6 +401,36 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
   return simt_attn(q, dtype, q_stride_token, q_stride_head, Q, heads, dk, dv, hist_k, hist_v, wk,
                    bias_k, wv, bias_v, nullptr, nullptr, 0, 0, hist_k->tokens, scale, out, lse, s,
                    rope, camera_k, camera_v);
+}
+
+static bool reads_by_rows(int dtype, int dk, int dv, int rank, int group) {
+  return dtype == NKV_BF16 && !simt_forced() && group > 0 && tc_attn_by_rows(dk, dv, rank, group);
+}
+
+size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, int dv, int tokens, int rank,
+                                           int group, int splits) {
+  if (!reads_by_rows(dtype, dk, dv, rank, group) || splits < 0 || splits > 16) return 0;
+  return tc_attn_rows_workspace_bytes(Q, heads, dk, tokens, splits == 0 ? 16 : splits, true) + 256;
+}
+
+int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
+                        int Q, int heads, int dk, int dv, const nkv_history* hist_k,
+                        const nkv_history* hist_v, const void* wk, const float* bias_k,
+                        const void* wv, const float* bias_v, int weight_order, const nkv_rope* rope,
+                        const nkv_camera* camera_k, const nkv_camera* camera_v, float scale,
+                        void* out, float* lse, int32_t* status_word, int splits, void* workspace,
+                        size_t workspace_bytes, void* stream) {
+  int rc = check_read(dtype, Q, heads, dk, dv, hist_k, hist_v, weight_order, rope, camera_k, camera_v);
+  if (rc != NKV_OK) return rc;
+  NKV_REQUIRE(splits >= 0 && splits <= 16, NKV_ERR_INVALID, "attn_codec_rows: splits=%d (0..16)", splits);
+  NKV_REQUIRE(reads_by_rows(dtype, dk, dv, hist_k->rank, hist_k->group), NKV_ERR_UNSUPPORTED,
+              "attn_codec_rows: dtype %d, dk=%d dv=%d rank=%d group=%d", dtype, dk, dv, hist_k->rank, hist_k->group);
+  NKV_REQUIRE(workspace && workspace_bytes >= nkv_attn_codec_rows_workspace_bytes(
+                               dtype, Q, heads, dk, dv, hist_k->tokens, hist_k->rank, hist_k->group, splits),
+              NKV_ERR_INVALID, "attn_codec_rows: workspace of %zu bytes is too small", workspace_bytes);
+  return tc_attn_by_rows_run(q, q_stride_token, q_stride_head, Q, heads, dk, hist_k, hist_v, wk, bias_k, wv, bias_v,
+                             weight_order == NKV_WEIGHTS_KERNEL_ORDER, rope, camera_k, camera_v, scale, out, lse,
+                             status_word, splits == 0 ? 16 : splits, workspace, static_cast<cudaStream_t>(stream));
 }
 
 int nkv_attn_codec_split(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
@@ -425,6 +464,25 @@ int nkv_attention_lse(const void* q, const void* k, const void* v, int dtype,
   return simt_attn(q, dtype, q_stride_token, q_stride_head, Q, heads, d, dv, nullptr, nullptr,
                    nullptr, nullptr, nullptr, nullptr, k, v, kv_stride_token, kv_stride_head, N,
                    scale, out, lse, static_cast<cudaStream_t>(stream));
+}
+
+size_t nkv_attention_lse_workspace_bytes(int Q, int heads, int d, int N) {
+  if (d != 64 && d != 128) return 0;
+  return tc_attn_rows_workspace_bytes(Q, heads, d, N, 16, false) + 256;
+}
+
+int nkv_attention_lse_bf16(const void* q, const void* k, const void* v, int64_t q_stride_token,
+                           int64_t q_stride_head, int64_t kv_stride_token, int64_t kv_stride_head,
+                           int Q, int N, int heads, int d, int dv, float scale, void* out, float* lse,
+                           int32_t* status_word, void* workspace, size_t workspace_bytes, void* stream) {
+  NKV_REQUIRE(Q >= 0 && N > 0 && heads >= 0, NKV_ERR_INVALID, "attention_lse_bf16: Q=%d N=%d heads=%d", Q, N, heads);
+  NKV_REQUIRE(tc_attention_rows_supported(q, k, v, q_stride_token, q_stride_head, kv_stride_token, kv_stride_head, d, dv),
+              NKV_ERR_INVALID, "attention_lse_bf16: needs d == dv in {64, 128}, 16-byte aligned rows and strides in "
+              "multiples of 8 elements (d=%d dv=%d)", d, dv);
+  NKV_REQUIRE(workspace == nullptr || workspace_bytes >= nkv_attention_lse_workspace_bytes(Q, heads, d, N),
+              NKV_ERR_INVALID, "attention_lse_bf16: workspace of %zu bytes is too small", workspace_bytes);
+  return tc_attention_rows(q, k, v, q_stride_token, q_stride_head, kv_stride_token, kv_stride_head, Q, N, heads, d,
+                           scale, out, lse, status_word, 16, workspace, static_cast<cudaStream_t>(stream));
 }
 
 int nkv_lse_merge(const void* const* outs, const float* const* lses, int parts, int64_t rows,

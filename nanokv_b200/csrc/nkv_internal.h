@@ -69,6 +69,19 @@ int tc_attn_codec(const void* q, int64_t q_stride_token, int64_t q_stride_head, 
                   int32_t* status_word, int splits, void* workspace, cudaStream_t stream,
                   const nkv_rope* rope = nullptr, const nkv_camera* cam_k = nullptr,
                   const nkv_camera* cam_v = nullptr, bool prepared_weights = false);
+// the read in two kernels per batch of heads (rows rebuilt, then attended); nkv_tc_attn.cu
+bool tc_attn_by_rows(int dk, int dv, int rank, int group);
+size_t tc_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens, int max_splits, bool rebuild);
+int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int d,
+                        const nkv_history* hist_k, const nkv_history* hist_v, const void* wk, const float* bias_k,
+                        const void* wv, const float* bias_v, bool prepared_weights, const nkv_rope* rope,
+                        const nkv_camera* cam_k, const nkv_camera* cam_v, float scale, void* out, float* lse,
+                        int32_t* status, int max_splits, void* workspace, cudaStream_t stream);
+bool tc_attention_rows_supported(const void* q, const void* k, const void* v, int64_t q_stride_token,
+                                 int64_t q_stride_head, int64_t kv_stride_token, int64_t kv_stride_head, int d, int dv);
+int tc_attention_rows(const void* q, const void* k, const void* v, int64_t q_stride_token, int64_t q_stride_head,
+                      int64_t kv_stride_token, int64_t kv_stride_head, int Q, int N, int heads, int d, float scale,
+                      void* out, float* lse, int32_t* status, int max_splits, void* workspace, cudaStream_t stream);
 int tc_prepare_decoder(const void* w_bf16, int64_t rows, int rank, void* out_bf16, cudaStream_t stream);
 bool tc_attn_supported(int dk, int dv, int rank);
 int tc_wait_expiry_selftest(int kind, long long budget_cycles, int32_t* status_word, cudaStream_t stream);

@@ -59,6 +59,7 @@ constexpr int NDONE = 8;          // "MMAs of pair g are complete" barriers, ind
 constexpr int KVS = 2;            // K / V stages of a consumer
 constexpr int META_BYTES = 3072;  // barriers, flags and per-token metadata at the head of shared memory
 constexpr int MAX_RING = 56;      // ring slots per group (GF - GF_DONE flag words)
+constexpr int P_FIRST = 64;       // tokens of a tile whose weights are handed to the PV MMAs ahead of the rest
 constexpr int NMETA = 4;          // metadata buffers of a producer (it prepares up to four jobs ahead)
 constexpr float RESCALE_THRESHOLD = 8.0f;
 constexpr float SCORE_WINDOW = 96.0f;   // log2 units a score may exceed the row's reference point by
@@ -73,7 +74,7 @@ enum Bar {
   PV_DONE = 14, O_FREE = 16,
   // producer
   W_FULL = 18, PAIR_DONE = 26, LAT_FULL = 34, META_FULL = 38, META_FREE = 42, CODES_FULL = 46,
-  CODES_FREE = 47, OUT_DONE = 48, NUM_BARS = 52
+  CODES_FREE = 47, OUT_DONE = 48, P_LAST = 52, NUM_BARS = 54
 };
 
 // meta block
@@ -91,6 +92,7 @@ constexpr int MAX_PROD = 8;
 
 struct Params {
   int Q, heads, N, rank, nchunks, npairs, ngroups, group;
+  int out_heads;     // heads of a result row (attn_rows_kernel attends a batch of `heads` of them)
   int scale_dtype, nw, w_perm;
   int tiles, tiles_per_split, splits, qchunks;
   int groups, cons, prod, prod_k, ring, units;   // prod producers per group, the first prod_k of them rebuild K tiles
@@ -123,10 +125,23 @@ __device__ __forceinline__ Unit unit_of(const Params& p, int u) {
   return r;
 }
 
+// Order of the units over K / V rows in memory: the query blocks of one (head, history split) follow one
+// another, so the blocks that run at the same time read the same rows and all but one find them in L2.
+__device__ __forceinline__ Unit row_unit_of(const Params& p, int u) {
+  Unit r;
+  r.qc = u % p.qchunks;
+  const int rest = u / p.qchunks;
+  r.z = rest % p.splits;
+  r.head = rest / p.splits;
+  r.tile0 = r.z * p.tiles_per_split;
+  r.nt = min(p.tiles_per_split, p.tiles - r.tile0);
+  return r;
+}
+
 // ---- bounded waits ------------------------------------------------------------------------------
 struct Ctx {
   volatile int* abort_flag;   // this CTA's (shared memory)
-  int32_t* gabort;            // the launch's (global memory)
+  int32_t* gabort;            // the launch's (global memory); NULL: no wait crosses thread blocks
   long long budget;           // SM cycles per wait
 };
 
@@ -162,12 +177,12 @@ __device__ __forceinline__ void red_release_add(int32_t* p, int v) {
 
 __device__ __noinline__ void raise_abort(const Ctx& c, int code) {
   atomicCAS(const_cast<int*>(c.abort_flag), 0, code);
-  atomicCAS(c.gabort, 0, code);
+  if (c.gabort != nullptr) atomicCAS(c.gabort, 0, code);
 }
 
 // slow path of both waits: true = give up
 __device__ __forceinline__ bool wait_expired(const Ctx& c, long long start, int code) {
-  if (ld_relaxed(c.gabort) != 0) {   // another CTA gave up: leave too
+  if (c.gabort != nullptr && ld_relaxed(c.gabort) != 0) {   // another CTA gave up: leave too
     atomicCAS(const_cast<int*>(c.abort_flag), 0, 900);
     return true;
   }
@@ -225,6 +240,29 @@ __device__ __forceinline__ float exp2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// two fp32 values in one 64-bit register pair: the packed operations issue once for both
+__device__ __forceinline__ uint64_t pair_bits(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
+  return pair_bits(__float_as_uint(lo), __float_as_uint(hi));
+}
+__device__ __forceinline__ void split_f32(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 // Lap timer of one thread (development builds only): adds the cycles since the previous lap to a
@@ -292,7 +330,9 @@ struct Layout {
 };
 
 // ================================================================================ consumer
-template <int D>
+// RING: K / V tiles come from the group's ring, behind the producers' counters; otherwise from K / V rows
+// in memory (map_rk / map_rv over [tokens][heads][D]) and every thread block is a group of one consumer.
+template <int D, bool RING>
 __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uint32_t tmem_base,
                                               const CUtensorMap* map_q, const CUtensorMap* map_rk,
                                               const CUtensorMap* map_rv, const Params& p, const Ctx& ctx,
@@ -301,7 +341,7 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
   constexpr int DCH = L::DCH;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int R = p.ring;
-  int32_t* gflags = p.flags + F_GROUPS + g * GF;
+  int32_t* gflags = RING ? p.flags + F_GROUPS + g * GF : nullptr;
   auto queries_of = [&](const Unit& un, int& q0) {
     q0 = (un.qc * p.cons + c) * (NQ * QT);
     return q0 >= p.Q ? 0 : ((q0 + QT < p.Q) ? 2 : 1);
@@ -321,7 +361,7 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
       Laps laps;
       laps.start(p.prof, p.prof != nullptr && g == 0 && c == 0);
       for (int u = g; u < p.units && ok; u += p.groups) {
-        const Unit un = unit_of(p, u);
+        const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
         int q0;
         const int nq = queries_of(un, q0);
         if (nq > 0) {
@@ -335,13 +375,13 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
           ++ucount;
         }
         for (int t = 0; t < un.nt && ok; ++t, ++seq) {
-          const int slot = seq % R;
+          const int slot = RING ? seq % R : 0;
           const int stage = cseq % KVS, use = cseq / KVS;
           const int row = (g * R + slot) * TOK;
           laps.lap(7);
+          if constexpr (RING) {
           // tile `seq` of K comes from K producer seq % PK as its job number seq / PK, V likewise from
           // V producer PK + seq % PV; the counters are re-read only when the cached copy falls short
-          {
             const int who = seq % PK, need = seq / PK + 1;
             const int who_v = PK + seq % PV, need_v = seq / PV + 1;
             if (pub[who] < need || pub[who_v] < need_v) {
@@ -363,26 +403,31 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
               fence_proxy_async_all();   // the tiles were written with ordinary stores, TMA reads them
             }
           }
+          const int first = (un.tile0 + t) * TOK;
           laps.lap(0);
           if (nq > 0) {
             if (use >= 1) ok = mwait(&bars[K_FREE + stage], (use - 1) & 1, ctx, 103);
             if (!ok) break;
             mbar_arrive_expect_tx(&bars[K_FULL + stage], DCH * TILE_BYTES);
-            for (int ch = 0; ch < DCH; ++ch)
-              tma_load_2d(smem + L::K_OFF + (stage * DCH + ch) * TILE_BYTES, map_rk, ch * 64, row,
-                          &bars[K_FULL + stage]);
+            for (int ch = 0; ch < DCH; ++ch) {
+              uint8_t* dst = smem + L::K_OFF + (stage * DCH + ch) * TILE_BYTES;
+              if constexpr (RING) tma_load_2d(dst, map_rk, ch * 64, row, &bars[K_FULL + stage]);
+              else tma_load_3d(dst, map_rk, ch * 64, un.head, first, &bars[K_FULL + stage]);
+            }
             laps.lap(1);
             if (use >= 1) ok = mwait(&bars[V_FREE + stage], (use - 1) & 1, ctx, 105);
             if (!ok) break;
             mbar_arrive_expect_tx(&bars[V_FULL + stage], DCH * TILE_BYTES);
-            for (int ch = 0; ch < DCH; ++ch)
-              tma_load_2d(smem + L::V_OFF + (stage * DCH + ch) * TILE_BYTES, map_rv, ch * 64, row,
-                          &bars[V_FULL + stage]);
+            for (int ch = 0; ch < DCH; ++ch) {
+              uint8_t* dst = smem + L::V_OFF + (stage * DCH + ch) * TILE_BYTES;
+              if constexpr (RING) tma_load_2d(dst, map_rv, ch * 64, row, &bars[V_FULL + stage]);
+              else tma_load_3d(dst, map_rv, ch * 64, un.head, first, &bars[V_FULL + stage]);
+            }
           }
           laps.lap(3);
           // the previous tile has landed in shared memory by now: hand its ring slot back.  The
           // slot's data has been read (the copies are complete), so a relaxed add is enough.
-          if (pend_slot >= 0) {
+          if (RING && pend_slot >= 0) {
             ok = mwait(&bars[K_FULL + pend_stage], pend_phase, ctx, 106) &&
                  mwait(&bars[V_FULL + pend_stage], pend_phase, ctx, 107);
             if (!ok) break;
@@ -394,12 +439,12 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
           if (nq > 0) {
             pend_slot = slot; pend_stage = stage; pend_phase = use & 1;
             ++cseq;
-          } else {   // nothing to load for this block of queries: the slot is not needed here
+          } else if (RING) {   // nothing to load for this block of queries: the slot is not needed here
             red_relaxed_add(gflags + GF_DONE + slot, 1);
           }
         }
       }
-      if (ok && pend_slot >= 0) {
+      if (RING && ok && pend_slot >= 0) {
         ok = mwait(&bars[K_FULL + pend_stage], pend_phase, ctx, 106) &&
              mwait(&bars[V_FULL + pend_stage], pend_phase, ctx, 107);
         if (ok) red_relaxed_add(gflags + GF_DONE + pend_slot, 1);
@@ -434,14 +479,20 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
     // operand in MN-major form: [tokens (K) x d (N)] with d contiguous, 64-column tiles 16 KB apart
     // (leading offset), 8-token groups 1 KB apart (stride offset); a K step of 16 tokens moves the
     // start by 2 KB (128 in the address field)
-    auto issue_pv = [&](int i, int stage, bool accumulate) {
+    auto issue_pv = [&](int i, int stage, bool accumulate, int part) {
       const uint64_t b_desc = make_smem_desc_sw128_mn(smem_base + L::V_OFF + stage * DCH * TILE_BYTES, TILE_BYTES);
       const uint32_t p_addr = tmem_base + i * 128;
       const uint32_t o_addr = tmem_base + 256 + i * 128;
+      if (part == 0) {
 #pragma unroll
-      for (int ks = 0; ks < TOK / 16; ++ks)
-        if (leader) mma_bf16_ts(o_addr, p_addr + 8 * ks, b_desc + 128 * ks, idesc_pv, accumulate || ks > 0);
-      if (leader) mma_commit(&bars[PV_DONE + i]);
+        for (int ks = 0; ks < P_FIRST / 16; ++ks)
+          if (leader) mma_bf16_ts(o_addr, p_addr + 8 * ks, b_desc + 128 * ks, idesc_pv, accumulate || ks > 0);
+      } else {
+#pragma unroll
+        for (int ks = P_FIRST / 16; ks < TOK / 16; ++ks)
+          if (leader) mma_bf16_ts(o_addr, p_addr + 8 * ks, b_desc + 128 * ks, idesc_pv, accumulate || ks > 0);
+        if (leader) mma_commit(&bars[PV_DONE + i]);
+      }
     };
     bool ok = true;
     int cseq = 0, ucount = 0;
@@ -449,7 +500,7 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
     Laps laps;
     laps.start(p.prof + 8, p.prof != nullptr && g == 0 && c == 0 && leader);
     for (int u = g; u < p.units && ok; u += p.groups) {
-      const Unit un = unit_of(p, u);
+      const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
       int q0;
       const int nq = queries_of(un, q0);
       if (nq == 0) continue;
@@ -477,7 +528,11 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
           if (ok && t == 0 && cunit[i] > 0) ok = mwait_all(&bars[O_FREE + i], (cunit[i] - 1) & 1, ctx, 214 + i);
           if (!ok) break;
           tc_fence_after();
-          issue_pv(i, stage, t > 0);
+          issue_pv(i, stage, t > 0, 0);
+          ok = mwait_all(&bars[P_LAST + i], ci & 1, ctx, 218 + i);
+          if (!ok) break;
+          tc_fence_after();
+          issue_pv(i, stage, t > 0, 1);
           if (i == nq - 1 && leader) mma_commit(&bars[V_FREE + stage]);
           laps.lap(3);
           if (t + 1 < un.nt) {
@@ -511,7 +566,7 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
     Laps laps;
     laps.start(p.prof + 16, p.prof != nullptr && g == 0 && c == 0 && tid == 0);
     for (; u < p.units && ok; u += p.groups) {
-      const Unit un = unit_of(p, u);
+      const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
       int q0;
       const int nq = queries_of(un, q0);
       if (wg >= nq) continue;
@@ -566,9 +621,7 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
           m_seen = fmaxf(m_seen, mx * p.scale_log2);
         }
         if (__any_sync(0xffffffffu, m_seen > m_used + RESCALE_THRESHOLD)) move_reference(m_seen);
-        // One pass over the scores: P (bf16 pairs) replaces S in place -- the 16 cells written per
-        // step lie below the 32 read -- and the load of the next 32 scores stays in flight under the
-        // exponentials of the current ones.
+        // One pass over the scores: P (bf16 pairs) replaces S in place, below the cells still to be read.
         // Weights go to bf16 by dropping the low 16 bits (one byte permute per pair) instead of a
         // rounding conversion, which runs on the same quarter-rate unit as the exponentials and
         // would take a third of its time.  So that the dropped bits do not bias the weights, every
@@ -578,37 +631,67 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
         float sum = 0.f, sum_b = 0.f, sum_c = 0.f, sum_d = 0.f;   // four chains instead of one
         uint32_t pmax_a = 0u, pmax_b = 0u;
         if (valid == TOK) {
-          // The whole row at once: four 32-column loads, ONE wait, and then a single run of
-          // instructions without a fence in it, so that the exponential unit's work of one quarter
-          // overlaps the arithmetic and the packing of its neighbours (a wait per quarter kept every
-          // quarter a closed block: arguments, exponentials, sums, each draining before the next).
+          // The whole row at once: four 32-column loads, ONE wait, then blocks of eight scores in a
+          // software pipeline (exponentials of block b, arguments of b + 1, sums and packing of b - 1), so
+          // that the exponential unit always has work behind it; arguments and sums as packed fp32 pairs,
+          // which halves their issue slots.  The first half of the weights is handed over as soon as it is
+          // stored: its PV MMAs run under the second half's exponentials.  Per 256 x 128 tile pair (148 SMs
+          // busy, 1965 MHz): 2.11 us with scalar arithmetic and one hand-off, 1.97 with pairs and the
+          // pipeline, 1.81 / 1.77 / 1.80 handing over after 96 / 64 / 32 tokens.  Taking a sixteenth / an
+          // eighth / a quarter of the exponentials as a polynomial on the arithmetic pipes: 1.79 / 1.93 / 1.94.
           uint32_t raw[4][32];
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) tmem_ld32_issue(s_addr + cc * 32, raw[cc]);
           tmem_ld128_wait(raw[0], raw[1], raw[2], raw[3]);
+          const uint64_t scale2 = pair_f32(p.scale_log2, p.scale_log2), ref2 = pair_f32(neg_ref, neg_ref);
+          uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
+          uint32_t packed[16];
+          uint64_t arg[2][4];
+          float w[2][8];
+          auto args = [&](int b) {
 #pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            uint32_t (&cur)[32] = raw[cc];
-            uint32_t packed[16];
-            float w[32];
+            for (int i = 0; i < 4; ++i)
+              arg[b & 1][i] = fma_f32x2(pair_bits(raw[b >> 2][(b & 3) * 8 + 2 * i], raw[b >> 2][(b & 3) * 8 + 2 * i + 1]), scale2, ref2);
+          };
+          auto exps = [&](int b) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) w[j] = fmaf(__uint_as_float(cur[j]), p.scale_log2, neg_ref);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) w[j] = exp2_approx(w[j]);
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              sum += w[j]; sum_b += w[j + 1]; sum_c += w[j + 2]; sum_d += w[j + 3];
-              packed[j >> 1] = truncate_bf16x2(w[j], w[j + 1]);
-              packed[(j >> 1) + 1] = truncate_bf16x2(w[j + 2], w[j + 3]);
+            for (int i = 0; i < 4; ++i) {
+              float lo, hi;
+              split_f32(arg[b & 1][i], lo, hi);
+              w[b & 1][2 * i] = exp2_approx(lo);
+              w[b & 1][2 * i + 1] = exp2_approx(hi);
             }
-            // the largest weight of the quarter, on the packed pairs (weights are positive, so the
-            // bf16 bit patterns order like the numbers): half an instruction per score
+          };
+          auto finish = [&](int b) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-              pmax_a = bf16x2_max(pmax_a, packed[j]);
-              pmax_b = bf16x2_max(pmax_b, packed[j + 1]);
+            for (int i = 0; i < 4; ++i) {
+              sum2[i] = add_f32x2(sum2[i], pair_f32(w[b & 1][2 * i], w[b & 1][2 * i + 1]));
+              const uint32_t pk = truncate_bf16x2(w[b & 1][2 * i], w[b & 1][2 * i + 1]);
+              packed[(b & 3) * 4 + i] = pk;
+              if (i & 1) pmax_a = bf16x2_max(pmax_a, pk); else pmax_b = bf16x2_max(pmax_b, pk);
             }
-            tmem_st16(s_addr + cc * 16, packed);
+            if ((b & 3) == 3) {
+              tmem_st16(s_addr + (b >> 2) * 16, packed);
+              if ((b + 1) * 8 == P_FIRST) {
+                tmem_wait_st();
+                tc_fence_before();
+                warp_arrive(&bars[P_READY + wg], lane);
+              }
+            }
+          };
+          args(0);
+#pragma unroll
+          for (int b = 0; b < 16; ++b) {
+            exps(b);
+            if (b + 1 < 16) args(b + 1);
+            if (b >= 1) finish(b - 1);
+          }
+          finish(15);
+          {
+            float lo, hi;
+            split_f32(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), lo, hi);
+            sum = lo;
+            sum_b = hi;
           }
         } else {
           uint32_t raw[2][32];
@@ -629,20 +712,21 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
             tmem_st16(s_addr + cc * 16, packed);
           }
         }
+        laps.lap(1);
+        tmem_wait_st();
+        laps.lap(6);
+        l_run += (sum + sum_b) + (sum_c + sum_d);
+        tc_fence_before();
+        if (valid != TOK) warp_arrive(&bars[P_READY + wg], lane);
+        warp_arrive(&bars[P_LAST + wg], lane);
         if (valid == TOK) {
-          // largest weight 2^(score - reference) -> the largest score the tile saw (to 2^-8)
+          // behind the hand-off: largest weight 2^(score - reference) -> the largest score the tile saw (to 2^-8)
           const uint32_t pm = bf16x2_max(pmax_a, pmax_b);
           const float wmax = fmaxf(__uint_as_float(pm << 16), __uint_as_float(pm & 0xFFFF0000u));
           m_seen = fmaxf(m_seen, m_used + log2f(wmax));
           // a weight beyond the window has overflowed or lost its meaning: the row cannot be trusted
           saturated = saturated || !(wmax < exp2f(SCORE_WINDOW));
         }
-        laps.lap(1);
-        tmem_wait_st();
-        laps.lap(6);
-        l_run += (sum + sum_b) + (sum_c + sum_d);
-        tc_fence_before();
-        warp_arrive(&bars[P_READY + wg], lane);
       }
       if (!ok) break;
       // ---- the unit's rows: O / l and the natural-log LSE (partial number z when the history is split)
@@ -653,8 +737,8 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
       l_run *= HALF_STEP_INV;    // the weights were summed with the half-step factor on them
       const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
       const uint32_t o_addr = tmem_base + lane_sel + 256 + wg * 128;
-      const size_t split_rows = static_cast<size_t>(un.z) * p.Q * p.heads;
-      uint16_t* dst = p.out + (split_rows + static_cast<size_t>(qrow) * p.heads + un.head) * D;
+      const size_t split_rows = static_cast<size_t>(un.z) * p.Q * p.out_heads;
+      uint16_t* dst = p.out + (split_rows + static_cast<size_t>(qrow) * p.out_heads + un.head) * D;
 #pragma unroll 1
       for (int cc = 0; cc < D / 32; ++cc) {
         float v[32];
@@ -672,7 +756,7 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
         }
       }
       if (qrow < p.Q) {
-        p.lse[split_rows + static_cast<size_t>(qrow) * p.heads + un.head] =
+        p.lse[split_rows + static_cast<size_t>(qrow) * p.out_heads + un.head] =
             saturated ? __int_as_float(0x7fc00000)
                       : (l_run > 0.f ? (m_used + log2f(l_run)) * 0.6931471805599453f : -INFINITY);
         if (saturated && p.status) atomicCAS(p.status, 0, STATUS_SCORE_RANGE);
@@ -686,12 +770,12 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
     // and every later one get NaN in their LSE
     if (!ok) {
       for (; u < p.units; u += p.groups) {
-        const Unit un = unit_of(p, u);
+        const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
         int q0;
         const int nq = queries_of(un, q0);
         const int qrow = q0 + wg * QT + row;
         if (wg < nq && qrow < p.Q)
-          p.lse[static_cast<size_t>(un.z) * p.Q * p.heads + static_cast<size_t>(qrow) * p.heads + un.head] =
+          p.lse[static_cast<size_t>(un.z) * p.Q * p.out_heads + static_cast<size_t>(qrow) * p.out_heads + un.head] =
               __int_as_float(0x7fc00000);
       }
     }
@@ -1249,6 +1333,56 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* bars, uin
   }
 }
 
+__device__ __forceinline__ void init_consumer_barriers(uint64_t* bars) {
+  mbar_init(&bars[Q_FULL], 1);
+  mbar_init(&bars[Q_FREE], 1);
+  for (int s = 0; s < 2; ++s) {
+    mbar_init(&bars[K_FULL + s], 1);
+    mbar_init(&bars[K_FREE + s], 1);
+    mbar_init(&bars[V_FULL + s], 1);
+    mbar_init(&bars[V_FREE + s], 1);
+    mbar_init(&bars[S_FULL + s], 1);
+    mbar_init(&bars[P_READY + s], QT / 32);
+    mbar_init(&bars[P_LAST + s], QT / 32);
+    mbar_init(&bars[PV_DONE + s], 1);
+    mbar_init(&bars[O_FREE + s], QT / 32);
+  }
+}
+
+// Attention over K / V rows in memory (rebuilt a batch of heads at a time by decode_gemm_kernel, or a
+// caller's own): the consumer of the fused kernel without its ring.  Every SM attends -- in the fused
+// kernel a fifth to a half of them rebuild tiles -- no wait crosses thread blocks, and launches share no
+// state.  Bound: the chain S -> softmax -> P -> PV of two 128-query tiles per SM.
+template <int D>
+__global__ void __launch_bounds__(THREADS, 1)
+attn_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                 const __grid_constant__ CUtensorMap map_v, Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + M_SLOT);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + M_ABORT);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (tid == 0) {
+    init_consumer_barriers(bars);
+    *abort_flag = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  if (warp == 9) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const Ctx ctx{abort_flag, nullptr, p.wait_budget};
+  consumer_role<D, false>(smem, bars, tmem_base, &map_q, &map_k, &map_v, p, ctx, blockIdx.x, 0);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) tmem_dealloc(tmem_base, 512);
+  if (tid == 0 && *abort_flag && p.status) atomicCAS(p.status, 0, *abort_flag);
+}
+
 template <int D, bool ROPE, bool CAM>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_codec_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -1269,18 +1403,7 @@ attn_codec_kernel(const __grid_constant__ CUtensorMap map_q,
   const int g = blockIdx.x / per_group, role = blockIdx.x % per_group;
 
   if (tid == 0) {
-    mbar_init(&bars[Q_FULL], 1);
-    mbar_init(&bars[Q_FREE], 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&bars[K_FULL + s], 1);
-      mbar_init(&bars[K_FREE + s], 1);
-      mbar_init(&bars[V_FULL + s], 1);
-      mbar_init(&bars[V_FREE + s], 1);
-      mbar_init(&bars[S_FULL + s], 1);
-      mbar_init(&bars[P_READY + s], QT / 32);
-      mbar_init(&bars[PV_DONE + s], 1);
-      mbar_init(&bars[O_FREE + s], QT / 32);
-    }
+    init_consumer_barriers(bars);
     for (int s = 0; s < NMETA; ++s) {
       mbar_init(&bars[META_FULL + s], 1);
       mbar_init(&bars[META_FREE + s], COMPUTE_WARPS);
@@ -1305,7 +1428,7 @@ attn_codec_kernel(const __grid_constant__ CUtensorMap map_q,
 
   if (g < p.groups) {
     if (role < p.cons) {
-      consumer_role<D>(smem, bars, tmem_base, &map_q, &map_rk, &map_rv, p, ctx, g, role);
+      consumer_role<D, true>(smem, bars, tmem_base, &map_q, &map_rk, &map_rv, p, ctx, g, role);
     } else {
       const int pidx = role - p.cons;
       const bool value = pidx >= p.prod_k;
@@ -1643,7 +1766,7 @@ int tc_attn_codec(const void* q, int64_t q_stride_token, int64_t q_stride_head, 
     int rc = encode_tensor_map(&maps[5 + w], 2, rings[w], 2, dims, strides, box, 128);
     if (rc != NKV_OK) return rc;
   }
-  p.Q = Q; p.heads = heads; p.N = N; p.rank = rank; p.nchunks = rank / CHUNK;
+  p.Q = Q; p.heads = heads; p.out_heads = heads; p.N = N; p.rank = rank; p.nchunks = rank / CHUNK;
   p.npairs = (p.nchunks + 1) / 2;
   p.group = group; p.ngroups = rank / group; p.scale_dtype = hk.scale_dtype;
   p.scale_log2 = scale * 1.4426950408889634f;
@@ -1694,6 +1817,225 @@ int tc_attn_codec(const void* q, int64_t q_stride_token, int64_t q_stride_head, 
   dev->last_stream = stream;
   dev->used = true;
   return NKV_OK;
+}
+
+// ---- attention over K / V rows in memory ------------------------------------------------------------
+
+namespace {
+
+// Plan of a read that rebuilds K / V rows a batch of heads at a time and attends to them.
+struct RowPlan { int batches, heads, splits, tiles_per_split; size_t kv_bytes; };
+
+// K and V rows of a batch stay below this many bytes (one head at least): a multiple of the 126 MB L2
+// costs nothing -- the rows of the next few units are what is in flight -- while small batches end in
+// emptier last rounds.
+constexpr size_t ROW_BATCH_BYTES = 512u << 20;
+constexpr int MAX_SPLITS = 16;
+
+// Splits (at most `max_splits`) and head batches with the least estimated time.  A unit of 256 queries
+// costs about 2 us per tile of 128 tokens plus a fill of about three tiles; the partials of a split
+// history are written and read once at HBM rate and cost one more launch.
+RowPlan plan_rows(int sms, int Q, int heads, int d, int tokens, int max_splits, bool rebuild) {
+  const int tiles = ceil_div(tokens, TOK), qblocks = ceil_div(Q, NQ * QT);
+  const size_t head_bytes = rebuild ? static_cast<size_t>(tokens) * d * 4 : 0;
+  int first = 1;
+  while (first < heads && head_bytes * ceil_div(heads, first) > ROW_BATCH_BYTES) ++first;
+  if (max_splits > MAX_SPLITS) max_splits = MAX_SPLITS;
+  if (max_splits > tiles) max_splits = tiles;
+  RowPlan best{};
+  double best_cost = -1;
+  for (int nb = first; nb <= heads && nb < first + 4; ++nb) {
+    const int hb = ceil_div(heads, nb);
+    if (nb > first && (!rebuild || ceil_div(heads, hb) != nb)) continue;
+    for (int s = 1; s <= max_splits; ++s) {
+      const int tps = ceil_div(tiles, s);
+      if (ceil_div(tiles, tps) != s) continue;
+      const int tail = heads - hb * (ceil_div(heads, hb) - 1);
+      double cost = 0;
+      for (int b = 0; b < ceil_div(heads, hb); ++b) {
+        const long long units = static_cast<long long>(b + 1 < ceil_div(heads, hb) ? hb : tail) * qblocks * s;
+        cost += static_cast<double>((units + sms - 1) / sms) * (tps + 3) * 2.0 + 3.0;
+      }
+      if (s > 1) cost += 3.0 + static_cast<double>(s) * Q * heads * (d * 4 + 8) / 5e6;
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best = RowPlan{ceil_div(heads, hb), hb, s, tps, head_bytes * hb};
+      }
+    }
+  }
+  return best;
+}
+
+size_t partial_bytes(int splits, int Q, int heads, int d) {
+  const size_t bytes = splits > 1 ? static_cast<size_t>(splits) * Q * heads * (static_cast<size_t>(d) * 2 + 4) : 0;
+  return (bytes + 255) / 256 * 256;
+}
+
+template <int D>
+int launch_rows(const CUtensorMap maps[3], const Params& p, cudaStream_t stream) {
+  const size_t smem = Layout<D>::CONSUMER_BYTES + 1024;
+  auto kernel = attn_rows_kernel<D>;
+  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kernel<<<p.groups, THREADS, smem, stream>>>(maps[0], maps[1], maps[2], p);
+  NKV_LAUNCH_CHECK("attn_rows_kernel");
+  return NKV_OK;
+}
+
+// rows of one tensor: element (token, head, column) at token * stride_token + head * stride_head + column
+int row_map(CUtensorMap* map, const void* base, int d, int heads, int tokens, int64_t stride_token, int64_t stride_head) {
+  uint64_t dims[3] = {static_cast<uint64_t>(d), static_cast<uint64_t>(heads), static_cast<uint64_t>(tokens)};
+  uint64_t strides[2] = {static_cast<uint64_t>(stride_head) * 2, static_cast<uint64_t>(stride_token) * 2};
+  uint32_t box[3] = {64, 1, TOK};
+  return encode_tensor_map(map, 2, base, 3, dims, strides, box, 128);
+}
+
+// one launch over `heads` heads; out / lse are the batch's first head inside rows of out_heads heads
+int attend_rows(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int out_heads,
+                int d, const void* k, const void* v, int64_t kv_stride_token, int64_t kv_stride_head, int N,
+                float scale, int splits, int tiles_per_split, uint16_t* out, float* lse, int32_t* status,
+                cudaStream_t stream) {
+  CUtensorMap maps[3];
+  int rc = row_map(&maps[0], q, d, heads, Q, q_stride_token, q_stride_head);
+  if (rc == NKV_OK) rc = row_map(&maps[1], k, d, heads, N, kv_stride_token, kv_stride_head);
+  if (rc == NKV_OK) rc = row_map(&maps[2], v, d, heads, N, kv_stride_token, kv_stride_head);
+  if (rc != NKV_OK) return rc;
+  Params p{};
+  p.Q = Q; p.heads = heads; p.out_heads = out_heads; p.N = N;
+  p.tiles = ceil_div(N, TOK);
+  p.splits = splits;
+  p.tiles_per_split = tiles_per_split;
+  p.qchunks = ceil_div(Q, NQ * QT);
+  p.units = p.qchunks * heads * splits;
+  const int sms = sm_count();
+  p.groups = p.units < sms ? p.units : sms;
+  p.cons = 1;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.wait_budget = 1ll << 31;
+  p.out = out; p.lse = lse; p.status = status;
+#ifdef NKV_DEV
+  p.prof = g_profile;
+#endif
+  return d == 128 ? launch_rows<128>(maps, p, stream) : launch_rows<64>(maps, p, stream);
+}
+
+int merge_splits(uint16_t* part_out, float* part_lse, int splits, int Q, int heads, int d, void* out, float* lse,
+                 cudaStream_t stream) {
+  const size_t rows = static_cast<size_t>(Q) * heads;
+  const void* outs[MAX_SPLITS];
+  const float* lses[MAX_SPLITS];
+  for (int z = 0; z < splits; ++z) {
+    outs[z] = part_out + static_cast<size_t>(z) * rows * d;
+    lses[z] = part_lse + static_cast<size_t>(z) * rows;
+  }
+  return lse_merge(outs, lses, splits, static_cast<int64_t>(rows), d, NKV_BF16, out, lse, stream);
+}
+
+bool aligned16(const void* pointer) { return (reinterpret_cast<uintptr_t>(pointer) & 15) == 0; }
+
+}  // namespace
+
+// Whether a read can rebuild rows first; false: the fused kernel (ranks above 640, odd layouts).
+bool tc_attn_by_rows(int dk, int dv, int rank, int group) {
+  return tc_attn_supported(dk, dv, rank) && rank <= 640 && (group == 32 || group % 64 == 0);
+}
+
+size_t tc_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens, int max_splits, bool rebuild) {
+  if (Q <= 0 || heads <= 0 || tokens <= 0) return 0;
+  const RowPlan plan = plan_rows(sm_count(), Q, heads, d, tokens, max_splits, rebuild);
+  return partial_bytes(plan.splits, Q, heads, d) + plan.kv_bytes + 256;
+}
+
+// The read in two kernels per batch of heads: rows rebuilt into `workspace`, then attended.  Against the
+// fused kernel the rows make one trip through L2 / HBM (a tenth of the time they save): the rebuild
+// expands a token's codes once per batch instead of once per head and runs as a plain GEMM on all SMs,
+// and all SMs attend.
+int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int d,
+                        const nkv_history* hist_k, const nkv_history* hist_v, const void* wk, const float* bias_k,
+                        const void* wv, const float* bias_v, bool prepared_weights, const nkv_rope* rope,
+                        const nkv_camera* cam_k, const nkv_camera* cam_v, float scale, void* out, float* lse,
+                        int32_t* status, int max_splits, void* workspace, cudaStream_t stream) {
+  const int N = hist_k->tokens, rank = hist_k->rank;
+  NKV_REQUIRE(q_stride_head % 8 == 0 && q_stride_token % 8 == 0 && aligned16(q), NKV_ERR_INVALID,
+              "queries must be 16-byte aligned with strides in multiples of 8 elements");
+  NKV_REQUIRE(hist_k->center_width % 8 == 0 && hist_v->center_width % 8 == 0, NKV_ERR_INVALID,
+              "centre row pitch must be a multiple of 8 elements");
+  NKV_REQUIRE(aligned16(bias_k) && aligned16(bias_v), NKV_ERR_INVALID, "bias arrays must be 16-byte aligned");
+  NKV_REQUIRE(aligned16(hist_k->codes) && aligned16(hist_v->codes), NKV_ERR_INVALID,
+              "code arrays must be 16-byte aligned");
+  NKV_REQUIRE(aligned16(hist_k->centers) && aligned16(hist_v->centers), NKV_ERR_INVALID,
+              "centre tables must be 16-byte aligned");
+  if (Q == 0 || heads == 0) return NKV_OK;
+  if (N == 0) {
+    const size_t rows = static_cast<size_t>(Q) * heads;
+    fill_empty_kernel<<<static_cast<unsigned>((rows * d + 255) / 256), 256, 0, stream>>>(
+        static_cast<uint16_t*>(out), lse, rows, d);
+    NKV_LAUNCH_CHECK("fill_empty_kernel");
+    return NKV_OK;
+  }
+  const int sms = sm_count();
+  const RowPlan plan = plan_rows(sms, Q, heads, d, N, max_splits, true);
+  uint8_t* space = static_cast<uint8_t*>(workspace);
+  space += (256 - (reinterpret_cast<uintptr_t>(space) & 255)) & 255;
+  uint16_t* part_out = plan.splits > 1 ? reinterpret_cast<uint16_t*>(space) : static_cast<uint16_t*>(out);
+  float* part_lse = plan.splits > 1
+      ? reinterpret_cast<float*>(part_out + static_cast<size_t>(plan.splits) * Q * heads * d) : lse;
+  uint16_t* rows_k = reinterpret_cast<uint16_t*>(space + partial_bytes(plan.splits, Q, heads, d));
+  uint16_t* rows_v = rows_k + static_cast<size_t>(plan.heads) * N * d;
+  for (int h0 = 0; h0 < heads; h0 += plan.heads) {
+    const int hb = heads - h0 < plan.heads ? heads - h0 : plan.heads;
+    const size_t col0 = static_cast<size_t>(h0) * d;
+    nkv_history hk = *hist_k, hv = *hist_v;
+    hk.centers = static_cast<const uint16_t*>(hk.centers) + col0;
+    hv.centers = static_cast<const uint16_t*>(hv.centers) + col0;
+    nkv_rope batch_rope{};
+    if (rope != nullptr) {
+      batch_rope = *rope;
+      if (batch_rope.pair_index != nullptr) batch_rope.pair_index += static_cast<size_t>(h0) * (d / 2);
+    }
+    nkv_camera cams[2] = {};
+    const nkv_camera* sources[2] = {cam_k, cam_v};
+    for (int i = 0; i < 2; ++i)
+      if (sources[i] != nullptr) {
+        cams[i] = *sources[i];
+        cams[i].cam_index += static_cast<size_t>(h0) * (d / 8);
+      }
+    const int64_t head_stride = static_cast<int64_t>(N) * d;
+    const DecodeTensor tensors[2] = {
+        {&hk, static_cast<const uint16_t*>(wk) + col0 * rank, bias_k + col0, nullptr, rows_k, d, head_stride,
+         rope != nullptr ? &batch_rope : nullptr, cam_k != nullptr ? &cams[0] : nullptr},
+        {&hv, static_cast<const uint16_t*>(wv) + col0 * rank, bias_v + col0, nullptr, rows_v, d, head_stride,
+         nullptr, cam_v != nullptr ? &cams[1] : nullptr}};
+    int rc = tc_decode(tensors, 2, N, hb * d, d, prepared_weights, false, status, sms, stream);
+    if (rc == NKV_OK)
+      rc = attend_rows(static_cast<const uint16_t*>(q) + h0 * q_stride_head, q_stride_token, q_stride_head, Q, hb,
+                       heads, d, rows_k, rows_v, d, head_stride, N, scale, plan.splits, plan.tiles_per_split,
+                       part_out + col0, part_lse + h0, status, stream);
+    if (rc != NKV_OK) return rc;
+  }
+  return plan.splits > 1 ? merge_splits(part_out, part_lse, plan.splits, Q, heads, d, out, lse, stream) : NKV_OK;
+}
+
+bool tc_attention_rows_supported(const void* q, const void* k, const void* v, int64_t q_stride_token,
+                                 int64_t q_stride_head, int64_t kv_stride_token, int64_t kv_stride_head, int d, int dv) {
+  return d == dv && (d == 64 || d == 128) && aligned16(q) && aligned16(k) && aligned16(v) &&
+         (q_stride_token | q_stride_head | kv_stride_token | kv_stride_head) % 8 == 0;
+}
+
+// Plain attention over a caller's bf16 rows.
+int tc_attention_rows(const void* q, const void* k, const void* v, int64_t q_stride_token, int64_t q_stride_head,
+                      int64_t kv_stride_token, int64_t kv_stride_head, int Q, int N, int heads, int d, float scale,
+                      void* out, float* lse, int32_t* status, int max_splits, void* workspace, cudaStream_t stream) {
+  if (Q == 0 || heads == 0) return NKV_OK;
+  const RowPlan plan = plan_rows(sm_count(), Q, heads, d, N, workspace != nullptr ? max_splits : 1, false);
+  uint8_t* space = static_cast<uint8_t*>(workspace);
+  space += (256 - (reinterpret_cast<uintptr_t>(space) & 255)) & 255;
+  uint16_t* part_out = plan.splits > 1 ? reinterpret_cast<uint16_t*>(space) : static_cast<uint16_t*>(out);
+  float* part_lse = plan.splits > 1
+      ? reinterpret_cast<float*>(part_out + static_cast<size_t>(plan.splits) * Q * heads * d) : lse;
+  int rc = attend_rows(q, q_stride_token, q_stride_head, Q, heads, heads, d, k, v, kv_stride_token, kv_stride_head, N,
+                       scale, plan.splits, plan.tiles_per_split, part_out, part_lse, status, stream);
+  if (rc == NKV_OK && plan.splits > 1) rc = merge_splits(part_out, part_lse, plan.splits, Q, heads, d, out, lse, stream);
+  return rc;
 }
 
 }  // namespace nkv

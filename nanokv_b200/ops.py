@@ -268,9 +268,17 @@ def attn_codec(q, view_k: HistoryView, view_v: HistoryView, wk, bias_k, wv, bias
         status = status_word(device)
     sk, sv = view_k.struct(), view_v.struct()
     lib = _lib.library()
-    if splits is None:
-        splits = default_splits(view_k.tokens) if q.dtype == torch.bfloat16 else 1
-    nbytes = lib.nkv_attn_codec_workspace_bytes(Q, H, dv, splits)
+    # rows rebuilt in scratch memory a batch of heads at a time, then attended; 0 bytes: this form does
+    # not apply and the fused kernel (or the fp32 one) reads the history
+    nbytes = lib.nkv_attn_codec_rows_workspace_bytes(dtype_code(q.dtype), Q, H, dk, dv, view_k.tokens, view_k.rank,
+                                                     view_k.group, 0 if splits is None else splits)
+    read = lib.nkv_attn_codec_rows if nbytes else lib.nkv_attn_codec_pos
+    if nbytes:
+        splits = 0 if splits is None else splits
+    else:
+        if splits is None:
+            splits = default_splits(view_k.tokens) if q.dtype == torch.bfloat16 else 1
+        nbytes = lib.nkv_attn_codec_workspace_bytes(Q, H, dv, splits)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
     rope_struct = None
     if rope is not None:
@@ -286,7 +294,7 @@ def attn_codec(q, view_k: HistoryView, view_v: HistoryView, wk, bias_k, wv, bias
         if camera is not None and tuple(camera.cam_index.shape) != (H, width // 8):
             raise ValueError("camera index must be [heads, head_dim/8]")
         cameras.append(None if camera is None else ctypes.byref(camera.struct()))
-    _lib.check(lib.nkv_attn_codec_pos(
+    _lib.check(read(
         _ptr(q), dtype_code(q.dtype), q.stride(0), q.stride(1), Q, H, dk, dv, ctypes.byref(sk),
         ctypes.byref(sv), _ptr(wk), _ptr(bias_k), _ptr(wv), _ptr(bias_v), 1 if prepared else 0,
         rope_struct, cameras[0],
@@ -394,56 +402,26 @@ def rope_rows(x: torch.Tensor, rope: RopeView) -> torch.Tensor:
     return out
 
 
-_PLAIN_CACHE: dict = {}
-
-
-def _plain_history(k: torch.Tensor) -> HistoryView:
-    """Full-width rows [N,H,D] dressed as a compressed history the fused kernel rebuilds exactly:
-    rank-64 codes that all mean zero with zero scales (latent = 0), and the rows themselves as the
-    centre table with ids 0, 1, 2 ... (segments of 32,768 tokens keep the ids in 16 bits), so that
-    bf16(bf16(0 + 0) + centre) is the row."""
-    N, H, D = k.shape
-    key = (k.device, N)
-    if key not in _PLAIN_CACHE:
-        span = 32768
-        segments = max(1, -(-N // span))
-        index = torch.arange(N, device=k.device)
-        for stale in [name for name in _PLAIN_CACHE if isinstance(name[0], torch.device)][:-7]:
-            del _PLAIN_CACHE[stale]   # keep a handful of history lengths
-        _PLAIN_CACHE[key] = dict(
-            codes=torch.full((max(N, 1), 32), 0x77, dtype=torch.uint8, device=k.device),
-            scales=torch.zeros(max(N, 1), 1, dtype=torch.bfloat16, device=k.device),
-            ids=(index % span).to(torch.int16),
-            seg_start=torch.tensor([min(s * span, N) for s in range(segments + 1)], dtype=torch.int32,
-                                   device=k.device),
-            seg_center_row=torch.arange(segments, dtype=torch.int32, device=k.device) * span,
-            segments=segments)
-    c = _PLAIN_CACHE[key]
-    return HistoryView(codes=c["codes"], scales=c["scales"], ids=c["ids"], centers=k.view(N, H * D),
-                       seg_start=c["seg_start"], seg_center_row=c["seg_center_row"], tokens=N,
-                       segments=c["segments"], rank=64, group=64)
-
-
 def attention_lse(q, k, v, *, scale: float):
     """Plain attention: q [Q,H,d], k [N,H,d], v [N,H,dv] -> (O [Q,H,dv], lse [Q,H]).
 
-    bf16 rows of width 64 or 128 run on the tcgen05 kernel of the fused read (the rows enter as
-    its centre table, see ``_plain_history``); everything else on the fp32 CUDA-core kernel."""
+    bf16 rows of width 64 or 128 run on the tensor cores; everything else on the fp32 CUDA-core
+    kernel."""
     device = _require_cuda(q, k, v)
     Q, H, d = q.shape
     N, dv = k.shape[0], v.shape[2]
     if (q.dtype == torch.bfloat16 and k.dtype == v.dtype == torch.bfloat16 and d == dv
-            and d in (64, 128) and N > 0 and k.is_contiguous() and v.is_contiguous()
-            and q.stride(2) == 1 and q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0):
-        zero_w = _PLAIN_CACHE.setdefault(("w", device, H, d),
-                                         torch.zeros(H, d, 64, dtype=torch.bfloat16, device=device))
-        zero_b = _PLAIN_CACHE.setdefault(("b", device, H, d),
-                                         torch.zeros(H, d, dtype=torch.float32, device=device))
-        view_k = _plain_history(k)
-        view_v = _plain_history(v)
-        # all-zero weights are their own kernel-order copy
-        return attn_codec(q, view_k, view_v, zero_w, zero_b, zero_w, zero_b, scale=scale,
-                          prepared=tensor_core_read(q.dtype, d, dv, 64))
+            and d in (64, 128) and N > 0 and q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0
+            and not _SIMT_FORCED[0]):
+        lib = _lib.library()
+        out = torch.empty(Q, H, dv, dtype=q.dtype, device=device)
+        lse = torch.empty(Q, H, dtype=torch.float32, device=device)
+        nbytes = lib.nkv_attention_lse_workspace_bytes(Q, H, d, N)
+        workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        _lib.check(lib.nkv_attention_lse_bf16(
+            _ptr(q), _ptr(k), _ptr(v), q.stride(0), q.stride(1), k.stride(0), k.stride(1), Q, N, H, d, dv,
+            float(scale), _ptr(out), _ptr(lse), _ptr(status_word(device)), _ptr(workspace), nbytes, _stream(device)))
+        return out, lse
     out = torch.empty(Q, H, dv, dtype=q.dtype, device=device)
     lse = torch.empty(Q, H, dtype=torch.float32, device=device)
     if k.stride() != v.stride() and d == dv:
