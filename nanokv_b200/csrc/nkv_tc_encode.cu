@@ -15,6 +15,11 @@
 //            memory), quantises to INT4, packs two codes per byte and writes codes and scale to
 //            their place in the history: the bf16 coefficients never travel to HBM.
 // A CTA covers up to 512 output columns as 1 or 2 accumulators of NB <= 256.
+// Calls of a few thousand tokens have too few token tiles for 148 SMs, and a tile's time is the length
+// of its K loop (J / 64 stages of operand latency).  Such calls cut K over a cluster of up to eight CTAs:
+// each sums its stretch in TMEM, the fp32 partials of a row travel to the CTA that owns the row (shared
+// memory to shared memory), which adds them in the order of K and finishes the row on its own: nearest
+// centre, or maximum, codes and scale.  See plan_split for the rule and figures.
 // Warps 0-7 compute, warp 8 lane 0 issues TMA, warp 9 lane 0 issues MMA.
 #include <atomic>
 
@@ -22,6 +27,9 @@
 #include "nkv_tc.cuh"
 
 namespace nkv {
+
+int pick_rows(int S, int column_parts);
+
 namespace {
 
 using namespace tc;
@@ -36,11 +44,15 @@ enum Bar { TMA_FULL = 0, A_FULL = 4, STAGE_FREE = 8, ACC_DONE = 12, SIDE_READY =
            PEER_READY = 15, NUM_BARS = 16 };
 enum Mode { PROJECT = 0, ASSIGN_IDS = 1, PROJECT_QUANT = 2 };
 constexpr int META_HEAD = 256;      // barriers, TMEM slot, abort flag
+constexpr int WARPS = COMPUTE_THREADS / 32;
+constexpr int MAX_CENTER_ROWS = 512 / 32;   // centre rows whose norms one thread group accumulates
 
 struct Params {
   int S, J, NB, NACC, n_total;      // n_total = r (project) or C (assign)
   int nstages;                      // depth of the shared-memory operand ring (2..4)
-  int rows;                         // tokens owned by one CTA (<= TM)
+  int rows;                         // tokens of a tile (<= TM)
+  int ksplit, parts;                // CTAs along K, CTAs per tile (ksplit * column_parts)
+  int meta_off;                     // shared memory: operand ring (then the exchange area), then barriers
   // project
   const uint16_t* x; const uint16_t* centers; const void* ids; int id_bytes;
   const float* mean; uint16_t* coeff;
@@ -77,28 +89,32 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   const int b_bytes = p.NB * 128;                       // one accumulator's B tile
   const int stage_bytes = A_BYTES + p.NACC * b_bytes;
   const int nst = p.nstages;
-  uint8_t* meta = smem + nst * stage_bytes;
+  uint8_t* meta = smem + p.meta_off;
   uint64_t* bars = reinterpret_cast<uint64_t*>(meta);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + NUM_BARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + NUM_BARS * 8 + 4);
-  float* xn_part = reinterpret_cast<float*>(meta + META_HEAD);    // [128][2]
+  float* xn_part = reinterpret_cast<float*>(meta + META_HEAD);    // [256]
   float* cand_d = xn_part + 256;                                  // [128]
   int* cand_i = reinterpret_cast<int*>(cand_d + 128);             // [128]
-  float* cn_part = reinterpret_cast<float*>(cand_i + 128);        // [C][2]
+  float* cn_part = reinterpret_cast<float*>(cand_i + 128);        // [C]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * p.rows;                   // this CTA's tokens: [m0, m_end)
+  const int part = blockIdx.x % p.parts;                // place in the tile's cluster
+  const int half = part % p.column_parts, kpart = part / p.column_parts;
+  const int m0 = (blockIdx.x / p.parts) * p.rows;       // this tile's tokens: [m0, m_end)
   const int m_end = min(p.S, m0 + p.rows);
-  const int n_base = blockIdx.y * p.NACC * p.NB;
+  const int n_base = half * p.NACC * p.NB;
   // assign against fp32 centres: B is the centres split into bf16 planes laid side by side along
   // K, A (the token rows) is walked once per plane
-  const int nchunks = ASSIGN ? p.a_chunks * (p.cnorm != nullptr ? 3 : 1) : p.J / 64;
+  const int total_chunks = ASSIGN ? p.a_chunks * (p.cnorm != nullptr ? 3 : 1) : p.J / 64;
+  const int c_first = total_chunks * kpart / p.ksplit;
+  const int nchunks = total_chunks * (kpart + 1) / p.ksplit - c_first;
 
   if (tid == 0) {
     for (int s = 0; s < MAX_STAGES; ++s) {
       mbar_init(&bars[TMA_FULL + s], 1);
-      mbar_init(&bars[A_FULL + s], COMPUTE_THREADS);
-      mbar_init(&bars[STAGE_FREE + s], ASSIGN ? 1 + COMPUTE_THREADS : 1);
+      mbar_init(&bars[A_FULL + s], WARPS);
+      mbar_init(&bars[STAGE_FREE + s], ASSIGN ? 1 + WARPS : 1);
     }
     mbar_init(&bars[ACC_DONE], 1);
     mbar_init(&bars[SIDE_READY], COMPUTE_THREADS);
@@ -115,16 +131,19 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   const uint32_t tmem_base = *tmem_slot;
   // the column-half CTAs of one token tile write into each other's shared memory: nobody may do so
   // before the peer's barriers exist
-  const bool paired = QUANT && p.column_parts == 2;
+  const bool split = p.ksplit > 1;
+  const bool paired = QUANT && !split && p.column_parts == 2;
   if (paired) cluster_sync_all();
+  bool ok = true;
+  float xs[4] = {0.f, 0.f, 0.f, 0.f};        // assign: squared-norm partials of this thread's rows
+  float cs[ASSIGN ? MAX_CENTER_ROWS : 1];
 
   if (warp == 8) {
     if (lane == 0) {
       prefetch_tensormap(&map_b);
       if (ASSIGN) prefetch_tensormap(&map_a);
-      bool ok = true;
-      for (int c = 0; c < nchunks && ok; ++c) {
-        const int s = c % nst, u = c / nst;
+      for (int i = 0; i < nchunks && ok; ++i) {
+        const int s = i % nst, u = i / nst, c = c_first + i;
         if (u >= 1) ok = mbar_wait(&bars[STAGE_FREE + s], (u - 1) & 1, abort_flag, 400 + s);
         if (!ok) break;
         uint8_t* stage = smem + s * stage_bytes;
@@ -145,7 +164,6 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     const bool leader = elect_one();
     const uint32_t idesc = make_idesc_bf16(128, p.NB);
     const uint32_t smem_base = smem_u32(smem);
-    bool ok = true;
     for (int c = 0; c < nchunks && ok; ++c) {
       const int s = c % nst, u = c / nst;
       ok = mbar_wait(&bars[TMA_FULL + s], u & 1, abort_flag, 410 + s);
@@ -171,48 +189,57 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   } else {
     const int row = tid & 127, wg = tid >> 7;
     const uint32_t lane_sel = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-    bool ok = true;
+    // eight threads share a 128-byte row chunk (16 bytes each), a thread serves rows r0 + 32 i: loads and
+    // the swizzled stores touch whole lines
+    const int r0 = tid >> 3, piece = tid & 7;
     if (ASSIGN) {
       // ---- squared norms from the resident tiles
       const int C = p.n_total;
-      float xs = 0.f, cs[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int c = 0; c < nchunks && ok; ++c) {
-        const int s = c % nst, u = c / nst;
-        ok = mbar_wait(&bars[TMA_FULL + s], u & 1, abort_flag, 420 + s);
+#pragma unroll
+      for (int i = 0; i < MAX_CENTER_ROWS; ++i) cs[i] = 0.f;
+      for (int i = 0; i < nchunks && ok; ++i) {
+        const int s = i % nst, u = i / nst;
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars[TMA_FULL + s], u & 1, abort_flag, 420 + s) ? 1 : 0) != 0;
         if (!ok) break;
-        const uint8_t* stage = smem + s * stage_bytes;
-        if (c < p.a_chunks) {
-          const uint4* src = reinterpret_cast<const uint4*>(stage + (tid >> 1) * 128 + (tid & 1) * 64);
+        const uint8_t* stage = smem + s * stage_bytes + r0 * 128 + piece * 16;
+        if (c_first + i < p.a_chunks) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) xs += sumsq8(src[j]);
+          for (int j = 0; j < 4; ++j) xs[j] += sumsq8(*reinterpret_cast<const uint4*>(stage + j * 32 * 128));
         }
+        if (p.cnorm == nullptr) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int item = tid + i * COMPUTE_THREADS;
-          if (p.cnorm == nullptr && item < 2 * C) {
-            const uint4* src = reinterpret_cast<const uint4*>(stage + A_BYTES + (item >> 1) * 128 + (item & 1) * 64);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) cs[i] += sumsq8(src[j]);
-          }
+          for (int j = 0; j < MAX_CENTER_ROWS; ++j)
+            if (r0 + 32 * j < C) cs[j] += sumsq8(*reinterpret_cast<const uint4*>(stage + A_BYTES + j * 32 * 128));
         }
-        mbar_arrive(&bars[STAGE_FREE + s]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[STAGE_FREE + s]);
       }
-      if (ok) {
-        xn_part[tid] = xs;
+      // the eight threads of a row hold an eighth of its sum each
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int item = tid + i * COMPUTE_THREADS;
-          if (item < 2 * C) cn_part[item] = cs[i];
+      for (int off = 1; off < 8; off <<= 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xs[j] += __shfl_xor_sync(0xffffffffu, xs[j], off);
+#pragma unroll
+        for (int j = 0; j < MAX_CENTER_ROWS; ++j) cs[j] += __shfl_xor_sync(0xffffffffu, cs[j], off);
+      }
+      if (ok && split) ok = mbar_wait(&bars[ACC_DONE], 0, abort_flag, 431);
+      if (ok && !split) {
+        if (piece == 0) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) xn_part[r0 + 32 * j] = xs[j];
+#pragma unroll
+          for (int j = 0; j < MAX_CENTER_ROWS; ++j)
+            if (r0 + 32 * j < C) cn_part[r0 + 32 * j] = cs[j];
         }
         mbar_arrive(&bars[SIDE_READY]);
         ok = mbar_wait(&bars[SIDE_READY], 0, abort_flag, 430) &&
              mbar_wait(&bars[ACC_DONE], 0, abort_flag, 431);
       }
-      if (ok) {
+      if (ok && !split) {
         tc_fence_after();
-        const float xn = xn_part[2 * row] + xn_part[2 * row + 1];
-        const int chunks = (C + 31) / 32, split = (chunks + 1) / 2;
-        const int first = wg == 0 ? 0 : split, last = wg == 0 ? split : chunks;
+        const float xn = xn_part[row];
+        const int chunks = (C + 31) / 32, middle = (chunks + 1) / 2;
+        const int first = wg == 0 ? 0 : middle, last = wg == 0 ? middle : chunks;
         float best = INFINITY;
         int best_i = 0x7fffffff;
 #pragma unroll 1
@@ -224,7 +251,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           for (int j = 0; j < 32; ++j) {
             const int cidx = col + j;
             if (cidx < C) {
-              const float cn = p.cnorm != nullptr ? __ldg(p.cnorm + cidx) : cn_part[2 * cidx] + cn_part[2 * cidx + 1];
+              const float cn = p.cnorm != nullptr ? __ldg(p.cnorm + cidx) : cn_part[cidx];
               const float dist = __fsub_rn(__fadd_rn(xn, cn), __fmul_rn(2.0f, v[j]));
               if (dist < best) { best = dist; best_i = cidx; }
             }
@@ -250,63 +277,73 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         }
       }
     } else {
-      // ---- residual operand: bf16((x - centre[id]) - mean), 32 columns per thread
-      const int r = tid >> 1, half = tid & 1;
-      const int t = m0 + r;
-      const bool in = t < m_end;
-      const uint16_t* xrow = p.x + static_cast<size_t>(in ? t : 0) * p.J;
-      const uint16_t* crow = p.centers + static_cast<size_t>(in ? load_id(p.ids, p.id_bytes, t) : 0) * p.J;
-      // raw operands of one chunk for this thread: 32 columns of x and of the centre row
-      uint4 xn[4], cn[4];
-      auto fetch = [&](int c) {
+      // ---- residual operand: bf16((x - centre[id]) - mean), 8 columns of four rows per thread and
+      // chunk; the operands of two chunks are in flight while one is formed
+      const uint16_t* xrow[4];
+      const uint16_t* crow[4];
+      bool in[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          xn[j] = make_uint4(0, 0, 0, 0);
-          cn[j] = make_uint4(0, 0, 0, 0);
-          if (in && c < nchunks) {
-            xn[j] = __ldg(reinterpret_cast<const uint4*>(xrow + c * 64 + half * 32) + j);
-            cn[j] = __ldg(reinterpret_cast<const uint4*>(crow + c * 64 + half * 32) + j);
+      for (int j = 0; j < 4; ++j) {
+        const int r = r0 + 32 * j, t = m0 + r;
+        in[j] = r < p.rows && t < m_end;
+        xrow[j] = p.x + static_cast<size_t>(in[j] ? t : 0) * p.J + piece * 8;
+        crow[j] = p.centers + static_cast<size_t>(in[j] ? load_id(p.ids, p.id_bytes, t) : 0) * p.J + piece * 8;
+      }
+      uint4 xq[2][4], cq[2][4];
+      float4 mq[2][2];
+      auto fetch = [&](int buf, int i) {
+        if (i >= nchunks) return;
+        const int j0 = (c_first + i) * 64;
+        mq[buf][0] = __ldg(reinterpret_cast<const float4*>(p.mean + j0 + piece * 8));
+        mq[buf][1] = __ldg(reinterpret_cast<const float4*>(p.mean + j0 + piece * 8) + 1);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (in[j]) {
+            xq[buf][j] = __ldg(reinterpret_cast<const uint4*>(xrow[j] + j0));
+            cq[buf][j] = __ldg(reinterpret_cast<const uint4*>(crow[j] + j0));
           }
-        }
       };
-      fetch(0);
-      for (int c = 0; c < nchunks && ok; ++c) {
-        const int s = c % nst, u = c / nst;
-        uint4 xc[4], cc4[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { xc[j] = xn[j]; cc4[j] = cn[j]; }
-        fetch(c + 1);                       // in flight while this chunk is formed
-        if (u >= 1) ok = mbar_wait(&bars[STAGE_FREE + s], (u - 1) & 1, abort_flag, 440 + s);
-        if (!ok) break;
-        uint8_t* stage = smem + s * stage_bytes;
-        const int j0 = c * 64 + half * 32;
-        const float4* ms = reinterpret_cast<const float4*>(p.mean + j0);
+      auto step = [&](int buf, int i) {
+        const int s = i % nst, u = i / nst;
+        const float mv[8] = {mq[buf][0].x, mq[buf][0].y, mq[buf][0].z, mq[buf][0].w,
+                             mq[buf][1].x, mq[buf][1].y, mq[buf][1].z, mq[buf][1].w};
+        uint4 out[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          uint4 out = make_uint4(0, 0, 0, 0);
-          if (in) {
-            const uint4 xw = xc[j], cw = cc4[j];
-            const float4 m0v = __ldg(ms + 2 * j), m1v = __ldg(ms + 2 * j + 1);
-            const uint32_t xwords[4] = {xw.x, xw.y, xw.z, xw.w};
-            const uint32_t cwords[4] = {cw.x, cw.y, cw.z, cw.w};
-            const float mv[8] = {m0v.x, m0v.y, m0v.z, m0v.w, m1v.x, m1v.y, m1v.z, m1v.w};
-            uint32_t* o = &out.x;
+          out[j] = make_uint4(0, 0, 0, 0);
+          if (in[j]) {
+            const uint32_t xw[4] = {xq[buf][j].x, xq[buf][j].y, xq[buf][j].z, xq[buf][j].w};
+            const uint32_t cw[4] = {cq[buf][j].x, cq[buf][j].y, cq[buf][j].z, cq[buf][j].w};
+            uint32_t* o = &out[j].x;
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
-              float lo = __fsub_rn(__fsub_rn(__uint_as_float(xwords[w] << 16),
-                                             __uint_as_float(cwords[w] << 16)), mv[2 * w]);
-              float hi = __fsub_rn(__fsub_rn(__uint_as_float(xwords[w] & 0xFFFF0000u),
-                                             __uint_as_float(cwords[w] & 0xFFFF0000u)), mv[2 * w + 1]);
+              const float lo = __fsub_rn(__fsub_rn(__uint_as_float(xw[w] << 16), __uint_as_float(cw[w] << 16)), mv[2 * w]);
+              const float hi = __fsub_rn(__fsub_rn(__uint_as_float(xw[w] & 0xFFFF0000u),
+                                                   __uint_as_float(cw[w] & 0xFFFF0000u)), mv[2 * w + 1]);
               o[w] = pack_bf16x2(lo, hi);
             }
           }
-          *reinterpret_cast<uint4*>(stage + sw128_offset(r, half * 32 + j * 8)) = out;
         }
+        fetch(buf, i + 2);
+        if (u >= 1) ok = __all_sync(0xffffffffu, mbar_wait(&bars[STAGE_FREE + s], (u - 1) & 1, abort_flag, 440 + s) ? 1 : 0) != 0;
+        if (!ok) return;
+        uint8_t* stage = smem + s * stage_bytes + r0 * 128 + ((piece ^ (r0 & 7)) << 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(stage + j * 32 * 128) = out[j];
         fence_proxy_async();
-        mbar_arrive(&bars[A_FULL + s]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[A_FULL + s]);
+      };
+      fetch(0, 0);
+      fetch(1, 1);
+      for (int i = 0; i < nchunks && ok; i += 2) {
+        step(0, i);
+        if (i + 1 < nchunks && ok) step(1, i + 1);
       }
       if (ok) ok = mbar_wait(&bars[ACC_DONE], 0, abort_flag, 450);
-      if (ok && QUANT) {
+      if (split) {
+        // the partial sums are exchanged below
+      } else if (ok && QUANT) {
         // ---- quantise + pack from TMEM.  Pass 1: |max| of the bf16-rounded coefficients of this
         // thread's column chunks; the two warpgroups, then the two column-half CTAs, combine.
         tc_fence_after();
@@ -363,7 +400,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               *reinterpret_cast<uint4*>(p.codes + static_cast<size_t>(tok) * (p.n_total >> 1) +
                                         ((n_base + col) >> 1)) = make_uint4(words[0], words[1], words[2], words[3]);
           }
-          if (wg == 0 && blockIdx.y == 0 && tok < m_end) store_float(p.scales, p.scale_dtype, tok, scale);
+          if (wg == 0 && half == 0 && tok < m_end) store_float(p.scales, p.scale_dtype, tok, scale);
         }
       } else if (ok) {
         tc_fence_after();
@@ -390,6 +427,133 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       }
     }
   }
+  if (split) {
+    // Every CTA of the cluster is behind its last MMA: the operand rings are free, and hold the partial
+    // sums of the rows a CTA owns, one slot per sender.
+    const int own = p.rows / p.parts;                  // rows per CTA
+    const int ncols = p.NACC * p.NB, pitch = ncols + 4;   // 16 bytes of padding: a row per bank group
+    float* slots = reinterpret_cast<float*>(smem);     // [parts][own][pitch]
+    float* xn_slots = slots + p.rows * pitch;          // [parts][own]
+    float* cn_slots = xn_slots + p.rows;               // [parts][C]
+    cluster_sync_all();
+    if (warp < WARPS) {
+      const int row = tid & 127, wg = tid >> 7;
+      tc_fence_after();
+      const uint32_t lane_sel = static_cast<uint32_t>(32 * (warp & 3)) << 16;
+      const bool live = row < p.rows;
+      const uint32_t dst = map_to_cta(smem_u32(slots + (part * own + row % own) * pitch), live ? row / own : 0);
+#pragma unroll 1
+      for (int cc = wg; cc * 32 < ncols; cc += 2) {
+        const int col = cc * 32, acc = col / p.NB;
+        float v[32];
+        tmem_ld32(tmem_base + lane_sel + acc * 256 + (col - acc * p.NB), v);
+        if (live) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            if (col + j < ncols)
+              st_cluster_v4(dst + (col + j) * 4, make_uint4(__float_as_uint(v[j]), __float_as_uint(v[j + 1]),
+                                                            __float_as_uint(v[j + 2]), __float_as_uint(v[j + 3])));
+        }
+      }
+      if (ASSIGN && (tid & 7) == 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int r = (tid >> 3) + 32 * j;
+          if (r < p.rows)
+            st_cluster_b32(map_to_cta(smem_u32(xn_slots + part * own + r % own), r / own), __float_as_uint(xs[j]));
+        }
+        if (p.cnorm == nullptr) {
+#pragma unroll
+          for (int j = 0; j < MAX_CENTER_ROWS; ++j) {
+            const int c = (tid >> 3) + 32 * j;
+            if (c < p.n_total)
+              for (int peer = 0; peer < p.parts; ++peer)
+                st_cluster_b32(map_to_cta(smem_u32(cn_slots + part * p.n_total + c), peer), __float_as_uint(cs[j]));
+          }
+        }
+      }
+    }
+    cluster_sync_all();
+    if (warp < WARPS) {
+      const int tpr = COMPUTE_THREADS / own;           // threads per row, 4 .. 32, inside one warp
+      const int r = tid / tpr, j = tid % tpr;
+      const int tok = m0 + part * own + r;
+      const bool live = tok < m_end;
+      if (ASSIGN) {
+        const int C = p.n_total;
+        float xn = 0.f;
+        for (int k = 0; k < p.ksplit; ++k) xn += xn_slots[k * own + r];
+        float best = INFINITY;
+        int best_i = 0x7fffffff;
+        for (int c = j; c < C; c += tpr) {
+          float dot = 0.f, cn = 0.f;
+          for (int k = 0; k < p.ksplit; ++k) dot += slots[(k * own + r) * pitch + c];
+          if (p.cnorm != nullptr) cn = __ldg(p.cnorm + c);
+          else for (int k = 0; k < p.ksplit; ++k) cn += cn_slots[k * C + c];
+          const float dist = __fsub_rn(__fadd_rn(xn, cn), __fmul_rn(2.0f, dot));
+          if (dist < best) { best = dist; best_i = c; }
+        }
+        for (int off = 1; off < tpr; off <<= 1) {      // smallest distance, first index among equals
+          const float od = __shfl_xor_sync(0xffffffffu, best, off);
+          const int oi = __shfl_xor_sync(0xffffffffu, best_i, off);
+          if (od < best || (od == best && oi < best_i)) { best = od; best_i = oi; }
+        }
+        if (j == 0 && live) {
+          if (p.ids_out != nullptr) {
+            if (p.id_bytes == 1) static_cast<uint8_t*>(p.ids_out)[tok] = static_cast<uint8_t>(best_i);
+            else static_cast<uint16_t*>(p.ids_out)[tok] = static_cast<uint16_t>(best_i);
+          }
+          if (p.labels_out != nullptr) p.labels_out[tok] = best_i;
+        }
+      } else {
+        // columns 8 g .. 8 g + 8 of the row: partials added in the order of K, rounded to bf16
+        const int groups = p.n_total / 8;
+        float amax = 0.f;
+        for (int g = j; g < groups; g += tpr) {
+          const int hh = g * 8 / ncols, col = g * 8 - hh * ncols;
+          float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          for (int k = 0; k < p.ksplit; ++k) {
+            const float4* src = reinterpret_cast<const float4*>(slots + ((k * p.column_parts + hh) * own + r) * pitch + col);
+            const float4 lo = src[0], hi = src[1];
+            z[0] += lo.x; z[1] += lo.y; z[2] += lo.z; z[3] += lo.w;
+            z[4] += hi.x; z[5] += hi.y; z[6] += hi.z; z[7] += hi.w;
+          }
+          if (QUANT) {
+            float* keep = slots + (hh * own + r) * pitch + col;   // this thread's alone: read again below
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              z[i] = round_to_bf16(z[i]);
+              amax = fmaxf(amax, fabsf(z[i]));
+            }
+            reinterpret_cast<float4*>(keep)[0] = make_float4(z[0], z[1], z[2], z[3]);
+            reinterpret_cast<float4*>(keep)[1] = make_float4(z[4], z[5], z[6], z[7]);
+          } else if (live) {
+            *reinterpret_cast<uint4*>(p.coeff + static_cast<size_t>(tok) * p.n_total + g * 8) =
+                make_uint4(pack_bf16x2(z[0], z[1]), pack_bf16x2(z[2], z[3]), pack_bf16x2(z[4], z[5]), pack_bf16x2(z[6], z[7]));
+          }
+        }
+        if (QUANT) {
+          for (int off = 1; off < tpr; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+          float scale;
+          if (p.in_bf16) scale = round_to_bf16(__fdiv_rn(fmaxf(amax, round_to_bf16(p.eps)), 7.0f));
+          else scale = __fdiv_rn(fmaxf(amax, p.eps), 7.0f);
+          const float inv = __frcp_rn(scale);
+          for (int g = j; g < groups; g += tpr) {
+            const int hh = g * 8 / ncols, col = g * 8 - hh * ncols;
+            const float* z = slots + (hh * own + r) * pitch + col;
+            uint32_t word = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int code = p.in_bf16 ? quant_code<true>(z[i], scale, inv) : quant_code<false>(z[i], scale, inv);
+              word |= static_cast<uint32_t>(code) << (4 * i);
+            }
+            if (live) *reinterpret_cast<uint32_t*>(p.codes + static_cast<size_t>(tok) * (p.n_total >> 1) + g * 4) = word;
+          }
+          if (j == 0 && live) store_float(p.scales, p.scale_dtype, tok, scale);
+        }
+      }
+    }
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 9) tmem_dealloc(tmem_base, 512);
@@ -408,15 +572,102 @@ bool plan_columns(int n_total, int* gy, int* nacc, int* nb) {
   return false;
 }
 
+size_t meta_bytes(int n_total) { return META_HEAD + 4 * (256 + 128 + 128) + 4 * static_cast<size_t>(n_total); }
+
+size_t ring_bytes(int nacc, int nb, int stages) { return stages * static_cast<size_t>(A_BYTES + nacc * nb * 128); }
+
 size_t smem_bytes(int nacc, int nb, int n_total, int stages = 2) {
-  return stages * static_cast<size_t>(A_BYTES + nacc * nb * 128) + META_HEAD + 4 * (256 + 128 + 128) +
-         8 * static_cast<size_t>(n_total) + 1024;
+  return ring_bytes(nacc, nb, stages) + meta_bytes(n_total) + 1024;
 }
 
-int pick_stages(int nacc, int nb, int n_total) {
-  int stages = MAX_STAGES;
-  while (stages > 2 && smem_bytes(nacc, nb, n_total, stages) > 232448) --stages;
-  return stages;
+// partial sums of a tile's rows with their norms (split form)
+size_t exchange_bytes(int rows, int columns, int parts, int n_norms) {
+  return 4 * (static_cast<size_t>(rows) * (columns + 4) + rows + static_cast<size_t>(parts) * n_norms);
+}
+
+constexpr size_t SMEM_LIMIT = 232448;
+
+// Fills in stages, the barrier block's place and the launch's shared memory.
+size_t place_smem(Params& p, int n_norms) {
+  p.nstages = MAX_STAGES;
+  while (p.nstages > 2 && smem_bytes(p.NACC, p.NB, n_norms, p.nstages) > SMEM_LIMIT) --p.nstages;
+  size_t front = ring_bytes(p.NACC, p.NB, p.nstages);
+  if (p.ksplit > 1) {
+    const size_t exchange = exchange_bytes(p.rows, p.NACC * p.NB, p.parts, n_norms);
+    if (exchange > front) front = exchange;
+  }
+  p.meta_off = static_cast<int>((front + 255) / 256 * 256);
+  return p.meta_off + meta_bytes(n_norms) + 1024;
+}
+
+// How a GEMM of S tokens x `columns` over `chunks` stages is cut: tokens per tile, column parts, K parts.
+// The estimate counts SM cycles: a stage costs the bytes it takes from L2 (token rows, centre rows, B) at
+// 48 bytes per clock, at least 350 cycles of latency; exchanging partials costs 15 bytes per clock, the
+// SM-to-SM rate, plus the barriers.  Clusters of 8 fit 128 of the 148 SMs at a time, of 4 about 144.
+// Bound of the undivided form: 880 tokens x 3,072 columns x rank 384 kept 14 SMs busy for 48 stages of
+// operand latency.  Undivided -> cut, us per call: projection of 880 x 3,072 x 384 107 -> 20 (64 tokens, 2
+// column parts, 4 K parts), of 1,560 x 3,072 x 384 84 -> 23, of 4,680 x 5,120 x 640 128 -> 75 (not cut:
+// operand prefetch alone); assignment of 1,560 x 3,072 to 256 centres 60 -> 30, of 880 x 3,072 to 64 fp32
+// centres 70 -> 16.  Only the order in which K is summed depends on the cut, and the projection
+// and its quantising form take the same one.
+struct Split { int rows, column_parts, ksplit; };
+
+Split plan_split(int S, int chunks, int columns, int column_parts, int n_norms, bool residual) {
+  const int sms = sm_count();
+  Split best{pick_rows(S, column_parts), column_parts, 1};
+  auto stage_cost = [&](int rows, int cols) {
+    const double bytes = rows * (residual ? 256.0 : 128.0) + cols * 128.0;
+    return bytes / 48 > 350 ? bytes / 48 : 350.0;
+  };
+  auto rounds = [](long long ctas, int room) { return static_cast<double>((ctas + room - 1) / room); };
+  double best_cost = rounds(static_cast<long long>(ceil_div(S, best.rows)) * column_parts, sms) *
+                     (chunks * stage_cost(best.rows, columns / column_parts) + 3000);
+  for (int rows = 64; rows <= TM; rows *= 2)
+    for (int h = column_parts; h <= 2 * column_parts && h <= 4; h *= 2)
+      for (int k = 2; k * h <= 8; k *= 2) {
+        const int cols = columns / h;
+        if (columns % h || cols > 512 || chunks < 2 * k) continue;
+        if (h > column_parts && (!residual || cols % 64)) continue;
+        if (exchange_bytes(rows, cols, k * h, n_norms) + meta_bytes(n_norms) + 2048 > SMEM_LIMIT) continue;
+        const int room = k * h == 8 ? sms - 20 : (k * h == 4 ? sms - 4 : sms);
+        const double cost = rounds(static_cast<long long>(ceil_div(S, rows)) * k * h, room) *
+                            (ceil_div(chunks, k) * stage_cost(rows, cols) + rows * cols * 4.0 / 15 + 5000);
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = Split{rows, h, k};
+        }
+      }
+  return best;
+}
+
+// accumulators of one CTA's columns
+void set_columns(Params& p, int columns) {
+  p.NACC = columns > 256 ? 2 : 1;
+  p.NB = columns / p.NACC;
+}
+
+template <int MODE>
+int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, Params& p, int n_norms, const char* name,
+                cudaStream_t stream) {
+  p.parts = p.ksplit * p.column_parts;
+  const size_t smem = place_smem(p, n_norms);
+  NKV_REQUIRE(smem <= SMEM_LIMIT, NKV_ERR_UNSUPPORTED, "%s needs %zu bytes of shared memory", name, smem);
+  auto kernel = encode_gemm_kernel<MODE>;
+  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(static_cast<unsigned>(ceil_div(p.S, p.rows)) * p.parts);
+  config.blockDim = dim3(THREADS);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = p.ksplit > 1 || (MODE == PROJECT_QUANT && p.column_parts == 2) ? p.parts : 1;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  NKV_CUDA(cudaLaunchKernelEx(&config, kernel, map_a, map_b, p));
+  return NKV_OK;
 }
 
 }  // namespace
@@ -469,6 +720,9 @@ int tc_project(const void* x_bf16, const void* centers_bf16, const void* ids, in
   int gy;
   NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB), NKV_ERR_UNSUPPORTED,
               "projection rank %d cannot be tiled", r);
+  const Split cut = plan_split(S, J / 64, r, gy, 0, true);
+  p.rows = cut.rows; p.column_parts = cut.column_parts; p.ksplit = cut.ksplit;
+  set_columns(p, r / p.column_parts);
   NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(centers_bf16) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(mean) & 15) == 0 &&
@@ -485,16 +739,7 @@ int tc_project(const void* x_bf16, const void* centers_bf16, const void* ids, in
   uint32_t box[2] = {64, static_cast<uint32_t>(p.NB)};
   int rc = encode_tensor_map(&map_b, 2, encoder_bf16, 2, dims, strides, box, 128);
   if (rc != NKV_OK) return rc;
-  p.nstages = pick_stages(p.NACC, p.NB, 0);
-  size_t smem = smem_bytes(p.NACC, p.NB, 0, p.nstages);
-  auto kernel = encode_gemm_kernel<PROJECT>;
-  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
-  p.rows = pick_rows(S, gy);
-  dim3 grid(ceil_div(S, p.rows), gy);
-  kernel<<<grid, THREADS, smem, stream>>>(map_b, map_b, p);
-  NKV_LAUNCH_CHECK("encode_gemm_kernel<project>");
-  return NKV_OK;
+  return launch_gemm<PROJECT>(map_b, map_b, p, 0, "encode_gemm_kernel<project>", stream);
 }
 
 bool tc_project_quant_supported(int J, int r, int group) {
@@ -510,6 +755,9 @@ int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* i
   int gy;
   NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB) && gy <= 2, NKV_ERR_UNSUPPORTED,
               "fused projection: rank %d cannot be tiled over at most two column parts", r);
+  const Split cut = plan_split(S, J / 64, r, gy, 0, true);
+  p.rows = cut.rows; p.column_parts = cut.column_parts; p.ksplit = cut.ksplit;
+  set_columns(p, r / p.column_parts);
   NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(centers_bf16) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(mean) & 15) == 0 &&
@@ -522,34 +770,13 @@ int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* i
   p.codes = codes; p.scales = scales; p.eps = eps;
   p.in_bf16 = quant_mode == NKV_QUANT_IN_BF16 ? 1 : 0;
   p.scale_dtype = scale_dtype;
-  p.column_parts = gy;
   CUtensorMap map_b;
   uint64_t dims[2] = {static_cast<uint64_t>(J), static_cast<uint64_t>(r)};
   uint64_t strides[1] = {static_cast<uint64_t>(J) * 2};
   uint32_t box[2] = {64, static_cast<uint32_t>(p.NB)};
   int rc = encode_tensor_map(&map_b, 2, encoder_bf16, 2, dims, strides, box, 128);
   if (rc != NKV_OK) return rc;
-  p.nstages = pick_stages(p.NACC, p.NB, 0);
-  size_t smem = smem_bytes(p.NACC, p.NB, 0, p.nstages);
-  auto kernel = encode_gemm_kernel<PROJECT_QUANT>;
-  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
-  p.rows = pick_rows(S, gy);
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(ceil_div(S, p.rows), gy);
-  config.blockDim = dim3(THREADS);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = 1;
-  attribute.val.clusterDim.y = gy;
-  attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  NKV_CUDA(cudaLaunchKernelEx(&config, kernel, map_b, map_b, p));
-  NKV_LAUNCH_CHECK("encode_gemm_kernel<project + quantise>");
-  return NKV_OK;
+  return launch_gemm<PROJECT_QUANT>(map_b, map_b, p, 0, "encode_gemm_kernel<project + quantise>", stream);
 }
 
 int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C, void* ids,
@@ -557,8 +784,9 @@ int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C,
   if (S == 0) return NKV_OK;
   Params p{};
   p.S = S; p.J = J; p.n_total = C;
-  p.NACC = C > 256 ? 2 : 1;
-  p.NB = C / p.NACC;
+  const Split cut = plan_split(S, J / 64, C, 1, C, false);
+  p.rows = cut.rows; p.column_parts = 1; p.ksplit = cut.ksplit;
+  set_columns(p, C);
   p.ids_out = ids; p.id_bytes = id_bytes;
   p.a_chunks = J / 64;
   CUtensorMap map_a, map_b;
@@ -576,16 +804,7 @@ int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C,
     int rc = encode_tensor_map(&map_b, 2, centers_bf16, 2, dims, strides, box, 128);
     if (rc != NKV_OK) return rc;
   }
-  p.nstages = pick_stages(p.NACC, p.NB, C);
-  size_t smem = smem_bytes(p.NACC, p.NB, C, p.nstages);
-  auto kernel = encode_gemm_kernel<ASSIGN_IDS>;
-  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
-  p.rows = pick_rows(S, 1);
-  dim3 grid(ceil_div(S, p.rows), 1);
-  kernel<<<grid, THREADS, smem, stream>>>(map_a, map_b, p);
-  NKV_LAUNCH_CHECK("encode_gemm_kernel<assign>");
-  return NKV_OK;
+  return launch_gemm<ASSIGN_IDS>(map_a, map_b, p, C, "encode_gemm_kernel<assign>", stream);
 }
 
 namespace {
@@ -639,8 +858,9 @@ int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, in
   NKV_LAUNCH_CHECK("split_centers_kernel");
   Params p{};
   p.S = S; p.J = J; p.n_total = C;
-  p.NACC = C > 256 ? 2 : 1;
-  p.NB = C / p.NACC;
+  const Split cut = plan_split(S, 3 * (J / 64), C, 1, C, false);
+  p.rows = cut.rows; p.column_parts = 1; p.ksplit = cut.ksplit;
+  set_columns(p, C);
   p.labels_out = labels; p.id_bytes = 1;
   p.a_chunks = J / 64;
   p.cnorm = cnorm;
@@ -659,16 +879,7 @@ int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, in
     int rc = encode_tensor_map(&map_b, 2, planes, 2, dims, strides, box, 128);
     if (rc != NKV_OK) return rc;
   }
-  p.nstages = pick_stages(p.NACC, p.NB, C);
-  size_t smem = smem_bytes(p.NACC, p.NB, C, p.nstages);
-  auto kernel = encode_gemm_kernel<ASSIGN_IDS>;
-  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)));
-  p.rows = pick_rows(S, 1);
-  dim3 grid(ceil_div(S, p.rows), 1);
-  kernel<<<grid, THREADS, smem, stream>>>(map_a, map_b, p);
-  NKV_LAUNCH_CHECK("encode_gemm_kernel<assign, fp32 centres>");
-  return NKV_OK;
+  return launch_gemm<ASSIGN_IDS>(map_a, map_b, p, C, "encode_gemm_kernel<assign, fp32 centres>", stream);
 }
 
 }  // namespace nkv
