@@ -496,33 +496,53 @@ __global__ void gather_init_kernel(const void* x, int x_dtype, int J, const int3
     centers[static_cast<size_t>(c) * J + j] = load_float(x, x_dtype, src + j);
 }
 
-// centre c, column j: sum of member rows in token order / member count;
+// columns j, j + 1 (COLS 2) or j (COLS 1) of a row, as floats
+template <int COLS>
+__device__ __forceinline__ float2 load_columns(const void* base, int dtype, size_t i) {
+  if (COLS == 1) return make_float2(load_float(base, dtype, i), 0.f);
+  if (dtype == NKV_F32) return __ldg(reinterpret_cast<const float2*>(static_cast<const float*>(base) + i));
+  const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(base) + i));
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+
+// centre c, columns j ..: sum of member rows in token order / member count;
 // an empty cluster keeps its centre.
+constexpr int UPDATE_LABELS = 32;                       // labels a thread looks at per round
+constexpr int UPDATE_SPAN = 256 * UPDATE_LABELS;        // tokens per round
+template <int COLS>
 __global__ void __launch_bounds__(256)
 kmeans_update_kernel(const void* x, int x_dtype, int S, int J, const int32_t* labels,
                      float* centers) {
   // Block (c, column block): the mean of the rows labelled c, summed in increasing token order (one
   // fp32 addition per row, the order a sequential scatter-add takes) so that the result does not
-  // depend on the launch shape.  Labels are taken 2,048 at a time: every thread looks at eight of
-  // them, a block-wide exclusive scan turns the match counts into positions, and the matching
-  // tokens land in shared memory in order; the columns are then summed over that short list only,
-  // four loads in flight at a time.
-  __shared__ int list[2048];
+  // depend on the launch shape.  Labels are taken 8,192 at a time: every thread looks at 32 of them, a
+  // block-wide exclusive scan turns the match counts into positions, and the matching tokens land in
+  // shared memory in order; the columns are then summed over that short list only.  Bound: the latency
+  // of the list's row loads, eight of which are in flight (two columns each: a block covers 512 columns
+  // and the grid is one wave).  4,680 x 5,120, 64 centres: 68 us (cold) / 50 us (rows in L2); with
+  // 2,048 labels a round, one column per thread and four loads in flight 97 / 73.
+  __shared__ uint16_t list[UPDATE_SPAN];
   __shared__ int warp_total[8];
-  const int c = blockIdx.x, j = blockIdx.y * 256 + threadIdx.x;
+  const int c = blockIdx.x, j = (blockIdx.y * 256 + threadIdx.x) * COLS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float sum = 0.f;
+  const bool vector = (reinterpret_cast<uintptr_t>(labels) & 15) == 0;
+  float2 sum = make_float2(0.f, 0.f);
   int count = 0;
-  for (int s0 = 0; s0 < S; s0 += 2048) {
-    const int len = min(2048, S - s0);
-    int mine[8], n = 0;
-    const int first = threadIdx.x * 8;
+  for (int s0 = 0; s0 < S; s0 += UPDATE_SPAN) {
+    const int len = min(UPDATE_SPAN, S - s0);
+    const int first = threadIdx.x * UPDATE_LABELS;
+    uint32_t match = 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int i = first + k;
-      mine[k] = (i < len && __ldg(labels + s0 + i) == c) ? 1 : 0;
-      n += mine[k];
+    for (int k = 0; k < UPDATE_LABELS; k += 4) {
+      if (vector && first + k + 4 <= len) {
+        const int4 l = __ldg(reinterpret_cast<const int4*>(labels + s0 + first + k));
+        match |= ((l.x == c ? 1u : 0u) | (l.y == c ? 2u : 0u) | (l.z == c ? 4u : 0u) | (l.w == c ? 8u : 0u)) << k;
+      } else {
+        for (int i = k; i < k + 4; ++i)
+          if (first + i < len && __ldg(labels + s0 + first + i) == c) match |= 1u << i;
+      }
     }
+    const int n = __popc(match);
     int scan = n;                                           // inclusive scan inside the warp
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -539,24 +559,32 @@ kmeans_update_kernel(const void* x, int x_dtype, int S, int J, const int32_t* la
       total += warp_total[w];
     }
     int at = base + scan - n;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (mine[k]) list[at++] = s0 + first + k;
+    for (; match != 0; match &= match - 1) list[at++] = static_cast<uint16_t>(first + __ffs(match) - 1);
     __syncthreads();
     count += total;
     if (j < J) {
       int i = 0;
-      for (; i + 4 <= total; i += 4) {
-        const float a = load_float(x, x_dtype, static_cast<size_t>(list[i]) * J + j);
-        const float b = load_float(x, x_dtype, static_cast<size_t>(list[i + 1]) * J + j);
-        const float d = load_float(x, x_dtype, static_cast<size_t>(list[i + 2]) * J + j);
-        const float e = load_float(x, x_dtype, static_cast<size_t>(list[i + 3]) * J + j);
-        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, a), b), d), e);
+      for (; i + 8 <= total; i += 8) {
+        float2 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = load_columns<COLS>(x, x_dtype, static_cast<size_t>(s0 + list[i + k]) * J + j);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          sum.x = __fadd_rn(sum.x, v[k].x);
+          sum.y = __fadd_rn(sum.y, v[k].y);
+        }
       }
-      for (; i < total; ++i) sum = __fadd_rn(sum, load_float(x, x_dtype, static_cast<size_t>(list[i]) * J + j));
+      for (; i < total; ++i) {
+        const float2 v = load_columns<COLS>(x, x_dtype, static_cast<size_t>(s0 + list[i]) * J + j);
+        sum.x = __fadd_rn(sum.x, v.x);
+        sum.y = __fadd_rn(sum.y, v.y);
+      }
     }
   }
-  if (j < J && count > 0) centers[static_cast<size_t>(c) * J + j] = __fdiv_rn(sum, static_cast<float>(count));
+  if (j < J && count > 0) {
+    centers[static_cast<size_t>(c) * J + j] = __fdiv_rn(sum.x, static_cast<float>(count));
+    if (COLS == 2) centers[static_cast<size_t>(c) * J + j + 1] = __fdiv_rn(sum.y, static_cast<float>(count));
+  }
 }
 
 __global__ void kmeans_store_kernel(const float* centers, const int32_t* labels, int S, size_t CJ,
@@ -763,8 +791,10 @@ int kmeans_gather_init(const void* x, int x_dtype, int J, int C, const int32_t* 
 
 int kmeans_update(const void* x, int x_dtype, int S, int J, int C, const int32_t* labels,
                   float* centers, cudaStream_t stream) {
-  dim3 grid(C, ceil_div(J, 256));
-  kmeans_update_kernel<<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
+  // two columns per thread: rows start 4 (bf16) or 8 (fp32) byte aligned and have an even length
+  const bool pairs = J % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & (x_dtype == NKV_F32 ? 7 : 3)) == 0;
+  if (pairs) kmeans_update_kernel<2><<<dim3(C, ceil_div(J, 512)), 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
+  else kmeans_update_kernel<1><<<dim3(C, ceil_div(J, 256)), 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
   NKV_LAUNCH_CHECK("kmeans_update_kernel");
   return NKV_OK;
 }
