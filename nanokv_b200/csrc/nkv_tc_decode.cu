@@ -55,6 +55,7 @@ struct Tensor {
 struct Params {
   Tensor t[2];
   int tensors, n, J, D, nchunks, ngroups, group, w_perm, round_bias, nstages;
+  int rope_pairs;             // rotation tables may be read two pairs (16 bytes) at a time
   int m_tiles, n_tiles, total;
   int32_t* status;
 };
@@ -111,10 +112,11 @@ __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatil
   return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code) ? 1 : 0) != 0;
 }
 
-template <bool POS>
+template <bool ROPE, bool CAM>
 __global__ void __launch_bounds__(THREADS, 1)
 decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_constant__ CUtensorMap map_1,
                    const __grid_constant__ Params p) {
+  constexpr bool POS = ROPE || CAM;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -287,120 +289,157 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       const int m0 = (r.m * 2 + static_cast<int>(cta)) * TM + wrow0;
       const int rounds = min(4, max(0, (p.J - nt * TN - wg * 128) / 32));
       // centre rows: 4 lanes read the 16-byte pieces of one row, 8 rows per load instruction; all
-      // rounds are requested ahead of the accumulator wait
+      // rounds (one, where the restore needs the registers) are requested ahead of the accumulator wait
       int crow_of[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) crow_of[i] = __shfl_sync(0xffffffffu, tok < 0 ? -1 : crow, i * 8 + lane / 4);
-      uint4 cen_all[4][4];
-#pragma unroll
-      for (int sub = 0; sub < 4; ++sub) {
+      auto load_centers = [&](int sub, uint4 (&dst)[4]) {
         const uint16_t* cbase = static_cast<const uint16_t*>(t.h.centers) + nt * TN + wg * 128 + sub * 32 + (lane & 3) * 8;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          cen_all[sub][i] = make_uint4(0, 0, 0, 0);
+          dst[i] = make_uint4(0, 0, 0, 0);
           if (sub < rounds && crow_of[i] >= 0)
-            cen_all[sub][i] = __ldg(reinterpret_cast<const uint4*>(cbase + static_cast<size_t>(crow_of[i]) * t.h.center_width));
+            dst[i] = __ldg(reinterpret_cast<const uint4*>(cbase + static_cast<size_t>(crow_of[i]) * t.h.center_width));
         }
-      }
-      // positional restore: this token's table rows
-      const bool rotate = POS && t.rope.cos_sin != nullptr;
-      int coord_t = 0, coord_h = 0, coord_w = 0;
+      };
+      uint4 cen_all[POS ? 1 : 4][4];
+#pragma unroll
+      for (int sub = 0; sub < (POS ? 1 : 4); ++sub) load_centers(sub, cen_all[sub]);
+      // positional restore: table rows and frame of the four tokens this lane stores a piece of
+      const bool rotate = ROPE && t.rope.cos_sin != nullptr;
+      const bool transform = CAM && t.cam.matrices != nullptr;
       const int band_a = t.rope.table_half - 2 * (t.rope.table_half / 3);
       const int band_b = band_a + t.rope.table_half / 3;
+      int coord_t[4], coord_h[4], coord_w[4], frame_of[4];
       if (rotate) {
         const int pos = tok >= 0 ? max(__ldg(t.rope.positions + tok), 0) : 0;
         const int last = t.rope.table_rows - 1;
-        if (t.rope.frame_seqlen == 0) {
-          coord_t = coord_h = coord_w = min(pos, last);
-        } else {
+        int ct = min(pos, last), ch = ct, cw = ct;   // frame_seqlen 0: one table row per token
+        if (t.rope.frame_seqlen > 0) {
           const int frame = pos / t.rope.frame_seqlen, spatial = pos - frame * t.rope.frame_seqlen;
           const int prow = spatial / t.rope.width;
-          coord_t = min(frame, last);
-          coord_h = min(prow, last);
-          coord_w = min(spatial - prow * t.rope.width, last);
+          ct = min(frame, last);
+          ch = min(prow, last);
+          cw = min(spatial - prow * t.rope.width, last);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          coord_t[i] = __shfl_sync(0xffffffffu, ct, i * 8 + lane / 4) * t.rope.table_half;
+          coord_h[i] = __shfl_sync(0xffffffffu, ch, i * 8 + lane / 4) * t.rope.table_half;
+          coord_w[i] = __shfl_sync(0xffffffffu, cw, i * 8 + lane / 4) * t.rope.table_half;
         }
       }
-      const bool transform = POS && t.cam.matrices != nullptr;
-      const float* cam_frame = nullptr;
-      if (transform)
-        cam_frame = t.cam.matrices + static_cast<size_t>(min(max(tok, 0) / t.cam.tokens_per_frame, t.cam.frames - 1)) * 64;
+      if (transform) {
+        const int frame = min(max(tok, 0) / t.cam.tokens_per_frame, t.cam.frames - 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) frame_of[i] = __shfl_sync(0xffffffffu, frame, i * 8 + lane / 4);
+      }
 
+      // The restore works on the 16-byte pieces a lane stores -- four pairs, or one camera block, of one
+      // token -- because four lanes then read 128 contiguous bytes of a token's table row; a lane that
+      // kept a whole row of the accumulator would gather from 32 rows at a time.  26,917 rotated tokens x
+      // 5,120 columns, rank 640 (K and V): 805 us, 1,328 with the gather per row.
+      auto load_rotation = [&](int head, int dcol, float2* rot) {
+        const int local = dcol / 2 + (lane & 3) * 4;
+        const float2* table = reinterpret_cast<const float2*>(t.rope.cos_sin);
+#pragma unroll
+        for (int w = 0; w < 4; w += 2) {
+          int pg[2] = {local + w, local + w + 1};
+          if (t.rope.pair_index != nullptr) {
+            pg[0] = __ldg(t.rope.pair_index + head * (p.D / 2) + pg[0]);
+            pg[1] = __ldg(t.rope.pair_index + head * (p.D / 2) + pg[1]);
+          }
+          // both pairs of one band, adjacent and 16-byte aligned: one load
+          const bool together = p.rope_pairs != 0 && pg[1] == pg[0] + 1 && (pg[0] & 1) == 0 && pg[1] != band_a && pg[1] != band_b;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int row0 = pg[0] < band_a ? coord_t[i] : (pg[0] < band_b ? coord_h[i] : coord_w[i]);
+            if (together) {
+              const float4 both = __ldg(reinterpret_cast<const float4*>(table + row0 + pg[0]));
+              rot[i * 4 + w] = make_float2(both.x, both.y);
+              rot[i * 4 + w + 1] = make_float2(both.z, both.w);
+            } else {
+              const int row1 = pg[1] < band_a ? coord_t[i] : (pg[1] < band_b ? coord_h[i] : coord_w[i]);
+              rot[i * 4 + w] = __ldg(table + row0 + pg[0]);
+              rot[i * 4 + w + 1] = __ldg(table + row1 + pg[1]);
+            }
+          }
+        }
+      };
+      auto restore = [&](int i, int head, int dcol, const float2* rot, uint4& v) {
+        uint32_t word[4] = {v.x, v.y, v.z, v.w};
+        if (rotate) {
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {   // a pair of the rebuilt bf16 key is one complex number
+            const float k0 = __uint_as_float(word[w] << 16), k1 = __uint_as_float(word[w] & 0xFFFF0000u);
+            const float2 cs = rot[i * 4 + w];
+            word[w] = pack_bf16x2(fmaf(k0, cs.x, -(k1 * cs.y)), fmaf(k0, cs.y, k1 * cs.x));
+          }
+        }
+        if (transform) {   // the four two-element slots of the block, mixed by the frame's matrix
+          const int which = __ldg(t.cam.cam_index + head * (p.D / 8) + dcol / 8 + (lane & 3)) & 3;
+          const float4* m = reinterpret_cast<const float4*>(t.cam.matrices + static_cast<size_t>(frame_of[i]) * 64 + which * 16);
+          float block[8];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            block[2 * w] = __uint_as_float(word[w] << 16);
+            block[2 * w + 1] = __uint_as_float(word[w] & 0xFFFF0000u);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 mi = __ldg(m + k);
+            const float c0 = round_to_bf16(mi.x), c1 = round_to_bf16(mi.y);
+            const float c2 = round_to_bf16(mi.z), c3 = round_to_bf16(mi.w);
+            word[k] = pack_bf16x2(fmaf(c3, block[6], fmaf(c2, block[4], fmaf(c1, block[2], c0 * block[0]))),
+                                  fmaf(c3, block[7], fmaf(c2, block[5], fmaf(c1, block[3], c0 * block[1]))));
+          }
+        }
+        v = make_uint4(word[0], word[1], word[2], word[3]);
+      };
       ok = wait_all(&bars[ACC_FULL + b], use & 1, abort_flag, 740 + b);
       if (!ok) return;
       tc_fence_after();
-#pragma unroll
-      for (int sub = 0; sub < 4; ++sub) {
-        if (sub >= rounds) break;
+      auto round = [&](int sub) {
         const int col0 = nt * TN + wg * 128 + sub * 32;
+        const int head = col0 / p.D, dcol = col0 - head * p.D;
+        // rotation entries of the pieces this lane stores, in flight under the rebuild
+        float2 rot[ROPE ? 16 : 1];
+        if (rotate) load_rotation(head, dcol, rot);
         uint32_t acc_raw[32];
         tmem_ld32_issue(tmem_base + lane_sel + b * TN + wg * 128 + sub * 32, acc_raw);
-        float bias[32];
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          const float4 b4 = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j));
-          bias[j] = b4.x; bias[j + 1] = b4.y; bias[j + 2] = b4.z; bias[j + 3] = b4.w;
-        }
-        if (p.round_bias) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) bias[j] = round_to_bf16(bias[j]);
-        }
         uint4 cen[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int rloc = i * 8 + lane / 4, piece = lane & 3;
-          *reinterpret_cast<uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4)) = cen_all[sub][i];
+          *reinterpret_cast<uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4)) = cen_all[POS ? 0 : sub][i];
         }
+        if (POS) load_centers(sub + 1, cen_all[0]);
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           cen[j] = *reinterpret_cast<const uint4*>(stage + lane * 64 + ((j ^ (lane & 3)) << 4));
         __syncwarp();
         tmem_ld32_wait(acc_raw);
-        const int head = col0 / p.D, dcol = col0 - head * p.D;
         uint32_t packed[16];
 #pragma unroll
         for (int j4 = 0; j4 < 4; ++j4) {
           const uint32_t cwords[4] = {cen[j4].x, cen[j4].y, cen[j4].z, cen[j4].w};
-          float block[8];
+          const float4 b0 = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8));
+          const float4 b1 = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8 + 4));
+          float bias[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+          if (p.round_bias) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) bias[j] = round_to_bf16(bias[j]);
+          }
 #pragma unroll
           for (int w = 0; w < 4; ++w) {
             const int j = j4 * 8 + w * 2;
             // two bf16 roundings: of (product + bias), then of (+ centre); the packed addition of two
             // bf16 numbers rounds their exact sum once
-            const uint32_t first = pack_bf16x2(__uint_as_float(acc_raw[j]) + bias[j], __uint_as_float(acc_raw[j + 1]) + bias[j + 1]);
+            const uint32_t first = pack_bf16x2(__uint_as_float(acc_raw[j]) + bias[2 * w], __uint_as_float(acc_raw[j + 1]) + bias[2 * w + 1]);
             const __nv_bfloat162 sum = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&first),
                                                *reinterpret_cast<const __nv_bfloat162*>(&cwords[w]));
             packed[j4 * 4 + w] = *reinterpret_cast<const uint32_t*>(&sum);
-            if (POS) {
-              float x0 = __uint_as_float(packed[j4 * 4 + w] << 16), x1 = __uint_as_float(packed[j4 * 4 + w] & 0xFFFF0000u);
-              if (rotate) {   // the pair (x0, x1) of the rebuilt bf16 key is one complex number
-                const int local = dcol / 2 + j4 * 4 + w;
-                const int pg = t.rope.pair_index ? __ldg(t.rope.pair_index + head * (p.D / 2) + local) : local;
-                const int coord = pg < band_a ? coord_t : (pg < band_b ? coord_h : coord_w);
-                const float2 cs = __ldg(reinterpret_cast<const float2*>(t.rope.cos_sin) + static_cast<size_t>(coord) * t.rope.table_half + pg);
-                const float k0 = x0, k1 = x1;
-                x0 = fmaf(k0, cs.x, -(k1 * cs.y));
-                x1 = fmaf(k0, cs.y, k1 * cs.x);
-                packed[j4 * 4 + w] = pack_bf16x2(x0, x1);
-              }
-              block[2 * w] = x0;
-              block[2 * w + 1] = x1;
-            }
-          }
-          if (POS && transform) {   // the four two-element slots of the block, mixed by the frame's matrix
-            const int which = __ldg(t.cam.cam_index + head * (p.D / 8) + dcol / 8 + j4) & 3;
-            const float4* m = reinterpret_cast<const float4*>(cam_frame + which * 16);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) block[k] = round_to_bf16(block[k]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 mi = __ldg(m + i);
-              const float c0 = round_to_bf16(mi.x), c1 = round_to_bf16(mi.y);
-              const float c2 = round_to_bf16(mi.z), c3 = round_to_bf16(mi.w);
-              const float y0 = fmaf(c3, block[6], fmaf(c2, block[4], fmaf(c1, block[2], c0 * block[0])));
-              const float y1 = fmaf(c3, block[7], fmaf(c2, block[5], fmaf(c1, block[3], c0 * block[1])));
-              packed[j4 * 4 + i] = pack_bf16x2(y0, y1);
-            }
           }
         }
         // through the warp's staging area, so that a store instruction writes whole 64-byte row pieces
@@ -413,10 +452,19 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int rloc = i * 8 + lane / 4, piece = lane & 3;
-          const uint4 v = *reinterpret_cast<const uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4));
+          uint4 v = *reinterpret_cast<const uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4));
+          if (POS) restore(i, head, dcol, rot, v);
           if (crow_of[i] >= 0) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(m0 + rloc) * t.row_stride) = v;
         }
         __syncwarp();
+      };
+      if constexpr (POS) {
+#pragma unroll 1
+        for (int sub = 0; sub < rounds; ++sub) round(sub);
+      } else {
+#pragma unroll
+        for (int sub = 0; sub < 4; ++sub)
+          if (sub < rounds) round(sub);
       }
       tc_fence_before();
       arrive_even(&bars[ACC_FREE + b]);
@@ -470,7 +518,7 @@ int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool 
   if (n == 0) return NKV_OK;
   Params p{};
   CUtensorMap maps[2];
-  bool positional = false;
+  bool rotated = false, transformed = false;
   for (int i = 0; i < count; ++i) {
     const DecodeTensor& src = tensors[i];
     Tensor& t = p.t[i];
@@ -480,8 +528,12 @@ int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool 
     t.out = static_cast<uint16_t*>(src.out);
     t.row_stride = src.row_stride;
     t.head_stride = src.head_stride;
-    if (src.rope != nullptr) { t.rope = *src.rope; positional = true; }
-    if (src.camera != nullptr) { t.cam = *src.camera; positional = true; }
+    if (src.rope != nullptr) {
+      t.rope = *src.rope;
+      p.rope_pairs = t.rope.table_half % 2 == 0 && (reinterpret_cast<uintptr_t>(t.rope.cos_sin) & 15) == 0;
+      rotated = true;
+    }
+    if (src.camera != nullptr) { t.cam = *src.camera; transformed = true; }
     uint64_t dims[2] = {static_cast<uint64_t>(t.h.rank), static_cast<uint64_t>(J)};
     uint64_t strides[1] = {static_cast<uint64_t>(t.h.rank) * 2};
     uint32_t box[2] = {64, TM};
@@ -517,7 +569,8 @@ int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool 
   attr.val.clusterDim.z = 1;
   config.attrs = &attr;
   config.numAttrs = 1;
-  auto kernel = positional ? decode_gemm_kernel<true> : decode_gemm_kernel<false>;
+  auto kernel = transformed ? decode_gemm_kernel<true, true>      // a NULL table switches the rotation off
+                : (rotated ? decode_gemm_kernel<true, false> : decode_gemm_kernel<false, false>);
   NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   NKV_CUDA(cudaLaunchKernelEx(&config, kernel, maps[0], maps[1], p));
   return NKV_OK;
