@@ -375,8 +375,8 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
  * arithmetic, and no state shared between launches.  It is the faster form wherever its workspace is
  * affordable; nkv_attn_codec_pos stays for callers that hand out no such memory and for ranks above
  * 640.  `splits`: upper bound of the history splits, 0: the library's choice.
- * nkv_attn_codec_rows_workspace_bytes is 0 where this form does not apply (fp32, rank above 640,
- * head widths other than 64 and 128).
+ * nkv_attn_codec_rows_workspace_bytes is 0 where this form does not apply (rank above 640 in bf16, head
+ * widths other than 64 and 128); the fp32 form takes no positional restore and 16-byte aligned queries.
  */
 size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, int dv, int tokens,
                                            int rank, int group, int splits);

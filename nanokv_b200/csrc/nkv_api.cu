@@ -274,7 +274,7 @@ int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
     return tc_decode(&t, 1, n, J, J, false, true, nullptr, sm_count(), static_cast<cudaStream_t>(stream));
   }
   return simt_decode_rows(*hist, rows_index, n, decoder, decoder_dtype, mean, J, out, out_dtype,
-                          static_cast<cudaStream_t>(stream));
+                          J, static_cast<cudaStream_t>(stream));
 }
 
 size_t nkv_attn_codec_workspace_bytes(int Q, int heads, int dv, int splits) {
@@ -404,12 +404,14 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
 }
 
 static bool reads_by_rows(int dtype, int dk, int dv, int rank, int group) {
+  if (dtype == NKV_F32) return f32_attn_by_rows(dk, dv);
   return dtype == NKV_BF16 && !simt_forced() && group > 0 && tc_attn_by_rows(dk, dv, rank, group);
 }
 
 size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, int dv, int tokens, int rank,
                                            int group, int splits) {
   if (!reads_by_rows(dtype, dk, dv, rank, group) || splits < 0 || splits > 16) return 0;
+  if (dtype == NKV_F32) return f32_attn_rows_workspace_bytes(Q, heads, dk, tokens) + 256;
   return tc_attn_rows_workspace_bytes(Q, heads, dk, tokens, splits == 0 ? 16 : splits, true) + 256;
 }
 
@@ -428,6 +430,19 @@ int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_
   NKV_REQUIRE(workspace && workspace_bytes >= nkv_attn_codec_rows_workspace_bytes(
                                dtype, Q, heads, dk, dv, hist_k->tokens, hist_k->rank, hist_k->group, splits),
               NKV_ERR_INVALID, "attn_codec_rows: workspace of %zu bytes is too small", workspace_bytes);
+  if (dtype == NKV_F32) {
+    NKV_REQUIRE(rope == nullptr && camera_k == nullptr && camera_v == nullptr, NKV_ERR_UNSUPPORTED,
+                "attn_codec_rows: the fp32 form has no positional restore");
+    NKV_REQUIRE((reinterpret_cast<uintptr_t>(q) & 15) == 0 && q_stride_token % 4 == 0 && q_stride_head % 4 == 0,
+                NKV_ERR_INVALID, "attn_codec_rows: fp32 queries must be 16-byte aligned");
+    if (hist_k->tokens > 0)
+      return f32_attn_by_rows_run(static_cast<const float*>(q), q_stride_token, q_stride_head, Q, heads, dk, hist_k,
+                                  hist_v, static_cast<const float*>(wk), bias_k, static_cast<const float*>(wv), bias_v,
+                                  scale, static_cast<float*>(out), lse, workspace, static_cast<cudaStream_t>(stream));
+    return simt_attn(q, dtype, q_stride_token, q_stride_head, Q, heads, dk, dv, hist_k, hist_v, wk, bias_k, wv, bias_v,
+                     nullptr, nullptr, 0, 0, 0, scale, out, lse, static_cast<cudaStream_t>(stream), nullptr, nullptr,
+                     nullptr);
+  }
   return tc_attn_by_rows_run(q, q_stride_token, q_stride_head, Q, heads, dk, hist_k, hist_v, wk, bias_k, wv, bias_v,
                              weight_order == NKV_WEIGHTS_KERNEL_ORDER, rope, camera_k, camera_v, scale, out, lse,
                              status_word, splits == 0 ? 16 : splits, workspace, static_cast<cudaStream_t>(stream));

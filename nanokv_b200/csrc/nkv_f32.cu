@@ -1,0 +1,592 @@
+// fp32 GEMMs and attention on the CUDA cores: nearest-centre assignment, residual projection, row decode
+// and the attention of rebuilt rows.
+//
+// These carry the fp32 configuration (operators stored in fp32, where the reference runs true IEEE fp32
+// GEMMs and tensor cores have no matching mode) and the C-means of fp32 rows.  With bf16 operands they
+// reproduce the rounding points of the bf16 path, which the test-suite uses to cross-check the
+// tensor-core kernels at full size.
+//
+// A block owns a 64 x 64 tile of the product.  The calls of this configuration have few tiles (96 for a
+// projection of 2,048 tokens) and long sums, so the block's four groups of 64 threads take a quarter of K
+// each, with operand tiles and barriers of their own (the next tile's operands in registers while one is
+// multiplied), and add their sums in order at the end.  Multiply-adds are packed pairs, a thread owns
+// 8 x 8 of the tile.
+#include "nkv_internal.h"
+
+namespace nkv {
+namespace {
+
+constexpr int TILE = 64, BK = 16, GROUPS = 4, GROUP_THREADS = 64, THREADS = GROUPS * GROUP_THREADS;
+constexpr int OPERAND = BK * TILE;                       // floats of one operand tile
+constexpr int SMEM_FLOATS = GROUPS * 2 * 2 * OPERAND;    // two buffers of two operands per group
+static_assert(SMEM_FLOATS == GROUPS * TILE * TILE, "the partial sums reuse the operand tiles");
+
+__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void split_f32(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// elements k .. k + 3 of a row (0 past K); `vector`: rows start on 16 (fp32) or 8 (16-bit) bytes, K % 4 == 0
+__device__ __forceinline__ float4 load4(const void* base, int dtype, size_t row_start, int k, int K, bool vector) {
+  if (vector && k + 4 <= K) {
+    if (dtype == NKV_F32) return __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + row_start + k));
+    if (dtype == NKV_BF16) {
+      const uint2 w = __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + row_start + k));
+      return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xFFFF0000u),
+                         __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xFFFF0000u));
+    }
+  }
+  float v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = k + i < K ? load_float(base, dtype, row_start + k + i) : 0.f;
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+
+bool vector_rows(const void* base, int dtype, int K) {
+  return K % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & (dtype == NKV_F32 ? 15 : 7)) == 0;
+}
+
+__device__ __forceinline__ float sumsq4(float4 v, float acc) {
+  return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, acc))));
+}
+
+// The block's 64 x 64 tile of A B^T over K: load_a(k) / load_b(k) give elements k .. k + 3 of row
+// (thread number in its group) of either operand.  `a_norm` / `b_norm` collect the squares of what this
+// thread loaded.  Afterwards sums(row, column) of the tile lie in `sm` as GROUPS partial tiles.
+template <bool NORMS, class LA, class LB>
+__device__ __forceinline__ void gemm64(float* sm, int K, LA load_a, LB load_b, float& a_norm, float& b_norm) {
+  const int g = threadIdx.x / GROUP_THREADS, t = threadIdx.x % GROUP_THREADS;
+  const int tx = t & 7, ty = t >> 3;
+  const int chunks = (K + BK - 1) / BK;
+  const int first = chunks * g / GROUPS, last = chunks * (g + 1) / GROUPS;
+  float* mine = sm + g * 4 * OPERAND;
+  uint64_t acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+  float4 ra[4], rb[4];
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      ra[j] = load_a(c * BK + 4 * j);
+      rb[j] = load_b(c * BK + 4 * j);
+    }
+  };
+  if (first < last) fetch(first);
+  for (int c = first; c < last; ++c) {
+    float* as = mine + (c & 1) * 2 * OPERAND;
+    float* bs = as + OPERAND;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float av[4] = {ra[j].x, ra[j].y, ra[j].z, ra[j].w}, bv[4] = {rb[j].x, rb[j].y, rb[j].z, rb[j].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        as[(4 * j + i) * TILE + t] = av[i];
+        bs[(4 * j + i) * TILE + t] = bv[i];
+      }
+      if (NORMS) {
+        a_norm = sumsq4(ra[j], a_norm);
+        b_norm = sumsq4(rb[j], b_norm);
+      }
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(GROUP_THREADS) : "memory");
+    if (c + 1 < last) fetch(c + 1);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      const float4 a0 = *reinterpret_cast<const float4*>(as + k * TILE + ty * 8);
+      const float4 a1 = *reinterpret_cast<const float4*>(as + k * TILE + ty * 8 + 4);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(bs + k * TILE + tx * 8);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(bs + k * TILE + tx * 8 + 4);
+      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const uint64_t b[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint64_t a2 = pair_f32(a[i], a[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fma_f32x2(a2, b[j], acc[i][j]);
+      }
+    }
+  }
+  __syncthreads();
+  float* part = sm + g * TILE * TILE;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    ulonglong2* dst = reinterpret_cast<ulonglong2*>(part + (ty * 8 + i) * TILE + tx * 8);
+    dst[0] = make_ulonglong2(acc[i][0], acc[i][1]);
+    dst[1] = make_ulonglong2(acc[i][2], acc[i][3]);
+  }
+  __syncthreads();
+}
+
+// columns c .. c + 3 of a finished row: the groups' partial sums in the order of K
+__device__ __forceinline__ float4 tile_sum(const float* sm, int row, int c) {
+  float4 s = *reinterpret_cast<const float4*>(sm + row * TILE + c);
+#pragma unroll
+  for (int g = 1; g < GROUPS; ++g) {
+    const float4 v = *reinterpret_cast<const float4*>(sm + (g * TILE + row) * TILE + c);
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  return s;
+}
+
+// ---------------------------------------------------------------- assignment
+__global__ void __launch_bounds__(THREADS)
+assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c_dtype, bool c_vec, int S, int J, int C,
+              void* ids, int id_bytes, int32_t* labels32) {
+  extern __shared__ float sm[];
+  __shared__ float xn[GROUPS][TILE], cn[GROUPS][TILE];
+  const int g = threadIdx.x / GROUP_THREADS, t = threadIdx.x % GROUP_THREADS;
+  const int m0 = blockIdx.x * TILE;
+  const int row = threadIdx.x >> 2, quarter = threadIdx.x & 3;   // of the epilogue: 16 centres each
+  float best = INFINITY;
+  int best_i = 0;
+  for (int n0 = 0; n0 < C; n0 += TILE) {
+    const bool in_a = m0 + t < S, in_b = n0 + t < C;
+    const size_t a_row = static_cast<size_t>(in_a ? m0 + t : 0) * J, b_row = static_cast<size_t>(in_b ? n0 + t : 0) * J;
+    float a_norm = 0.f, b_norm = 0.f;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();        // the previous tile's sums and norms have been read
+    gemm64<true>(sm, J, [&](int k) { return in_a ? load4(x, x_dtype, a_row, k, J, x_vec) : zero; },
+                 [&](int k) { return in_b ? load4(centers, c_dtype, b_row, k, J, c_vec) : zero; }, a_norm, b_norm);
+    xn[g][t] = a_norm;
+    cn[g][t] = b_norm;
+    __syncthreads();
+    const float xr = (xn[0][row] + xn[1][row]) + (xn[2][row] + xn[3][row]);
+    float d = INFINITY;
+    int idx = 0x7fffffff;
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) {
+      const int c = quarter * 16 + j;
+      const float4 dot4 = tile_sum(sm, row, c);
+      const float dots[4] = {dot4.x, dot4.y, dot4.z, dot4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (n0 + c + i < C) {
+          const float norm = (cn[0][c + i] + cn[1][c + i]) + (cn[2][c + i] + cn[3][c + i]);
+          // (||x||^2 + ||c||^2) - 2 x.c, in that association, in fp32
+          const float dist = __fsub_rn(__fadd_rn(xr, norm), __fmul_rn(2.0f, dots[i]));
+          if (dist < d) { d = dist; idx = n0 + c + i; }
+        }
+    }
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1) {
+      const float od = __shfl_xor_sync(0xffffffffu, d, off);
+      const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
+      if (od < d || (od == d && oi < idx)) { d = od; idx = oi; }
+    }
+    if (d < best) { best = d; best_i = idx; }
+  }
+  const int token = m0 + row;
+  if (quarter == 0 && token < S) {
+    if (ids) {
+      if (id_bytes == 1) static_cast<uint8_t*>(ids)[token] = static_cast<uint8_t>(best_i);
+      else static_cast<uint16_t*>(ids)[token] = static_cast<uint16_t>(best_i);
+    }
+    if (labels32) labels32[token] = best_i;
+  }
+}
+
+// ---------------------------------------------------------------- projection
+template <bool BF16>
+__global__ void __launch_bounds__(THREADS)
+project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, bool c_vec, const void* ids, int id_bytes,
+               const float* mean, const void* encoder, bool e_vec, int S, int J, int r, void* coeff) {
+  extern __shared__ float sm[];
+  const int t = threadIdx.x % GROUP_THREADS;
+  const int m0 = blockIdx.x * TILE, n0 = blockIdx.y * TILE;
+  const bool in_a = m0 + t < S, in_b = n0 + t < r;
+  const size_t a_row = static_cast<size_t>(in_a ? m0 + t : 0) * J, b_row = static_cast<size_t>(in_b ? n0 + t : 0) * J;
+  const size_t c_row = static_cast<size_t>(in_a ? load_id(ids, id_bytes, m0 + t) : 0) * J;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto residual = [&](int k) {
+    if (!in_a) return zero;
+    const float4 v = load4(x, x_dtype, a_row, k, J, x_vec), c = load4(centers, NKV_BF16, c_row, k, J, c_vec);
+    const float4 m = load4(mean, NKV_F32, 0, k, J, e_vec);
+    float4 res = make_float4(__fsub_rn(__fsub_rn(v.x, c.x), m.x), __fsub_rn(__fsub_rn(v.y, c.y), m.y),
+                             __fsub_rn(__fsub_rn(v.z, c.z), m.z), __fsub_rn(__fsub_rn(v.w, c.w), m.w));
+    if (BF16) res = make_float4(round_to_bf16(res.x), round_to_bf16(res.y), round_to_bf16(res.z), round_to_bf16(res.w));
+    return res;
+  };
+  float unused_a = 0.f, unused_b = 0.f;
+  gemm64<false>(sm, J, residual,
+                [&](int k) { return in_b ? load4(encoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, J, e_vec) : zero; },
+                unused_a, unused_b);
+  const int row = threadIdx.x >> 2, token = m0 + row;
+  if (token >= S) return;
+#pragma unroll
+  for (int j = 0; j < 16; j += 4) {
+    const int c = (threadIdx.x & 3) * 4 + j * 4;   // four lanes write 64 contiguous bytes
+    const float4 s = tile_sum(sm, row, c);
+    const float v[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n0 + c + i < r)
+        store_float(coeff, BF16 ? NKV_BF16 : NKV_F32, static_cast<size_t>(token) * r + n0 + c + i, v[i]);
+  }
+}
+
+// -------------------------------------------------------------------- decode
+// decoder rows, bias and centre columns of `J` columns; out has rows of out_stride elements
+template <bool BF16>
+__global__ void __launch_bounds__(THREADS)
+decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* decoder, bool d_vec,
+                   const float* mean, int J, void* out, int out_dtype, long long out_stride) {
+  extern __shared__ float sm[];
+  __shared__ int tok[TILE], crow[TILE];
+  const int t = threadIdx.x % GROUP_THREADS;
+  const int m0 = blockIdx.x * TILE, n0 = blockIdx.y * TILE;
+  if (threadIdx.x < TILE) {
+    int token = -1, row = 0;
+    if (m0 + t < n) {
+      token = rows_index ? rows_index[m0 + t] : m0 + t;
+      if (token < 0 || token >= h.tokens) token = -1; else row = center_row_of(h, token);
+    }
+    tok[t] = token;
+    crow[t] = row;
+  }
+  __syncthreads();
+  const int token = tok[t];
+  const bool in_b = n0 + t < J;
+  const size_t b_row = static_cast<size_t>(in_b ? n0 + t : 0) * h.rank;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int ngroups = h.rank / h.group;
+  const bool quads = h.group % 4 == 0;      // four coefficients share a scale and two whole bytes
+  auto latent = [&](int k) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (token >= 0 && quads && k < h.rank) {
+      const uint8_t* code = h.codes + static_cast<size_t>(token) * (h.rank >> 1) + (k >> 1);
+      const int b0 = __ldg(code), b1 = __ldg(code + 1);
+      const float scale = load_float(h.scales, h.scale_dtype,
+                                     static_cast<size_t>(token) * ngroups + (ngroups == 1 ? 0 : k / h.group));
+      v[0] = static_cast<float>((b0 & 15) - 7) * scale;
+      v[1] = static_cast<float>((b0 >> 4) - 7) * scale;
+      v[2] = static_cast<float>((b1 & 15) - 7) * scale;
+      v[3] = static_cast<float>((b1 >> 4) - 7) * scale;
+    } else if (token >= 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (k + i < h.rank) v[i] = latent_value(h, token, k + i);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (BF16) v[i] = round_to_bf16(v[i]);
+    return make_float4(v[0], v[1], v[2], v[3]);
+  };
+  float unused_a = 0.f, unused_b = 0.f;
+  gemm64<false>(sm, h.rank, latent,
+                [&](int k) { return in_b ? load4(decoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, h.rank, d_vec) : zero; },
+                unused_a, unused_b);
+  const uint16_t* centers = static_cast<const uint16_t*>(h.centers);
+  const int row = threadIdx.x >> 2;
+  if (m0 + row >= n || tok[row] < 0) return;
+#pragma unroll
+  for (int j = 0; j < 16; j += 4) {
+    const int c0 = (threadIdx.x & 3) * 4 + j * 4;
+    const float4 s = tile_sum(sm, row, c0);
+    const float sums[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = n0 + c0 + i;
+      if (c >= J) continue;
+      const float center = bf16_bits_to_float(centers[static_cast<size_t>(crow[row]) * h.center_width + c]);
+      float v;
+      if (BF16) {
+        v = round_to_bf16(__fadd_rn(sums[i], round_to_bf16(mean[c])));
+        v = round_to_bf16(__fadd_rn(v, center));
+      } else {
+        v = __fadd_rn(__fadd_rn(sums[i], mean[c]), center);
+      }
+      store_float(out, out_dtype, static_cast<size_t>(m0 + row) * out_stride + c, v);
+    }
+  }
+}
+
+// ----------------------------------------------------------------- attention
+// Block = 64 queries of one head over one run of history tokens, 64 at a time: K and V tiles in shared
+// memory, online softmax in fp32, two blocks per SM.  A thread owns 4 x 4 scores and 4 queries x D / 16
+// columns of O; multiply-adds are packed pairs.
+struct RowAttn {
+  const float* q; const float* k; const float* v;
+  long long q_stride_token, q_stride_head, kv_stride_token, kv_stride_head;
+  int Q, heads, N, tokens_per_split, out_heads;
+  float scale;
+  float* out; float* lse;      // partial z at z * Q * out_heads rows
+};
+
+template <int D>
+__global__ void __launch_bounds__(256, 2)
+attn_rows_f32_kernel(RowAttn a) {
+  extern __shared__ float smem[];
+  float* Qs = smem;                  // [D][64]
+  float* Ks = Qs + D * 64;           // [D][64]
+  float* Vs = Ks + D * 64;           // [64][D]
+  float* Ps = Vs + 64 * D;           // [64 tokens][64 queries]
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int q0 = blockIdx.x * 64, head = blockIdx.y, z = blockIdx.z;
+  const int t_begin = z * a.tokens_per_split, t_end = min(a.N, t_begin + a.tokens_per_split);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // lane -> row, so that the transposed stores are consecutive
+  for (int idx = tid; idx < 64 * (D / 4); idx += 256) {
+    const int i = idx % 64, d = idx / 64 * 4;
+    const float4 v = q0 + i < a.Q ? *reinterpret_cast<const float4*>(a.q + static_cast<size_t>(q0 + i) * a.q_stride_token +
+                                                                    static_cast<size_t>(head) * a.q_stride_head + d) : zero;
+    Qs[d * 64 + i] = v.x; Qs[(d + 1) * 64 + i] = v.y; Qs[(d + 2) * 64 + i] = v.z; Qs[(d + 3) * 64 + i] = v.w;
+  }
+  constexpr int OP = D / 32;         // pairs of O columns per thread
+  uint64_t o[4][OP];
+  float m_run[4], l_run[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m_run[i] = -INFINITY;
+    l_run[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < OP; ++c) o[i][c] = 0ull;
+  }
+  for (int t0 = t_begin; t0 < t_end; t0 += 64) {
+    __syncthreads();                 // previous tile fully consumed
+    for (int idx = tid; idx < 64 * (D / 4); idx += 256) {
+      const int i = idx % 64, d = idx / 64 * 4;
+      const float4 v = t0 + i < t_end ? *reinterpret_cast<const float4*>(a.k + static_cast<size_t>(t0 + i) * a.kv_stride_token +
+                                                                        static_cast<size_t>(head) * a.kv_stride_head + d) : zero;
+      Ks[d * 64 + i] = v.x; Ks[(d + 1) * 64 + i] = v.y; Ks[(d + 2) * 64 + i] = v.z; Ks[(d + 3) * 64 + i] = v.w;
+    }
+    for (int idx = tid; idx < 64 * (D / 4); idx += 256) {
+      const int i = idx / (D / 4), d = idx % (D / 4) * 4;
+      *reinterpret_cast<float4*>(Vs + i * D + d) =
+          t0 + i < t_end ? *reinterpret_cast<const float4*>(a.v + static_cast<size_t>(t0 + i) * a.kv_stride_token +
+                                                           static_cast<size_t>(head) * a.kv_stride_head + d) : zero;
+    }
+    __syncthreads();
+    uint64_t s2[4][2] = {};
+#pragma unroll 8
+    for (int d = 0; d < D; ++d) {
+      const float4 qa = *reinterpret_cast<const float4*>(Qs + d * 64 + ty * 4);
+      const ulonglong2 kb = *reinterpret_cast<const ulonglong2*>(Ks + d * 64 + tx * 4);
+      const float qv[4] = {qa.x, qa.y, qa.z, qa.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint64_t q2 = pair_f32(qv[i], qv[i]);
+        s2[i][0] = fma_f32x2(q2, kb.x, s2[i][0]);
+        s2[i][1] = fma_f32x2(q2, kb.y, s2[i][1]);
+      }
+    }
+    float weight[4][4];              // [query][token]
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float s[4];
+      split_f32(s2[i][0], s[0], s[1]);
+      split_f32(s2[i][1], s[2], s[3]);
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[j] = t0 + tx * 4 + j < t_end ? s[j] * a.scale : -INFINITY;
+        mx = fmaxf(mx, s[j]);
+      }
+#pragma unroll
+      for (int off = 8; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const float m_new = fmaxf(m_run[i], mx);   // finite: every processed tile has a valid token
+      const float alpha = expf(m_run[i] - m_new);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        weight[i][j] = expf(s[j] - m_new);
+        sum += weight[i][j];
+      }
+#pragma unroll
+      for (int off = 8; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      l_run[i] = l_run[i] * alpha + sum;
+      m_run[i] = m_new;
+      const uint64_t alpha2 = pair_f32(alpha, alpha);
+#pragma unroll
+      for (int c = 0; c < OP; ++c) o[i][c] = fma_f32x2(o[i][c], alpha2, 0ull);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<float4*>(Ps + (tx * 4 + j) * 64 + ty * 4) =
+          make_float4(weight[0][j], weight[1][j], weight[2][j], weight[3][j]);
+    __syncthreads();
+#pragma unroll 4
+    for (int t = 0; t < 64; ++t) {
+      const float4 p4 = *reinterpret_cast<const float4*>(Ps + t * 64 + ty * 4);
+      const float pv[4] = {p4.x, p4.y, p4.z, p4.w};
+      uint64_t vv[OP];
+#pragma unroll
+      for (int c = 0; c < OP; ++c) vv[c] = *reinterpret_cast<const uint64_t*>(Vs + t * D + c * 32 + tx * 2);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint64_t p2 = pair_f32(pv[i], pv[i]);
+#pragma unroll
+        for (int c = 0; c < OP; ++c) o[i][c] = fma_f32x2(p2, vv[c], o[i][c]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int qi = q0 + ty * 4 + i;
+    if (qi >= a.Q) continue;
+    const float inv = l_run[i] > 0.f ? 1.0f / l_run[i] : 0.f;
+    const size_t row = (static_cast<size_t>(z) * a.Q + qi) * a.out_heads + head;
+#pragma unroll
+    for (int c = 0; c < OP; ++c) {
+      float lo, hi;
+      split_f32(o[i][c], lo, hi);
+      *reinterpret_cast<float2*>(a.out + row * D + c * 32 + tx * 2) = make_float2(lo * inv, hi * inv);
+    }
+    if (tx == 0) a.lse[row] = l_run[i] > 0.f ? m_run[i] + logf(l_run[i]) : -INFINITY;
+  }
+}
+
+template <class K>
+int allow_smem(K kernel) {
+  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_FLOATS * 4));
+  return NKV_OK;
+}
+
+}  // namespace
+
+int simt_assign(const void* x, int x_dtype, const void* centers, int c_dtype, int S, int J,
+                int C, void* ids, int id_bytes, int32_t* labels32, cudaStream_t stream) {
+  if (S == 0) return NKV_OK;
+  int rc = allow_smem(assign_kernel);
+  if (rc != NKV_OK) return rc;
+  assign_kernel<<<ceil_div(S, TILE), THREADS, SMEM_FLOATS * 4, stream>>>(
+      x, x_dtype, vector_rows(x, x_dtype, J), centers, c_dtype, vector_rows(centers, c_dtype, J), S, J, C, ids,
+      id_bytes, labels32);
+  NKV_LAUNCH_CHECK("assign_kernel");
+  return NKV_OK;
+}
+
+int simt_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
+                 int id_bytes, const float* mean, const void* encoder, int enc_dtype, int S,
+                 int J, int r, void* coeff, cudaStream_t stream) {
+  if (S == 0) return NKV_OK;
+  const dim3 grid(ceil_div(S, TILE), ceil_div(r, TILE));
+  const bool e_vec = vector_rows(encoder, enc_dtype, J) && vector_rows(mean, NKV_F32, J);
+  auto kernel = enc_dtype == NKV_BF16 ? project_kernel<true> : project_kernel<false>;
+  int rc = allow_smem(kernel);
+  if (rc != NKV_OK) return rc;
+  kernel<<<grid, THREADS, SMEM_FLOATS * 4, stream>>>(
+      x, x_dtype, vector_rows(x, x_dtype, J), static_cast<const uint16_t*>(centers_bf16),
+      vector_rows(centers_bf16, NKV_BF16, J), ids, id_bytes, mean, encoder, e_vec, S, J, r, coeff);
+  NKV_LAUNCH_CHECK("project_kernel");
+  return NKV_OK;
+}
+
+int simt_decode_rows(const nkv_history& hist, const int32_t* rows_index, int n,
+                     const void* decoder, int dec_dtype, const float* mean, int J, void* out,
+                     int out_dtype, int64_t out_stride, cudaStream_t stream) {
+  if (n == 0) return NKV_OK;
+  const dim3 grid(ceil_div(n, TILE), ceil_div(J, TILE));
+  auto kernel = dec_dtype == NKV_BF16 ? decode_rows_kernel<true> : decode_rows_kernel<false>;
+  int rc = allow_smem(kernel);
+  if (rc != NKV_OK) return rc;
+  kernel<<<grid, THREADS, SMEM_FLOATS * 4, stream>>>(hist, rows_index, n, decoder,
+                                                     vector_rows(decoder, dec_dtype, hist.rank), mean, J, out, out_dtype,
+                                                     out_stride);
+  NKV_LAUNCH_CHECK("decode_rows_kernel");
+  return NKV_OK;
+}
+
+// ---- the fp32 read: rows of a batch of heads rebuilt into scratch, then attended over history splits ----
+namespace {
+
+struct F32Plan { int batch_heads, splits, tokens_per_split; };
+
+constexpr size_t ROW_BATCH_BYTES = 512u << 20;
+
+// Splits: about two blocks per SM, at least two 64-token tiles each.
+F32Plan plan_f32(int Q, int heads, int d, int tokens, bool rebuild) {
+  F32Plan plan{};
+  const size_t head_bytes = static_cast<size_t>(tokens) * d * 8;
+  int batches = 1;
+  while (rebuild && batches < heads && head_bytes * ceil_div(heads, batches) > ROW_BATCH_BYTES) ++batches;
+  plan.batch_heads = ceil_div(heads, batches);
+  const int tiles = ceil_div(tokens, 64);
+  const long long blocks = static_cast<long long>(ceil_div(Q, 64)) * plan.batch_heads;
+  long long splits = (2ll * sm_count() + blocks / 2) / blocks;
+  if (splits > tiles / 2) splits = tiles / 2;
+  if (splits > 16) splits = 16;
+  if (splits < 1) splits = 1;
+  const int per = ceil_div(tiles, static_cast<int>(splits));
+  plan.splits = ceil_div(tiles, per);
+  plan.tokens_per_split = per * 64;
+  return plan;
+}
+
+size_t partial_bytes(const F32Plan& plan, int Q, int heads, int d) {
+  return plan.splits > 1 ? static_cast<size_t>(plan.splits) * Q * heads * (static_cast<size_t>(d) + 4) * 4 : 0;
+}
+
+template <int D>
+int launch_rows(const RowAttn& a, int heads, int splits, cudaStream_t stream) {
+  const size_t smem = sizeof(float) * (3 * D * 64 + 64 * 64);
+  NKV_CUDA(cudaFuncSetAttribute(attn_rows_f32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  attn_rows_f32_kernel<D><<<dim3(ceil_div(a.Q, 64), heads, splits), 256, smem, stream>>>(a);
+  NKV_LAUNCH_CHECK("attn_rows_f32_kernel");
+  return NKV_OK;
+}
+
+}  // namespace
+
+bool f32_attn_by_rows(int dk, int dv) { return dk == dv && (dk == 64 || dk == 128); }
+
+size_t f32_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens) {
+  if (Q <= 0 || heads <= 0 || tokens <= 0) return 0;
+  const F32Plan plan = plan_f32(Q, heads, d, tokens, true);
+  return partial_bytes(plan, Q, heads, d) + static_cast<size_t>(tokens) * plan.batch_heads * d * 8 + 512;
+}
+
+int f32_attn_by_rows_run(const float* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int d,
+                         const nkv_history* hist_k, const nkv_history* hist_v, const float* wk, const float* bias_k,
+                         const float* wv, const float* bias_v, float scale, float* out, float* lse, void* workspace,
+                         cudaStream_t stream) {
+  if (Q == 0 || heads == 0) return NKV_OK;
+  const int N = hist_k->tokens, rank = hist_k->rank;
+  const F32Plan plan = plan_f32(Q, heads, d, N, true);
+  uint8_t* space = static_cast<uint8_t*>(workspace);
+  space += (256 - (reinterpret_cast<uintptr_t>(space) & 255)) & 255;
+  const size_t rows = static_cast<size_t>(Q) * heads;
+  float* part_out = plan.splits > 1 ? reinterpret_cast<float*>(space) : out;
+  float* part_lse = plan.splits > 1 ? part_out + plan.splits * rows * d : lse;
+  float* rows_k = reinterpret_cast<float*>(space + (partial_bytes(plan, Q, heads, d) + 255) / 256 * 256);
+  float* rows_v = rows_k + static_cast<size_t>(N) * plan.batch_heads * d;
+  for (int h0 = 0; h0 < heads; h0 += plan.batch_heads) {
+    const int hb = heads - h0 < plan.batch_heads ? heads - h0 : plan.batch_heads;
+    const size_t col0 = static_cast<size_t>(h0) * d;
+    const int J = hb * d;
+    nkv_history hk = *hist_k, hv = *hist_v;
+    hk.centers = static_cast<const uint16_t*>(hk.centers) + col0;
+    hv.centers = static_cast<const uint16_t*>(hv.centers) + col0;
+    int rc = simt_decode_rows(hk, nullptr, N, wk + col0 * rank, NKV_F32, bias_k + col0, J, rows_k, NKV_F32, J, stream);
+    if (rc == NKV_OK)
+      rc = simt_decode_rows(hv, nullptr, N, wv + col0 * rank, NKV_F32, bias_v + col0, J, rows_v, NKV_F32, J, stream);
+    if (rc != NKV_OK) return rc;
+    RowAttn a{};
+    a.q = q + h0 * q_stride_head; a.q_stride_token = q_stride_token; a.q_stride_head = q_stride_head;
+    a.k = rows_k; a.v = rows_v; a.kv_stride_token = J; a.kv_stride_head = d;
+    a.Q = Q; a.heads = hb; a.out_heads = heads; a.N = N; a.tokens_per_split = plan.tokens_per_split; a.scale = scale;
+    a.out = part_out + col0; a.lse = part_lse + h0;
+    rc = d == 128 ? launch_rows<128>(a, hb, plan.splits, stream) : launch_rows<64>(a, hb, plan.splits, stream);
+    if (rc != NKV_OK) return rc;
+  }
+  if (plan.splits == 1) return NKV_OK;
+  const void* outs[16];
+  const float* lses[16];
+  for (int z = 0; z < plan.splits; ++z) {
+    outs[z] = part_out + z * rows * d;
+    lses[z] = part_lse + z * rows;
+  }
+  return lse_merge(outs, lses, plan.splits, static_cast<int64_t>(rows), d, NKV_F32, out, lse, stream);
+}
+
+}  // namespace nkv

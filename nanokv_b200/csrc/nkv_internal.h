@@ -14,7 +14,7 @@ int simt_project(const void* x, int x_dtype, const void* centers_bf16, const voi
                  int J, int r, void* coeff, cudaStream_t stream);
 int simt_decode_rows(const nkv_history& hist, const int32_t* rows_index, int n,
                      const void* decoder, int dec_dtype, const float* mean, int J, void* out,
-                     int out_dtype, cudaStream_t stream);
+                     int out_dtype, int64_t out_stride, cudaStream_t stream);
 int simt_attn(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head, int Q,
               int heads, int dk, int dv, const nkv_history* hist_k, const nkv_history* hist_v,
               const void* wk, const float* bias_k, const void* wv, const float* bias_v,
@@ -22,6 +22,13 @@ int simt_attn(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride
               int64_t kv_stride_head, int N, float scale, void* out, float* lse,
               cudaStream_t stream, const nkv_rope* rope = nullptr, const nkv_camera* cam_k = nullptr,
               const nkv_camera* cam_v = nullptr);
+// the fp32 read in two kernels per batch of heads (nkv_f32.cu)
+bool f32_attn_by_rows(int dk, int dv);
+size_t f32_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens);
+int f32_attn_by_rows_run(const float* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int d,
+                         const nkv_history* hist_k, const nkv_history* hist_v, const float* wk, const float* bias_k,
+                         const float* wv, const float* bias_v, float scale, float* out, float* lse, void* workspace,
+                         cudaStream_t stream);
 int camera_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head, int S, int heads,
                 int d, const nkv_camera& camera, void* out, cudaStream_t stream);
 int rope_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head, int S, int heads,

@@ -1,10 +1,7 @@
-// fp32 CUDA-core kernels of the compressed-KV path.
-//
-// These carry the fp32 configuration (operators stored in fp32, where the
-// reference runs true IEEE fp32 GEMMs and tensor cores have no matching
-// mode) and the online C-means, whose centres are fp32 running means.  With
-// `emulate_bf16` they reproduce the rounding points of the bf16 path, which
-// the test-suite uses to cross-check the tensor-core kernels at full size.
+// CUDA-core kernels of the compressed-KV path: the fused read that rebuilds K / V tiles in shared memory
+// (fp32 with a positional restore or narrow heads, and bf16 with the rounding points of the tensor-core
+// path, which the test-suite uses to cross-check it), plain attention, the online C-means' updates,
+// rotations and camera transforms of explicit rows.
 #include "nkv_internal.h"
 
 namespace nkv {
@@ -43,180 +40,6 @@ __device__ __forceinline__ void gemm_tile(float (&acc)[4][4], int K, FA loadA, F
         for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
     __syncthreads();
-  }
-}
-
-// squared norm of `rows` consecutive rows (<= 64) into out[0..64), 4 threads per row
-__device__ __forceinline__ void row_sqnorms(const void* base, int dtype, int first, int count,
-                                            int total, int J, float* out) {
-  const int tid = threadIdx.x, row = tid >> 2, part = tid & 3;
-  float sum = 0.f;
-  if (row < count && first + row < total) {
-    size_t off = static_cast<size_t>(first + row) * J;
-    for (int j = part; j < J; j += 4) {
-      float v = load_float(base, dtype, off + j);
-      sum = fmaf(v, v, sum);
-    }
-  }
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  if (part == 0) out[row] = sum;
-}
-
-// ---------------------------------------------------------------- assignment
-__global__ void __launch_bounds__(THREADS)
-assign_kernel(const void* x, int x_dtype, const void* centers, int c_dtype, int S, int J, int C,
-              void* ids, int id_bytes, int32_t* labels32) {
-  __shared__ float As[BK * (BM + PAD)], Bs[BK * (BN + PAD)];
-  __shared__ float xn[BM], cn[BN];
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int m0 = blockIdx.x * BM;
-  row_sqnorms(x, x_dtype, m0, BM, S, J, xn);
-  float best_d[4];
-  int best_i[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { best_d[i] = INFINITY; best_i[i] = 0; }
-  for (int n0 = 0; n0 < C; n0 += BN) {
-    __syncthreads();
-    row_sqnorms(centers, c_dtype, n0, BN, C, J, cn);
-    float acc[4][4] = {};
-    auto loadA = [&](int m, int k) {
-      int t = m0 + m;
-      return t < S ? load_float(x, x_dtype, static_cast<size_t>(t) * J + k) : 0.f;
-    };
-    auto loadB = [&](int n, int k) {
-      int c = n0 + n;
-      return c < C ? load_float(centers, c_dtype, static_cast<size_t>(c) * J + k) : 0.f;
-    };
-    gemm_tile(acc, J, loadA, loadB, As, Bs);  // ends with __syncthreads: xn / cn visible
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float d = INFINITY;
-      int idx = 0x7fffffff;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        int c = n0 + tx * 4 + j;
-        if (c < C) {
-          // (||x||^2 + ||c||^2) - 2 x.c, in that association, in fp32
-          float dist = __fsub_rn(__fadd_rn(xn[ty * 4 + i], cn[tx * 4 + j]),
-                                 __fmul_rn(2.0f, acc[i][j]));
-          if (dist < d) { d = dist; idx = c; }
-        }
-      }
-#pragma unroll
-      for (int off = 8; off >= 1; off >>= 1) {
-        float od = __shfl_xor_sync(0xffffffffu, d, off);
-        int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-        if (od < d || (od == d && oi < idx)) { d = od; idx = oi; }
-      }
-      if (d < best_d[i]) { best_d[i] = d; best_i[i] = idx; }
-    }
-  }
-  if (tx == 0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int t = m0 + ty * 4 + i;
-      if (t < S) {
-        if (ids) {
-          if (id_bytes == 1) static_cast<uint8_t*>(ids)[t] = static_cast<uint8_t>(best_i[i]);
-          else static_cast<uint16_t*>(ids)[t] = static_cast<uint16_t>(best_i[i]);
-        }
-        if (labels32) labels32[t] = best_i[i];
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- projection
-template <bool BF16>
-__global__ void __launch_bounds__(THREADS)
-project_kernel(const void* x, int x_dtype, const uint16_t* centers, const void* ids, int id_bytes,
-               const float* mean, const void* encoder, int S, int J, int r, void* coeff) {
-  __shared__ float As[BK * (BM + PAD)], Bs[BK * (BN + PAD)];
-  __shared__ int crow[BM];
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  if (tid < BM) crow[tid] = (m0 + tid < S) ? load_id(ids, id_bytes, m0 + tid) : 0;
-  __syncthreads();
-  float acc[4][4] = {};
-  auto loadA = [&](int m, int k) {
-    int t = m0 + m;
-    if (t >= S) return 0.f;
-    float v = load_float(x, x_dtype, static_cast<size_t>(t) * J + k);
-    float c = bf16_bits_to_float(centers[static_cast<size_t>(crow[m]) * J + k]);
-    float res = __fsub_rn(__fsub_rn(v, c), mean[k]);
-    return BF16 ? round_to_bf16(res) : res;
-  };
-  auto loadB = [&](int n, int k) {
-    int c = n0 + n;
-    return c < r ? load_float(encoder, BF16 ? NKV_BF16 : NKV_F32, static_cast<size_t>(c) * J + k)
-                 : 0.f;
-  };
-  gemm_tile(acc, J, loadA, loadB, As, Bs);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int t = m0 + ty * 4 + i;
-    if (t >= S) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int c = n0 + tx * 4 + j;
-      if (c < r) store_float(coeff, BF16 ? NKV_BF16 : NKV_F32, static_cast<size_t>(t) * r + c,
-                             acc[i][j]);
-    }
-  }
-}
-
-// -------------------------------------------------------------------- decode
-template <bool BF16>
-__global__ void __launch_bounds__(THREADS)
-decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* decoder,
-                   const float* mean, int J, void* out, int out_dtype) {
-  __shared__ float As[BK * (BM + PAD)], Bs[BK * (BN + PAD)];
-  __shared__ int tok[BM], crow[BM];
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  if (tid < BM) {
-    int t = -1, row = 0;
-    if (m0 + tid < n) {
-      t = rows_index ? rows_index[m0 + tid] : m0 + tid;
-      if (t < 0 || t >= h.tokens) t = -1; else row = center_row_of(h, t);
-    }
-    tok[tid] = t;
-    crow[tid] = row;
-  }
-  __syncthreads();
-  float acc[4][4] = {};
-  auto loadA = [&](int m, int k) {
-    int t = tok[m];
-    if (t < 0) return 0.f;
-    float v = latent_value(h, t, k);
-    return BF16 ? round_to_bf16(v) : v;
-  };
-  auto loadB = [&](int nn, int k) {
-    int c = n0 + nn;
-    return c < J ? load_float(decoder, BF16 ? NKV_BF16 : NKV_F32,
-                              static_cast<size_t>(c) * h.rank + k) : 0.f;
-  };
-  gemm_tile(acc, h.rank, loadA, loadB, As, Bs);
-  const uint16_t* centers = static_cast<const uint16_t*>(h.centers);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int m = ty * 4 + i;
-    if (m0 + m >= n || tok[m] < 0) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int c = n0 + tx * 4 + j;
-      if (c >= J) continue;
-      float center = bf16_bits_to_float(centers[static_cast<size_t>(crow[m]) * h.center_width + c]);
-      float v;
-      if (BF16) {
-        v = round_to_bf16(__fadd_rn(acc[i][j], round_to_bf16(mean[c])));
-        v = round_to_bf16(__fadd_rn(v, center));
-      } else {
-        v = __fadd_rn(__fadd_rn(acc[i][j], mean[c]), center);
-      }
-      store_float(out, out_dtype, static_cast<size_t>(m0 + m) * J + c, v);
-    }
   }
 }
 
@@ -598,46 +421,6 @@ __global__ void kmeans_store_kernel(const float* centers, const int32_t* labels,
 }
 
 }  // namespace
-
-int simt_assign(const void* x, int x_dtype, const void* centers, int c_dtype, int S, int J,
-                int C, void* ids, int id_bytes, int32_t* labels32, cudaStream_t stream) {
-  if (S == 0) return NKV_OK;
-  assign_kernel<<<ceil_div(S, BM), THREADS, 0, stream>>>(x, x_dtype, centers, c_dtype, S, J, C,
-                                                        ids, id_bytes, labels32);
-  NKV_LAUNCH_CHECK("assign_kernel");
-  return NKV_OK;
-}
-
-int simt_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
-                 int id_bytes, const float* mean, const void* encoder, int enc_dtype, int S,
-                 int J, int r, void* coeff, cudaStream_t stream) {
-  if (S == 0) return NKV_OK;
-  dim3 grid(ceil_div(S, BM), ceil_div(r, BN));
-  const uint16_t* centers = static_cast<const uint16_t*>(centers_bf16);
-  if (enc_dtype == NKV_BF16)
-    project_kernel<true><<<grid, THREADS, 0, stream>>>(x, x_dtype, centers, ids, id_bytes, mean,
-                                                       encoder, S, J, r, coeff);
-  else
-    project_kernel<false><<<grid, THREADS, 0, stream>>>(x, x_dtype, centers, ids, id_bytes, mean,
-                                                        encoder, S, J, r, coeff);
-  NKV_LAUNCH_CHECK("project_kernel");
-  return NKV_OK;
-}
-
-int simt_decode_rows(const nkv_history& hist, const int32_t* rows_index, int n,
-                     const void* decoder, int dec_dtype, const float* mean, int J, void* out,
-                     int out_dtype, cudaStream_t stream) {
-  if (n == 0) return NKV_OK;
-  dim3 grid(ceil_div(n, BM), ceil_div(J, BN));
-  if (dec_dtype == NKV_BF16)
-    decode_rows_kernel<true><<<grid, THREADS, 0, stream>>>(hist, rows_index, n, decoder, mean, J,
-                                                           out, out_dtype);
-  else
-    decode_rows_kernel<false><<<grid, THREADS, 0, stream>>>(hist, rows_index, n, decoder, mean, J,
-                                                            out, out_dtype);
-  NKV_LAUNCH_CHECK("decode_rows_kernel");
-  return NKV_OK;
-}
 
 int simt_attn(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head, int Q,
               int heads, int dk, int dv, const nkv_history* hist_k, const nkv_history* hist_v,
