@@ -952,6 +952,116 @@ head_linear_kernel(const void* x, long long stride_row, long long stride_head, c
   }
 }
 
+// ---- the same on the tensor cores (bf16, widths in multiples of 16 / 8) -------------------------------
+// Bound: memory (rows in, rows out; the map comes from L2).  Block = 128 rows of one head, four warps of
+// 32 rows; rows and map in shared memory with 16 bytes of padding per row (conflict-free ldmatrix), the
+// results leave through the rows' place in whole 16-byte pieces.  A 128 x 64 tcgen05 tile would spend more
+// time setting up tensor memory than multiplying.  4,680 rows of 18 heads 128 -> 32 and 6 heads
+// 128 -> 128, and back: 326 us on the CUDA cores (one fp32 chain per output) for the four calls.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9},"
+               " {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+constexpr int HL_ROWS = 128;
+template <int NPAIRS>   // pairs of 8-column tiles a thread accumulates: dout <= 16 * NPAIRS
+__global__ void __launch_bounds__(128)
+head_linear_mma_kernel(const uint16_t* x, long long stride_row, long long stride_head, const int32_t* heads,
+                       const uint16_t* w, long long rows, int din, int dout, int dout_pad, uint16_t* out) {
+  extern __shared__ __align__(16) uint8_t hl_smem[];
+  const int wide = din > dout_pad ? din : dout_pad;      // the rows' place also takes the results
+  const int xp = (wide + 8) * 2, wp = (NPAIRS * 16 + 8) * 2;   // row pitches in bytes
+  uint8_t* xs = hl_smem;                                 // [128][xp]
+  uint8_t* ws = hl_smem + HL_ROWS * xp;                  // [din][wp], columns past dout are zero
+  const int g = blockIdx.y, head = heads ? heads[g] : g;
+  const long long row0 = static_cast<long long>(blockIdx.x) * HL_ROWS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  const int pieces = din / 8, wpieces = NPAIRS * 2;
+  for (int i = tid; i < HL_ROWS * pieces; i += 128) {
+    const int r = i / pieces, c = i - r * pieces;
+    *reinterpret_cast<uint4*>(xs + r * xp + c * 16) =
+        row0 + r < rows ? __ldg(reinterpret_cast<const uint4*>(x + (row0 + r) * stride_row + head * stride_head) + c) : zero;
+  }
+  for (int i = tid; i < din * wpieces; i += 128) {
+    const int k = i / wpieces, c = i - k * wpieces;
+    *reinterpret_cast<uint4*>(ws + k * wp + c * 16) =
+        c * 8 < dout ? __ldg(reinterpret_cast<const uint4*>(w + (static_cast<size_t>(g) * din + k) * dout) + c) : zero;
+  }
+  __syncthreads();
+  float acc[2][NPAIRS * 2][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < NPAIRS * 2; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.f;
+  const uint32_t xbase = static_cast<uint32_t>(__cvta_generic_to_shared(xs));
+  const uint32_t wbase = static_cast<uint32_t>(__cvta_generic_to_shared(ws));
+  for (int k = 0; k < din; k += 16) {
+    uint32_t a[2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+      ldmatrix_x4(a[m], xbase + (warp * 32 + m * 16 + (lane & 15)) * xp + (k + (lane >> 4) * 8) * 2);
+#pragma unroll
+    for (int n = 0; n < NPAIRS; ++n) {
+      uint32_t b[4];
+      ldmatrix_x4_trans(b, wbase + (k + (lane & 15)) * wp + (n * 16 + (lane >> 4) * 8) * 2);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        mma_16816(acc[m][2 * n], a[m], b[0], b[1]);
+        mma_16816(acc[m][2 * n + 1], a[m], b[2], b[3]);
+      }
+    }
+  }
+  __syncwarp();     // a warp reads and rewrites its own rows only
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < NPAIRS * 2; ++n)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = warp * 32 + m * 16 + h * 8 + (lane >> 2), c = n * 8 + (lane & 3) * 2;
+        if (c < dout_pad) {
+          const uint32_t pair = float_to_bf16_bits(acc[m][n][2 * h]) |
+                                (static_cast<uint32_t>(float_to_bf16_bits(acc[m][n][2 * h + 1])) << 16);
+          *reinterpret_cast<uint32_t*>(xs + r * xp + c * 2) = pair;
+        }
+      }
+  __syncwarp();
+  const int opieces = dout_pad / 8, held = NPAIRS * 2;
+  for (int i = lane; i < 32 * opieces; i += 32) {
+    const int r = warp * 32 + i / opieces, c = i % opieces;
+    if (row0 + r < rows)
+      *reinterpret_cast<uint4*>(out + ((row0 + r) * gridDim.y + g) * static_cast<size_t>(dout_pad) + c * 8) =
+          c < held ? *reinterpret_cast<const uint4*>(xs + r * xp + c * 16) : zero;
+  }
+}
+
+template <int NPAIRS>
+int launch_head_linear_mma(const void* x, int64_t stride_row, int64_t stride_head, const int32_t* heads, const void* w,
+                           int64_t rows, int group_heads, int din, int dout, int dout_pad, void* out, cudaStream_t stream) {
+  const int wide = din > dout_pad ? din : dout_pad;
+  const size_t smem = static_cast<size_t>(HL_ROWS) * (wide + 8) * 2 + static_cast<size_t>(din) * (NPAIRS * 16 + 8) * 2;
+  auto kernel = head_linear_mma_kernel<NPAIRS>;
+  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  dim3 grid(static_cast<unsigned>((rows + HL_ROWS - 1) / HL_ROWS), static_cast<unsigned>(group_heads));
+  kernel<<<grid, 128, smem, stream>>>(static_cast<const uint16_t*>(x), stride_row, stride_head, heads,
+                                      static_cast<const uint16_t*>(w), rows, din, dout, dout_pad, static_cast<uint16_t*>(out));
+  NKV_LAUNCH_CHECK("head_linear_mma_kernel");
+  return NKV_OK;
+}
+
 int head_linear(const void* x, int dtype, int64_t stride_row, int64_t stride_head, const int32_t* heads,
                 const void* w, int64_t rows, int group_heads, int din, int dout, int dout_pad, void* out,
                 cudaStream_t stream) {
@@ -962,6 +1072,13 @@ int head_linear(const void* x, int dtype, int64_t stride_row, int64_t stride_hea
   NKV_REQUIRE(smem <= 200 * 1024 && dout_pad <= 128 && (din * dout) % 4 == 0, NKV_ERR_UNSUPPORTED,
               "head_linear: a %d x %d map (padded to %d) is beyond the built kernel", din, dout, dout_pad);
   if (rows == 0) return NKV_OK;
+  // whole 16-byte pieces in and out, K steps of 16: the tensor-core form
+  if (dtype == NKV_BF16 && din % 16 == 0 && din <= 128 && dout % 8 == 0 && dout_pad % 8 == 0 && stride_row % 8 == 0 &&
+      stride_head % 8 == 0 && !simt_forced() &&
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+    auto run = dout <= 32 ? launch_head_linear_mma<2> : (dout <= 64 ? launch_head_linear_mma<4> : launch_head_linear_mma<8>);
+    return run(x, stride_row, stride_head, heads, w, rows, group_heads, din, dout, dout_pad, out, stream);
+  }
   dim3 grid(static_cast<unsigned>((rows + 63) / 64), static_cast<unsigned>(group_heads));
   if (dtype == NKV_F32) {
     NKV_CUDA(cudaFuncSetAttribute(head_linear_kernel<NKV_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -14,9 +14,11 @@
 // contiguous run of equal length, so the last wave is never emptier than one tile and a run expands
 // two or three token tiles.  No wait crosses clusters.
 //
-// Bound: the decoder stream from L2 into three 16 KB stages (all that 160 KB of latents leave at rank
-// 640).  28,080 rows x 5,120 columns at rank 640, K and V (two calls): 0.545 ms = 675 TFLOP/s; the
-// CUDA-core kernel that served bf16 operators before took 17.9 ms.
+// Bound: the epilogue's chain of latencies per 32 columns (accumulator read, staging, store; without it the
+// same launch takes 145 us), then the decoder stream into three 16 KB stages, all that 160 KB of latents
+// leave at rank 640.  28,080 rows x 5,120 columns at rank 640: 191 us = 964 TFLOP/s; 255 with cluster-scope
+// waits and releases on every hand-off, bias and centres loaded where they are used, and the centres
+// staged; the CUDA-core kernel that served bf16 operators before took 8.9 ms.
 //
 // Warps 0-7: expansion and epilogue (warp w serves TMEM lanes 32 (w & 3) .. and column half w >> 2),
 // warp 8 lane 0: TMA, warp 9 of the even CTA: MMA.
@@ -40,7 +42,8 @@ constexpr int META = 1024;
 constexpr int SCRATCH = COMPUTE_WARPS * 2048;
 constexpr size_t SMEM_LIMIT = 232448;
 
-enum Bar { FULL = 0, FREE = 8, A_FULL = 16, ACC_FULL = 26, ACC_FREE = 28, NUM_BARS = 30 };
+constexpr int A_GROUP = 5;                  // latent chunks handed over together
+enum Bar { FULL = 0, FREE = 8, A_FULL = 16, ACC_FULL = 18, ACC_FREE = 20, NUM_BARS = 22 };
 
 struct Tensor {
   nkv_history h;
@@ -96,6 +99,18 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
       : "memory");
 }
 
+__device__ __forceinline__ uint4 add_bf16x8(uint4 a, const uint4& b) {
+  uint32_t* x = &a.x;
+  const uint32_t* y = &b.x;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 sum = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(x + i),
+                                       *reinterpret_cast<const __nv_bfloat162*>(y + i));
+    x[i] = *reinterpret_cast<const uint32_t*>(&sum);
+  }
+  return a;
+}
+
 // a run of column tiles of one token tile
 struct Run { int tensor, m, nt0, count; };
 __device__ __forceinline__ Run run_at(const Params& p, int w, int w_end) {
@@ -108,8 +123,19 @@ __device__ __forceinline__ Run run_at(const Params& p, int w, int w_end) {
   return r;
 }
 
+// Acquire at block scope: what is handed over lies in shared memory or TMEM.  (A cluster-scope acquire also
+// gives up the first-level cache's lines, which hold the epilogue's bias, centre and rotation rows.)
 __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code) ? 1 : 0) != 0;
+}
+// the same for latents, which the other CTA's threads wrote
+__device__ __forceinline__ bool wait_all_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
   return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code) ? 1 : 0) != 0;
+}
+// Arrival that hands back tensor memory whose loads have completed: nothing written is published by it, so
+// it does not wait for the stores under way (a releasing arrival would: a tile's rows to L2, every tile).
+__device__ __forceinline__ void arrive_relaxed(uint32_t bar_cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
 template <bool ROPE, bool CAM>
@@ -139,8 +165,8 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       mbar_init(&bars[FULL + s], 1);
       mbar_init(&bars[FREE + s], 1);
     }
-    for (int c = 0; c < MAX_CHUNKS; ++c) mbar_init(&bars[A_FULL + c], 2 * COMPUTE_WARPS);
     for (int b = 0; b < 2; ++b) {
+      mbar_init(&bars[A_FULL + b], 2 * COMPUTE_WARPS);
       mbar_init(&bars[ACC_FULL + b], 1);
       mbar_init(&bars[ACC_FREE + b], 2 * COMPUTE_WARPS);
     }
@@ -169,7 +195,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
           const int y = (r.nt0 + k) * TN + static_cast<int>(cta) * TM;
           for (int c = 0; c < nchunks; ++c, ++it) {
             const int s = it % nst, u = it / nst;
-            if (u >= 1) ok = mbar_wait_cluster(&bars[FREE + s], (u - 1) & 1, abort_flag, 700 + s);
+            if (u >= 1) ok = mbar_wait(&bars[FREE + s], (u - 1) & 1, abort_flag, 700 + s);
             if (!ok) break;
             // both halves land on the even CTA's barrier, whose MMA warp reads them
             if (cta == 0) mbar_arrive_expect_tx(&bars[FULL + s], 2 * CHUNK_BYTES);
@@ -200,7 +226,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
           const uint32_t acc = tmem_base + b * TN;
           for (int c = 0; c < nchunks && ok; ++c, ++it) {
             const int s = it % nst, u = it / nst;
-            if (k == 0) ok = wait_all(&bars[A_FULL + c], seg & 1, abort_flag, 720 + c);
+            if (k == 0 && c % A_GROUP == 0) ok = wait_all_cluster(&bars[A_FULL + c / A_GROUP], seg & 1, abort_flag, 720 + c);
             ok = ok && wait_all(&bars[FULL + s], u & 1, abort_flag, 730 + s);
             if (!ok) break;
             tc_fence_after();
@@ -229,10 +255,6 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
     uint8_t* stage = scratch + warp * 2048;
     bool ok = true;
     int tile = 0;                       // tiles whose epilogue is done or pending, in order
-    auto arrive_even = [&](uint64_t* bar) {   // one arrival per warp on the even CTA's barrier
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(bar), 0));
-    };
     // this lane's token of a run (its row of the tile): history row, or -1 past the end of the list
     auto token_of = [&](const Run& r) {
       const int m = (r.m * 2 + static_cast<int>(cta)) * TM + row;
@@ -241,44 +263,43 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       const int tok = t.rows != nullptr ? __ldg(t.rows + m) : m;
       return tok < 0 || tok >= t.h.tokens ? -1 : tok;
     };
-    auto expand = [&](const Run& r, int tok) {
+    // this thread's codes of its token, 16 bytes of every chunk, with their scales
+    struct Codes { uint4 word[MAX_CHUNKS]; uint16_t scale[MAX_CHUNKS]; };
+    auto fetch_codes = [&](const Run& r, int tok, Codes& in) {
       const nkv_history& h = p.t[r.tensor].h;
       const uint8_t* codes = h.codes + static_cast<size_t>(tok < 0 ? 0 : tok) * (h.rank >> 1) + wg * 16;
       const uint16_t* scales = static_cast<const uint16_t*>(h.scales) + static_cast<size_t>(tok < 0 ? 0 : tok) * p.ngroups;
-      // half of the codes in flight at a time: 16 bytes of five chunks
 #pragma unroll
-      for (int half = 0; half < MAX_CHUNKS / 5; ++half) {
-        uint4 code[5];
-        uint16_t sbits[5];
-#pragma unroll
-        for (int i = 0; i < 5; ++i) {
-          const int c = half * 5 + i;
-          code[i] = make_uint4(0, 0, 0, 0);
-          sbits[i] = 0;
-          if (c < nchunks && tok >= 0) {
-            code[i] = __ldg(reinterpret_cast<const uint4*>(codes + c * 32));
-            sbits[i] = __ldg(scales + (p.ngroups == 1 ? 0 : (c * 64 + wg * 32) / p.group));
-          }
+      for (int c = 0; c < MAX_CHUNKS; ++c) {
+        in.word[c] = make_uint4(0, 0, 0, 0);
+        in.scale[c] = 0;
+        if (c < nchunks && tok >= 0) {
+          in.word[c] = __ldg(reinterpret_cast<const uint4*>(codes + c * 32));
+          in.scale[c] = __ldg(scales + (p.ngroups == 1 ? 0 : (c * 64 + wg * 32) / p.group));
         }
+      }
+    };
+    auto expand = [&](const Run& r, const Codes& in) {
+      const int scale_dtype = p.t[r.tensor].h.scale_dtype;
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
-          const int c = half * 5 + i;
-          if (c < nchunks) {
-            const uint32_t words[4] = {code[i].x, code[i].y, code[i].z, code[i].w};
-            uint8_t* dst = a_tiles + c * CHUNK_BYTES;
-            const uint32_t pair = static_cast<uint32_t>(sbits[i]) * 0x00010001u;
-            const __nv_bfloat162 scale2 = *reinterpret_cast<const __nv_bfloat162*>(&pair);
-            const float sc = scale_to_float(sbits[i], h.scale_dtype);
+      for (int c = 0; c < MAX_CHUNKS; ++c) {
+        if (c >= nchunks) break;
+        const uint32_t words[4] = {in.word[c].x, in.word[c].y, in.word[c].z, in.word[c].w};
+        uint8_t* dst = a_tiles + c * CHUNK_BYTES;
+        const uint32_t pair = static_cast<uint32_t>(in.scale[c]) * 0x00010001u;
+        const __nv_bfloat162 scale2 = *reinterpret_cast<const __nv_bfloat162*>(&pair);
+        const float sc = scale_to_float(in.scale[c], scale_dtype);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              uint4 v;
-              if (h.scale_dtype == NKV_BF16) v = p.w_perm ? dequant8_bf16_perm(words[k], scale2) : dequant8_bf16(words[k], scale2);
-              else v = p.w_perm ? dequant8_perm(words[k], sc) : dequant8(words[k], sc);
-              *reinterpret_cast<uint4*>(dst + sw128_offset(row, wg * 32 + k * 8)) = v;
-            }
-            fence_proxy_async_all();       // the pair's MMAs read this through the async proxy
-            arrive_even(&bars[A_FULL + c]);
-          }
+        for (int k = 0; k < 4; ++k) {
+          uint4 v;
+          if (scale_dtype == NKV_BF16) v = p.w_perm ? dequant8_bf16_perm(words[k], scale2) : dequant8_bf16(words[k], scale2);
+          else v = p.w_perm ? dequant8_perm(words[k], sc) : dequant8(words[k], sc);
+          *reinterpret_cast<uint4*>(dst + sw128_offset(row, wg * 32 + k * 8)) = v;
+        }
+        if (c % A_GROUP == A_GROUP - 1 || c == nchunks - 1) {
+          fence_proxy_async();             // the pair's MMAs read this through the async proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bars[A_FULL + c / A_GROUP]), 0));
         }
       }
     };
@@ -288,8 +309,9 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       const int b = tile & 1, use = tile >> 1;
       const int m0 = (r.m * 2 + static_cast<int>(cta)) * TM + wrow0;
       const int rounds = min(4, max(0, (p.J - nt * TN - wg * 128) / 32));
-      // centre rows: 4 lanes read the 16-byte pieces of one row, 8 rows per load instruction; all
-      // rounds (one, where the restore needs the registers) are requested ahead of the accumulator wait
+      // centre rows: 4 lanes read the 16-byte pieces of one row, 8 rows per load instruction.  Centres and
+      // bias of a round are requested a round ahead (the first ones ahead of the accumulator wait): next to
+      // 220 KB of shared memory the first-level cache holds neither.
       int crow_of[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) crow_of[i] = __shfl_sync(0xffffffffu, tok < 0 ? -1 : crow, i * 8 + lane / 4);
@@ -302,9 +324,17 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
             dst[i] = __ldg(reinterpret_cast<const uint4*>(cbase + static_cast<size_t>(crow_of[i]) * t.h.center_width));
         }
       };
-      uint4 cen_all[POS ? 1 : 4][4];
+      // bias of a round's 32 columns (the same for every lane)
+      auto load_bias = [&](int sub, float4 (&dst)[8]) {
+        if (sub >= rounds) return;
+        const float4* src = reinterpret_cast<const float4*>(t.bias + nt * TN + wg * 128 + sub * 32);
 #pragma unroll
-      for (int sub = 0; sub < (POS ? 1 : 4); ++sub) load_centers(sub, cen_all[sub]);
+        for (int j = 0; j < 8; ++j) dst[j] = __ldg(src + j);
+      };
+      uint4 cen[4];
+      float4 bias[POS ? 1 : 8];
+      load_centers(0, cen);
+      if constexpr (!POS) load_bias(0, bias);
       // positional restore: table rows and frame of the four tokens this lane stores a piece of
       const bool rotate = ROPE && t.rope.cos_sin != nullptr;
       const bool transform = CAM && t.cam.matrices != nullptr;
@@ -338,7 +368,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       // The restore works on the 16-byte pieces a lane stores -- four pairs, or one camera block, of one
       // token -- because four lanes then read 128 contiguous bytes of a token's table row; a lane that
       // kept a whole row of the accumulator would gather from 32 rows at a time.  26,917 rotated tokens x
-      // 5,120 columns, rank 640 (K and V): 805 us, 1,328 with the gather per row.
+      // 5,120 columns, rank 640 (K and V): 627 us, 1,328 with the gather per row.
       auto load_rotation = [&](int head, int dcol, float2* rot) {
         const int local = dcol / 2 + (lane & 3) * 4;
         const float2* table = reinterpret_cast<const float2*>(t.rope.cos_sin);
@@ -405,93 +435,81 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
         // rotation entries of the pieces this lane stores, in flight under the rebuild
         float2 rot[ROPE ? 16 : 1];
         if (rotate) load_rotation(head, dcol, rot);
+        if (POS) asm volatile("prefetch.global.L1 [%0];" ::"l"(t.bias + col0 + (lane & 1) * 16));
         uint32_t acc_raw[32];
         tmem_ld32_issue(tmem_base + lane_sel + b * TN + wg * 128 + sub * 32, acc_raw);
-        uint4 cen[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int rloc = i * 8 + lane / 4, piece = lane & 3;
-          *reinterpret_cast<uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4)) = cen_all[POS ? 0 : sub][i];
-        }
-        if (POS) load_centers(sub + 1, cen_all[0]);
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          cen[j] = *reinterpret_cast<const uint4*>(stage + lane * 64 + ((j ^ (lane & 3)) << 4));
-        __syncwarp();
         tmem_ld32_wait(acc_raw);
         uint32_t packed[16];
 #pragma unroll
         for (int j4 = 0; j4 < 4; ++j4) {
-          const uint32_t cwords[4] = {cen[j4].x, cen[j4].y, cen[j4].z, cen[j4].w};
-          const float4 b0 = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8));
-          const float4 b1 = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8 + 4));
-          float bias[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+          float4 lo, hi;
+          if constexpr (POS) {     // the registers hold rotation entries instead: from the first-level cache
+            lo = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8));
+            hi = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8 + 4));
+          } else {
+            lo = bias[2 * j4];
+            hi = bias[2 * j4 + 1];
+          }
+          float add[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
           if (p.round_bias) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) bias[j] = round_to_bf16(bias[j]);
+            for (int j = 0; j < 8; ++j) add[j] = round_to_bf16(add[j]);
           }
 #pragma unroll
           for (int w = 0; w < 4; ++w) {
             const int j = j4 * 8 + w * 2;
-            // two bf16 roundings: of (product + bias), then of (+ centre); the packed addition of two
-            // bf16 numbers rounds their exact sum once
-            const uint32_t first = pack_bf16x2(__uint_as_float(acc_raw[j]) + bias[2 * w], __uint_as_float(acc_raw[j + 1]) + bias[2 * w + 1]);
-            const __nv_bfloat162 sum = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&first),
-                                               *reinterpret_cast<const __nv_bfloat162*>(&cwords[w]));
-            packed[j4 * 4 + w] = *reinterpret_cast<const uint32_t*>(&sum);
+            packed[j4 * 4 + w] = pack_bf16x2(__uint_as_float(acc_raw[j]) + add[2 * w],
+                                             __uint_as_float(acc_raw[j + 1]) + add[2 * w + 1]);
           }
         }
-        // through the warp's staging area, so that a store instruction writes whole 64-byte row pieces
+        if constexpr (!POS) load_bias(sub + 1, bias);
+        // Through the warp's staging area, so that four lanes hold 64 contiguous bytes of a row: they add
+        // the centre (the second bf16 rounding: the packed addition of two bf16 numbers rounds their exact
+        // sum once), restore positions and store.  Two rows fill the banks: the swizzle follows the row pair.
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          *reinterpret_cast<uint4*>(stage + lane * 64 + ((j ^ (lane & 3)) << 4)) =
+          *reinterpret_cast<uint4*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) =
               make_uint4(packed[j * 4], packed[j * 4 + 1], packed[j * 4 + 2], packed[j * 4 + 3]);
         __syncwarp();
         uint16_t* dst = t.out + head * t.head_stride + dcol + (lane & 3) * 8;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int rloc = i * 8 + lane / 4, piece = lane & 3;
-          uint4 v = *reinterpret_cast<const uint4*>(stage + rloc * 64 + ((piece ^ (rloc & 3)) << 4));
+          uint4 v = *reinterpret_cast<const uint4*>(stage + rloc * 64 + ((piece ^ ((rloc >> 1) & 3)) << 4));
+          v = add_bf16x8(v, cen[i]);
           if (POS) restore(i, head, dcol, rot, v);
           if (crow_of[i] >= 0) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(m0 + rloc) * t.row_stride) = v;
         }
+        load_centers(sub + 1, cen);
         __syncwarp();
       };
-      if constexpr (POS) {
 #pragma unroll 1
-        for (int sub = 0; sub < rounds; ++sub) round(sub);
-      } else {
-#pragma unroll
-        for (int sub = 0; sub < 4; ++sub)
-          if (sub < rounds) round(sub);
-      }
+      for (int sub = 0; sub < rounds; ++sub) round(sub);
       tc_fence_before();
-      arrive_even(&bars[ACC_FREE + b]);
+      __syncwarp();
+      if (lane == 0) arrive_relaxed(map_to_cta(smem_u32(&bars[ACC_FREE + b]), 0));
       ++tile;
     };
 
-    Run prev{};
-    int prev_tok = -1, prev_crow = 0;
-    bool pending = false;      // the last column tile of the previous run awaits its epilogue
-    for (int w = w_begin; w < w_end && ok;) {
-      const Run r = run_at(p, w, w_end);
-      const int tok = token_of(r);
-      const int crow = tok < 0 ? 0 : center_row_of(p.t[r.tensor].h, tok);
-      // the latents in shared memory are free once the previous run's last tile is complete; the new
-      // ones go in before that tile's epilogue, so that the MMAs of this run start under it
-      if (pending) ok = wait_all(&bars[ACC_FULL + (tile & 1)], (tile >> 1) & 1, abort_flag, 750);
-      if (!ok) break;
-      expand(r, tok);
-      if (pending) epilogue(prev, prev.nt0 + prev.count - 1, prev_tok, prev_crow);
-      for (int k = 0; k + 1 < r.count && ok; ++k) epilogue(r, r.nt0 + k, tok, crow);
-      prev = r;
-      prev_tok = tok;
-      prev_crow = crow;
-      pending = true;
-      w += r.count;
+    Run run{}, next{};
+    int tok = -1, crow = 0, next_tok = -1, next_crow = 0;
+    for (int w = w_begin; w <= w_end && ok; ++w) {
+      const bool starts = w < w_end && (w == w_begin || w % p.n_tiles == 0);
+      if (starts) {
+        next = run_at(p, w, w_end);
+        next_tok = token_of(next);
+        next_crow = next_tok < 0 ? 0 : center_row_of(p.t[next.tensor].h, next_tok);
+        Codes codes;
+        fetch_codes(next, next_tok, codes);
+        // the latents in shared memory are free once the previous run's last tile is complete; the new
+        // ones go in before that tile's epilogue, so that the MMAs of this run start under it
+        if (w > w_begin) ok = wait_all(&bars[ACC_FULL + (tile & 1)], (tile >> 1) & 1, abort_flag, 750);
+        if (!ok) break;
+        expand(next, codes);
+      }
+      if (w > w_begin) epilogue(run, (w - 1) % p.n_tiles, tok, crow);
+      if (starts) { run = next; tok = next_tok; crow = next_crow; }
     }
-    if (ok && pending) epilogue(prev, prev.nt0 + prev.count - 1, prev_tok, prev_crow);
   }
   tc_fence_before();
   __syncthreads();
