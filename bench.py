@@ -34,6 +34,15 @@ METRIC = "codec_attention_history_tokens_per_s"
 UNIT = "history-tokens/s"
 
 
+def read_batches(shape, tokens: int) -> int:
+    """Head batches of one read: K and V rows of a batch take at most 512 MB of scratch (one head at least)."""
+    per_head = tokens * shape.head_dim * 4
+    batches = 1
+    while batches < shape.heads and per_head * -(-shape.heads // batches) > 512 << 20:
+        batches += 1
+    return -(-shape.heads // -(-shape.heads // batches))
+
+
 def measured_traffic(kernel: str, workload: str):
     """DRAM bytes per launch of `kernel` on `workload`, from the figures file written next to the ncu
     summary of that kernel (dram__bytes_read.sum + dram__bytes_write.sum of one launch); None when
@@ -552,16 +561,17 @@ def run_ours(args) -> dict:
                 "h2d_bytes_per_step": q_bytes * layers, "d2h_bytes_per_step": o_bytes * layers},
         "e2e_inline": {"value": tokens_per_step / (inline_seconds / e2e_steps), "unit": UNIT,
                        "note": "copies in line on the compute stream, no overlap with other layers"},
-        # per layer: fused attention + LSE merge of its history splits (+ the CP merge when sharded)
-        "gpu_launches": args.steps * layers * (2 + (1 if world > 1 else 0)),
+        # per layer and batch of heads: row decode + attention (a merge of cut units where there are any is
+        # not counted) (+ the CP merge when sharded)
+        "gpu_launches": args.steps * layers * (2 * read_batches(shape, local_tokens) + (1 if world > 1 else 0)),
         "exchange_ms_per_layer": exchange_ms,
-        "roofline": {"bound": "tensor", "kernel": "attn_codec_kernel<128>", "achieved": achieved,
+        "roofline": {"bound": "tensor", "kernel": "decode_gemm_kernel + attn_rows_kernel<128>", "achieved": achieved,
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "peak_source": f"bf16_tflops_sustained of {peak_kind}",
                      "launch_ms": kernel_s * 1e3, "flops_per_launch": flops_launch,
                      # DRAM bytes of one launch over the full layer from an ncu capture of this
                      # kernel, when one is on record (per-rank shards are not captured separately)
-                     "traffic": (measured_traffic("attn_codec_kernel", shape.name)
+                     "traffic": (measured_traffic("attn_rows_kernel", shape.name)
                                  if world == 1 and not args.history_frames else None)},
         "encode": encode,
         "clocks": clocks,
@@ -808,7 +818,7 @@ def run_fast(args) -> dict:
     # algorithmic flops: per low-width token and head group 4 Q d + 4 r d, per protected token the full read
     flops = (low_tokens * (18 * (4.0 * Q * 32 + 4.0 * r * 32) + 6 * (4.0 * Q * D + 4.0 * r * D)) +
              prot_tokens * (4.0 * Q * shape.joint + 4.0 * r * shape.joint))
-    roofline = {"bound": "tensor", "kernel": "attn_codec_kernel<64> + attn_codec_kernel<128>",
+    roofline = {"bound": "tensor", "kernel": "attn_rows_kernel<64> + attn_rows_kernel<128>",
                 "achieved": flops / seconds / 1e12, "peak": float(peaks["bf16_tflops_sustained"]),
                 "unit": "TFLOP/s", "frac": flops / seconds / 1e12 / float(peaks["bf16_tflops_sustained"]),
                 "peak_source": f"bf16_tflops_sustained of {peak_kind}", "flops_per_layer": flops,
@@ -1017,7 +1027,7 @@ def time_rope(shape, device, layers: int = 2, launches: int = 4) -> dict:
     peaks, peak_kind = measured_peaks()
     flops = attention_flops(shape.history, shape.queries, shape.joint, shape.rank)
     return {"ms_per_layer": ms, "history_tokens_per_s": shape.history / (ms / 1e3),
-            "roofline": {"bound": "tensor", "kernel": "attn_codec_kernel<128, rope>",
+            "roofline": {"bound": "tensor", "kernel": "decode_gemm_kernel<rope> + attn_rows_kernel<128>",
                          "achieved": flops / (ms / 1e3) / 1e12, "peak": float(peaks["bf16_tflops_sustained"]),
                          "unit": "TFLOP/s",
                          "frac": flops / (ms / 1e3) / 1e12 / float(peaks["bf16_tflops_sustained"]),

@@ -230,6 +230,13 @@ int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
                     const void* decoder, int decoder_dtype, const float* mean, int J,
                     void* out, int out_dtype, void* stream);
 
+/*
+ * Enters segment `index` in a device segment table: seg_start[index + 1] = stop (tokens before the next
+ * segment), seg_center_row[index] = center_row.  One launch.  No counterpart in the reference.
+ */
+int nkv_segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int center_row,
+                       void* stream);
+
 /* ---------------------------------------------------------------- attention */
 
 /*

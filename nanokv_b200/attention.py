@@ -22,9 +22,9 @@ def codec_attention(q: torch.Tensor, hist_k, hist_v, op_k: Operator, op_v: Opera
                     positions: torch.Tensor | None = None):
     """Full-dimensional read: q [Q,H,D] -> (O [Q,H,D], lse f32 [Q,H]).
 
-    K and V of every history token are rebuilt on chip from codes, scales, the
-    decoder slice of each head and the token's centre; nothing full-width is
-    written to HBM.  Replaces decode + attention of the reference
+    K and V of every history token are rebuilt from codes, scales, the decoder slice of each head and
+    the token's centre, a bounded batch of heads at a time in scratch memory (nkv_attn_codec_rows) or,
+    at ranks above 640, tile by tile inside the fused kernel.  Replaces decode + attention of the reference
     (MGM/nanokv_codec.py:393-455 + MGC/core.py:45-72).  With ``rope`` and the history tokens'
     absolute ``positions`` the rebuilt keys are rotated inside the kernel, which also replaces
     rope_pre_key_by_positions (LB/lingbot_v2_cache_runtime.py:19-76); q arrives rotated.

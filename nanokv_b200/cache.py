@@ -80,9 +80,12 @@ class CompressedHistory:
         self._starts.append(offset + count)
         self._center_rows.append(row)
         index = self.segments - 1
-        # two tiny async H2D-free updates of the device segment table
-        self.seg_start[index + 1].fill_(offset + count)
-        self.seg_center_row[index].fill_(row)
+        if self.seg_start.is_cuda:
+            with torch.cuda.device(self.seg_start.device):
+                ops.segment_append(self.seg_start, self.seg_center_row, index, offset + count, row)
+        else:
+            self.seg_start[index + 1] = offset + count
+            self.seg_center_row[index] = row
         return offset, self.centers[row:row + clusters]
 
     def view(self, start_segment: int = 0, stop_segment: int | None = None) -> HistoryView:
@@ -92,9 +95,11 @@ class CompressedHistory:
             raise ValueError("bad segment range")
         t0, t1 = self._starts[start_segment], self._starts[stop_segment]
         if start_segment == 0:
-            seg_start = self.seg_start
-        else:  # token offsets relative to the sliced arrays
-            seg_start = (self.seg_start[start_segment:stop_segment + 1] - t0).to(torch.int32)
+            return HistoryView(
+                codes=self.codes, scales=self.scales, ids=self.ids, centers=self.centers, seg_start=self.seg_start,
+                seg_center_row=self.seg_center_row, tokens=t1, segments=stop_segment, rank=self.rank, group=self.group)
+        # token offsets relative to the sliced arrays
+        seg_start = (self.seg_start[start_segment:stop_segment + 1] - t0).to(torch.int32)
         return HistoryView(
             codes=self.codes[t0:], scales=self.scales[t0:], ids=self.ids[t0:],
             centers=self.centers, seg_start=seg_start,

@@ -100,10 +100,10 @@ def encode_append(hist: CompressedHistory, rows: torch.Tensor, op: Operator,
     if clusters > hist.centers_per_segment:
         raise ValueError("more centres than the cache reserves per segment")
     offset, center_rows = hist.reserve_segment(S, clusters)
-    ids = hist.ids[offset:offset + S]
-    codes = hist.codes[offset:offset + S]
-    scales = hist.scales[offset:offset + S]
     if centers is None:
+        ids = hist.ids[offset:offset + S]
+        codes = hist.codes[offset:offset + S]
+        scales = hist.scales[offset:offset + S]
         init = kmeans_init_rows(S, clusters, seed).to(rows.device)
         ops.kmeans(rows, clusters, iters, init, centers=center_rows, ids=ids)
         ops.project_quant(rows, center_rows, ids, op.mean, op.encoder, group=hist.group, eps=quant.eps,

@@ -176,18 +176,25 @@ int nkv_kmeans(const void* x, int x_dtype, int S, int J, int C, int iters,
   return kmeans_store(centers, labels, S, J, C, centers_bf16, ids, id_bytes, s);
 }
 
-int nkv_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
-                int id_bytes, const float* mean, const void* encoder, int encoder_dtype, int S,
-                int J, int r, void* coeff, void* stream) {
+static int project_rows(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
+                        int id_bytes, const float* mean, const void* encoder, int encoder_dtype, int S,
+                        int J, int r, void* coeff, bool ordered, void* stream) {
   NKV_REQUIRE(S >= 0 && J > 0 && r > 0, NKV_ERR_INVALID, "project: S=%d J=%d r=%d", S, J, r);
   NKV_REQUIRE(encoder_dtype == NKV_F32 || encoder_dtype == NKV_BF16, NKV_ERR_INVALID,
               "project: encoder dtype");
   auto s = static_cast<cudaStream_t>(stream);
   if (encoder_dtype == NKV_BF16 && x_dtype == NKV_BF16 && !simt_forced() &&
       tc_project_supported(J, r))
-    return tc_project(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, coeff, s);
+    return tc_project(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, coeff, ordered, s);
   return simt_project(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J,
                       r, coeff, s);
+}
+
+int nkv_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
+                int id_bytes, const float* mean, const void* encoder, int encoder_dtype, int S,
+                int J, int r, void* coeff, void* stream) {
+  return project_rows(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r, coeff, true,
+                      stream);
 }
 
 int nkv_quant_pack(const void* coeff, int coeff_dtype, int S, int r, int group, float eps,
@@ -206,10 +213,10 @@ int nkv_quant_pack(const void* coeff, int coeff_dtype, int S, int r, int group, 
                     static_cast<cudaStream_t>(stream));
 }
 
-int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
+static int project_quant_rows(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
                       const float* mean, const void* encoder, int encoder_dtype, int S, int J, int r,
                       int group, float eps, int quant_mode, int scale_dtype, uint8_t* codes,
-                      void* scales, void* workspace, size_t workspace_bytes, void* stream) {
+                      void* scales, void* workspace, size_t workspace_bytes, bool ordered, void* stream) {
   NKV_REQUIRE(S >= 0 && J > 0 && r > 0 && group > 0 && r % group == 0, NKV_ERR_INVALID,
               "project_quant: S=%d J=%d r=%d group=%d", S, J, r, group);
   NKV_REQUIRE(encoder_dtype == NKV_F32 || encoder_dtype == NKV_BF16, NKV_ERR_INVALID,
@@ -225,14 +232,22 @@ int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, cons
   if (encoder_dtype == NKV_BF16 && x_dtype == NKV_BF16 && !simt_forced() &&
       tc_project_quant_supported(J, r, group) && (reinterpret_cast<uintptr_t>(codes) & 15) == 0)
     return tc_project_quant(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, eps, quant_mode,
-                            scale_dtype, codes, scales, static_cast<cudaStream_t>(stream));
+                            scale_dtype, codes, scales, ordered, static_cast<cudaStream_t>(stream));
   NKV_REQUIRE(workspace && workspace_bytes >= static_cast<size_t>(S) * r * dtype_bytes(encoder_dtype),
               NKV_ERR_INVALID, "project_quant: workspace of %zu bytes is too small", workspace_bytes);
-  int rc = nkv_project(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r,
-                       workspace, stream);
+  int rc = project_rows(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r,
+                        workspace, ordered, stream);
   if (rc != NKV_OK) return rc;
   return nkv_quant_pack(workspace, encoder_dtype, S, r, group, eps, quant_mode, scale_dtype, codes,
                         scales, stream);
+}
+
+int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
+                      const float* mean, const void* encoder, int encoder_dtype, int S, int J, int r,
+                      int group, float eps, int quant_mode, int scale_dtype, uint8_t* codes,
+                      void* scales, void* workspace, size_t workspace_bytes, void* stream) {
+  return project_quant_rows(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r, group, eps,
+                            quant_mode, scale_dtype, codes, scales, workspace, workspace_bytes, true, stream);
 }
 
 int nkv_encode_append(const void* x, int x_dtype, const void* centers_bf16, int C,
@@ -250,9 +265,16 @@ int nkv_encode_append(const void* x, int x_dtype, const void* centers_bf16, int 
   void* scales_at = static_cast<uint8_t*>(scales) + static_cast<size_t>(offset) * (r / group) * 2;
   int rc = nkv_assign(x, x_dtype, centers_bf16, NKV_BF16, S, J, C, ids_at, id_bytes, stream);
   if (rc != NKV_OK) return rc;
-  return nkv_project_quant(x, x_dtype, centers_bf16, ids_at, id_bytes, mean, encoder, encoder_dtype, S,
-                           J, r, group, eps, quant_mode, scale_dtype, codes_at, scales_at, workspace,
-                           workspace_bytes, stream);
+  return project_quant_rows(x, x_dtype, centers_bf16, ids_at, id_bytes, mean, encoder, encoder_dtype, S,
+                            J, r, group, eps, quant_mode, scale_dtype, codes_at, scales_at, workspace,
+                            workspace_bytes, false, stream);
+}
+
+int nkv_segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int center_row,
+                       void* stream) {
+  NKV_REQUIRE(seg_start && seg_center_row && index >= 0 && stop > 0 && center_row >= 0, NKV_ERR_INVALID,
+              "segment_append: index=%d stop=%d center_row=%d", index, stop, center_row);
+  return segment_append(seg_start, seg_center_row, index, stop, center_row, static_cast<cudaStream_t>(stream));
 }
 
 int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
@@ -412,7 +434,7 @@ size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, 
                                            int group, int splits) {
   if (!reads_by_rows(dtype, dk, dv, rank, group) || splits < 0 || splits > 16) return 0;
   if (dtype == NKV_F32) return f32_attn_rows_workspace_bytes(Q, heads, dk, tokens) + 256;
-  return tc_attn_rows_workspace_bytes(Q, heads, dk, tokens, splits == 0 ? 16 : splits, true) + 256;
+  return tc_attn_rows_workspace_bytes(Q, heads, dk, tokens, splits, true) + 256;
 }
 
 int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
@@ -445,7 +467,7 @@ int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_
   }
   return tc_attn_by_rows_run(q, q_stride_token, q_stride_head, Q, heads, dk, hist_k, hist_v, wk, bias_k, wv, bias_v,
                              weight_order == NKV_WEIGHTS_KERNEL_ORDER, rope, camera_k, camera_v, scale, out, lse,
-                             status_word, splits == 0 ? 16 : splits, workspace, static_cast<cudaStream_t>(stream));
+                             status_word, splits, workspace, static_cast<cudaStream_t>(stream));
 }
 
 int nkv_attn_codec_split(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
@@ -483,7 +505,7 @@ int nkv_attention_lse(const void* q, const void* k, const void* v, int dtype,
 
 size_t nkv_attention_lse_workspace_bytes(int Q, int heads, int d, int N) {
   if (d != 64 && d != 128) return 0;
-  return tc_attn_rows_workspace_bytes(Q, heads, d, N, 16, false) + 256;
+  return tc_attn_rows_workspace_bytes(Q, heads, d, N, 0, false) + 256;
 }
 
 int nkv_attention_lse_bf16(const void* q, const void* k, const void* v, int64_t q_stride_token,
@@ -497,7 +519,7 @@ int nkv_attention_lse_bf16(const void* q, const void* k, const void* v, int64_t 
   NKV_REQUIRE(workspace == nullptr || workspace_bytes >= nkv_attention_lse_workspace_bytes(Q, heads, d, N),
               NKV_ERR_INVALID, "attention_lse_bf16: workspace of %zu bytes is too small", workspace_bytes);
   return tc_attention_rows(q, k, v, q_stride_token, q_stride_head, kv_stride_token, kv_stride_head, Q, N, heads, d,
-                           scale, out, lse, status_word, 16, workspace, static_cast<cudaStream_t>(stream));
+                           scale, out, lse, status_word, 0, workspace, static_cast<cudaStream_t>(stream));
 }
 
 int nkv_lse_merge(const void* const* outs, const float* const* lses, int parts, int64_t rows,

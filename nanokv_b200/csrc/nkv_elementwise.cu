@@ -1095,6 +1095,17 @@ int head_linear(const void* x, int dtype, int64_t stride_row, int64_t stride_hea
   return NKV_OK;
 }
 
+__global__ void segment_append_kernel(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int row) {
+  seg_start[index + 1] = stop;
+  seg_center_row[index] = row;
+}
+
+int segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int row, cudaStream_t stream) {
+  segment_append_kernel<<<1, 1, 0, stream>>>(seg_start, seg_center_row, index, stop, row);
+  NKV_LAUNCH_CHECK("segment_append_kernel");
+  return NKV_OK;
+}
+
 size_t history_moments_workspace_bytes(int tokens, int rank) {
   const size_t slabs = (static_cast<size_t>(tokens > 0 ? tokens : 0) + MOMENT_SLAB - 1) / MOMENT_SLAB;
   return slabs * static_cast<size_t>(rank) * sizeof(float);

@@ -140,7 +140,7 @@ __device__ __forceinline__ float4 tile_sum(const float* sm, int row, int c) {
 }
 
 // ---------------------------------------------------------------- assignment
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)
 assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c_dtype, bool c_vec, int S, int J, int C,
               void* ids, int id_bytes, int32_t* labels32) {
   extern __shared__ float sm[];
@@ -198,7 +198,7 @@ assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c
 
 // ---------------------------------------------------------------- projection
 template <bool BF16>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)
 project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, bool c_vec, const void* ids, int id_bytes,
                const float* mean, const void* encoder, bool e_vec, int S, int J, int r, void* coeff) {
   extern __shared__ float sm[];
@@ -238,7 +238,7 @@ project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, 
 // -------------------------------------------------------------------- decode
 // decoder rows, bias and centre columns of `J` columns; out has rows of out_stride elements
 template <bool BF16>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)
 decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* decoder, bool d_vec,
                    const float* mean, int J, void* out, int out_dtype, long long out_stride) {
   extern __shared__ float sm[];

@@ -313,26 +313,43 @@ int launch_attn(const AttnArgs& a, cudaStream_t stream) {
 // -------------------------------------------------------------------- k-means
 __global__ void gather_init_kernel(const void* x, int x_dtype, int J, const int32_t* init_rows,
                                    float* centers) {
-  int c = blockIdx.x;
-  size_t src = static_cast<size_t>(init_rows[c]) * J;
-  for (int j = threadIdx.x; j < J; j += blockDim.x)
-    centers[static_cast<size_t>(c) * J + j] = load_float(x, x_dtype, src + j);
+  const int c = blockIdx.x, j = blockIdx.y * blockDim.x + threadIdx.x;
+  if (j < J) centers[static_cast<size_t>(c) * J + j] = load_float(x, x_dtype, static_cast<size_t>(init_rows[c]) * J + j);
 }
 
-// columns j, j + 1 (COLS 2) or j (COLS 1) of a row, as floats
-template <int COLS>
-__device__ __forceinline__ float2 load_columns(const void* base, int dtype, size_t i) {
-  if (COLS == 1) return make_float2(load_float(base, dtype, i), 0.f);
-  if (dtype == NKV_F32) return __ldg(reinterpret_cast<const float2*>(static_cast<const float*>(base) + i));
-  const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(base) + i));
-  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-}
+// Columns of a row as a thread of the update holds them in flight: a bf16 pair, an fp32 pair, or one
+// column of either type.
+struct PairBf16 {
+  static constexpr int COLS = 2;
+  uint32_t w;
+  __device__ __forceinline__ void load(const void* base, int, size_t i) {
+    w = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(base) + i));
+  }
+  __device__ __forceinline__ float2 value() const {
+    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+  }
+};
+struct PairF32 {
+  static constexpr int COLS = 2;
+  float2 v;
+  __device__ __forceinline__ void load(const void* base, int, size_t i) {
+    v = __ldg(reinterpret_cast<const float2*>(static_cast<const float*>(base) + i));
+  }
+  __device__ __forceinline__ float2 value() const { return v; }
+};
+struct Single {
+  static constexpr int COLS = 1;
+  float v;
+  __device__ __forceinline__ void load(const void* base, int dtype, size_t i) { v = load_float(base, dtype, i); }
+  __device__ __forceinline__ float2 value() const { return make_float2(v, 0.f); }
+};
 
 // centre c, columns j ..: sum of member rows in token order / member count;
 // an empty cluster keeps its centre.
 constexpr int UPDATE_LABELS = 32;                       // labels a thread looks at per round
 constexpr int UPDATE_SPAN = 256 * UPDATE_LABELS;        // tokens per round
-template <int COLS>
+constexpr int UPDATE_FLIGHT = 32;                       // row loads in flight per thread
+template <class Columns>
 __global__ void __launch_bounds__(256)
 kmeans_update_kernel(const void* x, int x_dtype, int S, int J, const int32_t* labels,
                      float* centers) {
@@ -340,12 +357,13 @@ kmeans_update_kernel(const void* x, int x_dtype, int S, int J, const int32_t* la
   // fp32 addition per row, the order a sequential scatter-add takes) so that the result does not
   // depend on the launch shape.  Labels are taken 8,192 at a time: every thread looks at 32 of them, a
   // block-wide exclusive scan turns the match counts into positions, and the matching tokens land in
-  // shared memory in order; the columns are then summed over that short list only.  Bound: the latency
-  // of the list's row loads, eight of which are in flight (two columns each: a block covers 512 columns
-  // and the grid is one wave).  4,680 x 5,120, 64 centres: 68 us (cold) / 50 us (rows in L2); with
-  // 2,048 labels a round, one column per thread and four loads in flight 97 / 73.
+  // shared memory in order; the columns are then summed over that short list only.  Bound: the chain of
+  // row loads of the largest cluster -- start rows drawn from one true cluster leave others to be shared,
+  // so a cluster can hold several times the mean -- hence 32 loads in flight, two columns each.
+  // 4,680 x 5,120, 64 centres, us per call with 4 / 8 / 32 loads in flight: 97 / 68 / 41.
   __shared__ uint16_t list[UPDATE_SPAN];
   __shared__ int warp_total[8];
+  constexpr int COLS = Columns::COLS;
   const int c = blockIdx.x, j = (blockIdx.y * 256 + threadIdx.x) * COLS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool vector = (reinterpret_cast<uintptr_t>(labels) & 15) == 0;
@@ -386,21 +404,18 @@ kmeans_update_kernel(const void* x, int x_dtype, int S, int J, const int32_t* la
     __syncthreads();
     count += total;
     if (j < J) {
-      int i = 0;
-      for (; i + 8 <= total; i += 8) {
-        float2 v[8];
+      for (int i = 0; i < total; i += UPDATE_FLIGHT) {
+        Columns v[UPDATE_FLIGHT];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = load_columns<COLS>(x, x_dtype, static_cast<size_t>(s0 + list[i + k]) * J + j);
+        for (int k = 0; k < UPDATE_FLIGHT; ++k)
+          if (i + k < total) v[k].load(x, x_dtype, static_cast<size_t>(s0 + list[i + k]) * J + j);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          sum.x = __fadd_rn(sum.x, v[k].x);
-          sum.y = __fadd_rn(sum.y, v[k].y);
-        }
-      }
-      for (; i < total; ++i) {
-        const float2 v = load_columns<COLS>(x, x_dtype, static_cast<size_t>(s0 + list[i]) * J + j);
-        sum.x = __fadd_rn(sum.x, v.x);
-        sum.y = __fadd_rn(sum.y, v.y);
+        for (int k = 0; k < UPDATE_FLIGHT; ++k)
+          if (i + k < total) {
+            const float2 pair = v[k].value();
+            sum.x = __fadd_rn(sum.x, pair.x);
+            sum.y = __fadd_rn(sum.y, pair.y);
+          }
       }
     }
   }
@@ -567,7 +582,7 @@ int rope_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head,
 
 int kmeans_gather_init(const void* x, int x_dtype, int J, int C, const int32_t* init_rows,
                        float* centers, cudaStream_t stream) {
-  gather_init_kernel<<<C, 256, 0, stream>>>(x, x_dtype, J, init_rows, centers);
+  gather_init_kernel<<<dim3(C, ceil_div(J, 256)), 256, 0, stream>>>(x, x_dtype, J, init_rows, centers);
   NKV_LAUNCH_CHECK("gather_init_kernel");
   return NKV_OK;
 }
@@ -576,8 +591,10 @@ int kmeans_update(const void* x, int x_dtype, int S, int J, int C, const int32_t
                   float* centers, cudaStream_t stream) {
   // two columns per thread: rows start 4 (bf16) or 8 (fp32) byte aligned and have an even length
   const bool pairs = J % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & (x_dtype == NKV_F32 ? 7 : 3)) == 0;
-  if (pairs) kmeans_update_kernel<2><<<dim3(C, ceil_div(J, 512)), 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
-  else kmeans_update_kernel<1><<<dim3(C, ceil_div(J, 256)), 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
+  const dim3 grid(C, ceil_div(J, pairs ? 512 : 256));
+  if (!pairs) kmeans_update_kernel<Single><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
+  else if (x_dtype == NKV_F32) kmeans_update_kernel<PairF32><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
+  else kmeans_update_kernel<PairBf16><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
   NKV_LAUNCH_CHECK("kmeans_update_kernel");
   return NKV_OK;
 }

@@ -109,6 +109,10 @@ struct Params {
   uint16_t* ring_k;  // [groups * ring * 128][D]
   uint16_t* ring_v;
   int32_t* flags;
+  // K / V rows: whole rounds of units, then the tail_units left over, cut into tail_blocks runs of tiles whose fp32 partials are merged by merge_tail_kernel
+  int tail_units, tail_blocks;
+  float* tail_out;   // [2 * tail_blocks][NQ * QT][D]
+  float* tail_lse;   // [2 * tail_blocks][NQ * QT]
   long long* prof;   // development builds: cycle buckets of group 0's first consumer and first producer
 };
 
@@ -137,6 +141,49 @@ __device__ __forceinline__ Unit row_unit_of(const Params& p, int u) {
   r.nt = min(p.tiles_per_split, p.tiles - r.tile0);
   return r;
 }
+
+// The units of one consumer in order; every role of the thread block walks the same list.  slot >= 0: a
+// run of tiles inside a unit of the tail, whose partial result goes to that slot.
+// (A thread block of the whole-unit rounds is not in step with its neighbours in the tail, where units are
+// few and their rows shared by several blocks.)
+template <bool RING>
+struct Walk {
+  int u;           // next whole unit
+  int w, w_end;    // tail: tiles of the left-over units, in order
+  int slot;
+  __device__ __forceinline__ Walk(const Params& p, int g) {
+    u = g;
+    slot = -1;
+    w = w_end = 0;
+    if (!RING && g < p.tail_blocks) {
+      const long long total = static_cast<long long>(p.tail_units) * p.tiles;
+      w = static_cast<int>(total * g / p.tail_blocks);
+      w_end = static_cast<int>(total * (g + 1) / p.tail_blocks);
+    }
+  }
+  __device__ __forceinline__ bool next(const Params& p, Unit& un) {
+    if (RING) {
+      if (u >= p.units) return false;
+      un = unit_of(p, u);
+      u += p.groups;
+      return true;
+    }
+    if (u < p.units - p.tail_units) {
+      un = row_unit_of(p, u);
+      u += gridDim.x;
+      return true;
+    }
+    if (w >= w_end) return false;
+    const int index = w / p.tiles, first = w - index * p.tiles;
+    un = row_unit_of(p, p.units - p.tail_units + index);
+    un.tile0 = first;
+    un.nt = min(p.tiles - first, w_end - w);
+    // a block holds at most one run that starts inside a unit and one that starts with it
+    slot = un.nt == p.tiles ? -1 : 2 * static_cast<int>(blockIdx.x) + (first == 0 ? 1 : 0);
+    w += un.nt;
+    return true;
+  }
+};
 
 // ---- bounded waits ------------------------------------------------------------------------------
 struct Ctx {
@@ -360,8 +407,9 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
       const int PK = p.prod_k, PV = p.prod - p.prod_k;
       Laps laps;
       laps.start(p.prof, p.prof != nullptr && g == 0 && c == 0);
-      for (int u = g; u < p.units && ok; u += p.groups) {
-        const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
+      Walk<RING> walk(p, g);
+      Unit un;
+      while (ok && walk.next(p, un)) {
         int q0;
         const int nq = queries_of(un, q0);
         if (nq > 0) {
@@ -499,8 +547,9 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
     int ctile[NQ] = {0, 0}, cunit[NQ] = {0, 0};   // tiles / units each query tile's chain has done
     Laps laps;
     laps.start(p.prof + 8, p.prof != nullptr && g == 0 && c == 0 && leader);
-    for (int u = g; u < p.units && ok; u += p.groups) {
-      const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
+    Walk<RING> walk(p, g);
+    Unit un;
+    while (ok && walk.next(p, un)) {
       int q0;
       const int nq = queries_of(un, q0);
       if (nq == 0) continue;
@@ -517,13 +566,21 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
       for (int t = 0; t < un.nt && ok; ++t) {
         const int cur = cseq + t, stage = cur % KVS, phase = (cur / KVS) & 1;
         const int nstage = (cur + 1) % KVS;
+        laps.lap(7);
+        // 64-wide heads: the stages (there long before the weights) are waited for while there is nothing
+        // to issue, not between the MMAs, which are half as long there: 1.80 -> 1.67 us per tile pair.
+        // For 128-wide heads it is the other way round: 1.79 -> 1.83.
+        constexpr bool STAGES_FIRST = D == 64;
+        if (STAGES_FIRST) {
+          ok = mwait_all(&bars[V_FULL + stage], phase, ctx, 212);
+          if (ok && t + 1 < un.nt) ok = mwait_all(&bars[K_FULL + nstage], ((cur + 1) / KVS) & 1, ctx, 216);
+        }
+        laps.lap(2);
         for (int i = 0; i < nq && ok; ++i) {
           const int ci = ctile[i] + t;
-          laps.lap(7);
-          ok = mwait_all(&bars[P_READY + i], ci & 1, ctx, 210 + i);
+          ok = ok && mwait_all(&bars[P_READY + i], ci & 1, ctx, 210 + i);
           laps.lap(i);
-          if (ok && i == 0) ok = mwait_all(&bars[V_FULL + stage], phase, ctx, 212);
-          laps.lap(2);
+          if (!STAGES_FIRST && ok && i == 0) ok = mwait_all(&bars[V_FULL + stage], phase, ctx, 212);
           // the first PV of a unit overwrites O: the previous unit's rows must have been read out
           if (ok && t == 0 && cunit[i] > 0) ok = mwait_all(&bars[O_FREE + i], (cunit[i] - 1) & 1, ctx, 214 + i);
           if (!ok) break;
@@ -538,7 +595,7 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
           if (t + 1 < un.nt) {
             // S of the next tile overwrites P of this one.  It is issued right behind the PV that
             // reads P: the tensor core executes the MMAs of one issuing thread in order
-            if (i == 0) ok = mwait_all(&bars[K_FULL + nstage], ((cur + 1) / KVS) & 1, ctx, 216);
+            if (!STAGES_FIRST && i == 0) ok = mwait_all(&bars[K_FULL + nstage], ((cur + 1) / KVS) & 1, ctx, 216);
             if (!ok) break;
             laps.lap(4);
             issue_s(i, nstage);
@@ -562,11 +619,18 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
     const uint32_t lane_sel = static_cast<uint32_t>(32 * (warp & 3)) << 16;
     bool ok = true;
     int ci = 0;
-    int u = g;
+    Walk<RING> walk(p, g);
+    Unit un;
     Laps laps;
     laps.start(p.prof + 16, p.prof != nullptr && g == 0 && c == 0 && tid == 0);
-    for (; u < p.units && ok; u += p.groups) {
-      const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
+    // where the rows of the unit at hand go: results (one row per query and head), or a slot of the tail
+    auto lse_of = [&](int q0) {
+      return walk.slot >= 0 ? p.tail_lse + static_cast<size_t>(walk.slot) * (NQ * QT) + wg * QT + row
+                            : p.lse + static_cast<size_t>(un.z) * p.Q * p.out_heads +
+                                  static_cast<size_t>(q0 + wg * QT + row) * p.out_heads + un.head;
+    };
+    bool more = true;
+    while (ok && (more = walk.next(p, un))) {
       int q0;
       const int nq = queries_of(un, q0);
       if (wg >= nq) continue;
@@ -737,28 +801,40 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
       l_run *= HALF_STEP_INV;    // the weights were summed with the half-step factor on them
       const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
       const uint32_t o_addr = tmem_base + lane_sel + 256 + wg * 128;
-      const size_t split_rows = static_cast<size_t>(un.z) * p.Q * p.out_heads;
-      uint16_t* dst = p.out + (split_rows + static_cast<size_t>(qrow) * p.out_heads + un.head) * D;
+      if (!RING && walk.slot >= 0) {
+        float* dst = p.tail_out + (static_cast<size_t>(walk.slot) * (NQ * QT) + wg * QT + row) * D;
 #pragma unroll 1
-      for (int cc = 0; cc < D / 32; ++cc) {
-        float v[32];
-        tmem_ld32(o_addr + cc * 32, v);
-        if (qrow < p.Q) {
+        for (int cc = 0; cc < D / 32; ++cc) {
+          float v[32];
+          tmem_ld32(o_addr + cc * 32, v);
+          if (qrow < p.Q) {
 #pragma unroll
-          for (int j4 = 0; j4 < 4; ++j4) {
-            uint4 w;
-            w.x = pack_bf16x2(v[j4 * 8 + 0] * inv, v[j4 * 8 + 1] * inv);
-            w.y = pack_bf16x2(v[j4 * 8 + 2] * inv, v[j4 * 8 + 3] * inv);
-            w.z = pack_bf16x2(v[j4 * 8 + 4] * inv, v[j4 * 8 + 5] * inv);
-            w.w = pack_bf16x2(v[j4 * 8 + 6] * inv, v[j4 * 8 + 7] * inv);
-            *reinterpret_cast<uint4*>(dst + cc * 32 + j4 * 8) = w;
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<float4*>(dst + cc * 32 + j) = make_float4(v[j] * inv, v[j + 1] * inv, v[j + 2] * inv, v[j + 3] * inv);
+          }
+        }
+      } else {
+        uint16_t* dst = p.out + (static_cast<size_t>(un.z) * p.Q * p.out_heads + static_cast<size_t>(qrow) * p.out_heads + un.head) * D;
+#pragma unroll 1
+        for (int cc = 0; cc < D / 32; ++cc) {
+          float v[32];
+          tmem_ld32(o_addr + cc * 32, v);
+          if (qrow < p.Q) {
+#pragma unroll
+            for (int j4 = 0; j4 < 4; ++j4) {
+              uint4 w;
+              w.x = pack_bf16x2(v[j4 * 8 + 0] * inv, v[j4 * 8 + 1] * inv);
+              w.y = pack_bf16x2(v[j4 * 8 + 2] * inv, v[j4 * 8 + 3] * inv);
+              w.z = pack_bf16x2(v[j4 * 8 + 4] * inv, v[j4 * 8 + 5] * inv);
+              w.w = pack_bf16x2(v[j4 * 8 + 6] * inv, v[j4 * 8 + 7] * inv);
+              *reinterpret_cast<uint4*>(dst + cc * 32 + j4 * 8) = w;
+            }
           }
         }
       }
       if (qrow < p.Q) {
-        p.lse[split_rows + static_cast<size_t>(qrow) * p.out_heads + un.head] =
-            saturated ? __int_as_float(0x7fc00000)
-                      : (l_run > 0.f ? (m_used + log2f(l_run)) * 0.6931471805599453f : -INFINITY);
+        *lse_of(q0) = saturated ? __int_as_float(0x7fc00000)
+                                : (l_run > 0.f ? (m_used + log2f(l_run)) * 0.6931471805599453f : -INFINITY);
         if (saturated && p.status) atomicCAS(p.status, 0, STATUS_SCORE_RANGE);
       }
       tc_fence_before();
@@ -769,14 +845,11 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
     // a launch that gave up must not hand back rows that look like results: the unit it stopped in
     // and every later one get NaN in their LSE
     if (!ok) {
-      for (; u < p.units; u += p.groups) {
-        const Unit un = RING ? unit_of(p, u) : row_unit_of(p, u);
+      while (more) {
         int q0;
         const int nq = queries_of(un, q0);
-        const int qrow = q0 + wg * QT + row;
-        if (wg < nq && qrow < p.Q)
-          p.lse[static_cast<size_t>(un.z) * p.Q * p.out_heads + static_cast<size_t>(qrow) * p.out_heads + un.head] =
-              __int_as_float(0x7fc00000);
+        if (wg < nq && q0 + wg * QT + row < p.Q) *lse_of(q0) = __int_as_float(0x7fc00000);
+        more = walk.next(p, un);
       }
     }
   }
@@ -1442,6 +1515,52 @@ attn_codec_kernel(const __grid_constant__ CUtensorMap map_q,
   if (tid == 0 && *abort_flag && p.status) atomicCAS(p.status, 0, *abort_flag);
 }
 
+// Merges the partials of the tail's cut units.  Block (b, part): the unit that the boundary between the runs
+// of blocks b and b + 1 cuts, if no earlier boundary lies in it; thread = (row, 8 columns).
+template <int D>
+__global__ void __launch_bounds__(256)
+merge_tail_kernel(Params p) {
+  const long long total = static_cast<long long>(p.tail_units) * p.tiles;
+  auto start_of = [&](int b) { return total * b / p.tail_blocks; };
+  const int b0 = blockIdx.x;
+  const long long cut = start_of(b0 + 1);
+  const int index = static_cast<int>(cut / p.tiles);
+  const long long unit_begin = static_cast<long long>(index) * p.tiles, unit_end = unit_begin + p.tiles;
+  if (cut == unit_begin || start_of(b0) > unit_begin) return;   // not inside a unit / not the unit's first cut
+  const Unit un = row_unit_of(p, p.units - p.tail_units + index);
+  constexpr int PER_ROW = D / 8, ROWS = 256 / PER_ROW;
+  const int row = blockIdx.y * ROWS + threadIdx.x / PER_ROW, col = (threadIdx.x % PER_ROW) * 8;
+  const int q = un.qc * (NQ * QT) + row;
+  if (q >= p.Q) return;
+  // first run: starts with the unit (slot 2 b + 1); the others start inside it (slot 2 b)
+  float top = -INFINITY;
+  bool nan = false;
+  for (int b = b0; b < p.tail_blocks && start_of(b) < unit_end; ++b) {
+    const float l = p.tail_lse[static_cast<size_t>(2 * b + (b == b0 ? 1 : 0)) * (NQ * QT) + row];
+    nan = nan || l != l;
+    top = fmaxf(top, l);
+  }
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, weight = 0.f;
+  for (int b = b0; b < p.tail_blocks && start_of(b) < unit_end; ++b) {
+    if (start_of(b) == start_of(b + 1)) continue;
+    const size_t at = static_cast<size_t>(2 * b + (b == b0 ? 1 : 0)) * (NQ * QT) + row;
+    const float w = expf(p.tail_lse[at] - top);
+    const float4 lo = *reinterpret_cast<const float4*>(p.tail_out + at * D + col);
+    const float4 hi = *reinterpret_cast<const float4*>(p.tail_out + at * D + col + 4);
+    weight += w;
+    acc[0] = fmaf(w, lo.x, acc[0]); acc[1] = fmaf(w, lo.y, acc[1]);
+    acc[2] = fmaf(w, lo.z, acc[2]); acc[3] = fmaf(w, lo.w, acc[3]);
+    acc[4] = fmaf(w, hi.x, acc[4]); acc[5] = fmaf(w, hi.y, acc[5]);
+    acc[6] = fmaf(w, hi.z, acc[6]); acc[7] = fmaf(w, hi.w, acc[7]);
+  }
+  const float inv = 1.0f / weight;
+  const size_t out_row = static_cast<size_t>(q) * p.out_heads + un.head;
+  *reinterpret_cast<uint4*>(p.out + out_row * D + col) =
+      make_uint4(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv),
+                 pack_bf16x2(acc[4] * inv, acc[5] * inv), pack_bf16x2(acc[6] * inv, acc[7] * inv));
+  if (col == 0) p.lse[out_row] = nan ? __int_as_float(0x7fc00000) : top + logf(weight);
+}
+
 __global__ void fill_empty_kernel(uint16_t* out, float* lse, size_t rows, int d) {
   size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < rows * d) out[i] = 0;
@@ -1832,39 +1951,58 @@ struct RowPlan { int batches, heads, splits, tiles_per_split; size_t kv_bytes; }
 constexpr size_t ROW_BATCH_BYTES = 512u << 20;
 constexpr int MAX_SPLITS = 16;
 
-// Splits (at most `max_splits`) and head batches with the least estimated time.  A unit of 256 queries
-// costs about 2 us per tile of 128 tokens plus a fill of about three tiles; the partials of a split
-// history are written and read once at HBM rate and cost one more launch.
+// A tail shorter than this many tiles per block is not worth another block's start.
+constexpr int MIN_TAIL_TILES = 2;
+
+struct Tail { int blocks, units; bool whole; };   // whole: some units run whole, on all blocks
+
+// Thread blocks of a launch of `units` whole units of `tiles` tiles, the rounds of whole units each takes,
+// and the units left over, which are cut evenly: 760 units on 148 SMs are five rounds and 20 units of
+// 183 tiles in runs of 25, where a sixth round of whole units would leave 128 SMs idle.
+Tail plan_tail(int sms, long long units, int tiles) {
+  Tail t{};
+  t.units = static_cast<int>(units % sms);
+  t.whole = units >= sms;
+  const long long work = static_cast<long long>(t.units) * tiles;
+  t.blocks = static_cast<int>(work / MIN_TAIL_TILES > sms ? sms : work / MIN_TAIL_TILES);
+  // about four tiles' time to fill, and to merge in a launch of its own
+  if (t.units > 0 && (t.blocks <= t.units || work / t.blocks + 4 >= tiles || work > 0x7fffffff)) {
+    t.units = t.blocks = 0;
+    t.whole = true;
+  }
+  return t;
+}
+
+// Head batches, and history splits where the caller bounds them (`max_splits` > 0: at most that many, with
+// the least estimated time: a unit of 256 queries costs about 1.8 us per tile of 128 tokens plus a fill of
+// about three tiles, the partials are written and read once and cost one more launch).  Otherwise the
+// history is not split but for the tail of a launch.
 RowPlan plan_rows(int sms, int Q, int heads, int d, int tokens, int max_splits, bool rebuild) {
   const int tiles = ceil_div(tokens, TOK), qblocks = ceil_div(Q, NQ * QT);
   const size_t head_bytes = rebuild ? static_cast<size_t>(tokens) * d * 4 : 0;
-  int first = 1;
-  while (first < heads && head_bytes * ceil_div(heads, first) > ROW_BATCH_BYTES) ++first;
+  int batches = 1;
+  while (batches < heads && head_bytes * ceil_div(heads, batches) > ROW_BATCH_BYTES) ++batches;
+  const int hb = ceil_div(heads, batches);
+  RowPlan best{ceil_div(heads, hb), hb, 1, tiles, head_bytes * hb};
   if (max_splits > MAX_SPLITS) max_splits = MAX_SPLITS;
   if (max_splits > tiles) max_splits = tiles;
-  RowPlan best{};
   double best_cost = -1;
-  for (int nb = first; nb <= heads && nb < first + 4; ++nb) {
-    const int hb = ceil_div(heads, nb);
-    if (nb > first && (!rebuild || ceil_div(heads, hb) != nb)) continue;
-    for (int s = 1; s <= max_splits; ++s) {
-      const int tps = ceil_div(tiles, s);
-      if (ceil_div(tiles, tps) != s) continue;
-      const int tail = heads - hb * (ceil_div(heads, hb) - 1);
-      double cost = 0;
-      for (int b = 0; b < ceil_div(heads, hb); ++b) {
-        const long long units = static_cast<long long>(b + 1 < ceil_div(heads, hb) ? hb : tail) * qblocks * s;
-        cost += static_cast<double>((units + sms - 1) / sms) * (tps + 3) * 2.0 + 3.0;
-      }
-      if (s > 1) cost += 3.0 + static_cast<double>(s) * Q * heads * (d * 4 + 8) / 5e6;
-      if (best_cost < 0 || cost < best_cost) {
-        best_cost = cost;
-        best = RowPlan{ceil_div(heads, hb), hb, s, tps, head_bytes * hb};
-      }
+  for (int s = 1; s <= max_splits; ++s) {
+    const int tps = ceil_div(tiles, s);
+    if (ceil_div(tiles, tps) != s) continue;
+    const long long units = static_cast<long long>(hb) * qblocks * s;
+    double cost = static_cast<double>((units + sms - 1) / sms) * (tps + 3) * 1.8 * best.batches;
+    if (s > 1) cost += 3.0 + static_cast<double>(s) * Q * heads * (d * 4 + 8) / 5e6;
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best.splits = s;
+      best.tiles_per_split = tps;
     }
   }
   return best;
 }
+
+size_t tail_bytes(int sms, int d) { return static_cast<size_t>(2 * sms) * (NQ * QT) * (d + 1) * 4; }
 
 size_t partial_bytes(int splits, int Q, int heads, int d) {
   const size_t bytes = splits > 1 ? static_cast<size_t>(splits) * Q * heads * (static_cast<size_t>(d) * 2 + 4) : 0;
@@ -1878,6 +2016,10 @@ int launch_rows(const CUtensorMap maps[3], const Params& p, cudaStream_t stream)
   NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   kernel<<<p.groups, THREADS, smem, stream>>>(maps[0], maps[1], maps[2], p);
   NKV_LAUNCH_CHECK("attn_rows_kernel");
+  if (p.tail_blocks > 1) {
+    merge_tail_kernel<D><<<dim3(p.tail_blocks - 1, NQ * QT * D / 2048), 256, 0, stream>>>(p);
+    NKV_LAUNCH_CHECK("merge_tail_kernel");
+  }
   return NKV_OK;
 }
 
@@ -1892,8 +2034,8 @@ int row_map(CUtensorMap* map, const void* base, int d, int heads, int tokens, in
 // one launch over `heads` heads; out / lse are the batch's first head inside rows of out_heads heads
 int attend_rows(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int out_heads,
                 int d, const void* k, const void* v, int64_t kv_stride_token, int64_t kv_stride_head, int N,
-                float scale, int splits, int tiles_per_split, uint16_t* out, float* lse, int32_t* status,
-                cudaStream_t stream) {
+                float scale, int splits, int tiles_per_split, float* tail, uint16_t* out, float* lse,
+                int32_t* status, cudaStream_t stream) {
   CUtensorMap maps[3];
   int rc = row_map(&maps[0], q, d, heads, Q, q_stride_token, q_stride_head);
   if (rc == NKV_OK) rc = row_map(&maps[1], k, d, heads, N, kv_stride_token, kv_stride_head);
@@ -1907,8 +2049,16 @@ int attend_rows(const void* q, int64_t q_stride_token, int64_t q_stride_head, in
   p.qchunks = ceil_div(Q, NQ * QT);
   p.units = p.qchunks * heads * splits;
   const int sms = sm_count();
-  p.groups = p.units < sms ? p.units : sms;
   p.cons = 1;
+  p.groups = p.units < sms ? p.units : sms;
+  if (tail != nullptr && splits == 1) {
+    const Tail t = plan_tail(sms, p.units, p.tiles);
+    p.tail_units = t.units;
+    p.tail_blocks = t.blocks;
+    if (!t.whole) p.groups = t.blocks;
+    p.tail_out = tail;
+    p.tail_lse = tail + static_cast<size_t>(2 * sms) * (NQ * QT) * d;
+  }
   p.scale_log2 = scale * 1.4426950408889634f;
   p.wait_budget = 1ll << 31;
   p.out = out; p.lse = lse; p.status = status;
@@ -1942,7 +2092,7 @@ bool tc_attn_by_rows(int dk, int dv, int rank, int group) {
 size_t tc_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens, int max_splits, bool rebuild) {
   if (Q <= 0 || heads <= 0 || tokens <= 0) return 0;
   const RowPlan plan = plan_rows(sm_count(), Q, heads, d, tokens, max_splits, rebuild);
-  return partial_bytes(plan.splits, Q, heads, d) + plan.kv_bytes + 256;
+  return partial_bytes(plan.splits, Q, heads, d) + tail_bytes(sm_count(), d) + plan.kv_bytes + 512;
 }
 
 // The read in two kernels per batch of heads: rows rebuilt into `workspace`, then attended.  Against the
@@ -1979,7 +2129,8 @@ int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_
   uint16_t* part_out = plan.splits > 1 ? reinterpret_cast<uint16_t*>(space) : static_cast<uint16_t*>(out);
   float* part_lse = plan.splits > 1
       ? reinterpret_cast<float*>(part_out + static_cast<size_t>(plan.splits) * Q * heads * d) : lse;
-  uint16_t* rows_k = reinterpret_cast<uint16_t*>(space + partial_bytes(plan.splits, Q, heads, d));
+  uint8_t* tail = space + partial_bytes(plan.splits, Q, heads, d);
+  uint16_t* rows_k = reinterpret_cast<uint16_t*>(tail + (tail_bytes(sms, d) + 255) / 256 * 256);
   uint16_t* rows_v = rows_k + static_cast<size_t>(plan.heads) * N * d;
   for (int h0 = 0; h0 < heads; h0 += plan.heads) {
     const int hb = heads - h0 < plan.heads ? heads - h0 : plan.heads;
@@ -2009,7 +2160,8 @@ int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_
     if (rc == NKV_OK)
       rc = attend_rows(static_cast<const uint16_t*>(q) + h0 * q_stride_head, q_stride_token, q_stride_head, Q, hb,
                        heads, d, rows_k, rows_v, d, head_stride, N, scale, plan.splits, plan.tiles_per_split,
-                       part_out + col0, part_lse + h0, status, stream);
+                       max_splits > 0 ? nullptr : reinterpret_cast<float*>(tail), part_out + col0, part_lse + h0,
+                       status, stream);
     if (rc != NKV_OK) return rc;
   }
   return plan.splits > 1 ? merge_splits(part_out, part_lse, plan.splits, Q, heads, d, out, lse, stream) : NKV_OK;
@@ -2027,13 +2179,15 @@ int tc_attention_rows(const void* q, const void* k, const void* v, int64_t q_str
                       void* out, float* lse, int32_t* status, int max_splits, void* workspace, cudaStream_t stream) {
   if (Q == 0 || heads == 0) return NKV_OK;
   const RowPlan plan = plan_rows(sm_count(), Q, heads, d, N, workspace != nullptr ? max_splits : 1, false);
+  const bool cut_tail = workspace != nullptr && max_splits == 0;
   uint8_t* space = static_cast<uint8_t*>(workspace);
   space += (256 - (reinterpret_cast<uintptr_t>(space) & 255)) & 255;
   uint16_t* part_out = plan.splits > 1 ? reinterpret_cast<uint16_t*>(space) : static_cast<uint16_t*>(out);
   float* part_lse = plan.splits > 1
       ? reinterpret_cast<float*>(part_out + static_cast<size_t>(plan.splits) * Q * heads * d) : lse;
+  float* tail = cut_tail ? reinterpret_cast<float*>(space + partial_bytes(plan.splits, Q, heads, d)) : nullptr;
   int rc = attend_rows(q, q_stride_token, q_stride_head, Q, heads, heads, d, k, v, kv_stride_token, kv_stride_head, N,
-                       scale, plan.splits, plan.tiles_per_split, part_out, part_lse, status, stream);
+                       scale, plan.splits, plan.tiles_per_split, tail, part_out, part_lse, status, stream);
   if (rc == NKV_OK && plan.splits > 1) rc = merge_splits(part_out, part_lse, plan.splits, Q, heads, d, out, lse, stream);
   return rc;
 }

@@ -186,20 +186,22 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
     if (lane == 0) {
       prefetch_tensormap(&map_0);
       if (p.tensors > 1) prefetch_tensormap(&map_1);
+      const uint32_t full_even = map_to_cta(smem_u32(&bars[FULL]), 0);
       bool ok = true;
-      int it = 0;
+      int s = 0, phase = 0;
+      bool wrapped = false;        // the ring has been filled once: stages must be handed back first
       for (int w = w_begin; w < w_end && ok;) {
         const Run r = run_at(p, w, w_end);
         const CUtensorMap* map = r.tensor ? &map_1 : &map_0;
         for (int k = 0; k < r.count && ok; ++k) {
           const int y = (r.nt0 + k) * TN + static_cast<int>(cta) * TM;
-          for (int c = 0; c < nchunks; ++c, ++it) {
-            const int s = it % nst, u = it / nst;
-            if (u >= 1) ok = mbar_wait(&bars[FREE + s], (u - 1) & 1, abort_flag, 700 + s);
+          for (int c = 0; c < nchunks; ++c) {
+            if (wrapped) ok = mbar_wait(&bars[FREE + s], phase ^ 1, abort_flag, 700 + s);
             if (!ok) break;
             // both halves land on the even CTA's barrier, whose MMA warp reads them
             if (cta == 0) mbar_arrive_expect_tx(&bars[FULL + s], 2 * CHUNK_BYTES);
-            tma_load_2d_pair(b_tiles + s * CHUNK_BYTES, map, c * 64, y, map_to_cta(smem_u32(&bars[FULL + s]), 0));
+            tma_load_2d_pair(b_tiles + s * CHUNK_BYTES, map, c * 64, y, full_even + s * 8);
+            if (++s == nst) { s = 0; phase ^= 1; wrapped = true; }
           }
         }
         w += r.count;
@@ -217,17 +219,16 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       const uint32_t idesc = make_idesc_bf16(2 * TM, TN);
       const uint32_t a_base = smem_u32(a_tiles), b_base = smem_u32(b_tiles);
       bool ok = true;
-      int it = 0, tile = 0, seg = 0;
+      int s = 0, phase = 0, tile = 0, seg = 0;   // the ring's place is counted: no division per stage
       for (int w = w_begin; w < w_end && ok; ++seg) {
         const Run r = run_at(p, w, w_end);
         for (int k = 0; k < r.count && ok; ++k, ++tile) {
           const int b = tile & 1, use = tile >> 1;
           if (use >= 1) ok = wait_all(&bars[ACC_FREE + b], (use - 1) & 1, abort_flag, 710 + b);
           const uint32_t acc = tmem_base + b * TN;
-          for (int c = 0; c < nchunks && ok; ++c, ++it) {
-            const int s = it % nst, u = it / nst;
+          for (int c = 0; c < nchunks && ok; ++c) {
             if (k == 0 && c % A_GROUP == 0) ok = wait_all_cluster(&bars[A_FULL + c / A_GROUP], seg & 1, abort_flag, 720 + c);
-            ok = ok && wait_all(&bars[FULL + s], u & 1, abort_flag, 730 + s);
+            ok = ok && wait_all(&bars[FULL + s], phase, abort_flag, 730 + s);
             if (!ok) break;
             tc_fence_after();
             const uint64_t a_desc = make_smem_desc_sw128(a_base + c * CHUNK_BYTES);
@@ -240,6 +241,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
               mma_commit_pair(&bars[FREE + s]);
             }
             __syncwarp();
+            if (++s == nst) { s = 0; phase ^= 1; }
           }
           if (ok && leader) mma_commit_pair(&bars[ACC_FULL + b]);
           __syncwarp();

@@ -39,13 +39,13 @@ constexpr int COMPUTE_THREADS = 256;
 constexpr int THREADS = COMPUTE_THREADS + 64;
 constexpr int A_BYTES = 128 * 128;
 
-constexpr int MAX_STAGES = 4;
-enum Bar { TMA_FULL = 0, A_FULL = 4, STAGE_FREE = 8, ACC_DONE = 12, SIDE_READY = 13, CAND_READY = 14,
-           PEER_READY = 15, NUM_BARS = 16 };
+constexpr int MAX_STAGES = 8;
+enum Bar { TMA_FULL = 0, A_FULL = 8, STAGE_FREE = 16, ACC_DONE = 24, SIDE_READY = 25, CAND_READY = 26,
+           PEER_READY = 27, NUM_BARS = 28 };
 enum Mode { PROJECT = 0, ASSIGN_IDS = 1, PROJECT_QUANT = 2 };
 constexpr int META_HEAD = 256;      // barriers, TMEM slot, abort flag
 constexpr int WARPS = COMPUTE_THREADS / 32;
-constexpr int MAX_CENTER_ROWS = 512 / 32;   // centre rows whose norms one thread group accumulates
+constexpr int MAX_PARTS = 8;        // thread blocks of one token tile that form a cluster
 
 struct Params {
   int S, J, NB, NACC, n_total;      // n_total = r (project) or C (assign)
@@ -77,6 +77,15 @@ __device__ __forceinline__ float sumsq8(uint4 w) {
   return s;
 }
 
+// place in the operand ring, kept by counting: a division by the run-time depth per stage, in the one thread
+// that issues the copies and the one that issues the MMAs, is a good part of a stage's time
+struct Ring {
+  int stage = 0, phase = 0;
+  __device__ __forceinline__ void advance(int depth) {
+    if (++stage == depth) { stage = 0; phase ^= 1; }
+  }
+};
+
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -96,7 +105,8 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   float* xn_part = reinterpret_cast<float*>(meta + META_HEAD);    // [256]
   float* cand_d = xn_part + 256;                                  // [128]
   int* cand_i = reinterpret_cast<int*>(cand_d + 128);             // [128]
-  float* cn_part = reinterpret_cast<float*>(cand_i + 128);        // [C]
+  float* cn_part = reinterpret_cast<float*>(cand_i + 128);        // [C][2]
+  float* peer_max = cn_part;                                      // project + quantise: [MAX_PARTS][128]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int part = blockIdx.x % p.parts;                // place in the tile's cluster
@@ -119,7 +129,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     mbar_init(&bars[ACC_DONE], 1);
     mbar_init(&bars[SIDE_READY], COMPUTE_THREADS);
     mbar_init(&bars[CAND_READY], 128);
-    mbar_init(&bars[PEER_READY], 128);
+    mbar_init(&bars[PEER_READY], 128 * (p.column_parts > 1 ? p.column_parts - 1 : 1));
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
@@ -129,26 +139,31 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // the column-half CTAs of one token tile write into each other's shared memory: nobody may do so
-  // before the peer's barriers exist
+  // the column parts of one token tile write into each other's shared memory: nobody may do so before
+  // the peers' barriers exist
   const bool split = p.ksplit > 1;
-  const bool paired = QUANT && !split && p.column_parts == 2;
-  if (paired) cluster_sync_all();
+  const bool joined = QUANT && !split && p.column_parts > 1;
+  if (joined) cluster_sync_all();
   bool ok = true;
-  float xs[4] = {0.f, 0.f, 0.f, 0.f};        // assign: squared-norm partials of this thread's rows
-  float cs[ASSIGN ? MAX_CENTER_ROWS : 1];
+  // assign: squared-norm partials of half a token row, and of half-rows tid + 256 i of the centres
+  float xs = 0.f, cs[4] = {0.f, 0.f, 0.f, 0.f};
 
   if (warp == 8) {
     if (lane == 0) {
       prefetch_tensormap(&map_b);
       if (ASSIGN) prefetch_tensormap(&map_a);
-      for (int i = 0; i < nchunks && ok; ++i) {
-        const int s = i % nst, u = i / nst, c = c_first + i;
-        if (u >= 1) ok = mbar_wait(&bars[STAGE_FREE + s], (u - 1) & 1, abort_flag, 400 + s);
+      int a_col = ASSIGN ? c_first % p.a_chunks : 0;
+      Ring at;
+      for (int i = 0; i < nchunks && ok; ++i, at.advance(nst)) {
+        const int s = at.stage, c = c_first + i;
+        if (i >= nst) ok = mbar_wait(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 400 + s);
         if (!ok) break;
         uint8_t* stage = smem + s * stage_bytes;
         mbar_arrive_expect_tx(&bars[TMA_FULL + s], p.NACC * b_bytes + (ASSIGN ? A_BYTES : 0));
-        if (ASSIGN) tma_load_2d(stage, &map_a, (c % p.a_chunks) * 64, m0, &bars[TMA_FULL + s]);
+        if (ASSIGN) {
+          tma_load_2d(stage, &map_a, a_col * 64, m0, &bars[TMA_FULL + s]);
+          if (++a_col == p.a_chunks) a_col = 0;
+        }
         for (int a = 0; a < p.NACC; ++a)
           tma_load_2d(stage + A_BYTES + a * b_bytes, &map_b, c * 64, n_base + a * p.NB,
                       &bars[TMA_FULL + s]);
@@ -164,10 +179,11 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     const bool leader = elect_one();
     const uint32_t idesc = make_idesc_bf16(128, p.NB);
     const uint32_t smem_base = smem_u32(smem);
-    for (int c = 0; c < nchunks && ok; ++c) {
-      const int s = c % nst, u = c / nst;
-      ok = mbar_wait(&bars[TMA_FULL + s], u & 1, abort_flag, 410 + s);
-      if (ok && !ASSIGN) ok = mbar_wait(&bars[A_FULL + s], u & 1, abort_flag, 412 + s);
+    Ring at;
+    for (int c = 0; c < nchunks && ok; ++c, at.advance(nst)) {
+      const int s = at.stage;
+      ok = mbar_wait(&bars[TMA_FULL + s], at.phase, abort_flag, 410 + s);
+      if (ok && !ASSIGN) ok = mbar_wait(&bars[A_FULL + s], at.phase, abort_flag, 412 + s);
       if (!ok) break;
       tc_fence_after();
       const uint32_t stage = smem_base + s * stage_bytes;
@@ -195,41 +211,38 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     if (ASSIGN) {
       // ---- squared norms from the resident tiles
       const int C = p.n_total;
-#pragma unroll
-      for (int i = 0; i < MAX_CENTER_ROWS; ++i) cs[i] = 0.f;
-      for (int i = 0; i < nchunks && ok; ++i) {
-        const int s = i % nst, u = i / nst;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars[TMA_FULL + s], u & 1, abort_flag, 420 + s) ? 1 : 0) != 0;
+      Ring at;
+      for (int i = 0; i < nchunks && ok; ++i, at.advance(nst)) {
+        const int s = at.stage;
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars[TMA_FULL + s], at.phase, abort_flag, 420 + s) ? 1 : 0) != 0;
         if (!ok) break;
-        const uint8_t* stage = smem + s * stage_bytes + r0 * 128 + piece * 16;
+        const uint8_t* stage = smem + s * stage_bytes;
         if (c_first + i < p.a_chunks) {
+          const uint4* src = reinterpret_cast<const uint4*>(stage + (tid >> 1) * 128 + (tid & 1) * 64);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) xs[j] += sumsq8(*reinterpret_cast<const uint4*>(stage + j * 32 * 128));
+          for (int j = 0; j < 4; ++j) xs += sumsq8(src[j]);
         }
         if (p.cnorm == nullptr) {
 #pragma unroll
-          for (int j = 0; j < MAX_CENTER_ROWS; ++j)
-            if (r0 + 32 * j < C) cs[j] += sumsq8(*reinterpret_cast<const uint4*>(stage + A_BYTES + j * 32 * 128));
+          for (int k = 0; k < 4; ++k) {
+            const int item = tid + k * COMPUTE_THREADS;
+            if (item < 2 * C) {
+              const uint4* src = reinterpret_cast<const uint4*>(stage + A_BYTES + (item >> 1) * 128 + (item & 1) * 64);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) cs[k] += sumsq8(src[j]);
+            }
+          }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[STAGE_FREE + s]);
       }
-      // the eight threads of a row hold an eighth of its sum each
-#pragma unroll
-      for (int off = 1; off < 8; off <<= 1) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) xs[j] += __shfl_xor_sync(0xffffffffu, xs[j], off);
-#pragma unroll
-        for (int j = 0; j < MAX_CENTER_ROWS; ++j) cs[j] += __shfl_xor_sync(0xffffffffu, cs[j], off);
-      }
       if (ok && split) ok = mbar_wait(&bars[ACC_DONE], 0, abort_flag, 431);
       if (ok && !split) {
-        if (piece == 0) {
+        xn_part[tid] = xs;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) xn_part[r0 + 32 * j] = xs[j];
-#pragma unroll
-          for (int j = 0; j < MAX_CENTER_ROWS; ++j)
-            if (r0 + 32 * j < C) cn_part[r0 + 32 * j] = cs[j];
+        for (int k = 0; k < 4; ++k) {
+          const int item = tid + k * COMPUTE_THREADS;
+          if (item < 2 * C) cn_part[item] = cs[k];
         }
         mbar_arrive(&bars[SIDE_READY]);
         ok = mbar_wait(&bars[SIDE_READY], 0, abort_flag, 430) &&
@@ -237,7 +250,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       }
       if (ok && !split) {
         tc_fence_after();
-        const float xn = xn_part[row];
+        const float xn = xn_part[2 * row] + xn_part[2 * row + 1];
         const int chunks = (C + 31) / 32, middle = (chunks + 1) / 2;
         const int first = wg == 0 ? 0 : middle, last = wg == 0 ? middle : chunks;
         float best = INFINITY;
@@ -251,7 +264,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           for (int j = 0; j < 32; ++j) {
             const int cidx = col + j;
             if (cidx < C) {
-              const float cn = p.cnorm != nullptr ? __ldg(p.cnorm + cidx) : cn_part[cidx];
+              const float cn = p.cnorm != nullptr ? __ldg(p.cnorm + cidx) : cn_part[2 * cidx] + cn_part[2 * cidx + 1];
               const float dist = __fsub_rn(__fadd_rn(xn, cn), __fmul_rn(2.0f, v[j]));
               if (dist < best) { best = dist; best_i = cidx; }
             }
@@ -303,8 +316,9 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
             cq[buf][j] = __ldg(reinterpret_cast<const uint4*>(crow[j] + j0));
           }
       };
+      Ring at;
       auto step = [&](int buf, int i) {
-        const int s = i % nst, u = i / nst;
+        const int s = at.stage;
         const float mv[8] = {mq[buf][0].x, mq[buf][0].y, mq[buf][0].z, mq[buf][0].w,
                              mq[buf][1].x, mq[buf][1].y, mq[buf][1].z, mq[buf][1].w};
         uint4 out[4];
@@ -325,8 +339,9 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           }
         }
         fetch(buf, i + 2);
-        if (u >= 1) ok = __all_sync(0xffffffffu, mbar_wait(&bars[STAGE_FREE + s], (u - 1) & 1, abort_flag, 440 + s) ? 1 : 0) != 0;
+        if (i >= nst) ok = __all_sync(0xffffffffu, mbar_wait(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 440 + s) ? 1 : 0) != 0;
         if (!ok) return;
+        at.advance(nst);
         uint8_t* stage = smem + s * stage_bytes + r0 * 128 + ((piece ^ (r0 & 7)) << 4);
 #pragma unroll
         for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(stage + j * 32 * 128) = out[j];
@@ -363,14 +378,18 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         ok = mbar_wait(&bars[SIDE_READY], 0, abort_flag, 451);
         if (ok) {
           amax = fmaxf(xn_part[row], xn_part[128 + row]);
-          if (paired) {
+          if (joined) {
             if (wg == 0) {
-              const uint32_t peer = cluster_ctarank() ^ 1u;
-              st_cluster_b32(map_to_cta(smem_u32(&cand_d[row]), peer), __float_as_uint(amax));
-              mbar_arrive_cluster(map_to_cta(smem_u32(&bars[PEER_READY]), peer));
+              for (int peer = 0; peer < p.column_parts; ++peer) {
+                if (peer == half) continue;
+                st_cluster_b32(map_to_cta(smem_u32(&peer_max[half * 128 + row]), peer), __float_as_uint(amax));
+                mbar_arrive_cluster(map_to_cta(smem_u32(&bars[PEER_READY]), peer));
+              }
             }
             ok = mbar_wait_cluster(&bars[PEER_READY], 0, abort_flag, 452);
-            if (ok) amax = fmaxf(amax, cand_d[row]);
+            if (ok)
+              for (int peer = 0; peer < p.column_parts; ++peer)
+                if (peer != half) amax = fmaxf(amax, peer_max[peer * 128 + row]);
           }
         }
         if (ok) {
@@ -455,21 +474,18 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                                                             __float_as_uint(v[j + 2]), __float_as_uint(v[j + 3])));
         }
       }
-      if (ASSIGN && (tid & 7) == 0) {
+      if (ASSIGN) {
+        xs += __shfl_xor_sync(0xffffffffu, xs, 1);     // two threads share a row
+        const int r = tid >> 1;
+        if ((tid & 1) == 0 && r < p.rows)
+          st_cluster_b32(map_to_cta(smem_u32(xn_slots + part * own + r % own), r / own), __float_as_uint(xs));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = (tid >> 3) + 32 * j;
-          if (r < p.rows)
-            st_cluster_b32(map_to_cta(smem_u32(xn_slots + part * own + r % own), r / own), __float_as_uint(xs[j]));
-        }
-        if (p.cnorm == nullptr) {
-#pragma unroll
-          for (int j = 0; j < MAX_CENTER_ROWS; ++j) {
-            const int c = (tid >> 3) + 32 * j;
-            if (c < p.n_total)
-              for (int peer = 0; peer < p.parts; ++peer)
-                st_cluster_b32(map_to_cta(smem_u32(cn_slots + part * p.n_total + c), peer), __float_as_uint(cs[j]));
-          }
+        for (int k = 0; k < 4; ++k) {
+          cs[k] += __shfl_xor_sync(0xffffffffu, cs[k], 1);
+          const int c = r + 128 * k;
+          if (p.cnorm == nullptr && (tid & 1) == 0 && c < p.n_total)
+            for (int peer = 0; peer < p.parts; ++peer)
+              st_cluster_b32(map_to_cta(smem_u32(cn_slots + part * p.n_total + c), peer), __float_as_uint(cs[k]));
         }
       }
     }
@@ -557,8 +573,8 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   tc_fence_before();
   __syncthreads();
   if (warp == 9) tmem_dealloc(tmem_base, 512);
-  // neither CTA of a pair leaves while the other may still write into its shared memory
-  if (paired) cluster_sync_all();
+  // no CTA of a tile leaves while another may still write into its shared memory
+  if (joined) cluster_sync_all();
 }
 
 // split n_total columns into grid.y CTAs x NACC accumulators x NB columns
@@ -572,7 +588,11 @@ bool plan_columns(int n_total, int* gy, int* nacc, int* nb) {
   return false;
 }
 
-size_t meta_bytes(int n_total) { return META_HEAD + 4 * (256 + 128 + 128) + 4 * static_cast<size_t>(n_total); }
+// n_norms: centres whose squared norms are kept (assign); 512 floats of them, or the parts' row maxima
+size_t meta_bytes(int n_norms) {
+  const size_t tail = 8 * static_cast<size_t>(n_norms);
+  return META_HEAD + 4 * (256 + 128 + 128) + (tail > 4 * MAX_PARTS * 128 ? tail : 4 * MAX_PARTS * 128);
+}
 
 size_t ring_bytes(int nacc, int nb, int stages) { return stages * static_cast<size_t>(A_BYTES + nacc * nb * 128); }
 
@@ -610,9 +630,12 @@ size_t place_smem(Params& p, int n_norms) {
 // operand prefetch alone); assignment of 1,560 x 3,072 to 256 centres 60 -> 30, of 880 x 3,072 to 64 fp32
 // centres 70 -> 16.  Only the order in which K is summed depends on the cut, and the projection
 // and its quantising form take the same one.
+// `ordered`: K is not cut, every sum runs in the order of K whatever the call's length, so that rows encode
+// to the same bytes in a chunk of any size (the online encoders, whose payloads are stored and compared, and
+// the projection entry points); such calls take more column parts instead.
 struct Split { int rows, column_parts, ksplit; };
 
-Split plan_split(int S, int chunks, int columns, int column_parts, int n_norms, bool residual) {
+Split plan_split(int S, int chunks, int columns, int column_parts, int n_norms, bool residual, bool ordered) {
   const int sms = sm_count();
   Split best{pick_rows(S, column_parts), column_parts, 1};
   auto stage_cost = [&](int rows, int cols) {
@@ -623,15 +646,18 @@ Split plan_split(int S, int chunks, int columns, int column_parts, int n_norms, 
   double best_cost = rounds(static_cast<long long>(ceil_div(S, best.rows)) * column_parts, sms) *
                      (chunks * stage_cost(best.rows, columns / column_parts) + 3000);
   for (int rows = 64; rows <= TM; rows *= 2)
-    for (int h = column_parts; h <= 2 * column_parts && h <= 4; h *= 2)
-      for (int k = 2; k * h <= 8; k *= 2) {
+    for (int h = column_parts; h <= MAX_PARTS; ++h)
+      for (int k = 1; k * h <= MAX_PARTS; k *= 2) {
         const int cols = columns / h;
-        if (columns % h || cols > 512 || chunks < 2 * k) continue;
-        if (h > column_parts && (!residual || cols % 64)) continue;
-        if (exchange_bytes(rows, cols, k * h, n_norms) + meta_bytes(n_norms) + 2048 > SMEM_LIMIT) continue;
-        const int room = k * h == 8 ? sms - 20 : (k * h == 4 ? sms - 4 : sms);
-        const double cost = rounds(static_cast<long long>(ceil_div(S, rows)) * k * h, room) *
-                            (ceil_div(chunks, k) * stage_cost(rows, cols) + rows * cols * 4.0 / 15 + 5000);
+        if (k > 1 && (ordered || chunks < 2 * k || h > 2 * column_parts || h > 4 || (h & (h - 1)) != 0)) continue;
+        if (columns % h || cols > 512 || cols % (cols > 256 ? 64 : 32)) continue;
+        if (h > column_parts && !residual) continue;
+        const int parts = k * h;
+        if (k > 1 && exchange_bytes(rows, cols, parts, n_norms) + meta_bytes(n_norms) + 2048 > SMEM_LIMIT) continue;
+        const int room = parts > 4 ? sms - 20 : (parts > 2 ? sms - 4 : sms);
+        const double cost = rounds(static_cast<long long>(ceil_div(S, rows)) * parts, room) *
+                            (ceil_div(chunks, k) * stage_cost(rows, cols) +
+                             (k > 1 ? rows * cols * 4.0 / 15 + 5000 : 3000 + 300 * h));
         if (cost < best_cost) {
           best_cost = cost;
           best = Split{rows, h, k};
@@ -661,7 +687,7 @@ int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, Params& p, i
   config.stream = stream;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = p.ksplit > 1 || (MODE == PROJECT_QUANT && p.column_parts == 2) ? p.parts : 1;
+  attr.val.clusterDim.x = p.ksplit > 1 || MODE == PROJECT_QUANT ? p.parts : 1;
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
   config.attrs = &attr;
@@ -714,13 +740,13 @@ bool tc_assign_supported(int J, int C) {
 
 int tc_project(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
                const float* mean, const void* encoder_bf16, int S, int J, int r, void* coeff,
-               cudaStream_t stream) {
+               bool ordered, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
   Params p{};
   int gy;
   NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB), NKV_ERR_UNSUPPORTED,
               "projection rank %d cannot be tiled", r);
-  const Split cut = plan_split(S, J / 64, r, gy, 0, true);
+  const Split cut = plan_split(S, J / 64, r, gy, 0, true, ordered);
   p.rows = cut.rows; p.column_parts = cut.column_parts; p.ksplit = cut.ksplit;
   set_columns(p, r / p.column_parts);
   NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
@@ -749,13 +775,14 @@ bool tc_project_quant_supported(int J, int r, int group) {
 
 int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
                      const float* mean, const void* encoder_bf16, int S, int J, int r, float eps,
-                     int quant_mode, int scale_dtype, uint8_t* codes, void* scales, cudaStream_t stream) {
+                     int quant_mode, int scale_dtype, uint8_t* codes, void* scales, bool ordered,
+                     cudaStream_t stream) {
   if (S == 0) return NKV_OK;
   Params p{};
   int gy;
   NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB) && gy <= 2, NKV_ERR_UNSUPPORTED,
               "fused projection: rank %d cannot be tiled over at most two column parts", r);
-  const Split cut = plan_split(S, J / 64, r, gy, 0, true);
+  const Split cut = plan_split(S, J / 64, r, gy, 0, true, ordered);
   p.rows = cut.rows; p.column_parts = cut.column_parts; p.ksplit = cut.ksplit;
   set_columns(p, r / p.column_parts);
   NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
@@ -784,7 +811,7 @@ int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C,
   if (S == 0) return NKV_OK;
   Params p{};
   p.S = S; p.J = J; p.n_total = C;
-  const Split cut = plan_split(S, J / 64, C, 1, C, false);
+  const Split cut = plan_split(S, J / 64, C, 1, C, false, false);
   p.rows = cut.rows; p.column_parts = 1; p.ksplit = cut.ksplit;
   set_columns(p, C);
   p.ids_out = ids; p.id_bytes = id_bytes;
@@ -858,7 +885,7 @@ int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, in
   NKV_LAUNCH_CHECK("split_centers_kernel");
   Params p{};
   p.S = S; p.J = J; p.n_total = C;
-  const Split cut = plan_split(S, 3 * (J / 64), C, 1, C, false);
+  const Split cut = plan_split(S, 3 * (J / 64), C, 1, C, false, true);
   p.rows = cut.rows; p.column_parts = 1; p.ksplit = cut.ksplit;
   set_columns(p, C);
   p.labels_out = labels; p.id_bytes = 1;

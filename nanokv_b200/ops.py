@@ -172,6 +172,12 @@ class HistoryView:
             self.ids.element_size(), self.centers.shape[0], self.centers.shape[1])
 
 
+def segment_append(seg_start: torch.Tensor, seg_center_row: torch.Tensor, index: int, stop: int, row: int) -> None:
+    """seg_start[index + 1] = stop, seg_center_row[index] = row on the current stream (nkv_segment_append)."""
+    _lib.check(_lib.library().nkv_segment_append(_ptr(seg_start), _ptr(seg_center_row), index, stop, row,
+                                                 _stream(seg_start.device)))
+
+
 def gather_view(view: HistoryView, index: torch.Tensor) -> HistoryView:
     """The history restricted to the tokens listed in ``index`` (increasing, device i64): codes,
     scales and ids are gathered, every segment keeps its centre rows and shrinks to its listed

@@ -62,3 +62,16 @@ def test_update_sums_members_in_token_order(S, J, dtype):
         for row in member:
             total += row
         assert torch.equal(centers[c].cpu(), (total / member.shape[0]).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("J,r", [(1536, 192), (3072, 384), (5120, 640)])
+def test_rows_encode_to_the_same_bytes_in_a_chunk_of_any_size(J, r):
+    """The projection entry points never cut K: a row's coefficients do not depend on its neighbours."""
+    rows, centers, pick, encoder, mean = _data(3000, J, 16, r, seed=2)
+    ids = pick.to(torch.uint8)
+    whole = ops.project(rows, centers, ids, mean, encoder)
+    codes, scales = ops.project_quant(rows, centers, ids, mean, encoder)
+    for a, b in ((0, 64), (64, 500), (500, 1700), (1700, 3000)):
+        assert torch.equal(ops.project(rows[a:b], centers, ids[a:b], mean, encoder), whole[a:b])
+        part = ops.project_quant(rows[a:b], centers, ids[a:b], mean, encoder)
+        assert torch.equal(part[0], codes[a:b]) and torch.equal(part[1].view(torch.int16), scales[a:b].view(torch.int16))

@@ -60,7 +60,7 @@ def compare(heads, D, rank, tokens, queries, *, rope=False, selected=False, came
                                          torch.randint(0, 4, (heads, D // 8), generator=gen, device="cuda",
                                                        dtype=torch.int32), -(-tokens // 5))
     got, got_lse = _read("nkv_attn_codec_rows", q, hk, hv, *weights, prepared=prepared, splits=splits, **extra)
-    want, want_lse = _read("nkv_attn_codec_pos", q, hk, hv, *weights, prepared=prepared, splits=splits, **extra)
+    want, want_lse = _read("nkv_attn_codec_pos", q, hk, hv, *weights, prepared=prepared, splits=max(splits, 1), **extra)
     # Both attend the same bf16 rows with bf16 weights (2^-9 each) and round O, and a split's partial O, to
     # bf16; a rebuilt value may sit one bf16 step apart where fp32 sums meet a rounding boundary.
     assert float((got - want).norm() / want.norm()) < 2.0 ** -7
@@ -70,7 +70,7 @@ def compare(heads, D, rank, tokens, queries, *, rope=False, selected=False, came
 
 @pytest.mark.parametrize("tokens,queries", [(1, 1), (127, 128), (129, 129), (1000, 300), (4100, 513)])
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("splits", [1, 5])
+@pytest.mark.parametrize("splits", [0, 1, 5])
 def test_sizes(tokens, queries, D, splits):
     compare(3, D, 192, tokens, queries, splits=splits, segments=min(2, tokens))
 
@@ -89,9 +89,16 @@ def test_positional_forms(D, position):
     compare(5, D, 128, 900, 260, **position)
 
 
+@pytest.mark.parametrize("heads,D,tokens,queries", [(12, 128, 2048, 256), (3, 128, 5000, 700), (8, 64, 3000, 5000),
+                                                    (40, 128, 1500, 1100), (1, 128, 20000, 64), (149, 64, 640, 100)])
+def test_left_over_units_are_cut(heads, D, tokens, queries):
+    """Units that do not fill a round of the SMs: none whole, one cut many ways, whole rounds and a tail."""
+    compare(heads, D, 64, tokens, queries, splits=0)
+
+
 def test_head_batches():
     """Rows of all heads exceed the scratch bound: the read goes through the heads in batches."""
-    compare(40, 128, 64, 30000, 64, rope=True, splits=3)
+    compare(40, 128, 64, 30000, 64, rope=True, splits=0)
 
 
 def test_reads_on_two_streams_do_not_share_state():
