@@ -32,6 +32,7 @@
 // TMEM columns, consumer: [0,128) S / P of query tile 0, [128,256) of tile 1, [256,384) O
 // tile 0, [384,512) O tile 1.  Producer: [0,D) the tile accumulator, [256,512) four latent
 // staging slots of 64 columns (a pair of 64-column latent chunks each).
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 
@@ -1532,21 +1533,25 @@ merge_tail_kernel(Params p) {
   const int row = blockIdx.y * ROWS + threadIdx.x / PER_ROW, col = (threadIdx.x % PER_ROW) * 8;
   const int q = un.qc * (NQ * QT) + row;
   if (q >= p.Q) return;
-  // first run: starts with the unit (slot 2 b + 1); the others start inside it (slot 2 b)
+  // runs b0 .. b_end: the first starts with the unit (slot 2 b + 1), the others inside it (slot 2 b)
+  const int b_end = static_cast<int>((unit_end * p.tail_blocks + total - 1) / total);
+  const float* lses = p.tail_lse + row;
+  auto slot_of = [&](int b) { return static_cast<size_t>(2 * b + (b == b0 ? 1 : 0)) * (NQ * QT); };
   float top = -INFINITY;
   bool nan = false;
-  for (int b = b0; b < p.tail_blocks && start_of(b) < unit_end; ++b) {
-    const float l = p.tail_lse[static_cast<size_t>(2 * b + (b == b0 ? 1 : 0)) * (NQ * QT) + row];
+#pragma unroll 4
+  for (int b = b0; b < b_end; ++b) {
+    const float l = lses[slot_of(b)];
     nan = nan || l != l;
     top = fmaxf(top, l);
   }
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, weight = 0.f;
-  for (int b = b0; b < p.tail_blocks && start_of(b) < unit_end; ++b) {
-    if (start_of(b) == start_of(b + 1)) continue;
-    const size_t at = static_cast<size_t>(2 * b + (b == b0 ? 1 : 0)) * (NQ * QT) + row;
-    const float w = expf(p.tail_lse[at] - top);
-    const float4 lo = *reinterpret_cast<const float4*>(p.tail_out + at * D + col);
-    const float4 hi = *reinterpret_cast<const float4*>(p.tail_out + at * D + col + 4);
+#pragma unroll 4
+  for (int b = b0; b < b_end; ++b) {
+    const size_t at = slot_of(b);
+    const float w = expf(lses[at] - top);
+    const float4 lo = *reinterpret_cast<const float4*>(p.tail_out + (at + row) * D + col);
+    const float4 hi = *reinterpret_cast<const float4*>(p.tail_out + (at + row) * D + col + 4);
     weight += w;
     acc[0] = fmaf(w, lo.x, acc[0]); acc[1] = fmaf(w, lo.y, acc[1]);
     acc[2] = fmaf(w, lo.z, acc[2]); acc[3] = fmaf(w, lo.w, acc[3]);
@@ -1951,9 +1956,6 @@ struct RowPlan { int batches, heads, splits, tiles_per_split; size_t kv_bytes; }
 constexpr size_t ROW_BATCH_BYTES = 512u << 20;
 constexpr int MAX_SPLITS = 16;
 
-// A tail shorter than this many tiles per block is not worth another block's start.
-constexpr int MIN_TAIL_TILES = 2;
-
 struct Tail { int blocks, units; bool whole; };   // whole: some units run whole, on all blocks
 
 // Thread blocks of a launch of `units` whole units of `tiles` tiles, the rounds of whole units each takes,
@@ -1964,9 +1966,17 @@ Tail plan_tail(int sms, long long units, int tiles) {
   t.units = static_cast<int>(units % sms);
   t.whole = units >= sms;
   const long long work = static_cast<long long>(t.units) * tiles;
-  t.blocks = static_cast<int>(work / MIN_TAIL_TILES > sms ? sms : work / MIN_TAIL_TILES);
-  // about four tiles' time to fill, and to merge in a launch of its own
-  if (t.units > 0 && (t.blocks <= t.units || work / t.blocks + 4 >= tiles || work > 0x7fffffff)) {
+  if (t.units == 0) return t;
+  // In tiles of time (1.8 us): a run costs its tiles and about three to fill -- twice where it crosses from
+  // one unit into the next -- and merging a launch, about two, and a 25th per run, whose 256 KB of partials
+  // are written and read.  Equal cuts of every unit never cross; one run for every SM may.
+  double best = tiles + 3;
+  for (int cuts = 2; cuts * t.units <= sms && cuts <= tiles; ++cuts) {
+    const double cost = (tiles + cuts - 1) / cuts + 3 + 2 + cuts * t.units / 25.0;
+    if (cost < best) { best = cost; t.blocks = cuts * t.units; }
+  }
+  if (work >= 4ll * sms && work / sms + 6 + 2 + sms / 25.0 < best) t.blocks = sms;
+  if (t.blocks == 0 || work > 0x7fffffff) {
     t.units = t.blocks = 0;
     t.whole = true;
   }
