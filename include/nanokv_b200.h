@@ -379,14 +379,18 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
 /*
  * The read of nkv_attn_codec_pos with K and V rows rebuilt in `workspace` a batch of heads at a time
  * (at most 512 MB of rows, at least one head) and then attended: two kernels per batch, same
- * arithmetic, and no state shared between launches.  It is the faster form wherever its workspace is
- * affordable; nkv_attn_codec_pos stays for callers that hand out no such memory and for ranks above
+ * arithmetic, and no state shared between launches.  It is the faster form nearly everywhere
+ * (nkv_attn_codec_rows_is_faster); nkv_attn_codec_pos stays for callers that hand out no such memory and for ranks above
  * 640.  `splits`: upper bound of the history splits, 0: the library's choice.
  * nkv_attn_codec_rows_workspace_bytes is 0 where this form does not apply (rank above 640 in bf16, head
  * widths other than 64 and 128); the fp32 form takes no positional restore and 16-byte aligned queries.
  */
 size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, int dv, int tokens,
                                            int rank, int group, int splits);
+/* 1 where this form applies and is the faster one, 0 where nkv_attn_codec_pos should run (short histories
+ * whose heads fill its groups of thread blocks in one round). */
+int nkv_attn_codec_rows_is_faster(int dtype, int Q, int heads, int dk, int dv, int tokens, int rank,
+                                  int group, int positional);
 int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
                         int Q, int heads, int dk, int dv,
                         const nkv_history* hist_k, const nkv_history* hist_v,

@@ -86,6 +86,7 @@ SIGNATURES = {
                                    c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_size_t,
                                    c_void_p]),
     "nkv_attn_codec_rows_workspace_bytes": (c_size_t, [c_int] * 9),
+    "nkv_attn_codec_rows_is_faster": (c_int, [c_int] * 9),
     "nkv_attn_codec_rows": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int, c_int, c_int, c_int,
                                     POINTER(History), POINTER(History), c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int, POINTER(Rope), POINTER(Camera), POINTER(Camera),

@@ -437,6 +437,13 @@ size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, 
   return tc_attn_rows_workspace_bytes(Q, heads, dk, tokens, splits, true) + 256;
 }
 
+int nkv_attn_codec_rows_is_faster(int dtype, int Q, int heads, int dk, int dv, int tokens, int rank, int group,
+                                  int positional) {
+  if (!reads_by_rows(dtype, dk, dv, rank, group)) return 0;
+  if (dtype == NKV_F32) return positional ? 0 : 1;
+  return tc_attn_fused_is_faster(Q, heads, dk, tokens, rank, positional != 0) ? 0 : 1;
+}
+
 int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
                         int Q, int heads, int dk, int dv, const nkv_history* hist_k,
                         const nkv_history* hist_v, const void* wk, const float* bias_k,

@@ -79,6 +79,7 @@ int tc_attn_codec(const void* q, int64_t q_stride_token, int64_t q_stride_head, 
                   const nkv_camera* cam_v = nullptr, bool prepared_weights = false);
 // the read in two kernels per batch of heads (rows rebuilt, then attended); nkv_tc_attn.cu
 bool tc_attn_by_rows(int dk, int dv, int rank, int group);
+bool tc_attn_fused_is_faster(int Q, int heads, int d, int tokens, int rank, bool positional);
 size_t tc_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens, int max_splits, bool rebuild);
 int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int d,
                         const nkv_history* hist_k, const nkv_history* hist_v, const void* wk, const float* bias_k,

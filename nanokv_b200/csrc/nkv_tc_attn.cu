@@ -29,6 +29,9 @@
 // drain and leave, and the wait-site code lands in the caller's status word.
 // No TMA load uses multicast; there are no clusters.
 //
+// attn_rows_kernel below is the consumer on its own, over K / V rows in memory: with decode_gemm_kernel it
+// is the read that most calls take (see tc_attn_by_rows_run and tc_attn_fused_is_faster).
+//
 // TMEM columns, consumer: [0,128) S / P of query tile 0, [128,256) of tile 1, [256,384) O
 // tile 0, [384,512) O tile 1.  Producer: [0,D) the tile accumulator, [256,512) four latent
 // staging slots of 64 columns (a pair of 64-column latent chunks each).
@@ -2097,6 +2100,25 @@ bool aligned16(const void* pointer) { return (reinterpret_cast<uintptr_t>(pointe
 // Whether a read can rebuild rows first; false: the fused kernel (ranks above 640, odd layouts).
 bool tc_attn_by_rows(int dk, int dv, int rank, int group) {
   return tc_attn_supported(dk, dv, rank) && rank <= 640 && (group == 32 || group % 64 == 0);
+}
+
+// Where the fused kernel is still the faster read: a short history whose heads fill one round of its groups
+// (or two exactly), so that a group rebuilds and attends its head without a launch in between.  us, by rows
+// / fused: 16 heads, rank 512, 1,024 queries: 500 tokens 39 / 38, 1,500 64 / 54, 2,500 80 / 71, 4,000
+// 96 / 97; 24 heads, rank 384, 512 queries: 1,000 tokens 48 / 46, 2,000 68 / 62, 3,000 77 / 77; 2,048
+// queries: 2,000 tokens 106 / 100.  Not with heads left over for a further round (24 heads, 1,024 queries,
+// 2,000 tokens: 73 / 99), few queries (16 heads, rank 512, 64 queries, 2,000 tokens: 52 / 60), small ranks
+// (12 heads, rank 192, 1,024 queries, 2,000 tokens: 58 / 74) or rotated keys (16 heads, rank 512, 1,024
+// queries, 2,500 tokens: 92 / 96).
+bool tc_attn_fused_is_faster(int Q, int heads, int d, int tokens, int rank, bool positional) {
+  if (positional || tokens > 2560 || !((rank >= 384 && Q > 256) || (rank >= 256 && Q > 768))) return false;
+  const int tiles = ceil_div(tokens, TOK);
+  if (tiles == 0 || heads == 0) return false;
+  const int sms = sm_count();
+  const Plan plan = make_plan(sms, Q, heads, tiles, rank, d, 1);
+  const int room = sms / (plan.cons + plan.prod);
+  const int units = plan.qchunks * heads;
+  return units <= room || units == 2 * room;
 }
 
 size_t tc_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens, int max_splits, bool rebuild) {

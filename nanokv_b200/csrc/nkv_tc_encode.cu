@@ -625,11 +625,12 @@ size_t place_smem(Params& p, int n_norms) {
 // 48 bytes per clock, at least 350 cycles of latency; exchanging partials costs 15 bytes per clock, the
 // SM-to-SM rate, plus the barriers.  Clusters of 8 fit 128 of the 148 SMs at a time, of 4 about 144.
 // Bound of the undivided form: 880 tokens x 3,072 columns x rank 384 kept 14 SMs busy for 48 stages of
-// operand latency.  Undivided -> cut, us per call: projection of 880 x 3,072 x 384 107 -> 20 (64 tokens, 2
-// column parts, 4 K parts), of 1,560 x 3,072 x 384 84 -> 23, of 4,680 x 5,120 x 640 128 -> 75 (not cut:
-// operand prefetch alone); assignment of 1,560 x 3,072 to 256 centres 60 -> 30, of 880 x 3,072 to 64 fp32
-// centres 70 -> 16.  Only the order in which K is summed depends on the cut, and the projection
-// and its quantising form take the same one.
+// operand latency (107 us).  us per call now: projection with K cut 880 x 3,072 x 384 18 (64 tokens, 2
+// column parts, 4 K parts), 1,560 x 3,072 x 384 23 (84 before); in order 880 x 3,072 x 384 39 (6 column
+// parts), 4,680 x 5,120 x 640 71 (128 before: operand prefetch alone); assignment of 1,560 x 3,072 to 256
+// centres 28 (60 before), to 64 fp32 centres in order 880 x 3,072 49 (70), 4,680 x 5,120 80 (116).  Only
+// the order in which K is summed depends on the cut, and the projection and its quantising form take the
+// same one.
 // `ordered`: K is not cut, every sum runs in the order of K whatever the call's length, so that rows encode
 // to the same bytes in a chunk of any size (the online encoders, whose payloads are stored and compared, and
 // the projection entry points); such calls take more column parts instead.

@@ -278,9 +278,12 @@ def attn_codec(q, view_k: HistoryView, view_v: HistoryView, wk, bias_k, wv, bias
     # not apply and the fused kernel (or the fp32 one) reads the history
     nbytes = lib.nkv_attn_codec_rows_workspace_bytes(dtype_code(q.dtype), Q, H, dk, dv, view_k.tokens, view_k.rank,
                                                      view_k.group, 0 if splits is None else splits)
-    if q.dtype == torch.float32 and (rope is not None or camera_k is not None or camera_v is not None
-                                     or q.data_ptr() % 16 or q.stride(0) % 4 or q.stride(1) % 4
+    positional = rope is not None or camera_k is not None or camera_v is not None
+    if q.dtype == torch.float32 and (positional or q.data_ptr() % 16 or q.stride(0) % 4 or q.stride(1) % 4
                                      or out.data_ptr() % 16):
+        nbytes = 0
+    if nbytes and not lib.nkv_attn_codec_rows_is_faster(dtype_code(q.dtype), Q, H, dk, dv, view_k.tokens, view_k.rank,
+                                                        view_k.group, int(positional)):
         nbytes = 0
     read = lib.nkv_attn_codec_rows if nbytes else lib.nkv_attn_codec_pos
     if nbytes:

@@ -133,3 +133,16 @@ def test_plain_rows_against_the_cuda_core_kernel(N, Q, H, D):
     # weights go to bf16 (2^-9) before the sum, results and split partials are rounded to bf16
     assert float((got.float() - want.float()).norm() / want.float().norm()) < 2.0 ** -7
     assert float((got_lse - want_lse).abs().max()) < 2.0 ** -9
+
+
+@pytest.mark.parametrize("heads,rank,queries,tokens,by_rows", [
+    (16, 512, 1024, 1500, 0), (16, 512, 1024, 2561, 1), (24, 384, 512, 1000, 0), (24, 384, 1024, 1000, 1),
+    (24, 384, 2048, 1000, 0), (16, 512, 256, 1000, 1), (12, 192, 1024, 1000, 1), (40, 640, 1024, 1000, 1)])
+def test_which_form_reads(heads, rank, queries, tokens, by_rows):
+    """The rule on 148 SMs, and the same result from either side of it through the public call."""
+    lib = _lib.library()
+    faster = lib.nkv_attn_codec_rows_is_faster(_lib.NKV_BF16, queries, heads, 128, 128, tokens, rank, rank, 0)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert faster == by_rows
+    assert lib.nkv_attn_codec_rows_is_faster(_lib.NKV_BF16, queries, heads, 128, 128, tokens, rank, rank, 1) == 1
+    compare(heads, 128, rank, tokens, queries, splits=0)
