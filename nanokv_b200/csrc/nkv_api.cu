@@ -176,25 +176,18 @@ int nkv_kmeans(const void* x, int x_dtype, int S, int J, int C, int iters,
   return kmeans_store(centers, labels, S, J, C, centers_bf16, ids, id_bytes, s);
 }
 
-static int project_rows(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
-                        int id_bytes, const float* mean, const void* encoder, int encoder_dtype, int S,
-                        int J, int r, void* coeff, bool ordered, void* stream) {
+int nkv_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
+                int id_bytes, const float* mean, const void* encoder, int encoder_dtype, int S,
+                int J, int r, void* coeff, void* stream) {
   NKV_REQUIRE(S >= 0 && J > 0 && r > 0, NKV_ERR_INVALID, "project: S=%d J=%d r=%d", S, J, r);
   NKV_REQUIRE(encoder_dtype == NKV_F32 || encoder_dtype == NKV_BF16, NKV_ERR_INVALID,
               "project: encoder dtype");
   auto s = static_cast<cudaStream_t>(stream);
   if (encoder_dtype == NKV_BF16 && x_dtype == NKV_BF16 && !simt_forced() &&
       tc_project_supported(J, r))
-    return tc_project(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, coeff, ordered, s);
+    return tc_project(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, coeff, s);
   return simt_project(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J,
                       r, coeff, s);
-}
-
-int nkv_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
-                int id_bytes, const float* mean, const void* encoder, int encoder_dtype, int S,
-                int J, int r, void* coeff, void* stream) {
-  return project_rows(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r, coeff, true,
-                      stream);
 }
 
 int nkv_quant_pack(const void* coeff, int coeff_dtype, int S, int r, int group, float eps,
@@ -213,10 +206,10 @@ int nkv_quant_pack(const void* coeff, int coeff_dtype, int S, int r, int group, 
                     static_cast<cudaStream_t>(stream));
 }
 
-static int project_quant_rows(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
+int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
                       const float* mean, const void* encoder, int encoder_dtype, int S, int J, int r,
                       int group, float eps, int quant_mode, int scale_dtype, uint8_t* codes,
-                      void* scales, void* workspace, size_t workspace_bytes, bool ordered, void* stream) {
+                      void* scales, void* workspace, size_t workspace_bytes, void* stream) {
   NKV_REQUIRE(S >= 0 && J > 0 && r > 0 && group > 0 && r % group == 0, NKV_ERR_INVALID,
               "project_quant: S=%d J=%d r=%d group=%d", S, J, r, group);
   NKV_REQUIRE(encoder_dtype == NKV_F32 || encoder_dtype == NKV_BF16, NKV_ERR_INVALID,
@@ -232,22 +225,14 @@ static int project_quant_rows(const void* x, int x_dtype, const void* centers_bf
   if (encoder_dtype == NKV_BF16 && x_dtype == NKV_BF16 && !simt_forced() &&
       tc_project_quant_supported(J, r, group) && (reinterpret_cast<uintptr_t>(codes) & 15) == 0)
     return tc_project_quant(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, eps, quant_mode,
-                            scale_dtype, codes, scales, ordered, static_cast<cudaStream_t>(stream));
+                            scale_dtype, codes, scales, static_cast<cudaStream_t>(stream));
   NKV_REQUIRE(workspace && workspace_bytes >= static_cast<size_t>(S) * r * dtype_bytes(encoder_dtype),
               NKV_ERR_INVALID, "project_quant: workspace of %zu bytes is too small", workspace_bytes);
-  int rc = project_rows(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r,
-                        workspace, ordered, stream);
+  int rc = nkv_project(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r,
+                       workspace, stream);
   if (rc != NKV_OK) return rc;
   return nkv_quant_pack(workspace, encoder_dtype, S, r, group, eps, quant_mode, scale_dtype, codes,
                         scales, stream);
-}
-
-int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
-                      const float* mean, const void* encoder, int encoder_dtype, int S, int J, int r,
-                      int group, float eps, int quant_mode, int scale_dtype, uint8_t* codes,
-                      void* scales, void* workspace, size_t workspace_bytes, void* stream) {
-  return project_quant_rows(x, x_dtype, centers_bf16, ids, id_bytes, mean, encoder, encoder_dtype, S, J, r, group, eps,
-                            quant_mode, scale_dtype, codes, scales, workspace, workspace_bytes, true, stream);
 }
 
 int nkv_encode_append(const void* x, int x_dtype, const void* centers_bf16, int C,
@@ -265,9 +250,9 @@ int nkv_encode_append(const void* x, int x_dtype, const void* centers_bf16, int 
   void* scales_at = static_cast<uint8_t*>(scales) + static_cast<size_t>(offset) * (r / group) * 2;
   int rc = nkv_assign(x, x_dtype, centers_bf16, NKV_BF16, S, J, C, ids_at, id_bytes, stream);
   if (rc != NKV_OK) return rc;
-  return project_quant_rows(x, x_dtype, centers_bf16, ids_at, id_bytes, mean, encoder, encoder_dtype, S,
-                            J, r, group, eps, quant_mode, scale_dtype, codes_at, scales_at, workspace,
-                            workspace_bytes, false, stream);
+  return nkv_project_quant(x, x_dtype, centers_bf16, ids_at, id_bytes, mean, encoder, encoder_dtype, S,
+                           J, r, group, eps, quant_mode, scale_dtype, codes_at, scales_at, workspace,
+                           workspace_bytes, stream);
 }
 
 int nkv_segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int center_row,

@@ -69,7 +69,7 @@ int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C,
               int id_bytes, cudaStream_t stream);
 int tc_project(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
                const float* mean, const void* encoder_bf16, int S, int J, int r, void* coeff,
-               bool ordered, cudaStream_t stream);
+               cudaStream_t stream);
 int tc_attn_codec(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q,
                   int heads, int dk, int dv, const nkv_history* hist_k,
                   const nkv_history* hist_v, const void* wk, const float* bias_k,
@@ -114,7 +114,7 @@ bool tc_project_supported(int J, int r);
 bool tc_project_quant_supported(int J, int r, int group);
 int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
                      const float* mean, const void* encoder_bf16, int S, int J, int r, float eps,
-                     int quant_mode, int scale_dtype, uint8_t* codes, void* scales, bool ordered, cudaStream_t stream);
+                     int quant_mode, int scale_dtype, uint8_t* codes, void* scales, cudaStream_t stream);
 bool tc_assign_supported(int J, int C);
 size_t tc_assign_f32_workspace_bytes(int J, int C);
 int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, int C, int32_t* labels,

@@ -16,10 +16,9 @@
 //            their place in the history: the bf16 coefficients never travel to HBM.
 // A CTA covers up to 512 output columns as 1 or 2 accumulators of NB <= 256.
 // Calls of a few thousand tokens have too few token tiles for 148 SMs, and a tile's time is the length
-// of its K loop (J / 64 stages of operand latency).  Such calls cut K over a cluster of up to eight CTAs:
-// each sums its stretch in TMEM, the fp32 partials of a row travel to the CTA that owns the row (shared
-// memory to shared memory), which adds them in the order of K and finishes the row on its own: nearest
-// centre, or maximum, codes and scale.  See plan_split for the rule and figures.
+// of its K loop (J / 64 stages of operand latency).  Such calls of the projection take more column parts
+// per tile (plan_split).  K itself is never cut: every sum runs in the order of K whatever the call's
+// length, so that a row gets the same id, codes and scale in a chunk of any size.
 // Warps 0-7 compute, warp 8 lane 0 issues TMA, warp 9 lane 0 issues MMA.
 #include <atomic>
 
@@ -49,10 +48,8 @@ constexpr int MAX_PARTS = 8;        // thread blocks of one token tile that form
 
 struct Params {
   int S, J, NB, NACC, n_total;      // n_total = r (project) or C (assign)
-  int nstages;                      // depth of the shared-memory operand ring (2..4)
+  int nstages;                      // depth of the shared-memory operand ring (2..MAX_STAGES)
   int rows;                         // tokens of a tile (<= TM)
-  int ksplit, parts;                // CTAs along K, CTAs per tile (ksplit * column_parts)
-  int meta_off;                     // shared memory: operand ring (then the exchange area), then barriers
   // project
   const uint16_t* x; const uint16_t* centers; const void* ids; int id_bytes;
   const float* mean; uint16_t* coeff;
@@ -98,7 +95,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   const int b_bytes = p.NB * 128;                       // one accumulator's B tile
   const int stage_bytes = A_BYTES + p.NACC * b_bytes;
   const int nst = p.nstages;
-  uint8_t* meta = smem + p.meta_off;
+  uint8_t* meta = smem + nst * stage_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(meta);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + NUM_BARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + NUM_BARS * 8 + 4);
@@ -109,16 +106,13 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   float* peer_max = cn_part;                                      // project + quantise: [MAX_PARTS][128]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int part = blockIdx.x % p.parts;                // place in the tile's cluster
-  const int half = part % p.column_parts, kpart = part / p.column_parts;
-  const int m0 = (blockIdx.x / p.parts) * p.rows;       // this tile's tokens: [m0, m_end)
+  const int part = blockIdx.x % p.column_parts;         // place in the tile's cluster
+  const int m0 = (blockIdx.x / p.column_parts) * p.rows;   // this tile's tokens: [m0, m_end)
   const int m_end = min(p.S, m0 + p.rows);
-  const int n_base = half * p.NACC * p.NB;
+  const int n_base = part * p.NACC * p.NB;
   // assign against fp32 centres: B is the centres split into bf16 planes laid side by side along
   // K, A (the token rows) is walked once per plane
-  const int total_chunks = ASSIGN ? p.a_chunks * (p.cnorm != nullptr ? 3 : 1) : p.J / 64;
-  const int c_first = total_chunks * kpart / p.ksplit;
-  const int nchunks = total_chunks * (kpart + 1) / p.ksplit - c_first;
+  const int nchunks = ASSIGN ? p.a_chunks * (p.cnorm != nullptr ? 3 : 1) : p.J / 64;
 
   if (tid == 0) {
     for (int s = 0; s < MAX_STAGES; ++s) {
@@ -141,22 +135,19 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   const uint32_t tmem_base = *tmem_slot;
   // the column parts of one token tile write into each other's shared memory: nobody may do so before
   // the peers' barriers exist
-  const bool split = p.ksplit > 1;
-  const bool joined = QUANT && !split && p.column_parts > 1;
+  const bool joined = QUANT && p.column_parts > 1;
   if (joined) cluster_sync_all();
   bool ok = true;
-  // assign: squared-norm partials of half a token row, and of half-rows tid + 256 i of the centres
-  float xs = 0.f, cs[4] = {0.f, 0.f, 0.f, 0.f};
 
   if (warp == 8) {
     if (lane == 0) {
       prefetch_tensormap(&map_b);
       if (ASSIGN) prefetch_tensormap(&map_a);
-      int a_col = ASSIGN ? c_first % p.a_chunks : 0;
+      int a_col = 0;
       Ring at;
-      for (int i = 0; i < nchunks && ok; ++i, at.advance(nst)) {
-        const int s = at.stage, c = c_first + i;
-        if (i >= nst) ok = mbar_wait(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 400 + s);
+      for (int c = 0; c < nchunks && ok; ++c, at.advance(nst)) {
+        const int s = at.stage;
+        if (c >= nst) ok = mbar_wait(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 400 + s);
         if (!ok) break;
         uint8_t* stage = smem + s * stage_bytes;
         mbar_arrive_expect_tx(&bars[TMA_FULL + s], p.NACC * b_bytes + (ASSIGN ? A_BYTES : 0));
@@ -211,13 +202,15 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     if (ASSIGN) {
       // ---- squared norms from the resident tiles
       const int C = p.n_total;
+      // partials of half a token row, and of half-rows tid + 256 k of the centres
+      float xs = 0.f, cs[4] = {0.f, 0.f, 0.f, 0.f};
       Ring at;
       for (int i = 0; i < nchunks && ok; ++i, at.advance(nst)) {
         const int s = at.stage;
         ok = __all_sync(0xffffffffu, mbar_wait(&bars[TMA_FULL + s], at.phase, abort_flag, 420 + s) ? 1 : 0) != 0;
         if (!ok) break;
         const uint8_t* stage = smem + s * stage_bytes;
-        if (c_first + i < p.a_chunks) {
+        if (i < p.a_chunks) {
           const uint4* src = reinterpret_cast<const uint4*>(stage + (tid >> 1) * 128 + (tid & 1) * 64);
 #pragma unroll
           for (int j = 0; j < 4; ++j) xs += sumsq8(src[j]);
@@ -236,8 +229,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[STAGE_FREE + s]);
       }
-      if (ok && split) ok = mbar_wait(&bars[ACC_DONE], 0, abort_flag, 431);
-      if (ok && !split) {
+      if (ok) {
         xn_part[tid] = xs;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -248,7 +240,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         ok = mbar_wait(&bars[SIDE_READY], 0, abort_flag, 430) &&
              mbar_wait(&bars[ACC_DONE], 0, abort_flag, 431);
       }
-      if (ok && !split) {
+      if (ok) {
         tc_fence_after();
         const float xn = xn_part[2 * row] + xn_part[2 * row + 1];
         const int chunks = (C + 31) / 32, middle = (chunks + 1) / 2;
@@ -306,7 +298,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       float4 mq[2][2];
       auto fetch = [&](int buf, int i) {
         if (i >= nchunks) return;
-        const int j0 = (c_first + i) * 64;
+        const int j0 = i * 64;
         mq[buf][0] = __ldg(reinterpret_cast<const float4*>(p.mean + j0 + piece * 8));
         mq[buf][1] = __ldg(reinterpret_cast<const float4*>(p.mean + j0 + piece * 8) + 1);
 #pragma unroll
@@ -356,9 +348,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         if (i + 1 < nchunks && ok) step(1, i + 1);
       }
       if (ok) ok = mbar_wait(&bars[ACC_DONE], 0, abort_flag, 450);
-      if (split) {
-        // the partial sums are exchanged below
-      } else if (ok && QUANT) {
+      if (ok && QUANT) {
         // ---- quantise + pack from TMEM.  Pass 1: |max| of the bf16-rounded coefficients of this
         // thread's column chunks; the two warpgroups, then the two column-half CTAs, combine.
         tc_fence_after();
@@ -381,15 +371,15 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           if (joined) {
             if (wg == 0) {
               for (int peer = 0; peer < p.column_parts; ++peer) {
-                if (peer == half) continue;
-                st_cluster_b32(map_to_cta(smem_u32(&peer_max[half * 128 + row]), peer), __float_as_uint(amax));
+                if (peer == part) continue;
+                st_cluster_b32(map_to_cta(smem_u32(&peer_max[part * 128 + row]), peer), __float_as_uint(amax));
                 mbar_arrive_cluster(map_to_cta(smem_u32(&bars[PEER_READY]), peer));
               }
             }
             ok = mbar_wait_cluster(&bars[PEER_READY], 0, abort_flag, 452);
             if (ok)
               for (int peer = 0; peer < p.column_parts; ++peer)
-                if (peer != half) amax = fmaxf(amax, peer_max[peer * 128 + row]);
+                if (peer != part) amax = fmaxf(amax, peer_max[peer * 128 + row]);
           }
         }
         if (ok) {
@@ -419,7 +409,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               *reinterpret_cast<uint4*>(p.codes + static_cast<size_t>(tok) * (p.n_total >> 1) +
                                         ((n_base + col) >> 1)) = make_uint4(words[0], words[1], words[2], words[3]);
           }
-          if (wg == 0 && half == 0 && tok < m_end) store_float(p.scales, p.scale_dtype, tok, scale);
+          if (wg == 0 && part == 0 && tok < m_end) store_float(p.scales, p.scale_dtype, tok, scale);
         }
       } else if (ok) {
         tc_fence_after();
@@ -442,130 +432,6 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               *reinterpret_cast<uint4*>(dst + j4 * 8) = w;
             }
           }
-        }
-      }
-    }
-  }
-  if (split) {
-    // Every CTA of the cluster is behind its last MMA: the operand rings are free, and hold the partial
-    // sums of the rows a CTA owns, one slot per sender.
-    const int own = p.rows / p.parts;                  // rows per CTA
-    const int ncols = p.NACC * p.NB, pitch = ncols + 4;   // 16 bytes of padding: a row per bank group
-    float* slots = reinterpret_cast<float*>(smem);     // [parts][own][pitch]
-    float* xn_slots = slots + p.rows * pitch;          // [parts][own]
-    float* cn_slots = xn_slots + p.rows;               // [parts][C]
-    cluster_sync_all();
-    if (warp < WARPS) {
-      const int row = tid & 127, wg = tid >> 7;
-      tc_fence_after();
-      const uint32_t lane_sel = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-      const bool live = row < p.rows;
-      const uint32_t dst = map_to_cta(smem_u32(slots + (part * own + row % own) * pitch), live ? row / own : 0);
-#pragma unroll 1
-      for (int cc = wg; cc * 32 < ncols; cc += 2) {
-        const int col = cc * 32, acc = col / p.NB;
-        float v[32];
-        tmem_ld32(tmem_base + lane_sel + acc * 256 + (col - acc * p.NB), v);
-        if (live) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            if (col + j < ncols)
-              st_cluster_v4(dst + (col + j) * 4, make_uint4(__float_as_uint(v[j]), __float_as_uint(v[j + 1]),
-                                                            __float_as_uint(v[j + 2]), __float_as_uint(v[j + 3])));
-        }
-      }
-      if (ASSIGN) {
-        xs += __shfl_xor_sync(0xffffffffu, xs, 1);     // two threads share a row
-        const int r = tid >> 1;
-        if ((tid & 1) == 0 && r < p.rows)
-          st_cluster_b32(map_to_cta(smem_u32(xn_slots + part * own + r % own), r / own), __float_as_uint(xs));
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          cs[k] += __shfl_xor_sync(0xffffffffu, cs[k], 1);
-          const int c = r + 128 * k;
-          if (p.cnorm == nullptr && (tid & 1) == 0 && c < p.n_total)
-            for (int peer = 0; peer < p.parts; ++peer)
-              st_cluster_b32(map_to_cta(smem_u32(cn_slots + part * p.n_total + c), peer), __float_as_uint(cs[k]));
-        }
-      }
-    }
-    cluster_sync_all();
-    if (warp < WARPS) {
-      const int tpr = COMPUTE_THREADS / own;           // threads per row, 4 .. 32, inside one warp
-      const int r = tid / tpr, j = tid % tpr;
-      const int tok = m0 + part * own + r;
-      const bool live = tok < m_end;
-      if (ASSIGN) {
-        const int C = p.n_total;
-        float xn = 0.f;
-        for (int k = 0; k < p.ksplit; ++k) xn += xn_slots[k * own + r];
-        float best = INFINITY;
-        int best_i = 0x7fffffff;
-        for (int c = j; c < C; c += tpr) {
-          float dot = 0.f, cn = 0.f;
-          for (int k = 0; k < p.ksplit; ++k) dot += slots[(k * own + r) * pitch + c];
-          if (p.cnorm != nullptr) cn = __ldg(p.cnorm + c);
-          else for (int k = 0; k < p.ksplit; ++k) cn += cn_slots[k * C + c];
-          const float dist = __fsub_rn(__fadd_rn(xn, cn), __fmul_rn(2.0f, dot));
-          if (dist < best) { best = dist; best_i = c; }
-        }
-        for (int off = 1; off < tpr; off <<= 1) {      // smallest distance, first index among equals
-          const float od = __shfl_xor_sync(0xffffffffu, best, off);
-          const int oi = __shfl_xor_sync(0xffffffffu, best_i, off);
-          if (od < best || (od == best && oi < best_i)) { best = od; best_i = oi; }
-        }
-        if (j == 0 && live) {
-          if (p.ids_out != nullptr) {
-            if (p.id_bytes == 1) static_cast<uint8_t*>(p.ids_out)[tok] = static_cast<uint8_t>(best_i);
-            else static_cast<uint16_t*>(p.ids_out)[tok] = static_cast<uint16_t>(best_i);
-          }
-          if (p.labels_out != nullptr) p.labels_out[tok] = best_i;
-        }
-      } else {
-        // columns 8 g .. 8 g + 8 of the row: partials added in the order of K, rounded to bf16
-        const int groups = p.n_total / 8;
-        float amax = 0.f;
-        for (int g = j; g < groups; g += tpr) {
-          const int hh = g * 8 / ncols, col = g * 8 - hh * ncols;
-          float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          for (int k = 0; k < p.ksplit; ++k) {
-            const float4* src = reinterpret_cast<const float4*>(slots + ((k * p.column_parts + hh) * own + r) * pitch + col);
-            const float4 lo = src[0], hi = src[1];
-            z[0] += lo.x; z[1] += lo.y; z[2] += lo.z; z[3] += lo.w;
-            z[4] += hi.x; z[5] += hi.y; z[6] += hi.z; z[7] += hi.w;
-          }
-          if (QUANT) {
-            float* keep = slots + (hh * own + r) * pitch + col;   // this thread's alone: read again below
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              z[i] = round_to_bf16(z[i]);
-              amax = fmaxf(amax, fabsf(z[i]));
-            }
-            reinterpret_cast<float4*>(keep)[0] = make_float4(z[0], z[1], z[2], z[3]);
-            reinterpret_cast<float4*>(keep)[1] = make_float4(z[4], z[5], z[6], z[7]);
-          } else if (live) {
-            *reinterpret_cast<uint4*>(p.coeff + static_cast<size_t>(tok) * p.n_total + g * 8) =
-                make_uint4(pack_bf16x2(z[0], z[1]), pack_bf16x2(z[2], z[3]), pack_bf16x2(z[4], z[5]), pack_bf16x2(z[6], z[7]));
-          }
-        }
-        if (QUANT) {
-          for (int off = 1; off < tpr; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-          float scale;
-          if (p.in_bf16) scale = round_to_bf16(__fdiv_rn(fmaxf(amax, round_to_bf16(p.eps)), 7.0f));
-          else scale = __fdiv_rn(fmaxf(amax, p.eps), 7.0f);
-          const float inv = __frcp_rn(scale);
-          for (int g = j; g < groups; g += tpr) {
-            const int hh = g * 8 / ncols, col = g * 8 - hh * ncols;
-            const float* z = slots + (hh * own + r) * pitch + col;
-            uint32_t word = 0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int code = p.in_bf16 ? quant_code<true>(z[i], scale, inv) : quant_code<false>(z[i], scale, inv);
-              word |= static_cast<uint32_t>(code) << (4 * i);
-            }
-            if (live) *reinterpret_cast<uint32_t*>(p.codes + static_cast<size_t>(tok) * (p.n_total >> 1) + g * 4) = word;
-          }
-          if (j == 0 && live) store_float(p.scales, p.scale_dtype, tok, scale);
         }
       }
     }
@@ -600,45 +466,23 @@ size_t smem_bytes(int nacc, int nb, int n_total, int stages = 2) {
   return ring_bytes(nacc, nb, stages) + meta_bytes(n_total) + 1024;
 }
 
-// partial sums of a tile's rows with their norms (split form)
-size_t exchange_bytes(int rows, int columns, int parts, int n_norms) {
-  return 4 * (static_cast<size_t>(rows) * (columns + 4) + rows + static_cast<size_t>(parts) * n_norms);
-}
-
 constexpr size_t SMEM_LIMIT = 232448;
 
-// Fills in stages, the barrier block's place and the launch's shared memory.
-size_t place_smem(Params& p, int n_norms) {
-  p.nstages = MAX_STAGES;
-  while (p.nstages > 2 && smem_bytes(p.NACC, p.NB, n_norms, p.nstages) > SMEM_LIMIT) --p.nstages;
-  size_t front = ring_bytes(p.NACC, p.NB, p.nstages);
-  if (p.ksplit > 1) {
-    const size_t exchange = exchange_bytes(p.rows, p.NACC * p.NB, p.parts, n_norms);
-    if (exchange > front) front = exchange;
-  }
-  p.meta_off = static_cast<int>((front + 255) / 256 * 256);
-  return p.meta_off + meta_bytes(n_norms) + 1024;
-}
-
-// How a GEMM of S tokens x `columns` over `chunks` stages is cut: tokens per tile, column parts, K parts.
+// How a GEMM of S tokens x `columns` over `chunks` stages is cut: tokens per tile and column parts.
 // The estimate counts SM cycles: a stage costs the bytes it takes from L2 (token rows, centre rows, B) at
-// 48 bytes per clock, at least 350 cycles of latency; exchanging partials costs 15 bytes per clock, the
-// SM-to-SM rate, plus the barriers.  Clusters of 8 fit 128 of the 148 SMs at a time, of 4 about 144.
-// Bound of the undivided form: 880 tokens x 3,072 columns x rank 384 kept 14 SMs busy for 48 stages of
-// operand latency (107 us).  us per call now: projection with K cut 880 x 3,072 x 384 18 (64 tokens, 2
-// column parts, 4 K parts), 1,560 x 3,072 x 384 23 (84 before); in order 880 x 3,072 x 384 39 (6 column
-// parts), 4,680 x 5,120 x 640 71 (128 before: operand prefetch alone); assignment of 1,560 x 3,072 to 256
-// centres 28 (60 before), to 64 fp32 centres in order 880 x 3,072 49 (70), 4,680 x 5,120 80 (116).  Only
-// the order in which K is summed depends on the cut, and the projection and its quantising form take the
-// same one.
-// `ordered`: K is not cut, every sum runs in the order of K whatever the call's length, so that rows encode
-// to the same bytes in a chunk of any size (the online encoders, whose payloads are stored and compared, and
-// the projection entry points); such calls take more column parts instead.
-struct Split { int rows, column_parts, ksplit; };
+// 48 bytes per clock, at least 350 cycles of latency.  Column parts of the projection form clusters of up
+// to eight, of which 128 of the 148 SMs hold whole ones at a time, of four about 144.
+// Bound of short calls: 880 tokens x 3,072 columns x rank 384 in tiles of 128 whole rows keep 14 SMs busy for
+// 48 stages of operand latency (107 us; 39 with six column parts); 4,680 x 5,120 x 640 71 (128 before the
+// operands of two chunks were in flight); assignment to 64 fp32 centres 880 x 3,072 49 (70), 4,680 x 5,120 80
+// (116).  Cutting K over a cluster as well was faster still for given centres (assignment of 1,560 x 3,072 to
+// 256 centres 28 us against 60), but then the order of a row's fp32 sums, and now and then a code or an id,
+// depends on the length of the call.
+struct Split { int rows, column_parts; };
 
-Split plan_split(int S, int chunks, int columns, int column_parts, int n_norms, bool residual, bool ordered) {
+Split plan_split(int S, int chunks, int columns, int column_parts, bool residual) {
   const int sms = sm_count();
-  Split best{pick_rows(S, column_parts), column_parts, 1};
+  Split best{pick_rows(S, column_parts), column_parts};
   auto stage_cost = [&](int rows, int cols) {
     const double bytes = rows * (residual ? 256.0 : 128.0) + cols * 128.0;
     return bytes / 48 > 350 ? bytes / 48 : 350.0;
@@ -647,23 +491,17 @@ Split plan_split(int S, int chunks, int columns, int column_parts, int n_norms, 
   double best_cost = rounds(static_cast<long long>(ceil_div(S, best.rows)) * column_parts, sms) *
                      (chunks * stage_cost(best.rows, columns / column_parts) + 3000);
   for (int rows = 64; rows <= TM; rows *= 2)
-    for (int h = column_parts; h <= MAX_PARTS; ++h)
-      for (int k = 1; k * h <= MAX_PARTS; k *= 2) {
-        const int cols = columns / h;
-        if (k > 1 && (ordered || chunks < 2 * k || h > 2 * column_parts || h > 4 || (h & (h - 1)) != 0)) continue;
-        if (columns % h || cols > 512 || cols % (cols > 256 ? 64 : 32)) continue;
-        if (h > column_parts && !residual) continue;
-        const int parts = k * h;
-        if (k > 1 && exchange_bytes(rows, cols, parts, n_norms) + meta_bytes(n_norms) + 2048 > SMEM_LIMIT) continue;
-        const int room = parts > 4 ? sms - 20 : (parts > 2 ? sms - 4 : sms);
-        const double cost = rounds(static_cast<long long>(ceil_div(S, rows)) * parts, room) *
-                            (ceil_div(chunks, k) * stage_cost(rows, cols) +
-                             (k > 1 ? rows * cols * 4.0 / 15 + 5000 : 3000 + 300 * h));
-        if (cost < best_cost) {
-          best_cost = cost;
-          best = Split{rows, h, k};
-        }
+    for (int h = column_parts; h <= (residual ? MAX_PARTS : column_parts); ++h) {
+      const int cols = columns / h;
+      if (columns % h || cols > 512 || cols % (cols > 256 ? 64 : 32)) continue;
+      const int room = h > 4 ? sms - 20 : (h > 2 ? sms - 4 : sms);
+      const double cost = rounds(static_cast<long long>(ceil_div(S, rows)) * h, room) *
+                          (chunks * stage_cost(rows, cols) + 3000 + 300 * h);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = Split{rows, h};
       }
+    }
   return best;
 }
 
@@ -676,19 +514,20 @@ void set_columns(Params& p, int columns) {
 template <int MODE>
 int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, Params& p, int n_norms, const char* name,
                 cudaStream_t stream) {
-  p.parts = p.ksplit * p.column_parts;
-  const size_t smem = place_smem(p, n_norms);
+  p.nstages = MAX_STAGES;
+  while (p.nstages > 2 && smem_bytes(p.NACC, p.NB, n_norms, p.nstages) > SMEM_LIMIT) --p.nstages;
+  const size_t smem = smem_bytes(p.NACC, p.NB, n_norms, p.nstages);
   NKV_REQUIRE(smem <= SMEM_LIMIT, NKV_ERR_UNSUPPORTED, "%s needs %zu bytes of shared memory", name, smem);
   auto kernel = encode_gemm_kernel<MODE>;
   NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   cudaLaunchConfig_t config{};
-  config.gridDim = dim3(static_cast<unsigned>(ceil_div(p.S, p.rows)) * p.parts);
+  config.gridDim = dim3(static_cast<unsigned>(ceil_div(p.S, p.rows)) * p.column_parts);
   config.blockDim = dim3(THREADS);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = p.ksplit > 1 || MODE == PROJECT_QUANT ? p.parts : 1;
+  attr.val.clusterDim.x = MODE == PROJECT_QUANT ? p.column_parts : 1;
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
   config.attrs = &attr;
@@ -741,14 +580,14 @@ bool tc_assign_supported(int J, int C) {
 
 int tc_project(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
                const float* mean, const void* encoder_bf16, int S, int J, int r, void* coeff,
-               bool ordered, cudaStream_t stream) {
+               cudaStream_t stream) {
   if (S == 0) return NKV_OK;
   Params p{};
   int gy;
   NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB), NKV_ERR_UNSUPPORTED,
               "projection rank %d cannot be tiled", r);
-  const Split cut = plan_split(S, J / 64, r, gy, 0, true, ordered);
-  p.rows = cut.rows; p.column_parts = cut.column_parts; p.ksplit = cut.ksplit;
+  const Split cut = plan_split(S, J / 64, r, gy, true);
+  p.rows = cut.rows; p.column_parts = cut.column_parts;
   set_columns(p, r / p.column_parts);
   NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(centers_bf16) & 15) == 0 &&
@@ -776,15 +615,14 @@ bool tc_project_quant_supported(int J, int r, int group) {
 
 int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
                      const float* mean, const void* encoder_bf16, int S, int J, int r, float eps,
-                     int quant_mode, int scale_dtype, uint8_t* codes, void* scales, bool ordered,
-                     cudaStream_t stream) {
+                     int quant_mode, int scale_dtype, uint8_t* codes, void* scales, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
   Params p{};
   int gy;
   NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB) && gy <= 2, NKV_ERR_UNSUPPORTED,
               "fused projection: rank %d cannot be tiled over at most two column parts", r);
-  const Split cut = plan_split(S, J / 64, r, gy, 0, true, ordered);
-  p.rows = cut.rows; p.column_parts = cut.column_parts; p.ksplit = cut.ksplit;
+  const Split cut = plan_split(S, J / 64, r, gy, true);
+  p.rows = cut.rows; p.column_parts = cut.column_parts;
   set_columns(p, r / p.column_parts);
   NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(centers_bf16) & 15) == 0 &&
@@ -812,8 +650,8 @@ int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C,
   if (S == 0) return NKV_OK;
   Params p{};
   p.S = S; p.J = J; p.n_total = C;
-  const Split cut = plan_split(S, J / 64, C, 1, C, false, false);
-  p.rows = cut.rows; p.column_parts = 1; p.ksplit = cut.ksplit;
+  const Split cut = plan_split(S, J / 64, C, 1, false);
+  p.rows = cut.rows; p.column_parts = 1;
   set_columns(p, C);
   p.ids_out = ids; p.id_bytes = id_bytes;
   p.a_chunks = J / 64;
@@ -886,8 +724,8 @@ int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, in
   NKV_LAUNCH_CHECK("split_centers_kernel");
   Params p{};
   p.S = S; p.J = J; p.n_total = C;
-  const Split cut = plan_split(S, 3 * (J / 64), C, 1, C, false, true);
-  p.rows = cut.rows; p.column_parts = 1; p.ksplit = cut.ksplit;
+  const Split cut = plan_split(S, 3 * (J / 64), C, 1, false);
+  p.rows = cut.rows; p.column_parts = 1;
   set_columns(p, C);
   p.labels_out = labels; p.id_bytes = 1;
   p.a_chunks = J / 64;
