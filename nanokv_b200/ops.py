@@ -416,23 +416,35 @@ def rope_rows(x: torch.Tensor, rope: RopeView) -> torch.Tensor:
 
 
 def attention_lse(q, k, v, *, scale: float):
-    """Plain attention: q [Q,H,d], k [N,H,d], v [N,H,dv] -> (O [Q,H,dv], lse [Q,H]).
+    """Plain attention: q [Q,H,d], k [N,H,d], v [N,H,dv] -> (O [Q,H,dv], lse [Q,H]).  K and V rows may
+    have more heads than the queries: the first H are attended.
 
     bf16 rows of width 64 or 128 run on the tensor cores; everything else on the fp32 CUDA-core
     kernel."""
     device = _require_cuda(q, k, v)
     Q, H, d = q.shape
     N, dv = k.shape[0], v.shape[2]
-    if (q.dtype == torch.bfloat16 and k.dtype == v.dtype == torch.bfloat16 and d == dv
+    # the kernels take one N and the widths of q and v: rows that do not agree would be read past their end
+    if v.shape[0] != N:
+        raise ValueError(f"K and V differ in tokens: {N} and {v.shape[0]}")
+    if k.shape[2] != d:
+        raise ValueError(f"keys are {k.shape[2]} wide, queries {d}")
+    if k.shape[1] < H or v.shape[1] < H:
+        raise ValueError(f"{H} query heads, but {k.shape[1]} of K and {v.shape[1]} of V")
+    if k.dtype != q.dtype or v.dtype != q.dtype:
+        raise ValueError("q, k and v must share a dtype")
+    if (q.dtype == torch.bfloat16 and d == dv
             and d in (64, 128) and N > 0 and q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0
             and not _SIMT_FORCED[0]):
         lib = _lib.library()
+        # rows with more heads than the queries: their first H
+        k, v = (x if x.shape[1] == H else x[:, :H].contiguous() for x in (k, v))
         out = torch.empty(Q, H, dv, dtype=q.dtype, device=device)
         lse = torch.empty(Q, H, dtype=torch.float32, device=device)
         nbytes = lib.nkv_attention_lse_workspace_bytes(Q, H, d, N)
         workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
         _lib.check(lib.nkv_attention_lse_bf16(
-            _ptr(q), _ptr(k), _ptr(v), q.stride(0), q.stride(1), k.stride(0), k.stride(1), Q, N, H, d, dv,
+            _ptr(q), _ptr(k), _ptr(v), q.stride(0), q.stride(1), H * d, d, Q, N, H, d, dv,
             float(scale), _ptr(out), _ptr(lse), _ptr(status_word(device)), _ptr(workspace), nbytes, _stream(device)))
         return out, lse
     out = torch.empty(Q, H, dv, dtype=q.dtype, device=device)
