@@ -589,11 +589,13 @@ int kmeans_gather_init(const void* x, int x_dtype, int J, int C, const int32_t* 
 
 int kmeans_update(const void* x, int x_dtype, int S, int J, int C, const int32_t* labels,
                   float* centers, cudaStream_t stream) {
-  // two columns per thread: rows start 4 (bf16) or 8 (fp32) byte aligned and have an even length
-  const bool pairs = J % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & (x_dtype == NKV_F32 ? 7 : 3)) == 0;
+  // two columns per thread for bf16 and fp32 rows of even length that start on 4 resp. 8 bytes; every other
+  // form (fp16 rows among them) one column, converted by load_float
+  const bool bf16 = x_dtype == NKV_BF16, f32 = x_dtype == NKV_F32;
+  const bool pairs = (bf16 || f32) && J % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & (f32 ? 7 : 3)) == 0;
   const dim3 grid(C, ceil_div(J, pairs ? 512 : 256));
   if (!pairs) kmeans_update_kernel<Single><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
-  else if (x_dtype == NKV_F32) kmeans_update_kernel<PairF32><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
+  else if (f32) kmeans_update_kernel<PairF32><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
   else kmeans_update_kernel<PairBf16><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
   NKV_LAUNCH_CHECK("kmeans_update_kernel");
   return NKV_OK;
