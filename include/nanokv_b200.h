@@ -100,6 +100,23 @@ int nkv_set_bf16_path(int path);
  */
 int nkv_selftest_bounded_wait(int kind, long long budget_cycles, int32_t* status_word, void* stream);
 
+/*
+ * Self-tests of what a give-up leaves behind: nkv_decode_rows_status with bf16 operators and rows, and
+ * nkv_attn_codec_rows in bf16 without a positional restore, with no decoder row ever loaded, so that the
+ * waits for them run out after `budget_cycles`.  The status word (not NULL) receives a wait site; the rows
+ * are NaN, resp. every LSE is.  No counterpart in the reference.
+ */
+int nkv_selftest_decode_gives_up(const nkv_history* hist, const int32_t* rows_index, int n,
+                                 const void* decoder, const float* mean, int J, void* out,
+                                 int32_t* status_word, long long budget_cycles, void* stream);
+int nkv_selftest_read_gives_up(const void* q, int64_t q_stride_token, int64_t q_stride_head,
+                               int Q, int heads, int d,
+                               const nkv_history* hist_k, const nkv_history* hist_v,
+                               const void* wk, const float* bias_k, const void* wv, const float* bias_v,
+                               float scale, void* out, float* lse, int32_t* status_word, int splits,
+                               void* workspace, size_t workspace_bytes, long long budget_cycles,
+                               void* stream);
+
 /* ------------------------------------------------------------------ encode */
 
 /*
@@ -225,10 +242,15 @@ int nkv_encode_append_static(const void* x, int x_dtype, const void* centers_bf1
  * Reference: decode_tensor MGM/nanokv_codec.py:369-390, _decode_method_segments
  * :393-455, LB/lingbot_v2_kv_codec.py:301-326,404-437 (row / slice forms).
  * decoder [J,r], mean f32 [J], out [n,J] (f32|bf16).
+ * The bf16 kernel has bounded waits (as the read): rows that it could not finish are NaN, and the _status
+ * form stores the wait's site in *status_word (device int32, cleared by the caller; NULL: not reported).
  */
 int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
                     const void* decoder, int decoder_dtype, const float* mean, int J,
                     void* out, int out_dtype, void* stream);
+int nkv_decode_rows_status(const nkv_history* hist, const int32_t* rows_index, int n,
+                           const void* decoder, int decoder_dtype, const float* mean, int J,
+                           void* out, int out_dtype, int32_t* status_word, void* stream);
 
 /*
  * Enters segment `index` in a device segment table: seg_start[index + 1] = stop (tokens before the next

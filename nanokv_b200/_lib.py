@@ -68,6 +68,8 @@ SIGNATURES = {
     "nkv_segment_append": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "nkv_decode_rows": (c_int, [POINTER(History), c_void_p, c_int, c_void_p, c_int, c_void_p,
                                 c_int, c_void_p, c_int, c_void_p]),
+    "nkv_decode_rows_status": (c_int, [POINTER(History), c_void_p, c_int, c_void_p, c_int, c_void_p,
+                                       c_int, c_void_p, c_int, c_void_p, c_void_p]),
     "nkv_attn_codec": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int, c_int, c_int, c_int,
                                POINTER(History), POINTER(History), c_void_p, c_void_p, c_void_p,
                                c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p]),
@@ -119,6 +121,12 @@ SIGNATURES = {
                                 c_int, c_int, c_void_p, c_void_p]),
     "nkv_set_bf16_path": (c_int, [c_int]),
     "nkv_selftest_bounded_wait": (c_int, [c_int, ctypes.c_longlong, c_void_p, c_void_p]),
+    "nkv_selftest_decode_gives_up": (c_int, [POINTER(History), c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p,
+                                             c_void_p, ctypes.c_longlong, c_void_p]),
+    "nkv_selftest_read_gives_up": (c_int, [c_void_p, c_int64, c_int64, c_int, c_int, c_int, POINTER(History),
+                                           POINTER(History), c_void_p, c_void_p, c_void_p, c_void_p, c_float,
+                                           c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_size_t,
+                                           ctypes.c_longlong, c_void_p]),
     "nkv_peer_open": (c_int, [c_char_p, POINTER(c_void_p)]),
     "nkv_peer_close": (c_int, [c_void_p]),
     "nkv_peer_free": (c_int, [c_void_p]),
@@ -162,8 +170,8 @@ STATUS_SCORE_RANGE = 950
 def check_device_status(word: int) -> None:
     """Raise for a non-zero status word that a kernel left behind.
 
-    The fused read writes the site code of a bounded wait that gave up (its rows are then not
-    results: their LSE is NaN), or STATUS_SCORE_RANGE when a row's scores left the window of the
+    The reads and the row decode write the site code of a bounded wait that gave up (its rows are then not
+    results: their LSE is NaN, decoded rows are NaN), or STATUS_SCORE_RANGE when a row's scores left the window of the
     online softmax (that row's LSE is NaN).  NKV_OK from the launching call only says that the
     launch was accepted; the word is valid once the stream has been synchronised."""
     if word == 0:

@@ -262,9 +262,15 @@ int nkv_segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, i
   return segment_append(seg_start, seg_center_row, index, stop, center_row, static_cast<cudaStream_t>(stream));
 }
 
-int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
-                    const void* decoder, int decoder_dtype, const float* mean, int J, void* out,
-                    int out_dtype, void* stream) {
+static int check_selftest(long long budget_cycles, const int32_t* status_word) {
+  NKV_REQUIRE(budget_cycles > 0 && budget_cycles <= (1ll << 28) && status_word, NKV_ERR_INVALID,
+              "wait self-test: budget=%lld", budget_cycles);
+  return NKV_OK;
+}
+
+static int decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
+                       const void* decoder, int decoder_dtype, const float* mean, int J, void* out,
+                       int out_dtype, int32_t* status_word, long long selftest_budget, void* stream) {
   int rc = check_history(hist, "decode");
   if (rc != NKV_OK) return rc;
   NKV_REQUIRE(n >= 0 && J > 0, NKV_ERR_INVALID, "decode_rows: n=%d J=%d", n, J);
@@ -278,10 +284,32 @@ int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
   if (decoder_dtype == NKV_BF16 && out_dtype == NKV_BF16 && !simt_forced() && hist->tokens > 0 &&
       tc_decode_supported(*hist, J) && aligned(decoder) && aligned(mean) && aligned(out)) {
     DecodeTensor t{hist, decoder, mean, rows_index, out, J, 0, nullptr, nullptr};
-    return tc_decode(&t, 1, n, J, J, false, true, nullptr, sm_count(), static_cast<cudaStream_t>(stream));
+    return tc_decode(&t, 1, n, J, J, false, true, status_word, nullptr, sm_count(), selftest_budget,
+                     static_cast<cudaStream_t>(stream));
   }
+  NKV_REQUIRE(selftest_budget == 0, NKV_ERR_UNSUPPORTED, "wait self-test: this decode has no waits");
   return simt_decode_rows(*hist, rows_index, n, decoder, decoder_dtype, mean, J, out, out_dtype,
                           J, static_cast<cudaStream_t>(stream));
+}
+
+int nkv_decode_rows(const nkv_history* hist, const int32_t* rows_index, int n,
+                    const void* decoder, int decoder_dtype, const float* mean, int J, void* out,
+                    int out_dtype, void* stream) {
+  return decode_rows(hist, rows_index, n, decoder, decoder_dtype, mean, J, out, out_dtype, nullptr, 0, stream);
+}
+
+int nkv_decode_rows_status(const nkv_history* hist, const int32_t* rows_index, int n,
+                           const void* decoder, int decoder_dtype, const float* mean, int J, void* out,
+                           int out_dtype, int32_t* status_word, void* stream) {
+  return decode_rows(hist, rows_index, n, decoder, decoder_dtype, mean, J, out, out_dtype, status_word, 0, stream);
+}
+
+int nkv_selftest_decode_gives_up(const nkv_history* hist, const int32_t* rows_index, int n,
+                                 const void* decoder, const float* mean, int J, void* out, int32_t* status_word,
+                                 long long budget_cycles, void* stream) {
+  int rc = check_selftest(budget_cycles, status_word);
+  if (rc != NKV_OK) return rc;
+  return decode_rows(hist, rows_index, n, decoder, NKV_BF16, mean, J, out, NKV_BF16, status_word, budget_cycles, stream);
 }
 
 size_t nkv_attn_codec_workspace_bytes(int Q, int heads, int dv, int splits) {
@@ -429,13 +457,13 @@ int nkv_attn_codec_rows_is_faster(int dtype, int Q, int heads, int dk, int dv, i
   return tc_attn_fused_is_faster(Q, heads, dk, tokens, rank, positional != 0) ? 0 : 1;
 }
 
-int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
-                        int Q, int heads, int dk, int dv, const nkv_history* hist_k,
-                        const nkv_history* hist_v, const void* wk, const float* bias_k,
-                        const void* wv, const float* bias_v, int weight_order, const nkv_rope* rope,
-                        const nkv_camera* camera_k, const nkv_camera* camera_v, float scale,
-                        void* out, float* lse, int32_t* status_word, int splits, void* workspace,
-                        size_t workspace_bytes, void* stream) {
+static int attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
+                           int Q, int heads, int dk, int dv, const nkv_history* hist_k,
+                           const nkv_history* hist_v, const void* wk, const float* bias_k,
+                           const void* wv, const float* bias_v, int weight_order, const nkv_rope* rope,
+                           const nkv_camera* camera_k, const nkv_camera* camera_v, float scale,
+                           void* out, float* lse, int32_t* status_word, int splits, void* workspace,
+                           size_t workspace_bytes, long long selftest_budget, void* stream) {
   int rc = check_read(dtype, Q, heads, dk, dv, hist_k, hist_v, weight_order, rope, camera_k, camera_v);
   if (rc != NKV_OK) return rc;
   NKV_REQUIRE(splits >= 0 && splits <= 16, NKV_ERR_INVALID, "attn_codec_rows: splits=%d (0..16)", splits);
@@ -459,7 +487,31 @@ int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_
   }
   return tc_attn_by_rows_run(q, q_stride_token, q_stride_head, Q, heads, dk, hist_k, hist_v, wk, bias_k, wv, bias_v,
                              weight_order == NKV_WEIGHTS_KERNEL_ORDER, rope, camera_k, camera_v, scale, out, lse,
-                             status_word, splits, workspace, static_cast<cudaStream_t>(stream));
+                             status_word, splits, workspace, selftest_budget, static_cast<cudaStream_t>(stream));
+}
+
+int nkv_attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,
+                        int Q, int heads, int dk, int dv, const nkv_history* hist_k,
+                        const nkv_history* hist_v, const void* wk, const float* bias_k,
+                        const void* wv, const float* bias_v, int weight_order, const nkv_rope* rope,
+                        const nkv_camera* camera_k, const nkv_camera* camera_v, float scale,
+                        void* out, float* lse, int32_t* status_word, int splits, void* workspace,
+                        size_t workspace_bytes, void* stream) {
+  return attn_codec_rows(q, dtype, q_stride_token, q_stride_head, Q, heads, dk, dv, hist_k, hist_v, wk, bias_k, wv, bias_v,
+                         weight_order, rope, camera_k, camera_v, scale, out, lse, status_word, splits, workspace,
+                         workspace_bytes, 0, stream);
+}
+
+int nkv_selftest_read_gives_up(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int d,
+                               const nkv_history* hist_k, const nkv_history* hist_v, const void* wk,
+                               const float* bias_k, const void* wv, const float* bias_v, float scale, void* out,
+                               float* lse, int32_t* status_word, int splits, void* workspace, size_t workspace_bytes,
+                               long long budget_cycles, void* stream) {
+  int rc = check_selftest(budget_cycles, status_word);
+  if (rc != NKV_OK) return rc;
+  return attn_codec_rows(q, NKV_BF16, q_stride_token, q_stride_head, Q, heads, d, d, hist_k, hist_v, wk, bias_k, wv, bias_v,
+                         NKV_WEIGHTS_NATURAL, nullptr, nullptr, nullptr, scale, out, lse, status_word, splits, workspace,
+                         workspace_bytes, budget_cycles, stream);
 }
 
 int nkv_attn_codec_split(const void* q, int dtype, int64_t q_stride_token, int64_t q_stride_head,

@@ -85,7 +85,8 @@ int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_
                         const nkv_history* hist_k, const nkv_history* hist_v, const void* wk, const float* bias_k,
                         const void* wv, const float* bias_v, bool prepared_weights, const nkv_rope* rope,
                         const nkv_camera* cam_k, const nkv_camera* cam_v, float scale, void* out, float* lse,
-                        int32_t* status, int max_splits, void* workspace, cudaStream_t stream);
+                        int32_t* status, int max_splits, void* workspace, long long selftest_budget,
+                        cudaStream_t stream);
 bool tc_attention_rows_supported(const void* q, const void* k, const void* v, int64_t q_stride_token,
                                  int64_t q_stride_head, int64_t kv_stride_token, int64_t kv_stride_head, int d, int dv);
 int tc_attention_rows(const void* q, const void* k, const void* v, int64_t q_stride_token, int64_t q_stride_head,
@@ -107,8 +108,11 @@ struct DecodeTensor {
   const nkv_camera* camera;  // or NULL
 };
 bool tc_decode_supported(const nkv_history& h, int J);
+// failed: tc_decode_blocks words that the launch sets to 0 or to the site of a wait that gave up, or NULL.
+// selftest_budget > 0: no decoder row is loaded and every wait gives up after that many cycles.
+int tc_decode_blocks(int count, int n, int J, int sms);
 int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool w_perm, bool round_bias,
-              int32_t* status, int sms, cudaStream_t stream);
+              int32_t* status, int32_t* failed, int sms, long long selftest_budget, cudaStream_t stream);
 int sm_count();
 bool tc_project_supported(int J, int r);
 bool tc_project_quant_supported(int J, int r, int group);

@@ -69,14 +69,14 @@ __device__ __forceinline__ bool mbar_try_wait_parked(uint64_t* bar, uint32_t par
 
 // Bounded wait.  `abort_flag` lives in shared memory; `code` identifies the
 // wait site in the status word the host reads.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          volatile int* abort_flag, int code) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                          long long budget = WAIT_BUDGET_CYCLES) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long start = clock64();
   while (true) {
     if (*abort_flag) return false;
     if (mbar_try_wait(bar, parity)) return true;
-    if (clock64() - start > WAIT_BUDGET_CYCLES) {
+    if (clock64() - start > budget) {
       atomicCAS(const_cast<int*>(abort_flag), 0, code);
       return false;
     }
@@ -149,14 +149,14 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
 }
 
 // bounded wait on a barrier that peer CTAs arrive on (cluster-scope acquire)
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity,
-                                                  volatile int* abort_flag, int code) {
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                                  long long budget = WAIT_BUDGET_CYCLES) {
   if (mbar_try_wait_cluster(bar, parity)) return true;
   const long long start = clock64();
   while (true) {
     if (*abort_flag) return false;
     if (mbar_try_wait_cluster(bar, parity)) return true;
-    if (clock64() - start > WAIT_BUDGET_CYCLES) {
+    if (clock64() - start > budget) {
       atomicCAS(const_cast<int*>(abort_flag), 0, code);
       return false;
     }

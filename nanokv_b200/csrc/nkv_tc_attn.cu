@@ -84,8 +84,9 @@ enum Bar {
 // meta block
 constexpr int M_SLOT = NUM_BARS * 8;              // TMEM base address
 constexpr int M_ABORT = M_SLOT + 4;
+constexpr int M_DECODE_FAILED = M_ABORT + 4;      // attn_rows_kernel: the decode in front of it gave up
 constexpr int M_CROW = 512;                       // [NMETA][128] centre row of every token of a tile
-static_assert(M_ABORT + 4 <= M_CROW && M_CROW + NMETA * TOK * 4 <= META_BYTES, "meta block layout");
+static_assert(M_DECODE_FAILED + 4 <= M_CROW && M_CROW + NMETA * TOK * 4 <= META_BYTES, "meta block layout");
 
 // global flag words
 constexpr int F_ABORT = 0;        // launch-wide abort (wait-site code)
@@ -117,6 +118,8 @@ struct Params {
   int tail_units, tail_blocks;
   float* tail_out;   // [2 * tail_blocks][NQ * QT][D]
   float* tail_lse;   // [2 * tail_blocks][NQ * QT]
+  const int32_t* decode_failed;   // words of the decode that rebuilt the rows; one that is not 0: it gave up
+  int decode_blocks;
   long long* prof;   // development builds: cycle buckets of group 0's first consumer and first producer
 };
 
@@ -836,8 +839,9 @@ __device__ __forceinline__ void consumer_role(uint8_t* smem, uint64_t* bars, uin
           }
         }
       }
+      const bool gave_up = !RING && *reinterpret_cast<volatile int*>(smem + M_DECODE_FAILED) != 0;
       if (qrow < p.Q) {
-        *lse_of(q0) = saturated ? __int_as_float(0x7fc00000)
+        *lse_of(q0) = saturated || gave_up ? __int_as_float(0x7fc00000)
                                 : (l_run > 0.f ? (m_used + log2f(l_run)) * 0.6931471805599453f : -INFINITY);
         if (saturated && p.status) atomicCAS(p.status, 0, STATUS_SCORE_RANGE);
       }
@@ -1441,6 +1445,12 @@ attn_rows_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + M_SLOT);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + M_ABORT);
   const int tid = threadIdx.x, warp = tid >> 5;
+  if (warp == 8) {   // did the decode in front of this launch give up?  (its rows are NaN then: so is every LSE)
+    int failed = 0;
+    for (int i = tid & 31; i < p.decode_blocks; i += 32) failed |= __ldg(p.decode_failed + i);
+    failed = __any_sync(0xffffffffu, failed != 0) ? 1 : 0;
+    if ((tid & 31) == 0) *reinterpret_cast<volatile int*>(smem + M_DECODE_FAILED) = failed;
+  }
   if (tid == 0) {
     init_consumer_barriers(bars);
     *abort_flag = 0;
@@ -2015,6 +2025,8 @@ RowPlan plan_rows(int sms, int Q, int heads, int d, int tokens, int max_splits, 
   return best;
 }
 
+size_t failed_bytes(int sms) { return (static_cast<size_t>(sms) * 4 + 255) / 256 * 256; }   // a word per decode block
+
 size_t tail_bytes(int sms, int d) { return static_cast<size_t>(2 * sms) * (NQ * QT) * (d + 1) * 4; }
 
 size_t partial_bytes(int splits, int Q, int heads, int d) {
@@ -2047,8 +2059,8 @@ int row_map(CUtensorMap* map, const void* base, int d, int heads, int tokens, in
 // one launch over `heads` heads; out / lse are the batch's first head inside rows of out_heads heads
 int attend_rows(const void* q, int64_t q_stride_token, int64_t q_stride_head, int Q, int heads, int out_heads,
                 int d, const void* k, const void* v, int64_t kv_stride_token, int64_t kv_stride_head, int N,
-                float scale, int splits, int tiles_per_split, float* tail, uint16_t* out, float* lse,
-                int32_t* status, cudaStream_t stream) {
+                float scale, int splits, int tiles_per_split, float* tail, const int32_t* decode_failed,
+                int decode_blocks, uint16_t* out, float* lse, int32_t* status, cudaStream_t stream) {
   CUtensorMap maps[3];
   int rc = row_map(&maps[0], q, d, heads, Q, q_stride_token, q_stride_head);
   if (rc == NKV_OK) rc = row_map(&maps[1], k, d, heads, N, kv_stride_token, kv_stride_head);
@@ -2074,6 +2086,8 @@ int attend_rows(const void* q, int64_t q_stride_token, int64_t q_stride_head, in
   }
   p.scale_log2 = scale * 1.4426950408889634f;
   p.wait_budget = 1ll << 31;
+  p.decode_failed = decode_failed;
+  p.decode_blocks = decode_blocks;
   p.out = out; p.lse = lse; p.status = status;
 #ifdef NKV_DEV
   p.prof = g_profile;
@@ -2124,7 +2138,8 @@ bool tc_attn_fused_is_faster(int Q, int heads, int d, int tokens, int rank, bool
 size_t tc_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens, int max_splits, bool rebuild) {
   if (Q <= 0 || heads <= 0 || tokens <= 0) return 0;
   const RowPlan plan = plan_rows(sm_count(), Q, heads, d, tokens, max_splits, rebuild);
-  return partial_bytes(plan.splits, Q, heads, d) + tail_bytes(sm_count(), d) + plan.kv_bytes + 512;
+  return partial_bytes(plan.splits, Q, heads, d) + tail_bytes(sm_count(), d) + plan.kv_bytes + 512 +
+         (rebuild ? failed_bytes(sm_count()) : 0);
 }
 
 // The read in two kernels per batch of heads: rows rebuilt into `workspace`, then attended.  Against the
@@ -2135,7 +2150,8 @@ int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_
                         const nkv_history* hist_k, const nkv_history* hist_v, const void* wk, const float* bias_k,
                         const void* wv, const float* bias_v, bool prepared_weights, const nkv_rope* rope,
                         const nkv_camera* cam_k, const nkv_camera* cam_v, float scale, void* out, float* lse,
-                        int32_t* status, int max_splits, void* workspace, cudaStream_t stream) {
+                        int32_t* status, int max_splits, void* workspace, long long selftest_budget,
+                        cudaStream_t stream) {
   const int N = hist_k->tokens, rank = hist_k->rank;
   NKV_REQUIRE(q_stride_head % 8 == 0 && q_stride_token % 8 == 0 && aligned16(q), NKV_ERR_INVALID,
               "queries must be 16-byte aligned with strides in multiples of 8 elements");
@@ -2158,6 +2174,8 @@ int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_
   const RowPlan plan = plan_rows(sms, Q, heads, d, N, max_splits, true);
   uint8_t* space = static_cast<uint8_t*>(workspace);
   space += (256 - (reinterpret_cast<uintptr_t>(space) & 255)) & 255;
+  int32_t* failed = reinterpret_cast<int32_t*>(space);
+  space += failed_bytes(sms);
   uint16_t* part_out = plan.splits > 1 ? reinterpret_cast<uint16_t*>(space) : static_cast<uint16_t*>(out);
   float* part_lse = plan.splits > 1
       ? reinterpret_cast<float*>(part_out + static_cast<size_t>(plan.splits) * Q * heads * d) : lse;
@@ -2188,12 +2206,12 @@ int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_
          rope != nullptr ? &batch_rope : nullptr, cam_k != nullptr ? &cams[0] : nullptr},
         {&hv, static_cast<const uint16_t*>(wv) + col0 * rank, bias_v + col0, nullptr, rows_v, d, head_stride,
          nullptr, cam_v != nullptr ? &cams[1] : nullptr}};
-    int rc = tc_decode(tensors, 2, N, hb * d, d, prepared_weights, false, status, sms, stream);
+    int rc = tc_decode(tensors, 2, N, hb * d, d, prepared_weights, false, status, failed, sms, selftest_budget, stream);
     if (rc == NKV_OK)
       rc = attend_rows(static_cast<const uint16_t*>(q) + h0 * q_stride_head, q_stride_token, q_stride_head, Q, hb,
                        heads, d, rows_k, rows_v, d, head_stride, N, scale, plan.splits, plan.tiles_per_split,
-                       max_splits > 0 ? nullptr : reinterpret_cast<float*>(tail), part_out + col0, part_lse + h0,
-                       status, stream);
+                       max_splits > 0 ? nullptr : reinterpret_cast<float*>(tail), failed,
+                       tc_decode_blocks(2, N, hb * d, sms), part_out + col0, part_lse + h0, status, stream);
     if (rc != NKV_OK) return rc;
   }
   return plan.splits > 1 ? merge_splits(part_out, part_lse, plan.splits, Q, heads, d, out, lse, stream) : NKV_OK;
@@ -2219,7 +2237,7 @@ int tc_attention_rows(const void* q, const void* k, const void* v, int64_t q_str
       ? reinterpret_cast<float*>(part_out + static_cast<size_t>(plan.splits) * Q * heads * d) : lse;
   float* tail = cut_tail ? reinterpret_cast<float*>(space + partial_bytes(plan.splits, Q, heads, d)) : nullptr;
   int rc = attend_rows(q, q_stride_token, q_stride_head, Q, heads, heads, d, k, v, kv_stride_token, kv_stride_head, N,
-                       scale, plan.splits, plan.tiles_per_split, tail, part_out, part_lse, status, stream);
+                       scale, plan.splits, plan.tiles_per_split, tail, nullptr, 0, part_out, part_lse, status, stream);
   if (rc == NKV_OK && plan.splits > 1) rc = merge_splits(part_out, part_lse, plan.splits, Q, heads, d, out, lse, stream);
   return rc;
 }

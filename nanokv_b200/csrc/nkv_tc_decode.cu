@@ -12,7 +12,9 @@
 //
 // Work is the list of (tensor, 256-token tile, 256-column tile) in that order; every cluster takes a
 // contiguous run of equal length, so the last wave is never emptier than one tile and a run expands
-// two or three token tiles.  No wait crosses clusters.
+// two or three token tiles.  No wait crosses clusters.  A wait that gives up leaves its site in the status
+// word and in the block's word of `failed` (which the attention behind a decode reads), and the rows that
+// were not finished become NaN.
 //
 // Bound: the epilogue's chain of latencies per 32 columns (accumulator read, staging, store; without it the
 // same launch takes 145 us), then the decoder stream into three 16 KB stages, all that 160 KB of latents
@@ -61,6 +63,9 @@ struct Params {
   int rope_pairs;             // rotation tables may be read two pairs (16 bytes) at a time
   int m_tiles, n_tiles, total;
   int32_t* status;
+  int32_t* failed;            // one word per block, written by every launch: 0, or the site of a wait that gave up; NULL: none
+  long long wait_budget;      // SM cycles per wait
+  int starve;                 // self-test: no decoder row is loaded, so that the waits for them run out
 };
 
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y,
@@ -125,17 +130,45 @@ __device__ __forceinline__ Run run_at(const Params& p, int w, int w_end) {
 
 // Acquire at block scope: what is handed over lies in shared memory or TMEM.  (A cluster-scope acquire also
 // gives up the first-level cache's lines, which hold the epilogue's bias, centre and rotation rows.)
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code) ? 1 : 0) != 0;
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                         long long budget) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code, budget) ? 1 : 0) != 0;
 }
 // the same for latents, which the other CTA's threads wrote
-__device__ __forceinline__ bool wait_all_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
-  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code) ? 1 : 0) != 0;
+__device__ __forceinline__ bool wait_all_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                                 long long budget) {
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code, budget) ? 1 : 0) != 0;
 }
 // Arrival that hands back tensor memory whose loads have completed: nothing written is published by it, so
 // it does not wait for the stores under way (a releasing arrival would: a tile's rows to L2, every tile).
 __device__ __forceinline__ void arrive_relaxed(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+}
+
+// history row of row `row` of this CTA's tile, or -1 past the end of the list
+__device__ __forceinline__ int token_at(const Params& p, const Run& r, uint32_t cta, int row) {
+  const int m = (r.m * 2 + static_cast<int>(cta)) * TM + row;
+  if (m >= p.n) return -1;
+  const Tensor& t = p.t[r.tensor];
+  const int tok = t.rows != nullptr ? __ldg(t.rows + m) : m;
+  return tok < 0 || tok >= t.h.tokens ? -1 : tok;
+}
+
+// After a wait gave up: NaN in this thread's row and column half of the tiles [w, w_end) it did not finish, so
+// that nothing unwritten looks like a result.
+__device__ __noinline__ void fill_unfinished(const Params& p, int w, int w_end, uint32_t cta, int row, int wg) {
+  const uint32_t nan2 = 0x7FC07FC0u;
+  for (; w < w_end; ++w) {
+    const Run r = run_at(p, w, w_end);
+    if (token_at(p, r, cta, row) < 0) continue;
+    const Tensor& t = p.t[r.tensor];
+    const int m = (r.m * 2 + static_cast<int>(cta)) * TM + row, first = r.nt0 * TN + wg * 128;
+    for (int col = first; col < min(first + 128, p.J); col += 8) {
+      const int head = col / p.D;
+      *reinterpret_cast<uint4*>(t.out + static_cast<size_t>(m) * t.row_stride + head * t.head_stride + (col - head * p.D)) =
+          make_uint4(nan2, nan2, nan2, nan2);
+    }
+  }
 }
 
 template <bool ROPE, bool CAM>
@@ -190,13 +223,13 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       bool ok = true;
       int s = 0, phase = 0;
       bool wrapped = false;        // the ring has been filled once: stages must be handed back first
-      for (int w = w_begin; w < w_end && ok;) {
+      for (int w = p.starve ? w_end : w_begin; w < w_end && ok;) {
         const Run r = run_at(p, w, w_end);
         const CUtensorMap* map = r.tensor ? &map_1 : &map_0;
         for (int k = 0; k < r.count && ok; ++k) {
           const int y = (r.nt0 + k) * TN + static_cast<int>(cta) * TM;
           for (int c = 0; c < nchunks; ++c) {
-            if (wrapped) ok = mbar_wait(&bars[FREE + s], phase ^ 1, abort_flag, 700 + s);
+            if (wrapped) ok = mbar_wait(&bars[FREE + s], phase ^ 1, abort_flag, 700 + s, p.wait_budget);
             if (!ok) break;
             // both halves land on the even CTA's barrier, whose MMA warp reads them
             if (cta == 0) mbar_arrive_expect_tx(&bars[FULL + s], 2 * CHUNK_BYTES);
@@ -224,11 +257,12 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
         const Run r = run_at(p, w, w_end);
         for (int k = 0; k < r.count && ok; ++k, ++tile) {
           const int b = tile & 1, use = tile >> 1;
-          if (use >= 1) ok = wait_all(&bars[ACC_FREE + b], (use - 1) & 1, abort_flag, 710 + b);
+          if (use >= 1) ok = wait_all(&bars[ACC_FREE + b], (use - 1) & 1, abort_flag, 710 + b, p.wait_budget);
           const uint32_t acc = tmem_base + b * TN;
           for (int c = 0; c < nchunks && ok; ++c) {
-            if (k == 0 && c % A_GROUP == 0) ok = wait_all_cluster(&bars[A_FULL + c / A_GROUP], seg & 1, abort_flag, 720 + c);
-            ok = ok && wait_all(&bars[FULL + s], phase, abort_flag, 730 + s);
+            if (k == 0 && c % A_GROUP == 0)
+              ok = wait_all_cluster(&bars[A_FULL + c / A_GROUP], seg & 1, abort_flag, 720 + c, p.wait_budget);
+            ok = ok && wait_all(&bars[FULL + s], phase, abort_flag, 730 + s, p.wait_budget);
             if (!ok) break;
             tc_fence_after();
             const uint64_t a_desc = make_smem_desc_sw128(a_base + c * CHUNK_BYTES);
@@ -257,14 +291,6 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
     uint8_t* stage = scratch + warp * 2048;
     bool ok = true;
     int tile = 0;                       // tiles whose epilogue is done or pending, in order
-    // this lane's token of a run (its row of the tile): history row, or -1 past the end of the list
-    auto token_of = [&](const Run& r) {
-      const int m = (r.m * 2 + static_cast<int>(cta)) * TM + row;
-      if (m >= p.n) return -1;
-      const Tensor& t = p.t[r.tensor];
-      const int tok = t.rows != nullptr ? __ldg(t.rows + m) : m;
-      return tok < 0 || tok >= t.h.tokens ? -1 : tok;
-    };
     // this thread's codes of its token, 16 bytes of every chunk, with their scales
     struct Codes { uint4 word[MAX_CHUNKS]; uint16_t scale[MAX_CHUNKS]; };
     auto fetch_codes = [&](const Run& r, int tok, Codes& in) {
@@ -428,7 +454,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
         }
         v = make_uint4(word[0], word[1], word[2], word[3]);
       };
-      ok = wait_all(&bars[ACC_FULL + b], use & 1, abort_flag, 740 + b);
+      ok = wait_all(&bars[ACC_FULL + b], use & 1, abort_flag, 740 + b, p.wait_budget);
       if (!ok) return;
       tc_fence_after();
       auto round = [&](int sub) {
@@ -499,27 +525,33 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       const bool starts = w < w_end && (w == w_begin || w % p.n_tiles == 0);
       if (starts) {
         next = run_at(p, w, w_end);
-        next_tok = token_of(next);
+        next_tok = token_at(p, next, cta, row);   // this lane's row of the tile
         next_crow = next_tok < 0 ? 0 : center_row_of(p.t[next.tensor].h, next_tok);
         Codes codes;
         fetch_codes(next, next_tok, codes);
         // the latents in shared memory are free once the previous run's last tile is complete; the new
         // ones go in before that tile's epilogue, so that the MMAs of this run start under it
-        if (w > w_begin) ok = wait_all(&bars[ACC_FULL + (tile & 1)], (tile >> 1) & 1, abort_flag, 750);
+        if (w > w_begin) ok = wait_all(&bars[ACC_FULL + (tile & 1)], (tile >> 1) & 1, abort_flag, 750, p.wait_budget);
         if (!ok) break;
         expand(next, codes);
       }
       if (w > w_begin) epilogue(run, (w - 1) % p.n_tiles, tok, crow);
       if (starts) { run = next; tok = next_tok; crow = next_crow; }
     }
+    if (!ok) fill_unfinished(p, w_begin + tile, w_end, cta, row, wg);
   }
   tc_fence_before();
   __syncthreads();
   // neither CTA leaves while the other may still arrive on its barriers or read its operands
   cluster_sync_all();
   if (warp == 9) tmem_dealloc_pair(tmem_base, 512);
-  if (tid == 0 && *abort_flag && p.status) atomicCAS(p.status, 0, *abort_flag);
+  if (tid == 0) {
+    if (p.failed != nullptr) p.failed[blockIdx.x] = *abort_flag;
+    if (*abort_flag && p.status) atomicCAS(p.status, 0, *abort_flag);
+  }
 }
+
+int tiles_of(int count, int n, int J) { return count * ceil_div(n, 2 * TM) * ceil_div(J, TN); }
 
 size_t smem_bytes(int nchunks, int stages) {
   return 1024 + META + static_cast<size_t>(nchunks + stages) * CHUNK_BYTES + SCRATCH;
@@ -533,8 +565,13 @@ bool tc_decode_supported(const nkv_history& h, int J) {
          ((reinterpret_cast<uintptr_t>(h.codes) | reinterpret_cast<uintptr_t>(h.centers)) & 15) == 0;
 }
 
+int tc_decode_blocks(int count, int n, int J, int sms) {
+  const int total = tiles_of(count, n, J);
+  return 2 * (total < sms / 2 ? total : sms / 2);
+}
+
 int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool w_perm, bool round_bias,
-              int32_t* status, int sms, cudaStream_t stream) {
+              int32_t* status, int32_t* failed, int sms, long long selftest_budget, cudaStream_t stream) {
   if (n == 0) return NKV_OK;
   Params p{};
   CUtensorMap maps[2];
@@ -574,11 +611,13 @@ int tc_decode(const DecodeTensor* tensors, int count, int n, int J, int D, bool 
   const size_t smem = smem_bytes(p.nchunks, p.nstages);
   p.m_tiles = ceil_div(n, 2 * TM);
   p.n_tiles = ceil_div(J, TN);
-  p.total = count * p.m_tiles * p.n_tiles;
+  p.total = tiles_of(count, n, J);
   p.status = status;
-  const int pairs = p.total < sms / 2 ? p.total : sms / 2;
+  p.failed = failed;
+  p.starve = selftest_budget > 0 ? 1 : 0;
+  p.wait_budget = selftest_budget > 0 ? selftest_budget : WAIT_BUDGET_CYCLES;
   cudaLaunchConfig_t config{};
-  config.gridDim = dim3(2 * pairs);
+  config.gridDim = dim3(tc_decode_blocks(count, n, J, sms));
   config.blockDim = dim3(THREADS);
   config.dynamicSmemBytes = smem;
   config.stream = stream;

@@ -204,9 +204,9 @@ def decode_rows(view: HistoryView, decoder, mean, *, rows=None, dtype=None) -> t
     if rows is not None:
         rows = rows.to(dtype=torch.int32).contiguous()
     struct = view.struct()
-    _lib.check(_lib.library().nkv_decode_rows(
+    _lib.check(_lib.library().nkv_decode_rows_status(
         ctypes.byref(struct), _ptr(rows), n, _ptr(decoder), dtype_code(decoder.dtype), _ptr(mean),
-        J, _ptr(out), dtype_code(dtype), _stream(device)))
+        J, _ptr(out), dtype_code(dtype), _ptr(status_word(device)), _stream(device)))
     return out
 
 
@@ -221,7 +221,7 @@ _STATUS_WORDS: dict = {}
 
 
 def status_word(device: torch.device) -> torch.Tensor:
-    """The per-device int32 word the fused read reports into when the caller passes none."""
+    """The per-device int32 word that a row decode, and a read whose caller passes none, report into."""
     key = torch.device(device)
     if key not in _STATUS_WORDS:
         _STATUS_WORDS[key] = torch.zeros(1, dtype=torch.int32, device=key)
@@ -229,7 +229,7 @@ def status_word(device: torch.device) -> torch.Tensor:
 
 
 def check_status(device=None) -> None:
-    """Synchronise and raise if a fused read on ``device`` (default: every device used so far) left a
+    """Synchronise and raise if a read or a row decode on ``device`` (default: every device used so far) left a
     status behind: a bounded device-side wait that gave up, or a row whose scores left the softmax
     window.  The word is cleared.  Results of launches since the last check are only to be trusted
     after this returns."""
