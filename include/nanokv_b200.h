@@ -406,6 +406,7 @@ int nkv_attn_codec_pos(const void* q, int dtype, int64_t q_stride_token, int64_t
  * 640.  `splits`: upper bound of the history splits, 0: the library's choice.
  * nkv_attn_codec_rows_workspace_bytes is 0 where this form does not apply (rank above 640 in bf16, head
  * widths other than 64 and 128); the fp32 form takes no positional restore and 16-byte aligned queries.
+ * out must be 16-byte aligned.
  */
 size_t nkv_attn_codec_rows_workspace_bytes(int dtype, int Q, int heads, int dk, int dv, int tokens,
                                            int rank, int group, int splits);
@@ -450,8 +451,8 @@ int nkv_attention_lse(const void* q, const void* k, const void* v, int dtype,
                       void* out, float* lse, void* stream);
 
 /*
- * The same on the tensor cores, for bf16 rows with d == dv in {64, 128}, N > 0, 16-byte aligned rows
- * and strides in multiples of 8 elements.  status_word as for nkv_attn_codec.  workspace:
+ * The same on the tensor cores, for bf16 rows with d == dv in {64, 128}, N > 0, 16-byte aligned rows and
+ * out, and strides in multiples of 8 elements.  status_word as for nkv_attn_codec.  workspace:
  * nkv_attention_lse_workspace_bytes bytes for history splits, or NULL (one split).
  */
 size_t nkv_attention_lse_workspace_bytes(int Q, int heads, int d, int N);

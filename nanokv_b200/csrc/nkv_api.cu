@@ -469,6 +469,8 @@ static int attn_codec_rows(const void* q, int dtype, int64_t q_stride_token, int
   NKV_REQUIRE(splits >= 0 && splits <= 16, NKV_ERR_INVALID, "attn_codec_rows: splits=%d (0..16)", splits);
   NKV_REQUIRE(reads_by_rows(dtype, dk, dv, hist_k->rank, hist_k->group), NKV_ERR_UNSUPPORTED,
               "attn_codec_rows: dtype %d, dk=%d dv=%d rank=%d group=%d", dtype, dk, dv, hist_k->rank, hist_k->group);
+  NKV_REQUIRE((reinterpret_cast<uintptr_t>(out) & 15) == 0, NKV_ERR_INVALID,
+              "attn_codec_rows: results must be 16-byte aligned");
   NKV_REQUIRE(workspace && workspace_bytes >= nkv_attn_codec_rows_workspace_bytes(
                                dtype, Q, heads, dk, dv, hist_k->tokens, hist_k->rank, hist_k->group, splits),
               NKV_ERR_INVALID, "attn_codec_rows: workspace of %zu bytes is too small", workspace_bytes);
@@ -560,6 +562,8 @@ int nkv_attention_lse_bf16(const void* q, const void* k, const void* v, int64_t 
   NKV_REQUIRE(tc_attention_rows_supported(q, k, v, q_stride_token, q_stride_head, kv_stride_token, kv_stride_head, d, dv),
               NKV_ERR_INVALID, "attention_lse_bf16: needs d == dv in {64, 128}, 16-byte aligned rows and strides in "
               "multiples of 8 elements (d=%d dv=%d)", d, dv);
+  NKV_REQUIRE((reinterpret_cast<uintptr_t>(out) & 15) == 0, NKV_ERR_INVALID,
+              "attention_lse_bf16: results must be 16-byte aligned");
   NKV_REQUIRE(workspace == nullptr || workspace_bytes >= nkv_attention_lse_workspace_bytes(Q, heads, d, N),
               NKV_ERR_INVALID, "attention_lse_bf16: workspace of %zu bytes is too small", workspace_bytes);
   return tc_attention_rows(q, k, v, q_stride_token, q_stride_head, kv_stride_token, kv_stride_head, Q, N, heads, d,
