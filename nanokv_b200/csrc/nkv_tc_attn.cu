@@ -2027,7 +2027,19 @@ RowPlan plan_rows(int sms, int Q, int heads, int d, int tokens, int max_splits, 
 
 size_t failed_bytes(int sms) { return (static_cast<size_t>(sms) * 4 + 255) / 256 * 256; }   // a word per decode block
 
-size_t tail_bytes(int sms, int d) { return static_cast<size_t>(2 * sms) * (NQ * QT) * (d + 1) * 4; }
+// fp32 partials of the left-over units of a launch over `heads` heads: two slots for each block that takes a run
+size_t tail_bytes(int sms, int Q, int heads, int tokens, int d) {
+  const Tail t = plan_tail(sms, static_cast<long long>(ceil_div(Q, NQ * QT)) * heads, ceil_div(tokens, TOK));
+  return (static_cast<size_t>(2 * t.blocks) * (NQ * QT) * (d + 1) * 4 + 255) / 256 * 256;
+}
+
+// the same for all batches of a plan (the last one may have fewer heads); none where the caller bounds the splits
+size_t tail_bytes(const RowPlan& plan, int sms, int Q, int heads, int tokens, int d, int max_splits) {
+  if (max_splits > 0) return 0;
+  const size_t full = tail_bytes(sms, Q, plan.heads, tokens, d);
+  const size_t last = tail_bytes(sms, Q, heads - plan.heads * (plan.batches - 1), tokens, d);
+  return full > last ? full : last;
+}
 
 size_t partial_bytes(int splits, int Q, int heads, int d) {
   const size_t bytes = splits > 1 ? static_cast<size_t>(splits) * Q * heads * (static_cast<size_t>(d) * 2 + 4) : 0;
@@ -2076,13 +2088,13 @@ int attend_rows(const void* q, int64_t q_stride_token, int64_t q_stride_head, in
   const int sms = sm_count();
   p.cons = 1;
   p.groups = p.units < sms ? p.units : sms;
-  if (tail != nullptr && splits == 1) {
+  if (tail != nullptr) {
     const Tail t = plan_tail(sms, p.units, p.tiles);
     p.tail_units = t.units;
     p.tail_blocks = t.blocks;
     if (!t.whole) p.groups = t.blocks;
     p.tail_out = tail;
-    p.tail_lse = tail + static_cast<size_t>(2 * sms) * (NQ * QT) * d;
+    p.tail_lse = tail + static_cast<size_t>(2 * t.blocks) * (NQ * QT) * d;
   }
   p.scale_log2 = scale * 1.4426950408889634f;
   p.wait_budget = 1ll << 31;
@@ -2138,7 +2150,8 @@ bool tc_attn_fused_is_faster(int Q, int heads, int d, int tokens, int rank, bool
 size_t tc_attn_rows_workspace_bytes(int Q, int heads, int d, int tokens, int max_splits, bool rebuild) {
   if (Q <= 0 || heads <= 0 || tokens <= 0) return 0;
   const RowPlan plan = plan_rows(sm_count(), Q, heads, d, tokens, max_splits, rebuild);
-  return partial_bytes(plan.splits, Q, heads, d) + tail_bytes(sm_count(), d) + plan.kv_bytes + 512 +
+  return partial_bytes(plan.splits, Q, heads, d) + tail_bytes(plan, sm_count(), Q, heads, tokens, d, max_splits) +
+         plan.kv_bytes + 512 +
          (rebuild ? failed_bytes(sm_count()) : 0);
 }
 
@@ -2180,7 +2193,7 @@ int tc_attn_by_rows_run(const void* q, int64_t q_stride_token, int64_t q_stride_
   float* part_lse = plan.splits > 1
       ? reinterpret_cast<float*>(part_out + static_cast<size_t>(plan.splits) * Q * heads * d) : lse;
   uint8_t* tail = space + partial_bytes(plan.splits, Q, heads, d);
-  uint16_t* rows_k = reinterpret_cast<uint16_t*>(tail + (tail_bytes(sms, d) + 255) / 256 * 256);
+  uint16_t* rows_k = reinterpret_cast<uint16_t*>(tail + tail_bytes(plan, sms, Q, heads, N, d, max_splits));
   uint16_t* rows_v = rows_k + static_cast<size_t>(plan.heads) * N * d;
   for (int h0 = 0; h0 < heads; h0 += plan.heads) {
     const int hb = heads - h0 < plan.heads ? heads - h0 : plan.heads;

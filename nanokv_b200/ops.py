@@ -285,14 +285,21 @@ def attn_codec(q, view_k: HistoryView, view_v: HistoryView, wk, bias_k, wv, bias
     if nbytes and not lib.nkv_attn_codec_rows_is_faster(dtype_code(q.dtype), Q, H, dk, dv, view_k.tokens, view_k.rank,
                                                         view_k.group, int(positional)):
         nbytes = 0
-    read = lib.nkv_attn_codec_rows if nbytes else lib.nkv_attn_codec_pos
+    workspace = None
     if nbytes:
+        try:
+            workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            pass      # the other forms hold no rows: slower, but they need next to no scratch
+    if workspace is not None:
+        read = lib.nkv_attn_codec_rows
         splits = 0 if splits is None else splits
     else:
+        read = lib.nkv_attn_codec_pos
         if splits is None:
             splits = default_splits(view_k.tokens) if q.dtype == torch.bfloat16 else 1
         nbytes = lib.nkv_attn_codec_workspace_bytes(Q, H, dv, splits)
-    workspace = torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
+        workspace = torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
     rope_struct = None
     if rope is not None:
         if rope.positions.numel() < view_k.tokens:
@@ -442,7 +449,10 @@ def attention_lse(q, k, v, *, scale: float):
         out = torch.empty(Q, H, dv, dtype=q.dtype, device=device)
         lse = torch.empty(Q, H, dtype=torch.float32, device=device)
         nbytes = lib.nkv_attention_lse_workspace_bytes(Q, H, d, N)
-        workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        try:
+            workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:   # without scratch no unit is cut
+            workspace, nbytes = None, 0
         _lib.check(lib.nkv_attention_lse_bf16(
             _ptr(q), _ptr(k), _ptr(v), q.stride(0), q.stride(1), H * d, d, Q, N, H, d, dv,
             float(scale), _ptr(out), _ptr(lse), _ptr(status_word(device)), _ptr(workspace), nbytes, _stream(device)))
