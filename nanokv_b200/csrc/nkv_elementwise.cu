@@ -1039,7 +1039,7 @@ head_linear_mma_kernel(const uint16_t* x, long long stride_row, long long stride
         }
       }
   __syncwarp();
-  const int opieces = dout_pad / 8, held = NPAIRS * 2;
+  const int opieces = dout_pad / 8, held = dout / 8;   // columns past dout are zero whatever the inputs (0 * inf is not)
   for (int i = lane; i < 32 * opieces; i += 32) {
     const int r = warp * 32 + i / opieces, c = i % opieces;
     if (row0 + r < rows)
