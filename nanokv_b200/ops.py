@@ -272,6 +272,8 @@ def attn_codec(q, view_k: HistoryView, view_v: HistoryView, wk, bias_k, wv, bias
     _require_cuda(out, lse)
     if status is None:   # a launch always has somewhere to report a wait that gave up: check_status()
         status = status_word(device)
+    if splits is not None and not 1 <= splits <= 16:
+        raise ValueError(f"splits must be in 1..16; got {splits}")
     sk, sv = view_k.struct(), view_v.struct()
     lib = _lib.library()
     # rows rebuilt in scratch memory a batch of heads at a time, then attended; 0 bytes: this form does
