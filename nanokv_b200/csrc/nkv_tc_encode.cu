@@ -246,7 +246,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         const int chunks = (C + 31) / 32, middle = (chunks + 1) / 2;
         const int first = wg == 0 ? 0 : middle, last = wg == 0 ? middle : chunks;
         float best = INFINITY;
-        int best_i = 0x7fffffff;
+        int best_i = 0;    // a row without a finite distance: centre 0, as in the CUDA-core kernel, never an id past C
 #pragma unroll 1
         for (int cc = first; cc < last; ++cc) {
           const int col = cc * 32, acc = col / p.NB;
