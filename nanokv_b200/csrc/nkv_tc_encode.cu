@@ -83,6 +83,15 @@ struct Ring {
   }
 };
 
+// Every wait of a whole warp gives one answer for all its lanes: what follows (tensor-memory loads, cluster
+// barriers, __syncwarp) takes converged warps, also when a wait gives up.
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code) ? 1 : 0) != 0;
+}
+__device__ __forceinline__ bool wait_all_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code) ? 1 : 0) != 0;
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -173,8 +182,8 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     Ring at;
     for (int c = 0; c < nchunks && ok; ++c, at.advance(nst)) {
       const int s = at.stage;
-      ok = mbar_wait(&bars[TMA_FULL + s], at.phase, abort_flag, 410 + s);
-      if (ok && !ASSIGN) ok = mbar_wait(&bars[A_FULL + s], at.phase, abort_flag, 412 + s);
+      ok = wait_all(&bars[TMA_FULL + s], at.phase, abort_flag, 410 + s);
+      if (ok && !ASSIGN) ok = wait_all(&bars[A_FULL + s], at.phase, abort_flag, 412 + s);
       if (!ok) break;
       tc_fence_after();
       const uint32_t stage = smem_base + s * stage_bytes;
@@ -207,7 +216,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       Ring at;
       for (int i = 0; i < nchunks && ok; ++i, at.advance(nst)) {
         const int s = at.stage;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars[TMA_FULL + s], at.phase, abort_flag, 420 + s) ? 1 : 0) != 0;
+        ok = wait_all(&bars[TMA_FULL + s], at.phase, abort_flag, 420 + s);
         if (!ok) break;
         const uint8_t* stage = smem + s * stage_bytes;
         if (i < p.a_chunks) {
@@ -237,8 +246,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           if (item < 2 * C) cn_part[item] = cs[k];
         }
         mbar_arrive(&bars[SIDE_READY]);
-        ok = mbar_wait(&bars[SIDE_READY], 0, abort_flag, 430) &&
-             mbar_wait(&bars[ACC_DONE], 0, abort_flag, 431);
+        ok = wait_all(&bars[SIDE_READY], 0, abort_flag, 430) && wait_all(&bars[ACC_DONE], 0, abort_flag, 431);
       }
       if (ok) {
         tc_fence_after();
@@ -267,7 +275,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           cand_i[row] = best_i;
           mbar_arrive(&bars[CAND_READY]);
         } else {
-          ok = mbar_wait(&bars[CAND_READY], 0, abort_flag, 432);
+          ok = wait_all(&bars[CAND_READY], 0, abort_flag, 432);
           if (ok) {
             if (cand_d[row] < best) { best = cand_d[row]; best_i = cand_i[row]; }
             const int t = m0 + row;
@@ -331,7 +339,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           }
         }
         fetch(buf, i + 2);
-        if (i >= nst) ok = __all_sync(0xffffffffu, mbar_wait(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 440 + s) ? 1 : 0) != 0;
+        if (i >= nst) ok = wait_all(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 440 + s);
         if (!ok) return;
         at.advance(nst);
         uint8_t* stage = smem + s * stage_bytes + r0 * 128 + ((piece ^ (r0 & 7)) << 4);
@@ -347,7 +355,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         step(0, i);
         if (i + 1 < nchunks && ok) step(1, i + 1);
       }
-      if (ok) ok = mbar_wait(&bars[ACC_DONE], 0, abort_flag, 450);
+      if (ok) ok = wait_all(&bars[ACC_DONE], 0, abort_flag, 450);
       if (ok && QUANT) {
         // ---- quantise + pack from TMEM.  Pass 1: |max| of the bf16-rounded coefficients of this
         // thread's column chunks; the two warpgroups, then the two column-half CTAs, combine.
@@ -365,7 +373,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         }
         xn_part[wg * 128 + row] = amax;
         mbar_arrive(&bars[SIDE_READY]);
-        ok = mbar_wait(&bars[SIDE_READY], 0, abort_flag, 451);
+        ok = wait_all(&bars[SIDE_READY], 0, abort_flag, 451);
         if (ok) {
           amax = fmaxf(xn_part[row], xn_part[128 + row]);
           if (joined) {
@@ -376,7 +384,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                 mbar_arrive_cluster(map_to_cta(smem_u32(&bars[PEER_READY]), peer));
               }
             }
-            ok = mbar_wait_cluster(&bars[PEER_READY], 0, abort_flag, 452);
+            ok = wait_all_cluster(&bars[PEER_READY], 0, abort_flag, 452);
             if (ok)
               for (int peer = 0; peer < p.column_parts; ++peer)
                 if (peer != part) amax = fmaxf(amax, peer_max[peer * 128 + row]);
