@@ -1558,11 +1558,12 @@ merge_tail_kernel(Params p) {
     nan = nan || l != l;
     top = fmaxf(top, l);
   }
+  const float origin = isfinite(top) ? top : 0.f;   // all of them -inf: weights of zero, not of -inf - -inf
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, weight = 0.f;
 #pragma unroll 4
   for (int b = b0; b < b_end; ++b) {
     const size_t at = slot_of(b);
-    const float w = expf(lses[at] - top);
+    const float w = expf(lses[at] - origin);
     const float4 lo = *reinterpret_cast<const float4*>(p.tail_out + (at + row) * D + col);
     const float4 hi = *reinterpret_cast<const float4*>(p.tail_out + (at + row) * D + col + 4);
     weight += w;
@@ -1571,12 +1572,12 @@ merge_tail_kernel(Params p) {
     acc[4] = fmaf(w, hi.x, acc[4]); acc[5] = fmaf(w, hi.y, acc[5]);
     acc[6] = fmaf(w, hi.z, acc[6]); acc[7] = fmaf(w, hi.w, acc[7]);
   }
-  const float inv = 1.0f / weight;
+  const float inv = weight == 0.f ? 1.0f : 1.0f / weight;
   const size_t out_row = static_cast<size_t>(q) * p.out_heads + un.head;
   *reinterpret_cast<uint4*>(p.out + out_row * D + col) =
       make_uint4(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv),
                  pack_bf16x2(acc[4] * inv, acc[5] * inv), pack_bf16x2(acc[6] * inv, acc[7] * inv));
-  if (col == 0) p.lse[out_row] = nan ? __int_as_float(0x7fc00000) : top + logf(weight);
+  if (col == 0) p.lse[out_row] = nan ? __int_as_float(0x7fc00000) : origin + logf(weight);
 }
 
 __global__ void fill_empty_kernel(uint16_t* out, float* lse, size_t rows, int d) {
