@@ -177,8 +177,8 @@ int nkv_quant_pack(const void* coeff, int coeff_dtype, int S, int r, int group, 
  * nkv_quant_pack of those coefficients, written to codes [S,r/2] and scales [S,r/group].
  * Reference: the second half of encode_tensor, MGM/nanokv_codec.py:345-351, LB/lingbot_v2_kv_codec.py:280-287.
  * With bf16 operands and one scale per token (group == r, r a multiple of 64 that tiles over at most
- * two column parts) one kernel does all of it: the coefficients stay in tensor memory, the per-token
- * maximum crosses the two column-half thread blocks through their shared memory, and `workspace`
+ * two column parts of at most 512) one kernel does all of it: the coefficients stay in tensor memory, the
+ * per-token maximum crosses the thread blocks of a token tile (up to eight) through their shared memory, and `workspace`
  * is not touched.  Otherwise it runs nkv_project into `workspace` (S * r elements of the encoder
  * dtype) followed by nkv_quant_pack.  Same bytes either way.
  */

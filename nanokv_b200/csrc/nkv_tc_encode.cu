@@ -1,7 +1,7 @@
 // Encoder GEMMs on tcgen05: nearest-centre assignment and residual projection.
 //
 // Both are [128 tokens x K=J] x [N x K]^T tiles with fp32 accumulators in TMEM,
-// K streamed 64 columns at a time through a shared-memory ring of up to four stages.
+// K streamed 64 columns at a time through a shared-memory ring of up to eight stages.
 //   assign : A = token rows (TMA), B = centre rows (TMA), N = C <= 512.  While
 //            a stage is resident the compute warps accumulate ||x||^2 and
 //            ||c||^2 from the same tiles; the epilogue evaluates
@@ -10,8 +10,8 @@
 //            the swizzled operand layout; B = encoder rows (TMA); the epilogue
 //            rounds once to bf16.
 //   project + quantise: the same GEMM, but the epilogue keeps the coefficients in TMEM, takes the
-//            token's absolute maximum over the whole rank row (the two column-half CTAs of a token
-//            tile form a cluster and swap their half-row maxima through each other's shared
+//            token's absolute maximum over the whole rank row (the up to eight column parts of a token
+//            tile form a cluster and swap the maxima of their columns through each other's shared
 //            memory), quantises to INT4, packs two codes per byte and writes codes and scale to
 //            their place in the history: the bf16 coefficients never travel to HBM.
 // A CTA covers up to 512 output columns as 1 or 2 accumulators of NB <= 256.
@@ -209,7 +209,9 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     // the swizzled stores touch whole lines
     const int r0 = tid >> 3, piece = tid & 7;
     if (ASSIGN) {
-      // ---- squared norms from the resident tiles
+      // ---- squared norms from the resident tiles.  Neighbouring threads read half-rows 64 bytes apart, four
+      // of which share their banks.  The order in which a half-row's sixteen squares are added is what the stored
+      // ids were made with, so a layout without the conflicts has to keep it.
       const int C = p.n_total;
       // partials of half a token row, and of half-rows tid + 256 k of the centres
       float xs = 0.f, cs[4] = {0.f, 0.f, 0.f, 0.f};
@@ -358,7 +360,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       if (ok) ok = wait_all(&bars[ACC_DONE], 0, abort_flag, 450);
       if (ok && QUANT) {
         // ---- quantise + pack from TMEM.  Pass 1: |max| of the bf16-rounded coefficients of this
-        // thread's column chunks; the two warpgroups, then the two column-half CTAs, combine.
+        // thread's column chunks; the two warpgroups, then the column parts' CTAs, combine.
         tc_fence_after();
         const int nc = p.NACC * p.NB;
         const int tok = m0 + row;
