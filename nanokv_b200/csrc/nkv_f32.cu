@@ -446,6 +446,38 @@ attn_rows_f32_kernel(RowAttn a) {
   }
 }
 
+// Merge of the history splits: thread = (row, 4 columns).  Weights against the largest LSE, one logarithm: the
+// pairwise fold of lse_merge rounds the LSE once per part (3,102 tokens in 16 parts: 4.9e-7 rms from float64,
+// where one part has 3.2e-7).
+__global__ void __launch_bounds__(256)
+merge_splits_kernel(const float* part_out, const float* part_lse, int splits, long long rows, int d, float* out,
+                    float* lse_out) {
+  const int per_row = d / 4;
+  const long long idx = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (idx >= rows * per_row) return;
+  const long long row = idx / per_row;
+  const int col = static_cast<int>(idx - row * per_row) * 4;
+  float top = -INFINITY;
+  bool nan = false;
+  for (int z = 0; z < splits; ++z) {
+    const float l = part_lse[z * rows + row];
+    nan = nan || l != l;
+    top = fmaxf(top, l);
+  }
+  const float origin = isfinite(top) ? top : 0.f;   // all of them -inf: weights of zero
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, weight = 0.f;
+  for (int z = 0; z < splits; ++z) {
+    const float w = expf(part_lse[z * rows + row] - origin);
+    const float4 v = *reinterpret_cast<const float4*>(part_out + (z * rows + row) * d + col);
+    weight += w;
+    acc[0] = fmaf(w, v.x, acc[0]); acc[1] = fmaf(w, v.y, acc[1]);
+    acc[2] = fmaf(w, v.z, acc[2]); acc[3] = fmaf(w, v.w, acc[3]);
+  }
+  const float inv = weight == 0.f ? 1.f : 1.0f / weight;
+  *reinterpret_cast<float4*>(out + row * d + col) = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
+  if (col == 0) lse_out[row] = nan ? __int_as_float(0x7fc00000) : origin + logf(weight);
+}
+
 template <class K>
 int allow_smem(K kernel) {
   NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_FLOATS * 4));
@@ -580,13 +612,10 @@ int f32_attn_by_rows_run(const float* q, int64_t q_stride_token, int64_t q_strid
     if (rc != NKV_OK) return rc;
   }
   if (plan.splits == 1) return NKV_OK;
-  const void* outs[16];
-  const float* lses[16];
-  for (int z = 0; z < plan.splits; ++z) {
-    outs[z] = part_out + z * rows * d;
-    lses[z] = part_lse + z * rows;
-  }
-  return lse_merge(outs, lses, plan.splits, static_cast<int64_t>(rows), d, NKV_F32, out, lse, stream);
+  merge_splits_kernel<<<static_cast<unsigned>((rows * (d / 4) + 255) / 256), 256, 0, stream>>>(
+      part_out, part_lse, plan.splits, static_cast<long long>(rows), d, out, lse);
+  NKV_LAUNCH_CHECK("merge_splits_kernel");
+  return NKV_OK;
 }
 
 }  // namespace nkv
