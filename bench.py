@@ -569,9 +569,10 @@ def run_ours(args) -> dict:
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "peak_source": f"bf16_tflops_sustained of {peak_kind}",
                      "launch_ms": kernel_s * 1e3, "flops_per_launch": flops_launch,
-                     # DRAM bytes of one launch over the full layer from an ncu capture of this
-                     # kernel, when one is on record (per-rank shards are not captured separately)
-                     "traffic": (measured_traffic("attn_rows_kernel", shape.name)
+                     # DRAM bytes of all launches over the full layer (decode, attention, merge of each
+                     # batch of heads) from an ncu capture, when one is on record (per-rank shards are
+                     # not captured separately)
+                     "traffic": (measured_traffic("decode_gemm_kernel + attn_rows_kernel", shape.name)
                                  if world == 1 and not args.history_frames else None)},
         "encode": encode,
         "clocks": clocks,
