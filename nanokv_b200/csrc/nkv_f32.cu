@@ -6,11 +6,11 @@
 // reproduce the rounding points of the bf16 path, which the test-suite uses to cross-check the
 // tensor-core kernels at full size.
 //
-// A block owns a 64 x 64 tile of the product.  The calls of this configuration have few tiles (96 for a
-// projection of 2,048 tokens) and long sums, so the block's four groups of 64 threads take a quarter of K
-// each, with operand tiles and barriers of their own (the next tile's operands in registers while one is
-// multiplied), and add their sums in order at the end.  Multiply-adds are packed pairs, a thread owns
-// 8 x 8 of the tile.
+// Two forms of the GEMM, both with packed multiply-adds and the next step's operands in registers while one is
+// multiplied.  Assignment and projection (gemm_ordered): every sum is one chain of fused multiply-adds in the
+// order of K, because what they give is stored -- ids, and codes that another order would move now and then.
+// Row decode (gemm64): 64 x 64 of the product per block; its four groups of 64 threads take a quarter of K each,
+// with operand tiles and barriers of their own, and add their sums in order at the end.
 #include "nkv_internal.h"
 
 namespace nkv {
@@ -55,15 +55,11 @@ bool vector_rows(const void* base, int dtype, int K) {
   return K % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & (dtype == NKV_F32 ? 15 : 7)) == 0;
 }
 
-__device__ __forceinline__ float sumsq4(float4 v, float acc) {
-  return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, acc))));
-}
-
 // The block's 64 x 64 tile of A B^T over K: load_a(k) / load_b(k) give elements k .. k + 3 of row
-// (thread number in its group) of either operand.  `a_norm` / `b_norm` collect the squares of what this
-// thread loaded.  Afterwards sums(row, column) of the tile lie in `sm` as GROUPS partial tiles.
-template <bool NORMS, class LA, class LB>
-__device__ __forceinline__ void gemm64(float* sm, int K, LA load_a, LB load_b, float& a_norm, float& b_norm) {
+// (thread number in its group) of either operand.  Afterwards sums(row, column) of the tile lie in `sm` as
+// GROUPS partial tiles.
+template <class LA, class LB>
+__device__ __forceinline__ void gemm64(float* sm, int K, LA load_a, LB load_b) {
   const int g = threadIdx.x / GROUP_THREADS, t = threadIdx.x % GROUP_THREADS;
   const int tx = t & 7, ty = t >> 3;
   const int chunks = (K + BK - 1) / BK;
@@ -93,10 +89,6 @@ __device__ __forceinline__ void gemm64(float* sm, int K, LA load_a, LB load_b, f
       for (int i = 0; i < 4; ++i) {
         as[(4 * j + i) * TILE + t] = av[i];
         bs[(4 * j + i) * TILE + t] = bv[i];
-      }
-      if (NORMS) {
-        a_norm = sumsq4(ra[j], a_norm);
-        b_norm = sumsq4(rb[j], b_norm);
       }
     }
     asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(GROUP_THREADS) : "memory");
@@ -139,74 +131,160 @@ __device__ __forceinline__ float4 tile_sum(const float* sm, int row, int c) {
   return s;
 }
 
+// ------------------------------------------------------- sums in the order of K
+// TM x 64 of A B^T per block: thread (ty, tx) owns TM / 16 rows x 4 columns, each sum one chain over K.  A step takes
+// 32 columns of K through one of two buffers; load_a(k) / load_b(k) give elements k .. k + 3 of row threadIdx.x % TM
+// resp. % 64.  Bound: 4,096 multiply-adds per column of K and 64 x 64 tile, 32 cycles of an SM.  us, 1,536 columns,
+// projection to 192 / assignment to 16 centres, against K cut in four as in gemm64: 300 tokens 109 / 90 (102 / 83),
+// 2,048 142 / 94 (103 / 84), 4,096 178 / 95 (160 / 84).
+constexpr int STEP = 32;
+template <int TM>
+constexpr int ORDERED_FLOATS = 2 * STEP * (TM + TILE);
+
+// NORMS: threads 0 .. TM - 1 / 128 .. 191 also square row threadIdx.x of A / threadIdx.x - 128 of B, elements
+// j, j + 4, j + 8 ... in chain j.
+template <int TM, bool NORMS, class LA, class LB>
+__device__ __forceinline__ void gemm_ordered(float* sm, int K, LA load_a, LB load_b, float (&sums)[TM / 16][4],
+                                             float (&norm)[4]) {
+  constexpr int ROWS = TM / 16, NA = TM * STEP / 4 / THREADS, NB = TILE * STEP / 4 / THREADS;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  const int ra = t % TM, ka = t / TM * 4, rb = t % TILE, kb = t / TILE * 4;   // first piece loaded; the others further along K
+  uint64_t acc[ROWS][2];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) acc[i][0] = acc[i][1] = 0ull;
+  float4 va[NA], vb[NB];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < NA; ++i) va[i] = load_a(k0 + ka + i * (STEP / NA));
+#pragma unroll
+    for (int i = 0; i < NB; ++i) vb[i] = load_b(k0 + kb + i * (STEP / NB));
+  };
+  fetch(0);
+  int buffer = 0;
+  for (int k0 = 0; k0 < K; k0 += STEP, buffer ^= 1) {
+    float* as = sm + buffer * STEP * (TM + TILE);
+    float* bs = as + STEP * TM;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      const float v[4] = {va[i].x, va[i].y, va[i].z, va[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) as[(ka + i * (STEP / NA) + j) * TM + ra] = v[j];
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const float v[4] = {vb[i].x, vb[i].y, vb[i].z, vb[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bs[(kb + i * (STEP / NB) + j) * TILE + rb] = v[j];
+    }
+    __syncthreads();      // one per step: whoever fills this buffer next is behind the barrier of the step between
+    if (k0 + STEP < K) fetch(k0 + STEP);
+#pragma unroll
+    for (int k = 0; k < STEP; ++k) {
+      float a[ROWS];
+      if constexpr (ROWS == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(as + k * TM + ty * 4);
+        a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
+      } else {
+        const float2 v = *reinterpret_cast<const float2*>(as + k * TM + ty * 2);
+        a[0] = v.x; a[1] = v.y;
+      }
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(bs + k * TILE + tx * 4);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const uint64_t a2 = pair_f32(a[i], a[i]);
+        acc[i][0] = fma_f32x2(a2, b.x, acc[i][0]);
+        acc[i][1] = fma_f32x2(a2, b.y, acc[i][1]);
+      }
+    }
+    if (NORMS && (t < TM || (t >= 128 && t < 128 + TILE))) {
+      const float* row = t < TM ? as + t : bs + (t - 128);
+      const int pitch = t < TM ? TM : TILE;
+#pragma unroll
+      for (int k = 0; k < STEP; ++k) norm[k & 3] = fmaf(row[k * pitch], row[k * pitch], norm[k & 3]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    split_f32(acc[i][0], sums[i][0], sums[i][1]);
+    split_f32(acc[i][1], sums[i][2], sums[i][3]);
+  }
+}
+
 // ---------------------------------------------------------------- assignment
+template <int TM>
 __global__ void __launch_bounds__(THREADS, 2)
 assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c_dtype, bool c_vec, int S, int J, int C,
               void* ids, int id_bytes, int32_t* labels32) {
-  extern __shared__ float sm[];
-  __shared__ float xn[GROUPS][TILE], cn[GROUPS][TILE];
-  const int g = threadIdx.x / GROUP_THREADS, t = threadIdx.x % GROUP_THREADS;
-  const int m0 = blockIdx.x * TILE;
-  const int row = threadIdx.x >> 2, quarter = threadIdx.x & 3;   // of the epilogue: 16 centres each
-  float best = INFINITY;
-  int best_i = 0;
+  __shared__ __align__(16) float sm[ORDERED_FLOATS<TM>];
+  __shared__ float xn[TM], cn[TILE];
+  constexpr int ROWS = TM / 16;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  const int m0 = blockIdx.x * TM;
+  const bool in_a = m0 + t % TM < S;
+  const size_t a_row = static_cast<size_t>(in_a ? m0 + t % TM : 0) * J;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float best[ROWS];
+  int best_i[ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) { best[i] = INFINITY; best_i[i] = 0; }
   for (int n0 = 0; n0 < C; n0 += TILE) {
-    const bool in_a = m0 + t < S, in_b = n0 + t < C;
-    const size_t a_row = static_cast<size_t>(in_a ? m0 + t : 0) * J, b_row = static_cast<size_t>(in_b ? n0 + t : 0) * J;
-    float a_norm = 0.f, b_norm = 0.f;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();        // the previous tile's sums and norms have been read
-    gemm64<true>(sm, J, [&](int k) { return in_a ? load4(x, x_dtype, a_row, k, J, x_vec) : zero; },
-                 [&](int k) { return in_b ? load4(centers, c_dtype, b_row, k, J, c_vec) : zero; }, a_norm, b_norm);
-    xn[g][t] = a_norm;
-    cn[g][t] = b_norm;
+    const bool in_b = n0 + t % TILE < C;
+    const size_t b_row = static_cast<size_t>(in_b ? n0 + t % TILE : 0) * J;
+    float dots[ROWS][4], norm[4] = {0.f, 0.f, 0.f, 0.f};
+    __syncthreads();        // the previous tile's operands and norms have been read
+    gemm_ordered<TM, true>(sm, J, [&](int k) { return in_a ? load4(x, x_dtype, a_row, k, J, x_vec) : zero; },
+                           [&](int k) { return in_b ? load4(centers, c_dtype, b_row, k, J, c_vec) : zero; }, dots, norm);
+    const float square = (norm[0] + norm[1]) + (norm[2] + norm[3]);
+    if (t < TM) xn[t] = square;
+    else if (t >= 128 && t < 128 + TILE) cn[t - 128] = square;
     __syncthreads();
-    const float xr = (xn[0][row] + xn[1][row]) + (xn[2][row] + xn[3][row]);
-    float d = INFINITY;
-    int idx = 0x7fffffff;
 #pragma unroll
-    for (int j = 0; j < 16; j += 4) {
-      const int c = quarter * 16 + j;
-      const float4 dot4 = tile_sum(sm, row, c);
-      const float dots[4] = {dot4.x, dot4.y, dot4.z, dot4.w};
+    for (int i = 0; i < ROWS; ++i) {
+      float d = INFINITY;
+      int idx = 0x7fffffff;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (n0 + c + i < C) {
-          const float norm = (cn[0][c + i] + cn[1][c + i]) + (cn[2][c + i] + cn[3][c + i]);
+      for (int j = 0; j < 4; ++j) {
+        const int c = n0 + tx * 4 + j;
+        if (c < C) {
           // (||x||^2 + ||c||^2) - 2 x.c, in that association, in fp32
-          const float dist = __fsub_rn(__fadd_rn(xr, norm), __fmul_rn(2.0f, dots[i]));
-          if (dist < d) { d = dist; idx = n0 + c + i; }
+          const float dist = __fsub_rn(__fadd_rn(xn[ty * ROWS + i], cn[tx * 4 + j]), __fmul_rn(2.0f, dots[i][j]));
+          if (dist < d) { d = dist; idx = c; }
         }
-    }
+      }
 #pragma unroll
-    for (int off = 1; off < 4; off <<= 1) {
-      const float od = __shfl_xor_sync(0xffffffffu, d, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-      if (od < d || (od == d && oi < idx)) { d = od; idx = oi; }
+      for (int off = 1; off < 16; off <<= 1) {
+        const float od = __shfl_xor_sync(0xffffffffu, d, off);
+        const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
+        if (od < d || (od == d && oi < idx)) { d = od; idx = oi; }
+      }
+      if (d < best[i]) { best[i] = d; best_i[i] = idx; }
     }
-    if (d < best) { best = d; best_i = idx; }
   }
-  const int token = m0 + row;
-  if (quarter == 0 && token < S) {
+  if (tx != 0) return;
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const int token = m0 + ty * ROWS + i;
+    if (token >= S) continue;
     if (ids) {
-      if (id_bytes == 1) static_cast<uint8_t*>(ids)[token] = static_cast<uint8_t>(best_i);
-      else static_cast<uint16_t*>(ids)[token] = static_cast<uint16_t>(best_i);
+      if (id_bytes == 1) static_cast<uint8_t*>(ids)[token] = static_cast<uint8_t>(best_i[i]);
+      else static_cast<uint16_t*>(ids)[token] = static_cast<uint16_t>(best_i[i]);
     }
-    if (labels32) labels32[token] = best_i;
+    if (labels32) labels32[token] = best_i[i];
   }
 }
 
 // ---------------------------------------------------------------- projection
-template <bool BF16>
+template <bool BF16, int TM>
 __global__ void __launch_bounds__(THREADS, 2)
 project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, bool c_vec, const void* ids, int id_bytes,
                const float* mean, const void* encoder, bool e_vec, int S, int J, int r, void* coeff) {
-  extern __shared__ float sm[];
-  const int t = threadIdx.x % GROUP_THREADS;
-  const int m0 = blockIdx.x * TILE, n0 = blockIdx.y * TILE;
-  const bool in_a = m0 + t < S, in_b = n0 + t < r;
-  const size_t a_row = static_cast<size_t>(in_a ? m0 + t : 0) * J, b_row = static_cast<size_t>(in_b ? n0 + t : 0) * J;
-  const size_t c_row = static_cast<size_t>(in_a ? load_id(ids, id_bytes, m0 + t) : 0) * J;
+  __shared__ __align__(16) float sm[ORDERED_FLOATS<TM>];
+  constexpr int ROWS = TM / 16;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TILE;
+  const bool in_a = m0 + t % TM < S, in_b = n0 + t % TILE < r;
+  const size_t a_row = static_cast<size_t>(in_a ? m0 + t % TM : 0) * J, b_row = static_cast<size_t>(in_b ? n0 + t % TILE : 0) * J;
+  const size_t c_row = static_cast<size_t>(in_a ? load_id(ids, id_bytes, m0 + t % TM) : 0) * J;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   auto residual = [&](int k) {
     if (!in_a) return zero;
@@ -217,21 +295,19 @@ project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, 
     if (BF16) res = make_float4(round_to_bf16(res.x), round_to_bf16(res.y), round_to_bf16(res.z), round_to_bf16(res.w));
     return res;
   };
-  float unused_a = 0.f, unused_b = 0.f;
-  gemm64<false>(sm, J, residual,
-                [&](int k) { return in_b ? load4(encoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, J, e_vec) : zero; },
-                unused_a, unused_b);
-  const int row = threadIdx.x >> 2, token = m0 + row;
-  if (token >= S) return;
+  float sums[ROWS][4], unused[4];
+  gemm_ordered<TM, false>(sm, J, residual,
+                          [&](int k) { return in_b ? load4(encoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, J, e_vec) : zero; },
+                          sums, unused);
 #pragma unroll
-  for (int j = 0; j < 16; j += 4) {
-    const int c = (threadIdx.x & 3) * 4 + j * 4;   // four lanes write 64 contiguous bytes
-    const float4 s = tile_sum(sm, row, c);
-    const float v[4] = {s.x, s.y, s.z, s.w};
+  for (int i = 0; i < ROWS; ++i) {
+    const int token = m0 + ty * ROWS + i;
+    if (token >= S) continue;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (n0 + c + i < r)
-        store_float(coeff, BF16 ? NKV_BF16 : NKV_F32, static_cast<size_t>(token) * r + n0 + c + i, v[i]);
+    for (int j = 0; j < 4; ++j) {
+      const int c = n0 + tx * 4 + j;
+      if (c < r) store_float(coeff, BF16 ? NKV_BF16 : NKV_F32, static_cast<size_t>(token) * r + c, sums[i][j]);
+    }
   }
 }
 
@@ -282,10 +358,8 @@ decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* 
       if (BF16) v[i] = round_to_bf16(v[i]);
     return make_float4(v[0], v[1], v[2], v[3]);
   };
-  float unused_a = 0.f, unused_b = 0.f;
-  gemm64<false>(sm, h.rank, latent,
-                [&](int k) { return in_b ? load4(decoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, h.rank, d_vec) : zero; },
-                unused_a, unused_b);
+  gemm64(sm, h.rank, latent,
+         [&](int k) { return in_b ? load4(decoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, h.rank, d_vec) : zero; });
   const uint16_t* centers = static_cast<const uint16_t*>(h.centers);
   const int row = threadIdx.x >> 2;
   if (m0 + row >= n || tok[row] < 0) return;
@@ -486,12 +560,18 @@ int allow_smem(K kernel) {
 
 }  // namespace
 
+// Rows of a tile in gemm_ordered: 32 while that still gives every block an SM of its own, else 64.  A tile of
+// half the rows takes three quarters of the time (K = 1,536: 109 against 142 us), so two on one SM would lose.
+static int ordered_rows(int S, int column_tiles) {
+  return static_cast<long long>(ceil_div(S, 32)) * column_tiles <= sm_count() ? 32 : 64;
+}
+
 int simt_assign(const void* x, int x_dtype, const void* centers, int c_dtype, int S, int J,
                 int C, void* ids, int id_bytes, int32_t* labels32, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
-  int rc = allow_smem(assign_kernel);
-  if (rc != NKV_OK) return rc;
-  assign_kernel<<<ceil_div(S, TILE), THREADS, SMEM_FLOATS * 4, stream>>>(
+  const int rows = ordered_rows(S, 1);
+  auto kernel = rows == 32 ? assign_kernel<32> : assign_kernel<64>;
+  kernel<<<ceil_div(S, rows), THREADS, 0, stream>>>(
       x, x_dtype, vector_rows(x, x_dtype, J), centers, c_dtype, vector_rows(centers, c_dtype, J), S, J, C, ids,
       id_bytes, labels32);
   NKV_LAUNCH_CHECK("assign_kernel");
@@ -502,12 +582,12 @@ int simt_project(const void* x, int x_dtype, const void* centers_bf16, const voi
                  int id_bytes, const float* mean, const void* encoder, int enc_dtype, int S,
                  int J, int r, void* coeff, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
-  const dim3 grid(ceil_div(S, TILE), ceil_div(r, TILE));
+  const int rows = ordered_rows(S, ceil_div(r, TILE));
+  const dim3 grid(ceil_div(S, rows), ceil_div(r, TILE));
   const bool e_vec = vector_rows(encoder, enc_dtype, J) && vector_rows(mean, NKV_F32, J);
-  auto kernel = enc_dtype == NKV_BF16 ? project_kernel<true> : project_kernel<false>;
-  int rc = allow_smem(kernel);
-  if (rc != NKV_OK) return rc;
-  kernel<<<grid, THREADS, SMEM_FLOATS * 4, stream>>>(
+  auto kernel = enc_dtype == NKV_BF16 ? (rows == 32 ? project_kernel<true, 32> : project_kernel<true, 64>)
+                                      : (rows == 32 ? project_kernel<false, 32> : project_kernel<false, 64>);
+  kernel<<<grid, THREADS, 0, stream>>>(
       x, x_dtype, vector_rows(x, x_dtype, J), static_cast<const uint16_t*>(centers_bf16),
       vector_rows(centers_bf16, NKV_BF16, J), ids, id_bytes, mean, encoder, e_vec, S, J, r, coeff);
   NKV_LAUNCH_CHECK("project_kernel");
