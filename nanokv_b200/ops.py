@@ -203,10 +203,15 @@ def decode_rows(view: HistoryView, decoder, mean, *, rows=None, dtype=None) -> t
     out = torch.empty(n, J, dtype=dtype, device=device)
     if rows is not None:
         rows = rows.to(dtype=torch.int32).contiguous()
+    # the word is not made inside a capture: a graph would clear it on every replay (the rows that a decode
+    # could not finish are NaN without it as well)
+    word = _STATUS_WORDS.get(device)
+    if word is None and not torch.cuda.is_current_stream_capturing():
+        word = status_word(device)
     struct = view.struct()
     _lib.check(_lib.library().nkv_decode_rows_status(
         ctypes.byref(struct), _ptr(rows), n, _ptr(decoder), dtype_code(decoder.dtype), _ptr(mean),
-        J, _ptr(out), dtype_code(dtype), _ptr(status_word(device)), _stream(device)))
+        J, _ptr(out), dtype_code(dtype), _ptr(word), _stream(device)))
     return out
 
 

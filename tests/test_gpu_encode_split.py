@@ -1,4 +1,4 @@
-"""Encoder GEMMs cut along K (and the C-means update) at the sizes where the cut changes."""
+"""Encoder GEMMs and the C-means update at the sizes where their tiles and column parts change."""
 import pytest
 import torch
 

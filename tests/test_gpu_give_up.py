@@ -91,3 +91,21 @@ def test_bad_arguments_are_refused():
                                                 budget, None) == _lib.NKV_ERR_INVALID
     assert lib.nkv_selftest_decode_gives_up(ctypes.byref(history), None, 0, None, None, 64, None, None, 1000,
                                             None) == _lib.NKV_ERR_INVALID
+
+
+@pytest.mark.gpu
+def test_a_captured_decode_makes_no_status_word(monkeypatch):
+    """A word made inside a capture would lie in the graph's pool and be cleared by every replay."""
+    view = random_history(300, 256, 64).view()
+    decoder, mean = operator(256, 64)
+    want = ops.decode_rows(view, decoder, mean)
+    torch.cuda.synchronize()
+    monkeypatch.setattr(ops, "_STATUS_WORDS", {})
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = ops.decode_rows(view, decoder, mean)
+    assert not ops._STATUS_WORDS
+    got.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
