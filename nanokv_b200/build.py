@@ -19,7 +19,7 @@ CSRC = PACKAGE / "csrc"
 BUILD = PACKAGE / "_build"
 LIBRARY = BUILD / "libnanokv_b200.so"
 SOURCES = ("nkv_api.cu", "nkv_simt.cu", "nkv_f32.cu", "nkv_elementwise.cu", "nkv_tc_attn.cu",
-           "nkv_tc_encode.cu", "nkv_tc_decode.cu", "nkv_static_scratch.cu")
+           "nkv_tc_assign.cu", "nkv_tc_encode.cu", "nkv_tc_decode.cu", "nkv_static_scratch.cu")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
 

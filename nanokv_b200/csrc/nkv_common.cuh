@@ -51,6 +51,29 @@ __device__ __forceinline__ uint16_t float_to_bf16_bits(float v) {
   return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 
+// two fp32 values in one 64-bit register pair: the packed operations issue once for both
+__device__ __forceinline__ uint64_t pair_bits(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
+  return pair_bits(__float_as_uint(lo), __float_as_uint(hi));
+}
+__device__ __forceinline__ void split_f32(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // INT4 code (0..14, i.e. the signed code plus 7) of coefficient z for a group scale, with the
 // reference's rounding points.  IN_BF16: the quotient is rounded to bf16 before rint (LingBot's
 // form).  Otherwise rint(z / scale) in fp32, taken through the reciprocal: z * inv is within 2 ulp

@@ -21,20 +21,6 @@ constexpr int OPERAND = BK * TILE;                       // floats of one operan
 constexpr int SMEM_FLOATS = GROUPS * 2 * 2 * OPERAND;    // two buffers of two operands per group
 static_assert(SMEM_FLOATS == GROUPS * TILE * TILE, "the partial sums reuse the operand tiles");
 
-__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void split_f32(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // elements k .. k + 3 of a row (0 past K); `vector`: rows start on 16 (fp32) or 8 (16-bit) bytes, K % 4 == 0
 __device__ __forceinline__ float4 load4(const void* base, int dtype, size_t row_start, int k, int K, bool vector) {
   if (vector && k + 4 <= K) {

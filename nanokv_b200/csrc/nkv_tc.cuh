@@ -131,6 +131,10 @@ __device__ __forceinline__ void fence_proxy_async_all() {
   asm volatile("fence.proxy.async;" ::: "memory");
 }
 
+// the two halves of a cluster-wide barrier, each for all threads of a block
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -163,6 +167,27 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
   }
 }
 
+// Place in an operand ring, kept by counting: a division by the run-time depth per stage, in the one thread that
+// issues the copies and the one that issues the MMAs, is a good part of a stage's time.
+struct Ring {
+  int stage = 0, phase = 0;
+  __device__ __forceinline__ void advance(int depth) {
+    if (++stage == depth) { stage = 0; phase ^= 1; }
+  }
+};
+
+// Waits of a whole warp that give one answer for all its lanes: what follows (tensor-memory loads, cluster
+// barriers, __syncwarp) takes converged warps, also when a wait gives up.  wait_all acquires at block scope (a
+// cluster-scope acquire also gives up the first-level cache's lines), wait_all_cluster what peers' threads wrote.
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                         long long budget = WAIT_BUDGET_CYCLES) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code, budget) ? 1 : 0) != 0;
+}
+__device__ __forceinline__ bool wait_all_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                                 long long budget = WAIT_BUDGET_CYCLES) {
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code, budget) ? 1 : 0) != 0;
+}
+
 // ---- TMA ---------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
                                             uint64_t* bar) {
@@ -189,6 +214,11 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
           smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+
+// asks L2 for `bytes` (a multiple of 16) from a 16-byte aligned address
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
 }
 
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {

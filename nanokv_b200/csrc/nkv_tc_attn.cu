@@ -296,29 +296,6 @@ __device__ __forceinline__ float exp2_approx(float x) {
   return y;
 }
 
-// two fp32 values in one 64-bit register pair: the packed operations issue once for both
-__device__ __forceinline__ uint64_t pair_bits(uint32_t lo, uint32_t hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-  return r;
-}
-__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
-  return pair_bits(__float_as_uint(lo), __float_as_uint(hi));
-}
-__device__ __forceinline__ void split_f32(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // Lap timer of one thread (development builds only): adds the cycles since the previous lap to a
 // bucket kept in registers; flush() adds the buckets to global memory once, at the end.
 #ifdef NKV_DEV

@@ -128,17 +128,6 @@ __device__ __forceinline__ Run run_at(const Params& p, int w, int w_end) {
   return r;
 }
 
-// Acquire at block scope: what is handed over lies in shared memory or TMEM.  (A cluster-scope acquire also
-// gives up the first-level cache's lines, which hold the epilogue's bias, centre and rotation rows.)
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
-                                         long long budget) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code, budget) ? 1 : 0) != 0;
-}
-// the same for latents, which the other CTA's threads wrote
-__device__ __forceinline__ bool wait_all_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
-                                                 long long budget) {
-  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code, budget) ? 1 : 0) != 0;
-}
 // Arrival that hands back tensor memory whose loads have completed: nothing written is published by it, so
 // it does not wait for the stores under way (a releasing arrival would: a tile's rows to L2, every tile).
 __device__ __forceinline__ void arrive_relaxed(uint32_t bar_cluster_addr) {

@@ -1,11 +1,5 @@
-// Encoder GEMMs on tcgen05: nearest-centre assignment and residual projection.
-//
-// Both are [128 tokens x K=J] x [N x K]^T tiles with fp32 accumulators in TMEM,
+// Encoder projection on tcgen05: [128 tokens x K=J] x [N x K]^T tiles with fp32 accumulators in TMEM,
 // K streamed 64 columns at a time through a shared-memory ring of up to eight stages.
-//   assign : A = token rows (TMA), B = centre rows (TMA), N = C <= 512.  While
-//            a stage is resident the compute warps accumulate ||x||^2 and
-//            ||c||^2 from the same tiles; the epilogue evaluates
-//            (||x||^2 + ||c||^2) - 2 x.c in fp32 and keeps the first minimum.
 //   project: A = bf16((x - centre[id]) - mean), formed by the compute warps in
 //            the swizzled operand layout; B = encoder rows (TMA); the epilogue
 //            rounds once to bf16.
@@ -41,7 +35,7 @@ constexpr int A_BYTES = 128 * 128;
 constexpr int MAX_STAGES = 8;
 enum Bar { TMA_FULL = 0, A_FULL = 8, STAGE_FREE = 16, ACC_DONE = 24, SIDE_READY = 25, CAND_READY = 26,
            PEER_READY = 27, NUM_BARS = 28 };
-enum Mode { PROJECT = 0, ASSIGN_IDS = 1, PROJECT_QUANT = 2 };
+enum Mode { PROJECT = 0, PROJECT_QUANT = 2 };
 constexpr int META_HEAD = 256;      // barriers, TMEM slot, abort flag
 constexpr int WARPS = COMPUTE_THREADS / 32;
 constexpr int MAX_PARTS = 8;        // thread blocks of one token tile that form a cluster
@@ -53,50 +47,14 @@ struct Params {
   // project
   const uint16_t* x; const uint16_t* centers; const void* ids; int id_bytes;
   const float* mean; uint16_t* coeff;
-  // assign
-  void* ids_out;
-  int32_t* labels_out;              // optional 32-bit copy of the ids (the C-means update reads it)
-  int a_chunks;                     // 64-column chunks of a token row; K runs over planes * a_chunks chunks
-  const float* cnorm;               // squared norms of the centres when B holds bf16 planes of fp32 centres
   // project + quantise: codes u8 [S, r/2] and scales [S] at the history's token offset
   uint8_t* codes; void* scales; float eps; int in_bf16; int scale_dtype; int column_parts;
 };
-
-__device__ __forceinline__ float sumsq8(uint4 w) {
-  const uint32_t words[4] = {w.x, w.y, w.z, w.w};
-  float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float a = __uint_as_float(words[i] << 16), b = __uint_as_float(words[i] & 0xFFFF0000u);
-    s = fmaf(a, a, s);
-    s = fmaf(b, b, s);
-  }
-  return s;
-}
-
-// place in the operand ring, kept by counting: a division by the run-time depth per stage, in the one thread
-// that issues the copies and the one that issues the MMAs, is a good part of a stage's time
-struct Ring {
-  int stage = 0, phase = 0;
-  __device__ __forceinline__ void advance(int depth) {
-    if (++stage == depth) { stage = 0; phase ^= 1; }
-  }
-};
-
-// Every wait of a whole warp gives one answer for all its lanes: what follows (tensor-memory loads, cluster
-// barriers, __syncwarp) takes converged warps, also when a wait gives up.
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code) ? 1 : 0) != 0;
-}
-__device__ __forceinline__ bool wait_all_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
-  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, code) ? 1 : 0) != 0;
-}
 
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
 encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                    const __grid_constant__ CUtensorMap map_b, Params p) {
-  constexpr bool ASSIGN = MODE == ASSIGN_IDS;
   constexpr bool QUANT = MODE == PROJECT_QUANT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
@@ -109,25 +67,20 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + NUM_BARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + NUM_BARS * 8 + 4);
   float* xn_part = reinterpret_cast<float*>(meta + META_HEAD);    // [256]
-  float* cand_d = xn_part + 256;                                  // [128]
-  int* cand_i = reinterpret_cast<int*>(cand_d + 128);             // [128]
-  float* cn_part = reinterpret_cast<float*>(cand_i + 128);        // [C][2]
-  float* peer_max = cn_part;                                      // project + quantise: [MAX_PARTS][128]
+  float* peer_max = xn_part + 512;                                // project + quantise: [MAX_PARTS][128]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int part = blockIdx.x % p.column_parts;         // place in the tile's cluster
   const int m0 = (blockIdx.x / p.column_parts) * p.rows;   // this tile's tokens: [m0, m_end)
   const int m_end = min(p.S, m0 + p.rows);
   const int n_base = part * p.NACC * p.NB;
-  // assign against fp32 centres: B is the centres split into bf16 planes laid side by side along
-  // K, A (the token rows) is walked once per plane
-  const int nchunks = ASSIGN ? p.a_chunks * (p.cnorm != nullptr ? 3 : 1) : p.J / 64;
+  const int nchunks = p.J / 64;
 
   if (tid == 0) {
     for (int s = 0; s < MAX_STAGES; ++s) {
       mbar_init(&bars[TMA_FULL + s], 1);
       mbar_init(&bars[A_FULL + s], WARPS);
-      mbar_init(&bars[STAGE_FREE + s], ASSIGN ? 1 + WARPS : 1);
+      mbar_init(&bars[STAGE_FREE + s], 1);
     }
     mbar_init(&bars[ACC_DONE], 1);
     mbar_init(&bars[SIDE_READY], COMPUTE_THREADS);
@@ -151,19 +104,13 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   if (warp == 8) {
     if (lane == 0) {
       prefetch_tensormap(&map_b);
-      if (ASSIGN) prefetch_tensormap(&map_a);
-      int a_col = 0;
       Ring at;
       for (int c = 0; c < nchunks && ok; ++c, at.advance(nst)) {
         const int s = at.stage;
         if (c >= nst) ok = mbar_wait(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 400 + s);
         if (!ok) break;
         uint8_t* stage = smem + s * stage_bytes;
-        mbar_arrive_expect_tx(&bars[TMA_FULL + s], p.NACC * b_bytes + (ASSIGN ? A_BYTES : 0));
-        if (ASSIGN) {
-          tma_load_2d(stage, &map_a, a_col * 64, m0, &bars[TMA_FULL + s]);
-          if (++a_col == p.a_chunks) a_col = 0;
-        }
+        mbar_arrive_expect_tx(&bars[TMA_FULL + s], p.NACC * b_bytes);
         for (int a = 0; a < p.NACC; ++a)
           tma_load_2d(stage + A_BYTES + a * b_bytes, &map_b, c * 64, n_base + a * p.NB,
                       &bars[TMA_FULL + s]);
@@ -183,7 +130,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     for (int c = 0; c < nchunks && ok; ++c, at.advance(nst)) {
       const int s = at.stage;
       ok = wait_all(&bars[TMA_FULL + s], at.phase, abort_flag, 410 + s);
-      if (ok && !ASSIGN) ok = wait_all(&bars[A_FULL + s], at.phase, abort_flag, 412 + s);
+      if (ok) ok = wait_all(&bars[A_FULL + s], at.phase, abort_flag, 412 + s);
       if (!ok) break;
       tc_fence_after();
       const uint32_t stage = smem_base + s * stage_bytes;
@@ -208,90 +155,7 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     // eight threads share a 128-byte row chunk (16 bytes each), a thread serves rows r0 + 32 i: loads and
     // the swizzled stores touch whole lines
     const int r0 = tid >> 3, piece = tid & 7;
-    if (ASSIGN) {
-      // ---- squared norms from the resident tiles.  Neighbouring threads read half-rows 64 bytes apart, four
-      // of which share their banks.  The order in which a half-row's sixteen squares are added is what the stored
-      // ids were made with, so a layout without the conflicts has to keep it.
-      const int C = p.n_total;
-      // partials of half a token row, and of half-rows tid + 256 k of the centres
-      float xs = 0.f, cs[4] = {0.f, 0.f, 0.f, 0.f};
-      Ring at;
-      for (int i = 0; i < nchunks && ok; ++i, at.advance(nst)) {
-        const int s = at.stage;
-        ok = wait_all(&bars[TMA_FULL + s], at.phase, abort_flag, 420 + s);
-        if (!ok) break;
-        const uint8_t* stage = smem + s * stage_bytes;
-        if (i < p.a_chunks) {
-          const uint4* src = reinterpret_cast<const uint4*>(stage + (tid >> 1) * 128 + (tid & 1) * 64);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) xs += sumsq8(src[j]);
-        }
-        if (p.cnorm == nullptr) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int item = tid + k * COMPUTE_THREADS;
-            if (item < 2 * C) {
-              const uint4* src = reinterpret_cast<const uint4*>(stage + A_BYTES + (item >> 1) * 128 + (item & 1) * 64);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) cs[k] += sumsq8(src[j]);
-            }
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[STAGE_FREE + s]);
-      }
-      if (ok) {
-        xn_part[tid] = xs;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int item = tid + k * COMPUTE_THREADS;
-          if (item < 2 * C) cn_part[item] = cs[k];
-        }
-        mbar_arrive(&bars[SIDE_READY]);
-        ok = wait_all(&bars[SIDE_READY], 0, abort_flag, 430) && wait_all(&bars[ACC_DONE], 0, abort_flag, 431);
-      }
-      if (ok) {
-        tc_fence_after();
-        const float xn = xn_part[2 * row] + xn_part[2 * row + 1];
-        const int chunks = (C + 31) / 32, middle = (chunks + 1) / 2;
-        const int first = wg == 0 ? 0 : middle, last = wg == 0 ? middle : chunks;
-        float best = INFINITY;
-        int best_i = 0;    // a row without a finite distance: centre 0, as in the CUDA-core kernel, never an id past C
-#pragma unroll 1
-        for (int cc = first; cc < last; ++cc) {
-          const int col = cc * 32, acc = col / p.NB;
-          float v[32];
-          tmem_ld32(tmem_base + lane_sel + acc * 256 + (col - acc * p.NB), v);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int cidx = col + j;
-            if (cidx < C) {
-              const float cn = p.cnorm != nullptr ? __ldg(p.cnorm + cidx) : cn_part[2 * cidx] + cn_part[2 * cidx + 1];
-              const float dist = __fsub_rn(__fadd_rn(xn, cn), __fmul_rn(2.0f, v[j]));
-              if (dist < best) { best = dist; best_i = cidx; }
-            }
-          }
-        }
-        if (wg == 1) {
-          cand_d[row] = best;
-          cand_i[row] = best_i;
-          mbar_arrive(&bars[CAND_READY]);
-        } else {
-          ok = wait_all(&bars[CAND_READY], 0, abort_flag, 432);
-          if (ok) {
-            if (cand_d[row] < best) { best = cand_d[row]; best_i = cand_i[row]; }
-            const int t = m0 + row;
-            if (t < m_end) {
-              if (p.ids_out != nullptr) {
-                if (p.id_bytes == 1) static_cast<uint8_t*>(p.ids_out)[t] = static_cast<uint8_t>(best_i);
-                else static_cast<uint16_t*>(p.ids_out)[t] = static_cast<uint16_t>(best_i);
-              }
-              if (p.labels_out != nullptr) p.labels_out[t] = best_i;
-            }
-          }
-        }
-      }
-    } else {
+    {
       // ---- residual operand: bf16((x - centre[id]) - mean), 8 columns of four rows per thread and
       // chunk; the operands of two chunks are in flight while one is formed
       const uint16_t* xrow[4];
@@ -583,11 +447,6 @@ int pick_rows(int S, int column_parts) {
   return static_cast<int>(rows);
 }
 
-bool tc_assign_supported(int J, int C) {
-  if (J % 64 || C % 16 || C > 512) return false;
-  return C <= 256 || C % 64 == 0;
-}
-
 int tc_project(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
                const float* mean, const void* encoder_bf16, int S, int J, int r, void* coeff,
                cudaStream_t stream) {
@@ -653,109 +512,6 @@ int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* i
   int rc = encode_tensor_map(&map_b, 2, encoder_bf16, 2, dims, strides, box, 128);
   if (rc != NKV_OK) return rc;
   return launch_gemm<PROJECT_QUANT>(map_b, map_b, p, 0, "encode_gemm_kernel<project + quantise>", stream);
-}
-
-int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C, void* ids,
-              int id_bytes, cudaStream_t stream) {
-  if (S == 0) return NKV_OK;
-  Params p{};
-  p.S = S; p.J = J; p.n_total = C;
-  const Split cut = plan_split(S, J / 64, C, 1, false);
-  p.rows = cut.rows; p.column_parts = 1;
-  set_columns(p, C);
-  p.ids_out = ids; p.id_bytes = id_bytes;
-  p.a_chunks = J / 64;
-  CUtensorMap map_a, map_b;
-  {
-    uint64_t dims[2] = {static_cast<uint64_t>(J), static_cast<uint64_t>(S)};
-    uint64_t strides[1] = {static_cast<uint64_t>(J) * 2};
-    uint32_t box[2] = {64, TM};
-    int rc = encode_tensor_map(&map_a, 2, x_bf16, 2, dims, strides, box, 128);
-    if (rc != NKV_OK) return rc;
-  }
-  {
-    uint64_t dims[2] = {static_cast<uint64_t>(J), static_cast<uint64_t>(C)};
-    uint64_t strides[1] = {static_cast<uint64_t>(J) * 2};
-    uint32_t box[2] = {64, static_cast<uint32_t>(p.NB)};
-    int rc = encode_tensor_map(&map_b, 2, centers_bf16, 2, dims, strides, box, 128);
-    if (rc != NKV_OK) return rc;
-  }
-  return launch_gemm<ASSIGN_IDS>(map_a, map_b, p, C, "encode_gemm_kernel<assign>", stream);
-}
-
-namespace {
-
-// fp32 centre rows -> three bf16 planes side by side ([C, 3 J]: c = hi + mid + lo exactly, up to the
-// last bit of the third term) and the rows' squared norms in fp32
-__global__ void __launch_bounds__(256)
-split_centers_kernel(const float* centers, int J, uint16_t* planes, float* cnorm) {
-  __shared__ float part[256];
-  const int c = blockIdx.x;
-  const float* row = centers + static_cast<size_t>(c) * J;
-  uint16_t* out = planes + static_cast<size_t>(c) * 3 * J;
-  float sum = 0.f;
-  for (int j = threadIdx.x; j < J; j += 256) {
-    const float v = row[j];
-    sum = fmaf(v, v, sum);
-    const uint16_t hi = float_to_bf16_bits(v);
-    const float r1 = __fsub_rn(v, bf16_bits_to_float(hi));
-    const uint16_t mid = float_to_bf16_bits(r1);
-    const float r2 = __fsub_rn(r1, bf16_bits_to_float(mid));
-    out[j] = hi;
-    out[J + j] = mid;
-    out[2 * J + j] = float_to_bf16_bits(r2);
-  }
-  part[threadIdx.x] = sum;
-  __syncthreads();
-  for (int width = 128; width >= 1; width >>= 1) {
-    if (threadIdx.x < width) part[threadIdx.x] += part[threadIdx.x + width];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) cnorm[c] = part[0];
-}
-
-}  // namespace
-
-size_t tc_assign_f32_workspace_bytes(int J, int C) {
-  return static_cast<size_t>(C) * 3 * J * 2 + static_cast<size_t>(C) * 4 + 256;
-}
-
-// Nearest centre against fp32 centres on the tensor cores: every bf16 x bf16 product is exact in the
-// fp32 accumulator, and the three planes restore the centres' 24 mantissa bits, so the distances
-// carry fp32 accuracy (the accumulation order is the tensor core's).  Writes 32-bit labels.
-int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, int C, int32_t* labels,
-                  void* workspace, cudaStream_t stream) {
-  if (S == 0) return NKV_OK;
-  NKV_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, NKV_ERR_INVALID,
-              "assign: plane workspace must be 256-byte aligned");
-  uint16_t* planes = static_cast<uint16_t*>(workspace);
-  float* cnorm = reinterpret_cast<float*>(planes + static_cast<size_t>(C) * 3 * J);
-  split_centers_kernel<<<C, 256, 0, stream>>>(centers_f32, J, planes, cnorm);
-  NKV_LAUNCH_CHECK("split_centers_kernel");
-  Params p{};
-  p.S = S; p.J = J; p.n_total = C;
-  const Split cut = plan_split(S, 3 * (J / 64), C, 1, false);
-  p.rows = cut.rows; p.column_parts = 1;
-  set_columns(p, C);
-  p.labels_out = labels; p.id_bytes = 1;
-  p.a_chunks = J / 64;
-  p.cnorm = cnorm;
-  CUtensorMap map_a, map_b;
-  {
-    uint64_t dims[2] = {static_cast<uint64_t>(J), static_cast<uint64_t>(S)};
-    uint64_t strides[1] = {static_cast<uint64_t>(J) * 2};
-    uint32_t box[2] = {64, TM};
-    int rc = encode_tensor_map(&map_a, 2, x_bf16, 2, dims, strides, box, 128);
-    if (rc != NKV_OK) return rc;
-  }
-  {
-    uint64_t dims[2] = {static_cast<uint64_t>(J) * 3, static_cast<uint64_t>(C)};
-    uint64_t strides[1] = {static_cast<uint64_t>(J) * 3 * 2};
-    uint32_t box[2] = {64, static_cast<uint32_t>(p.NB)};
-    int rc = encode_tensor_map(&map_b, 2, planes, 2, dims, strides, box, 128);
-    if (rc != NKV_OK) return rc;
-  }
-  return launch_gemm<ASSIGN_IDS>(map_a, map_b, p, C, "encode_gemm_kernel<assign, fp32 centres>", stream);
 }
 
 }  // namespace nkv
