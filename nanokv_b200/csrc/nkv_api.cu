@@ -224,7 +224,7 @@ int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, cons
   // coefficients stay on chip
   if (encoder_dtype == NKV_BF16 && x_dtype == NKV_BF16 && !simt_forced() &&
       tc_project_quant_supported(J, r, group) && (reinterpret_cast<uintptr_t>(codes) & 15) == 0)
-    return tc_project_quant(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, eps, quant_mode,
+    return tc_project_quant(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, group, eps, quant_mode,
                             scale_dtype, codes, scales, static_cast<cudaStream_t>(stream));
   NKV_REQUIRE(workspace && workspace_bytes >= static_cast<size_t>(S) * r * dtype_bytes(encoder_dtype),
               NKV_ERR_INVALID, "project_quant: workspace of %zu bytes is too small", workspace_bytes);

@@ -91,6 +91,103 @@ __device__ __forceinline__ int quant_code(float z, float scale, float inv) {
   return static_cast<int>(fminf(fmaxf(rintf(q), -7.f), 7.f)) + 7;
 }
 
+// The listed values of a word redone with the IEEE division, lane by lane: a warp takes as many rounds as its
+// lane with the most of them, not one per value that any of its lanes lists.
+template <bool IN_BF16>
+__device__ __forceinline__ uint32_t quant_word_exact(const uint32_t (&w)[4], float scale, float inv, uint32_t hits, uint32_t out) {
+  for (; hits != 0; hits &= hits - 1) {
+    const int e = __ffs(hits) - 1;
+    const uint32_t word = (e & 4) ? ((e & 2) ? w[3] : w[2]) : ((e & 2) ? w[1] : w[0]);
+    const float z = __uint_as_float((e & 1) ? (word & 0xFFFF0000u) : (word << 16));
+    out = (out & ~(0xFu << (4 * e))) | (static_cast<uint32_t>(quant_code<IN_BF16>(z, scale, inv)) << (4 * e));
+  }
+  return out;
+}
+
+// Codes of eight bf16 coefficients (two per word, the even one in the low half) as one 32-bit word, without a
+// conversion instruction per value.
+template <bool IN_BF16>
+__device__ __forceinline__ uint32_t quant_word(const uint32_t (&w)[4], float scale, float inv) {
+  uint32_t out = 0;
+  if (IN_BF16) {
+    // The quotient is rounded to bf16 before rint.  z * inv is within 2 ulp of the IEEE quotient,
+    // so both round to the same bf16 number unless the product's low 16 bits lie within 4 of the
+    // rounding boundary 0x8000; only such values take the division (an exact boundary case cannot
+    // occur: a ratio of two 8-bit mantissas is never a 9-bit midpoint).  rint of the bf16 quotient
+    // is again the addition of 1.5 * 2^23 (exact on a bf16 number, ties to even as rint has them).
+    constexpr float MAGIC = 12582912.0f;
+    constexpr uint32_t MAGIC_BITS = 0x4B400000u;
+    constexpr uint32_t PACK_BIAS = (MAGIC_BITS - 7u) * 0x11111111u;
+    bool ambiguous = false;
+    uint32_t acc = 0;
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      const float q1 = __uint_as_float(w[k] & 0xFFFF0000u) * inv;
+      const float q0 = __uint_as_float(w[k] << 16) * inv;
+      ambiguous |= ((__float_as_uint(q1) + 0x8004u) & 0xFFFFu) <= 8u;
+      ambiguous |= ((__float_as_uint(q0) + 0x8004u) & 0xFFFFu) <= 8u;
+      const __nv_bfloat162 rounded = __floats2bfloat162_rn(q0, q1);
+      const uint32_t both = *reinterpret_cast<const uint32_t*>(&rounded);
+      const float t1 = __uint_as_float(both & 0xFFFF0000u) + MAGIC;
+      const float t0 = __uint_as_float(both << 16) + MAGIC;
+      acc = (acc << 4) + __float_as_uint(t1);
+      acc = (acc << 4) + __float_as_uint(t0);
+    }
+    out = acc - PACK_BIAS;
+    if (ambiguous) {
+      uint32_t hits = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float z = __uint_as_float((e & 1) ? (w[e >> 1] & 0xFFFF0000u) : (w[e >> 1] << 16));
+        if (((__float_as_uint(z * inv) + 0x8004u) & 0xFFFFu) <= 8u) hits |= 1u << e;
+      }
+      out = quant_word_exact<true>(w, scale, inv, hits, out);
+    }
+  } else {
+    // whole piece through the reciprocal; a piece holding a value whose scaled form lies within
+    // 1e-5 of a half-integer (where the reciprocal and the IEEE quotient could round apart) is
+    // redone value by value with the exact rule.  Rounding to the nearest-even integer is the
+    // fp32 addition of 1.5 * 2^23 (the integer then sits in the low mantissa bits), which keeps
+    // the whole loop on the full-rate floating-point and integer pipes: no conversion
+    // instruction per value.  No clamp is needed here: |z| <= the group's maximum and
+    // scale = max(that, eps) / 7 bound |z * inv| by 7 (1 + 2^-22) for every finite row, and a row
+    // with a non-finite value has no defined codes in the reference either (the 32-bit word of
+    // such a piece may then hold arbitrary bits; nothing outside that word is touched).
+    constexpr float MAGIC = 12582912.0f;
+    constexpr uint32_t MAGIC_BITS = 0x4B400000u;
+    // the float bits of (q + MAGIC) are MAGIC_BITS + rint(q): eight of them, each shifted four
+    // bits further, add up (mod 2^32) to the packed word plus a constant
+    constexpr uint32_t PACK_BIAS = (MAGIC_BITS - 7u) * 0x11111111u;
+    float worst = 0.f;
+    uint32_t acc = 0;
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      const float q1 = __uint_as_float(w[k] & 0xFFFF0000u) * inv;
+      const float q0 = __uint_as_float(w[k] << 16) * inv;
+      const float t1 = q1 + MAGIC, t0 = q0 + MAGIC;
+      worst = fmaxf(worst, fabsf(q1 - (t1 - MAGIC)));
+      worst = fmaxf(worst, fabsf(q0 - (t0 - MAGIC)));
+      acc = (acc << 4) + __float_as_uint(t1);
+      acc = (acc << 4) + __float_as_uint(t0);
+    }
+    out = acc - PACK_BIAS;
+    const bool near_half = worst > 0.49999f;
+    if (near_half) {
+      // exact ties are not rare (a row whose maximum has a mantissa divisible by 7 holds many),
+      // so only the values that are near a half take the IEEE division; their nibble is replaced
+      uint32_t hits = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float z = __uint_as_float((e & 1) ? (w[e >> 1] & 0xFFFF0000u) : (w[e >> 1] << 16));
+        const float q = z * inv;
+        if (fabsf(q - ((q + MAGIC) - MAGIC)) > 0.49999f) hits |= 1u << e;
+      }
+      out = quant_word_exact<false>(w, scale, inv, hits, out);
+    }
+  }
+  return out;
+}
+
 // element i of an array of the given element type, as float (exact)
 __device__ __forceinline__ float load_float(const void* base, int dtype, size_t i) {
   if (dtype == NKV_F32) return static_cast<const float*>(base)[i];

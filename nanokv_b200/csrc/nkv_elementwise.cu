@@ -106,87 +106,7 @@ __device__ __forceinline__ void quant_pack_row(const uint4 (&v)[QP_MAXJ], int su
     if (i >= pieces) continue;
     const float scale = scale_of[j], inv = inv_of[j];
     const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-    uint32_t out = 0;
-    if (IN_BF16) {
-      // The quotient is rounded to bf16 before rint.  z * inv is within 2 ulp of the IEEE quotient,
-      // so both round to the same bf16 number unless the product's low 16 bits lie within 4 of the
-      // rounding boundary 0x8000; only such values take the division (an exact boundary case cannot
-      // occur: a ratio of two 8-bit mantissas is never a 9-bit midpoint).  rint of the bf16 quotient
-      // is again the addition of 1.5 * 2^23 (exact on a bf16 number, ties to even as rint has them).
-      constexpr float MAGIC = 12582912.0f;
-      constexpr uint32_t MAGIC_BITS = 0x4B400000u;
-      constexpr uint32_t PACK_BIAS = (MAGIC_BITS - 7u) * 0x11111111u;
-      bool ambiguous = false;
-      uint32_t acc = 0;
-#pragma unroll
-      for (int k = 3; k >= 0; --k) {
-        const float q1 = __uint_as_float(w[k] & 0xFFFF0000u) * inv;
-        const float q0 = __uint_as_float(w[k] << 16) * inv;
-        ambiguous |= ((__float_as_uint(q1) + 0x8004u) & 0xFFFFu) <= 8u;
-        ambiguous |= ((__float_as_uint(q0) + 0x8004u) & 0xFFFFu) <= 8u;
-        const __nv_bfloat162 rounded = __floats2bfloat162_rn(q0, q1);
-        const uint32_t both = *reinterpret_cast<const uint32_t*>(&rounded);
-        const float t1 = __uint_as_float(both & 0xFFFF0000u) + MAGIC;
-        const float t0 = __uint_as_float(both << 16) + MAGIC;
-        acc = (acc << 4) + __float_as_uint(t1);
-        acc = (acc << 4) + __float_as_uint(t0);
-      }
-      out = acc - PACK_BIAS;
-      if (ambiguous) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint32_t word = w[e >> 1];
-          const float z = __uint_as_float((e & 1) ? (word & 0xFFFF0000u) : (word << 16));
-          if (((__float_as_uint(z * inv) + 0x8004u) & 0xFFFFu) <= 8u) {
-            const uint32_t code = static_cast<uint32_t>(quant_code<true>(z, scale, inv));
-            out = (out & ~(0xFu << (4 * e))) | (code << (4 * e));
-          }
-        }
-      }
-    } else {
-      // whole piece through the reciprocal; a piece holding a value whose scaled form lies within
-      // 1e-5 of a half-integer (where the reciprocal and the IEEE quotient could round apart) is
-      // redone value by value with the exact rule.  Rounding to the nearest-even integer is the
-      // fp32 addition of 1.5 * 2^23 (the integer then sits in the low mantissa bits), which keeps
-      // the whole loop on the full-rate floating-point and integer pipes: no conversion
-      // instruction per value.  No clamp is needed here: |z| <= the group's maximum and
-      // scale = max(that, eps) / 7 bound |z * inv| by 7 (1 + 2^-22) for every finite row, and a row
-      // with a non-finite value has no defined codes in the reference either (the 32-bit word of
-      // such a piece may then hold arbitrary bits; nothing outside that word is touched).
-      constexpr float MAGIC = 12582912.0f;
-      constexpr uint32_t MAGIC_BITS = 0x4B400000u;
-      // the float bits of (q + MAGIC) are MAGIC_BITS + rint(q): eight of them, each shifted four
-      // bits further, add up (mod 2^32) to the packed word plus a constant
-      constexpr uint32_t PACK_BIAS = (MAGIC_BITS - 7u) * 0x11111111u;
-      float worst = 0.f;
-      uint32_t acc = 0;
-#pragma unroll
-      for (int k = 3; k >= 0; --k) {
-        const float q1 = __uint_as_float(w[k] & 0xFFFF0000u) * inv;
-        const float q0 = __uint_as_float(w[k] << 16) * inv;
-        const float t1 = q1 + MAGIC, t0 = q0 + MAGIC;
-        worst = fmaxf(worst, fabsf(q1 - (t1 - MAGIC)));
-        worst = fmaxf(worst, fabsf(q0 - (t0 - MAGIC)));
-        acc = (acc << 4) + __float_as_uint(t1);
-        acc = (acc << 4) + __float_as_uint(t0);
-      }
-      out = acc - PACK_BIAS;
-      const bool near_half = worst > 0.49999f;
-      if (near_half) {
-        // exact ties are not rare (a row whose maximum has a mantissa divisible by 7 holds many),
-        // so only the values that are near a half take the IEEE division; their nibble is replaced
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint32_t word = w[e >> 1];
-          const float z = __uint_as_float((e & 1) ? (word & 0xFFFF0000u) : (word << 16));
-          const float q = z * inv;
-          if (fabsf(q - ((q + MAGIC) - MAGIC)) > 0.49999f) {
-            const uint32_t code = static_cast<uint32_t>(quant_code<false>(z, scale, inv));
-            out = (out & ~(0xFu << (4 * e))) | (code << (4 * e));
-          }
-        }
-      }
-    }
+    const uint32_t out = quant_word<IN_BF16>(w, scale, inv);
     dst[i] = out;
     if (GROUP32) {
       if ((i & 3) == 0) store_float(scales, scale_dtype, static_cast<size_t>(t) * groups + (i >> 2), scale);

@@ -117,7 +117,7 @@ int sm_count();
 bool tc_project_supported(int J, int r);
 bool tc_project_quant_supported(int J, int r, int group);
 int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
-                     const float* mean, const void* encoder_bf16, int S, int J, int r, float eps,
+                     const float* mean, const void* encoder_bf16, int S, int J, int r, int group, float eps,
                      int quant_mode, int scale_dtype, uint8_t* codes, void* scales, cudaStream_t stream);
 bool tc_assign_supported(int J, int C);
 size_t tc_assign_f32_workspace_bytes(int J, int C);

@@ -1,19 +1,27 @@
-// Encoder projection on tcgen05: [128 tokens x K=J] x [N x K]^T tiles with fp32 accumulators in TMEM,
-// K streamed 64 columns at a time through a shared-memory ring of up to eight stages.
-//   project: A = bf16((x - centre[id]) - mean), formed by the compute warps in
-//            the swizzled operand layout; B = encoder rows (TMA); the epilogue
-//            rounds once to bf16.
-//   project + quantise: the same GEMM, but the epilogue keeps the coefficients in TMEM, takes the
-//            token's absolute maximum over the whole rank row (the up to eight column parts of a token
-//            tile form a cluster and swap the maxima of their columns through each other's shared
-//            memory), quantises to INT4, packs two codes per byte and writes codes and scale to
-//            their place in the history: the bf16 coefficients never travel to HBM.
-// A CTA covers up to 512 output columns as 1 or 2 accumulators of NB <= 256.
-// Calls of a few thousand tokens have too few token tiles for 148 SMs, and a tile's time is the length
-// of its K loop (J / 64 stages of operand latency).  Such calls of the projection take more column parts
-// per tile (plan_split).  K itself is never cut: every sum runs in the order of K whatever the call's
-// length, so that a row gets the same id, codes and scale in a chunk of any size.
-// Warps 0-7 compute, warp 8 lane 0 issues TMA, warp 9 lane 0 issues MMA.
+// Encoder projection on tcgen05: coefficients = bf16((x - centre[id]) - mean) encoder^T, fp32 accumulators in TMEM,
+// and the INT4 quantiser behind it.
+//
+// x and the encoder's rows come by TMA into a ring of stages along K = J; the compute warps turn x into the residual in
+// its place (the swizzled operand layout), the centres' pieces fetched into registers some stages ahead.  K is never
+// cut: every sum runs in the order of K whatever the call's length, so that a row gets the same codes and scale in a
+// chunk of any size.
+//   project            rounds the coefficients to bf16 and writes them.
+//   project + quantise keeps them in TMEM and writes packed codes and scales to their place in the history.  With one
+//                      scale per token the column parts of a token tile (a cluster of up to eight) swap the maxima of
+//                      their columns through each other's shared memory; with one per 32 coefficients a thread holds
+//                      whole groups.
+//
+// Bound: short calls the length of the K loop (a 64-column chunk costs 500 to 550 cycles: MMAs on one accumulator follow one
+// another at 86 cycles, forming the residual takes the load / store and conversion units about as long) and 10 us
+// of prologue and epilogue; long calls what a block takes from L2 (2.0 GB at about 14 TB/s for 12,480 x 5,120 x 640).
+// What counted, us for 1,560 x 3,072 x 384 / 4,680 x 5,120 x 640 / 12,480 x 5,120 x 640: 38 / 72 / 171 with x loaded by the
+// residual warps, the mean from L2, values quantised one by one; 32 / 72 / 192 with x by TMA and the mean in shared memory
+// read once per row (eight conflicting lines each: more than all else the residual reads); 27 / 67 / 162 read once
+// per chunk, in whole lines; 25 / 61 / 146 with packed quantising and without the rows that are nobody's in it.
+// Tried: the residual of a tile formed once and written to all its parts' shared memory 47 / 148 / 316 (every
+// stage waits for the slowest remote store); centres by TMA gathers of four rows 56 / 97 / 238 (about 100 cycles each); 16
+// residual warps 31 / 71 / 199; started ahead of the assignment's end (programmatic launch): no difference.
+// Warps 0-7: residual and epilogue, warp 8 lane 0: TMA, warp 9: MMA.
 #include <atomic>
 
 #include "nkv_internal.h"
@@ -29,122 +37,200 @@ using namespace tc;
 
 constexpr int TM = 128;
 constexpr int COMPUTE_THREADS = 256;
-constexpr int THREADS = COMPUTE_THREADS + 64;
-constexpr int A_BYTES = 128 * 128;
-
-constexpr int MAX_STAGES = 8;
-enum Bar { TMA_FULL = 0, A_FULL = 8, STAGE_FREE = 16, ACC_DONE = 24, SIDE_READY = 25, CAND_READY = 26,
-           PEER_READY = 27, NUM_BARS = 28 };
-enum Mode { PROJECT = 0, PROJECT_QUANT = 2 };
-constexpr int META_HEAD = 256;      // barriers, TMEM slot, abort flag
+constexpr int GROUPS = COMPUTE_THREADS / TM;   // warpgroups: a TMEM lane is served by one thread of each
 constexpr int WARPS = COMPUTE_THREADS / 32;
-constexpr int MAX_PARTS = 8;        // thread blocks of one token tile that form a cluster
+constexpr int THREADS = COMPUTE_THREADS + 64;
+constexpr int MAX_STAGES = 8;
+constexpr int MAX_PARTS = 8;            // thread blocks of one token tile that form a cluster
+constexpr int MAX_MEAN = 8192;          // widest row whose mean is kept in shared memory
+enum Bar { FULL = 0, FORMED = 8, FREE = 16, ACC_DONE = 24, SIDE_READY = 25, PEER_READY = 26, NUM_BARS = 27 };
 
-struct Params {
-  int S, J, NB, NACC, n_total;      // n_total = r (project) or C (assign)
-  int nstages;                      // depth of the shared-memory operand ring (2..MAX_STAGES)
-  int rows;                         // tokens of a tile (<= TM)
-  // project
-  const uint16_t* x; const uint16_t* centers; const void* ids; int id_bytes;
-  const float* mean; uint16_t* coeff;
-  // project + quantise: codes u8 [S, r/2] and scales [S] at the history's token offset
-  uint8_t* codes; void* scales; float eps; int in_bf16; int scale_dtype; int column_parts;
+struct Meta {
+  uint64_t bars[NUM_BARS];
+  uint32_t tmem_slot;
+  int abort_flag;
+  float row_max[GROUPS][TM];
+  float peer_max[MAX_PARTS][TM];
 };
 
-template <int MODE>
+struct Params {
+  int S, J, rows, rows_pad, NB, NACC, n_total;          // n_total = r
+  int parts, kc;            // column parts of a tile; 64-column chunks of a stage
+  int nstages, nchunks, tmem_columns, mean_bytes;       // mean_bytes 0: the mean is read where it lies
+  const uint16_t* centers; const void* ids; int id_bytes;
+  const float* mean; uint16_t* coeff;
+  // project + quantise: codes u8 [S, r/2] and scales [S, r/group] at the history's token offset
+  uint8_t* codes; void* scales; float eps; int in_bf16; int scale_dtype; int group32;
+};
+
+__device__ __forceinline__ float scale_of(float amax, const Params& p) {
+  return p.in_bf16 ? round_to_bf16(__fdiv_rn(fmaxf(amax, round_to_bf16(p.eps)), 7.0f))
+                   : __fdiv_rn(fmaxf(amax, p.eps), 7.0f);
+}
+
+// 32 coefficients of this thread's token, rounded to bf16 (two per word)
+__device__ __forceinline__ void round_chunk(const float (&v)[32], uint32_t (&w)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+}
+
+// largest magnitude of the 32, as bf16 bits in both halves (a NaN or an infinity gives 0x7F80 or more)
+__device__ __forceinline__ uint32_t max_bits(const uint32_t (&w)[16]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) m = __vmaxu2(m, w[i] & 0x7FFF7FFFu);
+  const uint32_t swapped = __byte_perm(m, m, 0x1032);
+  return __vmaxu2(m, swapped);
+}
+constexpr uint32_t NOT_FINITE = 0x7F807F80u;
+
+// the same with NaNs left out, for rows that are not finite
+__device__ __forceinline__ float max_of_numbers(const uint32_t (&w)[16]) {
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    amax = fmaxf(fmaxf(amax, fabsf(__uint_as_float(w[i] << 16))), fabsf(__uint_as_float(w[i] & 0xFFFF0000u)));
+  return amax;
+}
+__device__ __forceinline__ float max_magnitude(const uint32_t (&w)[16], uint32_t& worst) {
+  const uint32_t bits = max_bits(w);
+  worst = __vmaxu2(worst, bits);
+  return bits >= NOT_FINITE ? max_of_numbers(w) : __uint_as_float(bits << 16);
+}
+
+// value by value, with every rounding and clamp spelled out: NaN gives code 0.  By value: an array whose address
+// leaves the caller would live in local memory there, on the path that finite rows take too.
+__device__ __noinline__ uint32_t quant_word_any(uint4 v, float scale, float inv, bool in_bf16) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  uint32_t out = 0;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float z = __uint_as_float((e & 1) ? w[e >> 1] & 0xFFFF0000u : w[e >> 1] << 16);
+    const int code = in_bf16 ? quant_code<true>(z, scale, inv) : quant_code<false>(z, scale, inv);
+    out |= static_cast<uint32_t>(code) << (4 * e);
+  }
+  return out;
+}
+
+// packed codes of 32 coefficients; `finite`: none of them is a NaN or an infinity
+__device__ __forceinline__ uint4 pack_codes(const uint32_t (&w)[16], float scale, bool in_bf16, bool finite) {
+  const float inv = __frcp_rn(scale);
+  uint32_t words[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t part[4] = {w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]};
+    words[i] = !finite ? quant_word_any(make_uint4(part[0], part[1], part[2], part[3]), scale, inv, in_bf16)
+                       : (in_bf16 ? quant_word<true>(part, scale, inv) : quant_word<false>(part, scale, inv));
+  }
+  return make_uint4(words[0], words[1], words[2], words[3]);
+}
+
+// SLOTS: rows of a stage's residual of which a thread forms 16 bytes, their centres fetched DEPTH stages ahead
+template <bool QUANT, int SLOTS, int DEPTH>
 __global__ void __launch_bounds__(THREADS, 1)
-encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
-                   const __grid_constant__ CUtensorMap map_b, Params p) {
-  constexpr bool QUANT = MODE == PROJECT_QUANT;
+project_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b,
+                    const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const int b_bytes = p.NB * 128;                       // one accumulator's B tile
-  const int stage_bytes = A_BYTES + p.NACC * b_bytes;
-  const int nst = p.nstages;
-  uint8_t* meta = smem + nst * stage_bytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(meta);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + NUM_BARS * 8);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + NUM_BARS * 8 + 4);
-  float* xn_part = reinterpret_cast<float*>(meta + META_HEAD);    // [256]
-  float* peer_max = xn_part + 512;                                // project + quantise: [MAX_PARTS][128]
+  Meta& meta = *reinterpret_cast<Meta*>(smem_raw);
+  float* mean_smem = reinterpret_cast<float*>(smem_raw + (sizeof(Meta) + 15) / 16 * 16);
+  uint8_t* ring = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(mean_smem) + p.mean_bytes + 1023) & ~static_cast<uintptr_t>(1023));
+  const int a_tile = p.rows_pad * 128, b_tile = p.NB * 128;       // one 64-column chunk; of one accumulator
+  const int kc = p.kc, a_bytes = kc * a_tile, stage_bytes = a_bytes + kc * p.NACC * b_tile;
+  const int nst = p.nstages, nchunks = p.nchunks, steps = (nchunks + kc - 1) / kc;
+  uint64_t* bars = meta.bars;
+  volatile int* abort_flag = &meta.abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int part = blockIdx.x % p.column_parts;         // place in the tile's cluster
-  const int m0 = (blockIdx.x / p.column_parts) * p.rows;   // this tile's tokens: [m0, m_end)
-  const int m_end = min(p.S, m0 + p.rows);
-  const int n_base = part * p.NACC * p.NB;
-  const int nchunks = p.J / 64;
+  const int part = blockIdx.x % p.parts;                   // place in the tile's cluster
+  const int m0 = (blockIdx.x / p.parts) * p.rows, m_end = min(p.S, m0 + p.rows);
+  const int columns = p.NACC * p.NB, n_base = part * columns;
 
   if (tid == 0) {
     for (int s = 0; s < MAX_STAGES; ++s) {
-      mbar_init(&bars[TMA_FULL + s], 1);
-      mbar_init(&bars[A_FULL + s], WARPS);
-      mbar_init(&bars[STAGE_FREE + s], 1);
+      mbar_init(&bars[FULL + s], 1);
+      mbar_init(&bars[FORMED + s], WARPS);
+      mbar_init(&bars[FREE + s], 1);
     }
     mbar_init(&bars[ACC_DONE], 1);
     mbar_init(&bars[SIDE_READY], COMPUTE_THREADS);
-    mbar_init(&bars[CAND_READY], 128);
-    mbar_init(&bars[PEER_READY], 128 * (p.column_parts > 1 ? p.column_parts - 1 : 1));
+    mbar_init(&bars[PEER_READY], TM * (p.parts > 1 ? p.parts - 1 : 1));
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
   }
-  if (warp == 9) tmem_alloc(tmem_slot, 512);
+  if (warp == WARPS + 1) tmem_alloc(&meta.tmem_slot, p.tmem_columns);
+  // The slots of a compute thread: rows of one of the stage's chunks, eight threads (16 bytes each) to the 128-byte piece
+  // of a row.  Their ids and the mean come while the barriers and tensor memory are set up.
+  const int per_chunk = COMPUTE_THREADS / kc, chunk_of = tid / per_chunk, piece = tid & 7;
+  const int first_row = (tid % per_chunk) >> 3, row_step = per_chunk >> 3;
+  int ids[SLOTS];
+#pragma unroll
+  for (int j = 0; j < SLOTS; ++j) {
+    const int r = first_row + row_step * j, t = m0 + r;
+    ids[j] = tid < COMPUTE_THREADS && r < p.rows && t < m_end ? load_id(p.ids, p.id_bytes, t) : 0;
+  }
+  // the eight columns of a piece as two halves 128 bytes apart: a quarter of a warp reads whole lines
+  for (int i = tid; i < p.mean_bytes / 16; i += THREADS)
+    reinterpret_cast<float4*>(mean_smem)[(i & ~15) + (i & 1) * 8 + ((i & 15) >> 1)] = __ldg(reinterpret_cast<const float4*>(p.mean) + i);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = meta.tmem_slot;
   // the column parts of one token tile write into each other's shared memory: nobody may do so before
   // the peers' barriers exist
-  const bool joined = QUANT && p.column_parts > 1;
-  if (joined) cluster_sync_all();
-  bool ok = true;
+  const bool joined = QUANT && !p.group32 && p.parts > 1;
+  if (joined) cluster_arrive();
+  bool ok = true, met = false;
 
-  if (warp == 8) {
+  if (warp == WARPS) {
     if (lane == 0) {
+      prefetch_tensormap(&map_x);
       prefetch_tensormap(&map_b);
       Ring at;
-      for (int c = 0; c < nchunks && ok; ++c, at.advance(nst)) {
+      for (int i = 0; i < steps && ok; ++i, at.advance(nst)) {
         const int s = at.stage;
-        if (c >= nst) ok = mbar_wait(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 400 + s);
+        if (i >= nst) ok = mbar_wait(&bars[FREE + s], at.phase ^ 1, abort_flag, 400 + s);
         if (!ok) break;
-        uint8_t* stage = smem + s * stage_bytes;
-        mbar_arrive_expect_tx(&bars[TMA_FULL + s], p.NACC * b_bytes);
+        uint8_t* stage = ring + s * stage_bytes;
+        mbar_arrive_expect_tx(&bars[FULL + s], stage_bytes);   // chunks past the row's end arrive as zeros and are not used
+        tma_load_3d(stage, &map_x, 0, m0, i * kc, &bars[FULL + s]);
         for (int a = 0; a < p.NACC; ++a)
-          tma_load_2d(stage + A_BYTES + a * b_bytes, &map_b, c * 64, n_base + a * p.NB,
-                      &bars[TMA_FULL + s]);
+          tma_load_3d(stage + a_bytes + a * kc * b_tile, &map_b, 0, n_base + a * p.NB, i * kc, &bars[FULL + s]);
       }
-      if (!ok) {
+      if (!ok) {   // copies in flight land before the block goes away
         const long long start = clock64();
         while (clock64() - start < (1ll << 21)) {}
       }
     }
     __syncwarp();
-  } else if (warp == 9) {
+  } else if (warp == WARPS + 1) {
     // The whole warp walks the uniform control flow; one elected lane issues.
     const bool leader = elect_one();
-    const uint32_t idesc = make_idesc_bf16(128, p.NB);
-    const uint32_t smem_base = smem_u32(smem);
+    const uint32_t idesc = make_idesc_bf16(TM, p.NB);
+    const uint32_t ring_base = smem_u32(ring);
     Ring at;
-    for (int c = 0; c < nchunks && ok; ++c, at.advance(nst)) {
+    for (int i = 0; i < steps && ok; ++i, at.advance(nst)) {
       const int s = at.stage;
-      ok = wait_all(&bars[TMA_FULL + s], at.phase, abort_flag, 410 + s);
-      if (ok) ok = wait_all(&bars[A_FULL + s], at.phase, abort_flag, 412 + s);
+      ok = wait_all(&bars[FORMED + s], at.phase, abort_flag, 410 + s);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t stage = smem_base + s * stage_bytes;
-      const uint64_t a_desc = make_smem_desc_sw128(stage);
-      for (int a = 0; a < p.NACC; ++a) {
-        const uint64_t b_desc = make_smem_desc_sw128(stage + A_BYTES + a * b_bytes);
-        if (leader) {
-          mma_bf16(tmem_base + a * 256, a_desc, b_desc, idesc, c > 0);
-          mma_bf16(tmem_base + a * 256, a_desc + 2, b_desc + 2, idesc, true);
-          mma_bf16(tmem_base + a * 256, a_desc + 4, b_desc + 4, idesc, true);
-          mma_bf16(tmem_base + a * 256, a_desc + 6, b_desc + 6, idesc, true);
+      const uint32_t stage = ring_base + s * stage_bytes;
+      const int last = min(kc, nchunks - i * kc);
+      if (leader) {
+        // an accumulator's MMAs follow one another at 86 cycles at the least; two accumulators take turns
+        for (int q = 0; q < last; ++q) {
+          const uint64_t a_desc = make_smem_desc_sw128(stage + q * a_tile);
+          const uint64_t b_desc = make_smem_desc_sw128(stage + a_bytes + q * b_tile);
+          const uint64_t b_next = make_smem_desc_sw128(stage + a_bytes + (kc + q) * b_tile);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            mma_bf16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (i | q | k) != 0);
+            if (p.NACC == 2) mma_bf16(tmem_base + 256, a_desc + 2 * k, b_next + 2 * k, idesc, (i | q | k) != 0);
+          }
         }
+        mma_commit(&bars[FREE + s]);
       }
-      if (leader) mma_commit(&bars[STAGE_FREE + s]);
       __syncwarp();
     }
     if (ok && leader) mma_commit(&bars[ACC_DONE]);
@@ -152,167 +238,161 @@ encode_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
   } else {
     const int row = tid & 127, wg = tid >> 7;
     const uint32_t lane_sel = static_cast<uint32_t>(32 * (warp & 3)) << 16;
-    // eight threads share a 128-byte row chunk (16 bytes each), a thread serves rows r0 + 32 i: loads and
-    // the swizzled stores touch whole lines
-    const int r0 = tid >> 3, piece = tid & 7;
-    {
-      // ---- residual operand: bf16((x - centre[id]) - mean), 8 columns of four rows per thread and
-      // chunk; the operands of two chunks are in flight while one is formed
-      const uint16_t* xrow[4];
-      const uint16_t* crow[4];
-      bool in[4];
+    // ---- residual operand: bf16((x - centre[id]) - mean), in the place of x.  Loads carry no conditions: a row that
+    // is not the tile's takes centre 0, a chunk past the row's end the last one, and what comes of them is not used.
+    const uint16_t* crow[SLOTS];
+    uint32_t place[SLOTS];
+    bool stored[SLOTS];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = r0 + 32 * j, t = m0 + r;
-        in[j] = r < p.rows && t < m_end;
-        xrow[j] = p.x + static_cast<size_t>(in[j] ? t : 0) * p.J + piece * 8;
-        crow[j] = p.centers + static_cast<size_t>(in[j] ? load_id(p.ids, p.id_bytes, t) : 0) * p.J + piece * 8;
+    for (int j = 0; j < SLOTS; ++j) {
+      const int r = first_row + row_step * j;
+      stored[j] = r < p.rows_pad;
+      place[j] = chunk_of * a_tile + (stored[j] ? r : 0) * 128 + ((piece ^ (r & 7)) << 4);
+      crow[j] = p.centers + static_cast<size_t>(ids[j]) * p.J + piece * 8;
+    }
+    uint4 cq[DEPTH][SLOTS];
+    auto fetch = [&](int buf, int i) {
+      const int j0 = min((i * kc + chunk_of) * 64, p.J - 64);
+#pragma unroll
+      for (int j = 0; j < SLOTS; ++j) cq[buf][j] = __ldg(reinterpret_cast<const uint4*>(crow[j] + j0));
+    };
+#pragma unroll
+    for (int b = 0; b < DEPTH; ++b) fetch(b, b);
+    const uint64_t minus_one = pair_f32(-1.f, -1.f);
+    Ring at;
+    auto step = [&](int buf, int i) {
+      const int s = at.stage;
+      ok = wait_all(&bars[FULL + s], at.phase, abort_flag, 440 + s);
+      if (!ok) return;
+      uint8_t* stage = ring + s * stage_bytes;
+      uint4 xv[SLOTS];
+#pragma unroll
+      for (int j = 0; j < SLOTS; ++j) xv[j] = *reinterpret_cast<const uint4*>(stage + place[j]);
+      const int j0 = min((i * kc + chunk_of) * 64, p.J - 64);
+      ulonglong2 m01, m23;
+      if (p.mean_bytes > 0) {
+        m01 = *reinterpret_cast<const ulonglong2*>(mean_smem + j0 + piece * 4);
+        m23 = *reinterpret_cast<const ulonglong2*>(mean_smem + j0 + 32 + piece * 4);
+      } else {
+        m01 = __ldg(reinterpret_cast<const ulonglong2*>(p.mean + j0 + piece * 8));
+        m23 = __ldg(reinterpret_cast<const ulonglong2*>(p.mean + j0 + piece * 8 + 4));
       }
-      uint4 xq[2][4], cq[2][4];
-      float4 mq[2][2];
-      auto fetch = [&](int buf, int i) {
-        if (i >= nchunks) return;
-        const int j0 = i * 64;
-        mq[buf][0] = __ldg(reinterpret_cast<const float4*>(p.mean + j0 + piece * 8));
-        mq[buf][1] = __ldg(reinterpret_cast<const float4*>(p.mean + j0 + piece * 8) + 1);
+      const uint64_t m2[4] = {m01.x, m01.y, m23.x, m23.y};
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (in[j]) {
-            xq[buf][j] = __ldg(reinterpret_cast<const uint4*>(xrow[j] + j0));
-            cq[buf][j] = __ldg(reinterpret_cast<const uint4*>(crow[j] + j0));
-          }
-      };
-      Ring at;
-      auto step = [&](int buf, int i) {
-        const int s = at.stage;
-        const float mv[8] = {mq[buf][0].x, mq[buf][0].y, mq[buf][0].z, mq[buf][0].w,
-                             mq[buf][1].x, mq[buf][1].y, mq[buf][1].z, mq[buf][1].w};
-        uint4 out[4];
+      for (int j = 0; j < SLOTS; ++j) {
+        const uint32_t xw[4] = {xv[j].x, xv[j].y, xv[j].z, xv[j].w};
+        const uint32_t cw[4] = {cq[buf][j].x, cq[buf][j].y, cq[buf][j].z, cq[buf][j].w};
+        uint32_t out[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          out[j] = make_uint4(0, 0, 0, 0);
-          if (in[j]) {
-            const uint32_t xw[4] = {xq[buf][j].x, xq[buf][j].y, xq[buf][j].z, xq[buf][j].w};
-            const uint32_t cw[4] = {cq[buf][j].x, cq[buf][j].y, cq[buf][j].z, cq[buf][j].w};
-            uint32_t* o = &out[j].x;
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              const float lo = __fsub_rn(__fsub_rn(__uint_as_float(xw[w] << 16), __uint_as_float(cw[w] << 16)), mv[2 * w]);
-              const float hi = __fsub_rn(__fsub_rn(__uint_as_float(xw[w] & 0xFFFF0000u),
-                                                   __uint_as_float(cw[w] & 0xFFFF0000u)), mv[2 * w + 1]);
-              o[w] = pack_bf16x2(lo, hi);
-            }
-          }
+        for (int w = 0; w < 4; ++w) {
+          // (x - c) - m in fp32, each difference rounded once: a + (-1) b is a - b
+          const uint64_t x2 = pair_bits(xw[w] << 16, xw[w] & 0xFFFF0000u), c2 = pair_bits(cw[w] << 16, cw[w] & 0xFFFF0000u);
+          float lo, hi;
+          split_f32(fma_f32x2(m2[w], minus_one, fma_f32x2(c2, minus_one, x2)), lo, hi);
+          out[w] = pack_bf16x2(lo, hi);
         }
-        fetch(buf, i + 2);
-        if (i >= nst) ok = wait_all(&bars[STAGE_FREE + s], at.phase ^ 1, abort_flag, 440 + s);
-        if (!ok) return;
-        at.advance(nst);
-        uint8_t* stage = smem + s * stage_bytes + r0 * 128 + ((piece ^ (r0 & 7)) << 4);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(stage + j * 32 * 128) = out[j];
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[A_FULL + s]);
-      };
-      fetch(0, 0);
-      fetch(1, 1);
-      for (int i = 0; i < nchunks && ok; i += 2) {
-        step(0, i);
-        if (i + 1 < nchunks && ok) step(1, i + 1);
+        if (stored[j]) *reinterpret_cast<uint4*>(stage + place[j]) = make_uint4(out[0], out[1], out[2], out[3]);
       }
-      if (ok) ok = wait_all(&bars[ACC_DONE], 0, abort_flag, 450);
-      if (ok && QUANT) {
-        // ---- quantise + pack from TMEM.  Pass 1: |max| of the bf16-rounded coefficients of this
-        // thread's column chunks; the two warpgroups, then the column parts' CTAs, combine.
-        tc_fence_after();
-        const int nc = p.NACC * p.NB;
-        const int tok = m0 + row;
-        float amax = 0.f;
+      fetch(buf, i + DEPTH);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[FORMED + s]);
+      at.advance(nst);
+    };
 #pragma unroll 1
-        for (int cc = wg; cc < nc / 32; cc += 2) {
-          const int col = cc * 32, acc = col / p.NB;
-          float v[32];
-          tmem_ld32(tmem_base + lane_sel + acc * 256 + (col - acc * p.NB), v);
+    for (int i = 0; i < steps && ok; i += DEPTH) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) amax = fmaxf(amax, fabsf(round_to_bf16(v[j])));
-        }
-        xn_part[wg * 128 + row] = amax;
-        mbar_arrive(&bars[SIDE_READY]);
-        ok = wait_all(&bars[SIDE_READY], 0, abort_flag, 451);
-        if (ok) {
-          amax = fmaxf(xn_part[row], xn_part[128 + row]);
-          if (joined) {
-            if (wg == 0) {
-              for (int peer = 0; peer < p.column_parts; ++peer) {
-                if (peer == part) continue;
-                st_cluster_b32(map_to_cta(smem_u32(&peer_max[part * 128 + row]), peer), __float_as_uint(amax));
-                mbar_arrive_cluster(map_to_cta(smem_u32(&bars[PEER_READY]), peer));
-              }
-            }
-            ok = wait_all_cluster(&bars[PEER_READY], 0, abort_flag, 452);
-            if (ok)
-              for (int peer = 0; peer < p.column_parts; ++peer)
-                if (peer != part) amax = fmaxf(amax, peer_max[peer * 128 + row]);
-          }
-        }
-        if (ok) {
-          float scale;
-          if (p.in_bf16) scale = round_to_bf16(__fdiv_rn(fmaxf(amax, round_to_bf16(p.eps)), 7.0f));
-          else scale = __fdiv_rn(fmaxf(amax, p.eps), 7.0f);
-          const float inv = __frcp_rn(scale);
+      for (int b = 0; b < DEPTH; ++b)
+        if (i + b < steps && ok) step(b, i + b);
+    }
+    if (ok) ok = wait_all(&bars[ACC_DONE], 0, abort_flag, 450);
+    const int tok = m0 + row;
+    const bool mine = row < p.rows && tok < m_end;
+    const int column_chunks = __any_sync(0xffffffffu, mine) ? columns / 32 : 0;
+    auto chunk = [&](int cc, uint32_t (&w)[16]) {
+      const int col = cc * 32, acc = col / p.NB;
+      float v[32];
+      tmem_ld32(tmem_base + lane_sel + acc * 256 + (col - acc * p.NB), v);
+      round_chunk(v, w);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w[i] = mine ? w[i] : 0u;     // rows that are nobody's hold anything
+      return n_base + col;
+    };
+    if (ok) tc_fence_after();
+    if (ok && QUANT && p.group32) {
+      // ---- one scale per 32 coefficients: a thread's chunk is a group
 #pragma unroll 1
-          for (int cc = wg; cc < nc / 32; cc += 2) {
-            const int col = cc * 32, acc = col / p.NB;
-            float v[32];
-            tmem_ld32(tmem_base + lane_sel + acc * 256 + (col - acc * p.NB), v);
-            uint32_t words[4];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-              uint32_t out = 0;
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float z0 = round_to_bf16(v[w * 8 + 2 * k]), z1 = round_to_bf16(v[w * 8 + 2 * k + 1]);
-                const int c0 = p.in_bf16 ? quant_code<true>(z0, scale, inv) : quant_code<false>(z0, scale, inv);
-                const int c1 = p.in_bf16 ? quant_code<true>(z1, scale, inv) : quant_code<false>(z1, scale, inv);
-                out |= static_cast<uint32_t>(c0 | (c1 << 4)) << (8 * k);
-              }
-              words[w] = out;
-            }
-            if (tok < m_end)
-              *reinterpret_cast<uint4*>(p.codes + static_cast<size_t>(tok) * (p.n_total >> 1) +
-                                        ((n_base + col) >> 1)) = make_uint4(words[0], words[1], words[2], words[3]);
-          }
-          if (wg == 0 && part == 0 && tok < m_end) store_float(p.scales, p.scale_dtype, tok, scale);
+      for (int cc = wg; cc < column_chunks; cc += GROUPS) {
+        uint32_t w[16], worst = 0;
+        const int col = chunk(cc, w);
+        const float scale = scale_of(max_magnitude(w, worst), p);
+        const uint4 words = pack_codes(w, scale, p.in_bf16, worst < NOT_FINITE);
+        if (mine) {
+          *reinterpret_cast<uint4*>(p.codes + static_cast<size_t>(tok) * (p.n_total >> 1) + (col >> 1)) = words;
+          store_float(p.scales, p.scale_dtype, static_cast<size_t>(tok) * (p.n_total / 32) + col / 32, scale);
         }
-      } else if (ok) {
-        tc_fence_after();
-        const int nc = p.NACC * p.NB;
-        const int tok = m0 + row;
+      }
+    } else if (ok && QUANT) {
+      // ---- one scale per token.  Pass 1: |max| of the bf16-rounded coefficients of this thread's column chunks;
+      // the two warpgroups, then the column parts' CTAs, combine.
+      float amax = 0.f;
+      uint32_t worst = 0;
 #pragma unroll 1
-        for (int cc = wg; cc < nc / 32; cc += 2) {
-          const int col = cc * 32, acc = col / p.NB;
-          float v[32];
-          tmem_ld32(tmem_base + lane_sel + acc * 256 + (col - acc * p.NB), v);
-          if (tok < m_end) {
-            uint16_t* dst = p.coeff + static_cast<size_t>(tok) * p.n_total + n_base + col;
+      for (int cc = wg; cc < column_chunks; cc += GROUPS) {
+        uint32_t w[16];
+        chunk(cc, w);
+        amax = fmaxf(amax, max_magnitude(w, worst));
+      }
+      meta.row_max[wg][row] = amax;
+      mbar_arrive(&bars[SIDE_READY]);
+      ok = wait_all(&bars[SIDE_READY], 0, abort_flag, 451);
+      if (ok) {
 #pragma unroll
-            for (int j4 = 0; j4 < 4; ++j4) {
-              uint4 w;
-              w.x = pack_bf16x2(v[j4 * 8 + 0], v[j4 * 8 + 1]);
-              w.y = pack_bf16x2(v[j4 * 8 + 2], v[j4 * 8 + 3]);
-              w.z = pack_bf16x2(v[j4 * 8 + 4], v[j4 * 8 + 5]);
-              w.w = pack_bf16x2(v[j4 * 8 + 6], v[j4 * 8 + 7]);
-              *reinterpret_cast<uint4*>(dst + j4 * 8) = w;
+        for (int g = 0; g < GROUPS; ++g) amax = fmaxf(amax, meta.row_max[g][row]);
+        if (joined) {
+          cluster_wait();
+          met = true;
+          if (wg == 0) {
+            for (int peer = 0; peer < p.parts; ++peer) {
+              if (peer == part) continue;
+              st_cluster_b32(map_to_cta(smem_u32(&meta.peer_max[part][row]), peer), __float_as_uint(amax));
+              mbar_arrive_cluster(map_to_cta(smem_u32(&bars[PEER_READY]), peer));
             }
           }
+          ok = wait_all_cluster(&bars[PEER_READY], 0, abort_flag, 452);
+          if (ok)
+            for (int peer = 0; peer < p.parts; ++peer)
+              if (peer != part) amax = fmaxf(amax, meta.peer_max[peer][row]);
+        }
+      }
+      if (ok) {
+        const float scale = scale_of(amax, p);
+#pragma unroll 1
+        for (int cc = wg; cc < column_chunks; cc += GROUPS) {
+          uint32_t w[16];
+          const int col = chunk(cc, w);
+          const uint4 words = pack_codes(w, scale, p.in_bf16, worst < NOT_FINITE);
+          if (mine) *reinterpret_cast<uint4*>(p.codes + static_cast<size_t>(tok) * (p.n_total >> 1) + (col >> 1)) = words;
+        }
+        if (wg == 0 && part == 0 && mine) store_float(p.scales, p.scale_dtype, tok, scale);
+      }
+    } else if (ok) {
+#pragma unroll 1
+      for (int cc = wg; cc < column_chunks; cc += GROUPS) {
+        uint32_t w[16];
+        const int col = chunk(cc, w);
+        if (mine) {
+          uint4* dst = reinterpret_cast<uint4*>(p.coeff + static_cast<size_t>(tok) * p.n_total + col);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
         }
       }
     }
   }
+  if (joined && !met) cluster_wait();
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tmem_base, 512);
+  if (warp == WARPS + 1) tmem_dealloc(tmem_base, p.tmem_columns);
   // no CTA of a tile leaves while another may still write into its shared memory
   if (joined) cluster_sync_all();
 }
@@ -328,94 +408,118 @@ bool plan_columns(int n_total, int* gy, int* nacc, int* nb) {
   return false;
 }
 
-// n_norms: centres whose squared norms are kept (assign); 512 floats of them, or the parts' row maxima
-size_t meta_bytes(int n_norms) {
-  const size_t tail = 8 * static_cast<size_t>(n_norms);
-  return META_HEAD + 4 * (256 + 128 + 128) + (tail > 4 * MAX_PARTS * 128 ? tail : 4 * MAX_PARTS * 128);
-}
-
-size_t ring_bytes(int nacc, int nb, int stages) { return stages * static_cast<size_t>(A_BYTES + nacc * nb * 128); }
-
-size_t smem_bytes(int nacc, int nb, int n_total, int stages = 2) {
-  return ring_bytes(nacc, nb, stages) + meta_bytes(n_total) + 1024;
-}
-
 constexpr size_t SMEM_LIMIT = 232448;
 
-// How a GEMM of S tokens x `columns` over `chunks` stages is cut: tokens per tile and column parts.
-// The estimate counts SM cycles: a stage costs the bytes it takes from L2 (token rows, centre rows, B) at
-// 48 bytes per clock, at least 350 cycles of latency.  Column parts of the projection form clusters of up
-// to eight, of which 128 of the 148 SMs hold whole ones at a time, of four about 144.
-// Bound of short calls: 880 tokens x 3,072 columns x rank 384 in tiles of 128 whole rows keep 14 SMs busy for
-// 48 stages of operand latency (107 us; 39 with six column parts); 4,680 x 5,120 x 640 71 (128 before the
-// operands of two chunks were in flight); assignment to 64 fp32 centres 880 x 3,072 49 (70), 4,680 x 5,120 80
-// (116).  Cutting K over a cluster as well was faster still for given centres (assignment of 1,560 x 3,072 to
-// 256 centres 28 us against 60), but then the order of a row's fp32 sums, and now and then a code or an id,
-// depends on the length of the call.
-struct Split { int rows, column_parts; };
+size_t mean_bytes(int J) { return J <= MAX_MEAN ? static_cast<size_t>(J) * 4 : 0; }
 
-Split plan_split(int S, int chunks, int columns, int column_parts, bool residual) {
-  const int sms = sm_count();
-  Split best{pick_rows(S, column_parts), column_parts};
-  auto stage_cost = [&](int rows, int cols) {
-    const double bytes = rows * (residual ? 256.0 : 128.0) + cols * 128.0;
-    return bytes / 48 > 350 ? bytes / 48 : 350.0;
-  };
-  auto rounds = [](long long ctas, int room) { return static_cast<double>((ctas + room - 1) / room); };
-  double best_cost = rounds(static_cast<long long>(ceil_div(S, best.rows)) * column_parts, sms) *
-                     (chunks * stage_cost(best.rows, columns / column_parts) + 3000);
-  for (int rows = 64; rows <= TM; rows *= 2)
-    for (int h = column_parts; h <= (residual ? MAX_PARTS : column_parts); ++h) {
-      const int cols = columns / h;
-      if (columns % h || cols > 512 || cols % (cols > 256 ? 64 : 32)) continue;
-      const int room = h > 4 ? sms - 20 : (h > 2 ? sms - 4 : sms);
-      const double cost = rounds(static_cast<long long>(ceil_div(S, rows)) * h, room) *
-                          (chunks * stage_cost(rows, cols) + 3000 + 300 * h);
-      if (cost < best_cost) {
+// the MMA reads 128 rows from where the last token tile starts, which may reach past the ring
+size_t smem_bytes(int J, int rows_pad, int columns, int kc, int stages) {
+  const size_t stage = static_cast<size_t>(kc) * (rows_pad + columns) * 128;
+  const size_t end = stages * stage, last_a = (stages - 1) * stage + static_cast<size_t>(kc - 1) * rows_pad * 128;
+  const size_t reach = last_a + TM * 128;
+  return sizeof(Meta) + 16 + mean_bytes(J) + 1024 + (reach > end ? reach : end);
+}
+
+// Tokens per tile, column parts and chunks of a stage.  The estimate counts SM cycles.  A 64-column chunk costs the
+// longer of its bytes from L2 (encoder rows, x and centre rows) at 45 per clock and its MMAs (four in a chain of 86
+// cycles each at the least).  Clusters of more than four fill 128 of the 148 SMs, of three or four 144.
+struct Cut { int rows, parts, kc, stages; };
+
+Cut plan_project(int S, int J, int r, int first_parts, bool cluster) {
+  const int sms = sm_count(), chunks = J / 64;
+  Cut best{0, 0, 0, 0};
+  double best_cost = -1;
+  const int candidates[5] = {pick_rows(S, first_parts), 128, 96, 64, 32};
+  for (int rows : candidates)
+    for (int h = first_parts; h <= (cluster ? MAX_PARTS : 16); ++h) {
+      const int cols = r / h, nacc = cols > 256 ? 2 : 1;
+      if (r % h || cols > 512 || cols % (nacc == 2 ? 64 : 32)) continue;
+      const int rows_pad = (rows + 7) / 8 * 8;
+      Cut cut{rows, h, rows_pad <= 32 ? 4 : (rows_pad <= 64 ? 2 : 1), MAX_STAGES};
+      while (cut.kc > 1 && smem_bytes(J, rows_pad, cols, cut.kc, 3) > SMEM_LIMIT) cut.kc /= 2;
+      while (cut.stages > 2 && smem_bytes(J, rows_pad, cols, cut.kc, cut.stages) > SMEM_LIMIT) --cut.stages;
+      const int room = !cluster ? sms : h > 4 ? sms - 20 : (h > 2 ? sms - 4 : sms);
+      const double bytes = (rows * 256.0 + cols * 128.0) / 45;
+      const double mma = nacc == 2 ? (4.0 * cols / 2 > 390 ? 4.0 * cols / 2 : 390) : (2.0 * cols > 340 + cols / 4 ? 2.0 * cols : 340 + cols / 4);
+      const double chunk = bytes > mma ? bytes : mma;
+      const double cost = static_cast<double>((static_cast<long long>(ceil_div(S, rows)) * h + room - 1) / room) *
+                          (chunk * chunks + 18000 + cols * 20);
+      if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;
-        best = Split{rows, h};
+        best = cut;
       }
     }
   return best;
 }
 
-// accumulators of one CTA's columns
-void set_columns(Params& p, int columns) {
-  p.NACC = columns > 256 ? 2 : 1;
-  p.NB = columns / p.NACC;
-}
-
-template <int MODE>
-int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, Params& p, int n_norms, const char* name,
-                cudaStream_t stream) {
-  p.nstages = MAX_STAGES;
-  while (p.nstages > 2 && smem_bytes(p.NACC, p.NB, n_norms, p.nstages) > SMEM_LIMIT) --p.nstages;
-  const size_t smem = smem_bytes(p.NACC, p.NB, n_norms, p.nstages);
-  NKV_REQUIRE(smem <= SMEM_LIMIT, NKV_ERR_UNSUPPORTED, "%s needs %zu bytes of shared memory", name, smem);
-  auto kernel = encode_gemm_kernel<MODE>;
+template <bool QUANT, int SLOTS, int DEPTH>
+int launch_slots(const CUtensorMap (&maps)[2], const Params& p, size_t smem, cudaStream_t stream) {
+  auto kernel = project_gemm_kernel<QUANT, SLOTS, DEPTH>;
   NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   cudaLaunchConfig_t config{};
-  config.gridDim = dim3(static_cast<unsigned>(ceil_div(p.S, p.rows)) * p.column_parts);
+  config.gridDim = dim3(static_cast<unsigned>(ceil_div(p.S, p.rows)) * p.parts);
   config.blockDim = dim3(THREADS);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = MODE == PROJECT_QUANT ? p.column_parts : 1;
+  attr.val.clusterDim.x = QUANT && !p.group32 ? p.parts : 1;
   attr.val.clusterDim.y = 1;
   attr.val.clusterDim.z = 1;
   config.attrs = &attr;
   config.numAttrs = 1;
-  NKV_CUDA(cudaLaunchKernelEx(&config, kernel, map_a, map_b, p));
+  NKV_CUDA(cudaLaunchKernelEx(&config, kernel, maps[0], maps[1], p));
   return NKV_OK;
+}
+
+template <bool QUANT>
+int launch_project(const void* x, const void* centers, const void* encoder, Params& p, cudaStream_t stream) {
+  NKV_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(centers) & 15) == 0 &&
+                  (reinterpret_cast<uintptr_t>(p.mean) & 15) == 0 &&
+                  (reinterpret_cast<uintptr_t>(QUANT ? static_cast<const void*>(p.codes) : p.coeff) & 15) == 0 &&
+                  (!QUANT || (p.n_total / 2) % 16 == 0),
+              NKV_ERR_INVALID, "projection operands must be 16-byte aligned");
+  int gy, nacc, nb;
+  NKV_REQUIRE(plan_columns(p.n_total, &gy, &nacc, &nb), NKV_ERR_UNSUPPORTED, "projection rank %d cannot be tiled", p.n_total);
+  NKV_REQUIRE(!QUANT || p.group32 || gy <= 2, NKV_ERR_UNSUPPORTED,
+              "fused projection: rank %d cannot be tiled over at most two column parts", p.n_total);
+  const Cut cut = plan_project(p.S, p.J, p.n_total, gy, QUANT && !p.group32);
+  p.rows = cut.rows; p.parts = cut.parts; p.kc = cut.kc; p.nstages = cut.stages;
+  p.rows_pad = (p.rows + 7) / 8 * 8;
+  const int columns = p.n_total / p.parts;
+  p.NACC = columns > 256 ? 2 : 1;
+  p.NB = columns / p.NACC;
+  p.tmem_columns = p.NACC == 2 ? 512 : (p.NB > 128 ? 256 : (p.NB > 64 ? 128 : (p.NB > 32 ? 64 : 32)));
+  p.nchunks = p.J / 64;
+  p.mean_bytes = static_cast<int>(mean_bytes(p.J));
+  p.centers = static_cast<const uint16_t*>(centers);
+  const size_t smem = smem_bytes(p.J, p.rows_pad, columns, p.kc, p.nstages);
+  NKV_REQUIRE(smem <= SMEM_LIMIT, NKV_ERR_UNSUPPORTED, "projection: %zu bytes of shared memory", smem);
+  CUtensorMap maps[2];     // rows, encoder
+  const uint64_t chunk_strides[2] = {static_cast<uint64_t>(p.J) * 2, 128};
+  {
+    const uint64_t dims[3] = {64, static_cast<uint64_t>(p.S), static_cast<uint64_t>(p.nchunks)};
+    const uint32_t box[3] = {64, static_cast<uint32_t>(p.rows_pad), static_cast<uint32_t>(p.kc)};
+    const int rc = encode_tensor_map(&maps[0], 2, x, 3, dims, chunk_strides, box, 128);
+    if (rc != NKV_OK) return rc;
+  }
+  {
+    const uint64_t dims[3] = {64, static_cast<uint64_t>(p.n_total), static_cast<uint64_t>(p.nchunks)};
+    const uint32_t box[3] = {64, static_cast<uint32_t>(p.NB), static_cast<uint32_t>(p.kc)};
+    const int rc = encode_tensor_map(&maps[1], 2, encoder, 3, dims, chunk_strides, box, 128);
+    if (rc != NKV_OK) return rc;
+  }
+  const int slots = ceil_div(p.rows_pad, COMPUTE_THREADS / 8 / p.kc);
+  if (slots <= 1) return launch_slots<QUANT, 1, 6>(maps, p, smem, stream);
+  if (slots <= 2) return launch_slots<QUANT, 2, 4>(maps, p, smem, stream);
+  return launch_slots<QUANT, 4, 3>(maps, p, smem, stream);
 }
 
 }  // namespace
 
 bool tc_project_supported(int J, int r) {
   int gy, nacc, nb;
-  return J % 64 == 0 && plan_columns(r, &gy, &nacc, &nb) &&
-         smem_bytes(nacc, nb, 0) <= 232448;
+  return J % 64 == 0 && plan_columns(r, &gy, &nacc, &nb);
 }
 
 // SM count of the current device, cached per device ordinal
@@ -452,66 +556,30 @@ int tc_project(const void* x_bf16, const void* centers_bf16, const void* ids, in
                cudaStream_t stream) {
   if (S == 0) return NKV_OK;
   Params p{};
-  int gy;
-  NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB), NKV_ERR_UNSUPPORTED,
-              "projection rank %d cannot be tiled", r);
-  const Split cut = plan_split(S, J / 64, r, gy, true);
-  p.rows = cut.rows; p.column_parts = cut.column_parts;
-  set_columns(p, r / p.column_parts);
-  NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(centers_bf16) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(mean) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(coeff) & 15) == 0,
-              NKV_ERR_INVALID, "projection operands must be 16-byte aligned");
   p.S = S; p.J = J; p.n_total = r;
-  p.x = static_cast<const uint16_t*>(x_bf16);
-  p.centers = static_cast<const uint16_t*>(centers_bf16);
   p.ids = ids; p.id_bytes = id_bytes; p.mean = mean;
   p.coeff = static_cast<uint16_t*>(coeff);
-  CUtensorMap map_b;
-  uint64_t dims[2] = {static_cast<uint64_t>(J), static_cast<uint64_t>(r)};
-  uint64_t strides[1] = {static_cast<uint64_t>(J) * 2};
-  uint32_t box[2] = {64, static_cast<uint32_t>(p.NB)};
-  int rc = encode_tensor_map(&map_b, 2, encoder_bf16, 2, dims, strides, box, 128);
-  if (rc != NKV_OK) return rc;
-  return launch_gemm<PROJECT>(map_b, map_b, p, 0, "encode_gemm_kernel<project>", stream);
+  return launch_project<false>(x_bf16, centers_bf16, encoder_bf16, p, stream);
 }
 
 bool tc_project_quant_supported(int J, int r, int group) {
   int gy, nacc, nb;
-  return group == r && r % 64 == 0 && tc_project_supported(J, r) && plan_columns(r, &gy, &nacc, &nb) && gy <= 2;
+  if (!tc_project_supported(J, r) || !plan_columns(r, &gy, &nacc, &nb)) return false;
+  return group == r ? r % 64 == 0 && gy <= 2 : group == 32;
 }
 
 int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* ids, int id_bytes,
-                     const float* mean, const void* encoder_bf16, int S, int J, int r, float eps,
+                     const float* mean, const void* encoder_bf16, int S, int J, int r, int group, float eps,
                      int quant_mode, int scale_dtype, uint8_t* codes, void* scales, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
   Params p{};
-  int gy;
-  NKV_REQUIRE(plan_columns(r, &gy, &p.NACC, &p.NB) && gy <= 2, NKV_ERR_UNSUPPORTED,
-              "fused projection: rank %d cannot be tiled over at most two column parts", r);
-  const Split cut = plan_split(S, J / 64, r, gy, true);
-  p.rows = cut.rows; p.column_parts = cut.column_parts;
-  set_columns(p, r / p.column_parts);
-  NKV_REQUIRE((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(centers_bf16) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(mean) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(codes) & 15) == 0 && (r / 2) % 16 == 0,
-              NKV_ERR_INVALID, "fused projection operands must be 16-byte aligned");
   p.S = S; p.J = J; p.n_total = r;
-  p.x = static_cast<const uint16_t*>(x_bf16);
-  p.centers = static_cast<const uint16_t*>(centers_bf16);
   p.ids = ids; p.id_bytes = id_bytes; p.mean = mean;
   p.codes = codes; p.scales = scales; p.eps = eps;
   p.in_bf16 = quant_mode == NKV_QUANT_IN_BF16 ? 1 : 0;
   p.scale_dtype = scale_dtype;
-  CUtensorMap map_b;
-  uint64_t dims[2] = {static_cast<uint64_t>(J), static_cast<uint64_t>(r)};
-  uint64_t strides[1] = {static_cast<uint64_t>(J) * 2};
-  uint32_t box[2] = {64, static_cast<uint32_t>(p.NB)};
-  int rc = encode_tensor_map(&map_b, 2, encoder_bf16, 2, dims, strides, box, 128);
-  if (rc != NKV_OK) return rc;
-  return launch_gemm<PROJECT_QUANT>(map_b, map_b, p, 0, "encode_gemm_kernel<project + quantise>", stream);
+  p.group32 = group != r ? 1 : 0;
+  return launch_project<true>(x_bf16, centers_bf16, encoder_bf16, p, stream);
 }
 
 }  // namespace nkv

@@ -119,7 +119,8 @@ def project_quant(x, centers_bf16, ids, mean, encoder, *, group=None, eps=1.1920
                   in_coeff_dtype=False, scale_dtype=torch.bfloat16, codes=None, scales=None):
     """project + quant_pack of rows whose centre ids are known -> (codes u8 [S,r/2], scales
     [S,r/group]); one kernel (coefficients never leave the chip) for bf16 operands with one scale per
-    token, the two kernels through a scratch tensor otherwise.  Same bytes either way."""
+    token or per 32 coefficients, the two kernels through a scratch tensor otherwise.  Same bytes either way
+    (groups of finite coefficients: others have no defined codes)."""
     device = _require_cuda(x, centers_bf16, ids, mean, encoder, codes, scales)
     S, J = x.shape
     r = encoder.shape[0]
@@ -128,7 +129,8 @@ def project_quant(x, centers_bf16, ids, mean, encoder, *, group=None, eps=1.1920
         codes = torch.empty(S, r // 2, dtype=torch.uint8, device=device)
     if scales is None:
         scales = torch.empty(S, r // group, dtype=scale_dtype, device=device)
-    fused = (x.dtype == encoder.dtype == torch.bfloat16 and group == r and r % 64 == 0
+    fused = (x.dtype == encoder.dtype == torch.bfloat16
+             and (group == r and r % 64 == 0 or group == 32 and r % 32 == 0) and J % 64 == 0
              and not _SIMT_FORCED[0] and codes.data_ptr() % 16 == 0)
     workspace = None if fused else torch.empty(S, r, dtype=encoder.dtype, device=device)
     status = _lib.library().nkv_project_quant(

@@ -40,3 +40,30 @@ def test_long_calls_assign_every_row(S):
         pick = torch.randint(0, C, (S,), generator=gen, device="cuda")
         rows = (centers[pick].float() + 0.3 * torch.randn(S, 256, generator=gen, device="cuda")).to(torch.bfloat16)
         assert torch.equal(ops.assign(rows, centers).long() & 0xFFFF, pick)
+
+
+@pytest.mark.parametrize("S", [1, 31, 65, 400, 3000])
+@pytest.mark.parametrize("J,r", [(64, 32), (192, 96), (1536, 160), (448, 640), (8256, 64)])
+def test_groups_of_32_are_quantised_in_place(S, J, r):
+    rows, centers, encoder, mean = _data(S, J, 16, r, seed=S)
+    ids = ops.assign(rows, centers)
+    coeff = ops.project(rows, centers, ids, mean, encoder)
+    for in_coeff_dtype in (False, True):
+        for scale_dtype in (torch.float16, torch.bfloat16):
+            form = dict(group=32, in_coeff_dtype=in_coeff_dtype, scale_dtype=scale_dtype)
+            one, two = ops.project_quant(rows, centers, ids, mean, encoder, **form), ops.quant_pack(coeff, **form)
+            assert torch.equal(one[0], two[0]) and torch.equal(one[1].view(torch.int16), two[1].view(torch.int16))
+
+
+def test_rows_that_are_not_finite_leave_their_neighbours_alone():
+    rows, centers, encoder, mean = _data(300, 1536, 16, 192, seed=5)
+    ids = ops.assign(rows, centers)
+    clean = {g: ops.project_quant(rows, centers, ids, mean, encoder, group=g) for g in (192, 32)}
+    bad = rows.clone()
+    bad[7, 3], bad[64, 1000], bad[299, 0] = float("inf"), float("nan"), -float("inf")
+    keep = torch.ones(300, dtype=torch.bool, device="cuda")
+    keep[[7, 64, 299]] = False
+    for group, want in clean.items():
+        codes, scales = ops.project_quant(bad, centers, ids, mean, encoder, group=group)
+        assert torch.equal(codes[keep], want[0][keep]) and torch.equal(scales[keep], want[1][keep])
+        assert bool(((codes & 15) <= 14).all() and ((codes >> 4) <= 14).all())
