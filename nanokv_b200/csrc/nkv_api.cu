@@ -133,14 +133,13 @@ int nkv_assign(const void* x, int x_dtype, const void* centers, int centers_dtyp
   return simt_assign(x, x_dtype, centers, centers_dtype, S, J, C, ids, id_bytes, nullptr, s);
 }
 
-// fp32 centres, 32-bit labels, and (for the tensor-core assignment of bf16 rows) the centres' three
-// bf16 planes with their squared norms
+// fp32 centres, 32-bit labels, and (for the tensor-core assignment of bf16 rows) the centres' three bf16 planes
 static size_t kmeans_planes_offset(int S, int J, int C) {
   const size_t head = sizeof(float) * static_cast<size_t>(C) * J + sizeof(int32_t) * static_cast<size_t>(S);
   return (head + 255) / 256 * 256;
 }
 size_t nkv_kmeans_workspace_bytes(int S, int J, int C) {
-  return kmeans_planes_offset(S, J, C) + tc_assign_f32_workspace_bytes(J, C) + 256;
+  return kmeans_planes_offset(S, J, C) + static_cast<size_t>(C) * 3 * J * 2 + 256;
 }
 
 int nkv_kmeans(const void* x, int x_dtype, int S, int J, int C, int iters,
@@ -157,23 +156,30 @@ int nkv_kmeans(const void* x, int x_dtype, int S, int J, int C, int iters,
   auto s = static_cast<cudaStream_t>(stream);
   float* centers = static_cast<float*>(workspace);
   int32_t* labels = reinterpret_cast<int32_t*>(centers + static_cast<size_t>(C) * J);
-  int rc = kmeans_gather_init(x, x_dtype, J, C, init_rows, centers, s);
-  if (rc != NKV_OK) return rc;
-  NKV_CUDA(cudaMemsetAsync(labels, 0, sizeof(int32_t) * S, s));
   // bf16 rows: the assignment runs on the tensor cores against the fp32 centres split into bf16
   // planes (fp32-accurate distances); anything else on the fp32 CUDA-core kernel
-  const bool planes = x_dtype == NKV_BF16 && !simt_forced() && tc_assign_supported(J, C) &&
+  const bool tensor = x_dtype == NKV_BF16 && !simt_forced() && tc_assign_supported(J, C) &&
                       (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   uint8_t* plane_space = static_cast<uint8_t*>(workspace) + kmeans_planes_offset(S, J, C);
   plane_space += (256 - (reinterpret_cast<uintptr_t>(plane_space) & 255)) & 255;
+  uint16_t* planes = tensor ? reinterpret_cast<uint16_t*>(plane_space) : nullptr;
+  int rc = kmeans_gather_init(x, x_dtype, J, C, init_rows, centers, planes, s);
+  if (rc != NKV_OK) return rc;
+  if (iters == 0) {
+    NKV_CUDA(cudaMemsetAsync(labels, 0, sizeof(int32_t) * S, s));
+    return kmeans_store(centers, labels, S, J, C, centers_bf16, ids, id_bytes, s);
+  }
+  // the last pass stores what a caller keeps: the ids with the labels, the centres with the means
   for (int it = 0; it < iters; ++it) {
-    rc = planes ? tc_assign_f32(x, centers, S, J, C, labels, plane_space, s)
-                : simt_assign(x, x_dtype, centers, NKV_F32, S, J, C, nullptr, id_bytes, labels, s);
+    const bool last = it == iters - 1;
+    rc = tensor ? tc_assign_f32(x, centers, planes, S, J, C, labels, last ? ids : nullptr, id_bytes, s)
+                : simt_assign(x, x_dtype, centers, NKV_F32, S, J, C, last ? ids : nullptr, id_bytes, labels, s);
     if (rc != NKV_OK) return rc;
-    rc = kmeans_update(x, x_dtype, S, J, C, labels, centers, s);
+    rc = kmeans_update(x, x_dtype, S, J, C, labels, centers, last ? nullptr : planes,
+                       last ? static_cast<uint16_t*>(centers_bf16) : nullptr, s);
     if (rc != NKV_OK) return rc;
   }
-  return kmeans_store(centers, labels, S, J, C, centers_bf16, ids, id_bytes, s);
+  return NKV_OK;
 }
 
 int nkv_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,

@@ -34,9 +34,10 @@ int camera_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_hea
 int rope_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head, int S, int heads,
               int d, const nkv_rope& rope, void* out, cudaStream_t stream);
 int kmeans_gather_init(const void* x, int x_dtype, int J, int C, const int32_t* init_rows,
-                       float* centers, cudaStream_t stream);
+                       float* centers, uint16_t* planes, cudaStream_t stream);
+// planes: bf16 [C, 3 J] for the next tc_assign_f32, or NULL; stored: bf16 [C, J], or NULL
 int kmeans_update(const void* x, int x_dtype, int S, int J, int C, const int32_t* labels,
-                  float* centers, cudaStream_t stream);
+                  float* centers, uint16_t* planes, uint16_t* stored, cudaStream_t stream);
 int kmeans_store(const float* centers, const int32_t* labels, int S, int J, int C,
                  void* centers_bf16, void* ids, int id_bytes, cudaStream_t stream);
 
@@ -120,8 +121,7 @@ int tc_project_quant(const void* x_bf16, const void* centers_bf16, const void* i
                      const float* mean, const void* encoder_bf16, int S, int J, int r, int group, float eps,
                      int quant_mode, int scale_dtype, uint8_t* codes, void* scales, cudaStream_t stream);
 bool tc_assign_supported(int J, int C);
-size_t tc_assign_f32_workspace_bytes(int J, int C);
-int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, int C, int32_t* labels,
-                  void* workspace, cudaStream_t stream);
+int tc_assign_f32(const void* x_bf16, const float* centers_f32, const uint16_t* planes, int S, int J, int C,
+                  int32_t* labels, void* ids, int id_bytes, cudaStream_t stream);
 
 }  // namespace nkv

@@ -311,23 +311,192 @@ int launch_attn(const AttnArgs& a, cudaStream_t stream) {
 }
 
 // -------------------------------------------------------------------- k-means
-__global__ void gather_init_kernel(const void* x, int x_dtype, int J, const int32_t* init_rows,
-                                   float* centers) {
-  const int c = blockIdx.x, j = blockIdx.y * blockDim.x + threadIdx.x;
-  if (j < J) centers[static_cast<size_t>(c) * J + j] = load_float(x, x_dtype, static_cast<size_t>(init_rows[c]) * J + j);
+// One centre value as the assignment on the tensor cores takes it: three bf16 planes side by side along a row of
+// [C, 3 J] (v = hi + mid + lo exactly, up to the last bit of the third).
+__device__ __forceinline__ void split_planes(float v, uint16_t& hi, uint16_t& mid, uint16_t& lo) {
+  hi = float_to_bf16_bits(v);
+  const float r1 = __fsub_rn(v, bf16_bits_to_float(hi));
+  mid = float_to_bf16_bits(r1);
+  lo = float_to_bf16_bits(__fsub_rn(r1, bf16_bits_to_float(mid)));
 }
 
-// Columns of a row as a thread of the update holds them in flight: a bf16 pair, an fp32 pair, or one
-// column of either type.
+__global__ void gather_init_kernel(const void* x, int x_dtype, int J, const int32_t* init_rows,
+                                   float* centers, uint16_t* planes) {
+  const int c = blockIdx.x, j = blockIdx.y * blockDim.x + threadIdx.x;
+  if (j >= J) return;
+  const float v = load_float(x, x_dtype, static_cast<size_t>(init_rows[c]) * J + j);
+  centers[static_cast<size_t>(c) * J + j] = v;
+  if (planes != nullptr) {
+    uint16_t* out = planes + static_cast<size_t>(c) * 3 * J + j;
+    split_planes(v, out[0], out[J], out[2 * J]);
+  }
+}
+
+// The update: block (c, column block) sets centre c to the mean of the rows labelled c, summed in increasing token
+// order (one fp32 addition per row, the order a sequential scatter-add takes) so that the result does not depend on
+// the launch shape.  An empty cluster keeps its centre.  The new centre leaves as the next assignment's planes
+// (`planes`) or as the stored centre (`stored`) too.
+constexpr int UPDATE_SPAN = 8192;                       // labels taken at a time
+
+// The tokens of [s0, s0 + len) labelled c, in order, into `list`; gives their number.  A warp looks at a run of labels,
+// 128 at a time in whole lines (four per lane), keeps the matches as bits, and writes its tokens behind those of the
+// warps before it.
+template <int THREADS_>
+__device__ __forceinline__ int list_members(const int32_t* labels, int s0, int len, int c, uint16_t* list, int* warp_total) {
+  constexpr int WARPS_ = THREADS_ / 32;
+  static_assert(UPDATE_SPAN / WARPS_ <= 16 * 128, "a lane keeps 16 times four matches");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rounds = (len + WARPS_ * 128 - 1) / (WARPS_ * 128), first = warp * rounds * 128 + lane * 4;
+  const bool vector = (reinterpret_cast<uintptr_t>(labels) & 15) == 0;
+  uint64_t match = 0;
+#pragma unroll 4
+  for (int r = 0; r < rounds; ++r) {
+    const int at = first + r * 128;
+    uint32_t m = 0;
+    if (vector && at + 4 <= len) {
+      const int4 l = __ldg(reinterpret_cast<const int4*>(labels + s0 + at));
+      m = (l.x == c ? 1u : 0u) | (l.y == c ? 2u : 0u) | (l.z == c ? 4u : 0u) | (l.w == c ? 8u : 0u);
+    } else {
+      for (int i = 0; i < 4; ++i)
+        if (at + i < len && __ldg(labels + s0 + at + i) == c) m |= 1u << i;
+    }
+    match |= static_cast<uint64_t>(m) << (4 * r);
+  }
+  const int mine = __reduce_add_sync(0xffffffffu, __popcll(match));
+  __syncthreads();                                        // the previous list has been consumed
+  if (lane == 0) warp_total[warp] = mine;
+  __syncthreads();
+  int base = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < WARPS_; ++w) {
+    if (w < warp) base += warp_total[w];
+    total += warp_total[w];
+  }
+  for (int r = 0; r < rounds; ++r) {
+    const uint32_t m = static_cast<uint32_t>(match >> (4 * r)) & 15u;
+    int before = 0, all = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t votes = __ballot_sync(0xffffffffu, (m >> e) & 1u);
+      before += __popc(votes & ((1u << lane) - 1u));
+      all += __popc(votes);
+    }
+    int at = base + before;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if ((m >> e) & 1u) list[at++] = static_cast<uint16_t>(first + r * 128 + e);
+    base += all;
+  }
+  __syncthreads();
+  return total;
+}
+
+template <int COLS>
+__device__ __forceinline__ void store_centre(const float (&sum)[COLS], int count, int c, int j, int J, float* centers,
+                                             uint16_t* planes, uint16_t* stored) {
+  float* centre = centers + static_cast<size_t>(c) * J + j;
+  uint16_t* plane = planes == nullptr ? nullptr : planes + static_cast<size_t>(c) * 3 * J + j;
+#pragma unroll
+  for (int q = 0; q < COLS; ++q) {
+    float v = 0.f;
+    if (count > 0) {
+      v = __fdiv_rn(sum[q], static_cast<float>(count));
+      centre[q] = v;
+      if (plane != nullptr) split_planes(v, plane[q], plane[J + q], plane[2 * J + q]);
+    } else if (stored != nullptr) {
+      v = centre[q];
+    }
+    if (stored != nullptr) stored[static_cast<size_t>(c) * J + j + q] = float_to_bf16_bits(v);
+  }
+}
+
+// Rows of bf16 or fp32, four columns per thread.  Bound: the chain of row loads of the largest cluster -- start rows
+// drawn from one true cluster leave others to be shared, so a cluster can hold several times the mean.  The members'
+// pieces run through a ring in shared memory that every thread fills for itself: registers filled in
+// turn share a handful of scoreboards, and waiting for one waits for the ones filled after it.
+// us per call, 64 centres, 4,680 x 5,120 / 880 x 3,072 / 8,000 x 1,536: 41 / 9 / 52 with two columns per thread, 32 row
+// loads at a time and a thread's labels side by side (32 lines per load of a warp); 35 / 9 / 42 with this ring in groups
+// of four rows and labels in whole lines; 22 / 6 / 25 with groups of eight whose places come in one load.
+constexpr int RING_THREADS = 128, RING_GROUP = 8;
+template <int BYTES>     // of an element
+__global__ void __launch_bounds__(RING_THREADS)
+kmeans_update_ring_kernel(const void* x, int S, int J, const int32_t* labels, float* centers, uint16_t* planes,
+                          uint16_t* stored) {
+  constexpr int PIECE = 4 * BYTES, GROUPS = BYTES == 2 ? 3 : 2;   // 24 rows of bf16, 16 of fp32
+  constexpr int SPAN = BYTES == 2 ? UPDATE_SPAN : UPDATE_SPAN / 2;
+  __shared__ __align__(16) uint16_t list[SPAN];
+  __shared__ int warp_total[RING_THREADS / 32];
+  __shared__ __align__(16) uint8_t ring[GROUPS * RING_GROUP][RING_THREADS * PIECE];
+  const int c = blockIdx.x, j = (blockIdx.y * RING_THREADS + threadIdx.x) * 4;
+  const bool in = j < J;
+  const uint8_t* column = static_cast<const uint8_t*>(x) + static_cast<size_t>(in ? j : 0) * BYTES;
+  const uint32_t pitch = static_cast<uint32_t>(J) * BYTES;
+  const uint32_t my_ring = static_cast<uint32_t>(__cvta_generic_to_shared(&ring[0][threadIdx.x * PIECE]));
+  float sum[4] = {};
+  int count = 0;
+  for (int s0 = 0; s0 < S; s0 += SPAN) {
+    const int total = list_members<RING_THREADS>(labels, s0, min(SPAN, S - s0), c, list, warp_total);
+    count += total;
+    auto copy = [&](uint32_t dst, uint32_t member) {
+      const uint8_t* src = column + static_cast<uint64_t>(member) * pitch;
+      if constexpr (BYTES == 2) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+      else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    };
+    auto fetch = [&](int first, int slot) {       // members first .. first + RING_GROUP - 1, a group always
+      const uint32_t dst = my_ring + slot * RING_GROUP * RING_THREADS * PIECE;
+      if (first + RING_GROUP <= total) {
+        const uint4 four = *reinterpret_cast<const uint4*>(list + first);
+        const uint32_t pair[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+        for (int k = 0; k < RING_GROUP; ++k)
+          copy(dst + k * RING_THREADS * PIECE, s0 + ((k & 1) ? pair[k >> 1] >> 16 : pair[k >> 1] & 0xFFFFu));
+      } else {
+        for (int k = 0; first + k < total; ++k) copy(dst + k * RING_THREADS * PIECE, s0 + list[first + k]);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto add = [&](const uint8_t* piece) {
+      float v[4];
+      if constexpr (BYTES == 2) {
+        const uint2 w = *reinterpret_cast<const uint2*>(piece);
+        v[0] = __uint_as_float(w.x << 16); v[1] = __uint_as_float(w.x & 0xFFFF0000u);
+        v[2] = __uint_as_float(w.y << 16); v[3] = __uint_as_float(w.y & 0xFFFF0000u);
+      } else {
+        const float4 w = *reinterpret_cast<const float4*>(piece);
+        v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sum[q] = __fadd_rn(sum[q], v[q]);
+    };
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) fetch(g * RING_GROUP, g);
+    int slot = 0;
+    for (int i = 0; i < total; i += RING_GROUP) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(GROUPS - 1) : "memory");
+      const uint8_t* piece = &ring[slot * RING_GROUP][threadIdx.x * PIECE];
+      if (i + RING_GROUP <= total) {
+#pragma unroll
+        for (int k = 0; k < RING_GROUP; ++k) add(piece + k * RING_THREADS * PIECE);
+      } else {
+        for (int k = 0; i + k < total; ++k) add(piece + k * RING_THREADS * PIECE);
+      }
+      fetch(i + GROUPS * RING_GROUP, slot);
+      if (++slot == GROUPS) slot = 0;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+  if (in) store_centre(sum, count, c, j, J, centers, planes, stored);
+}
+
+// Other rows: two columns per thread (rows of even length on their own multiple), or one column of any type, 32 row
+// loads at a time.
 struct PairBf16 {
   static constexpr int COLS = 2;
   uint32_t w;
   __device__ __forceinline__ void load(const void* base, int, size_t i) {
     w = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(base) + i));
   }
-  __device__ __forceinline__ float2 value() const {
-    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-  }
+  __device__ __forceinline__ float value(int k) const { return __uint_as_float(k ? w & 0xFFFF0000u : w << 16); }
 };
 struct PairF32 {
   static constexpr int COLS = 2;
@@ -335,73 +504,28 @@ struct PairF32 {
   __device__ __forceinline__ void load(const void* base, int, size_t i) {
     v = __ldg(reinterpret_cast<const float2*>(static_cast<const float*>(base) + i));
   }
-  __device__ __forceinline__ float2 value() const { return v; }
+  __device__ __forceinline__ float value(int k) const { return k ? v.y : v.x; }
 };
 struct Single {
   static constexpr int COLS = 1;
   float v;
   __device__ __forceinline__ void load(const void* base, int dtype, size_t i) { v = load_float(base, dtype, i); }
-  __device__ __forceinline__ float2 value() const { return make_float2(v, 0.f); }
+  __device__ __forceinline__ float value(int) const { return v; }
 };
 
-// centre c, columns j ..: sum of member rows in token order / member count;
-// an empty cluster keeps its centre.
-constexpr int UPDATE_LABELS = 32;                       // labels a thread looks at per round
-constexpr int UPDATE_SPAN = 256 * UPDATE_LABELS;        // tokens per round
 constexpr int UPDATE_FLIGHT = 32;                       // row loads in flight per thread
 template <class Columns>
 __global__ void __launch_bounds__(256)
 kmeans_update_kernel(const void* x, int x_dtype, int S, int J, const int32_t* labels,
-                     float* centers) {
-  // Block (c, column block): the mean of the rows labelled c, summed in increasing token order (one
-  // fp32 addition per row, the order a sequential scatter-add takes) so that the result does not
-  // depend on the launch shape.  Labels are taken 8,192 at a time: every thread looks at 32 of them, a
-  // block-wide exclusive scan turns the match counts into positions, and the matching tokens land in
-  // shared memory in order; the columns are then summed over that short list only.  Bound: the chain of
-  // row loads of the largest cluster -- start rows drawn from one true cluster leave others to be shared,
-  // so a cluster can hold several times the mean -- hence 32 loads in flight, two columns each.
-  // 4,680 x 5,120, 64 centres, us per call with 4 / 8 / 32 loads in flight: 97 / 68 / 41.
+                     float* centers, uint16_t* planes, uint16_t* stored) {
   __shared__ uint16_t list[UPDATE_SPAN];
   __shared__ int warp_total[8];
   constexpr int COLS = Columns::COLS;
   const int c = blockIdx.x, j = (blockIdx.y * 256 + threadIdx.x) * COLS;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool vector = (reinterpret_cast<uintptr_t>(labels) & 15) == 0;
-  float2 sum = make_float2(0.f, 0.f);
+  float sum[COLS] = {};
   int count = 0;
   for (int s0 = 0; s0 < S; s0 += UPDATE_SPAN) {
-    const int len = min(UPDATE_SPAN, S - s0);
-    const int first = threadIdx.x * UPDATE_LABELS;
-    uint32_t match = 0;
-#pragma unroll
-    for (int k = 0; k < UPDATE_LABELS; k += 4) {
-      if (vector && first + k + 4 <= len) {
-        const int4 l = __ldg(reinterpret_cast<const int4*>(labels + s0 + first + k));
-        match |= ((l.x == c ? 1u : 0u) | (l.y == c ? 2u : 0u) | (l.z == c ? 4u : 0u) | (l.w == c ? 8u : 0u)) << k;
-      } else {
-        for (int i = k; i < k + 4; ++i)
-          if (first + i < len && __ldg(labels + s0 + first + i) == c) match |= 1u << i;
-      }
-    }
-    const int n = __popc(match);
-    int scan = n;                                           // inclusive scan inside the warp
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, scan, off);
-      if (lane >= off) scan += v;
-    }
-    __syncthreads();                                        // the previous list has been consumed
-    if (lane == 31) warp_total[warp] = scan;
-    __syncthreads();
-    int base = 0, total = 0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      if (w < warp) base += warp_total[w];
-      total += warp_total[w];
-    }
-    int at = base + scan - n;
-    for (; match != 0; match &= match - 1) list[at++] = static_cast<uint16_t>(first + __ffs(match) - 1);
-    __syncthreads();
+    const int total = list_members<256>(labels, s0, min(UPDATE_SPAN, S - s0), c, list, warp_total);
     count += total;
     if (j < J) {
       for (int i = 0; i < total; i += UPDATE_FLIGHT) {
@@ -412,17 +536,13 @@ kmeans_update_kernel(const void* x, int x_dtype, int S, int J, const int32_t* la
 #pragma unroll
         for (int k = 0; k < UPDATE_FLIGHT; ++k)
           if (i + k < total) {
-            const float2 pair = v[k].value();
-            sum.x = __fadd_rn(sum.x, pair.x);
-            sum.y = __fadd_rn(sum.y, pair.y);
+#pragma unroll
+            for (int q = 0; q < COLS; ++q) sum[q] = __fadd_rn(sum[q], v[k].value(q));
           }
       }
     }
   }
-  if (j < J && count > 0) {
-    centers[static_cast<size_t>(c) * J + j] = __fdiv_rn(sum.x, static_cast<float>(count));
-    if (COLS == 2) centers[static_cast<size_t>(c) * J + j + 1] = __fdiv_rn(sum.y, static_cast<float>(count));
-  }
+  if (j < J) store_centre(sum, count, c, j, J, centers, planes, stored);
 }
 
 __global__ void kmeans_store_kernel(const float* centers, const int32_t* labels, int S, size_t CJ,
@@ -581,22 +701,30 @@ int rope_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head,
 }
 
 int kmeans_gather_init(const void* x, int x_dtype, int J, int C, const int32_t* init_rows,
-                       float* centers, cudaStream_t stream) {
-  gather_init_kernel<<<dim3(C, ceil_div(J, 256)), 256, 0, stream>>>(x, x_dtype, J, init_rows, centers);
+                       float* centers, uint16_t* planes, cudaStream_t stream) {
+  gather_init_kernel<<<dim3(C, ceil_div(J, 256)), 256, 0, stream>>>(x, x_dtype, J, init_rows, centers, planes);
   NKV_LAUNCH_CHECK("gather_init_kernel");
   return NKV_OK;
 }
 
 int kmeans_update(const void* x, int x_dtype, int S, int J, int C, const int32_t* labels,
-                  float* centers, cudaStream_t stream) {
-  // two columns per thread for bf16 and fp32 rows of even length that start on 4 resp. 8 bytes; every other
+                  float* centers, uint16_t* planes, uint16_t* stored, cudaStream_t stream) {
+  // four or two columns per thread for bf16 and fp32 rows that start on a multiple of that many; every other
   // form (fp16 rows among them) one column, converted by load_float
   const bool bf16 = x_dtype == NKV_BF16, f32 = x_dtype == NKV_F32;
-  const bool pairs = (bf16 || f32) && J % 2 == 0 && (reinterpret_cast<uintptr_t>(x) & (f32 ? 7 : 3)) == 0;
-  const dim3 grid(C, ceil_div(J, pairs ? 512 : 256));
-  if (!pairs) kmeans_update_kernel<Single><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
-  else if (f32) kmeans_update_kernel<PairF32><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
-  else kmeans_update_kernel<PairBf16><<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers);
+  auto fits = [&](int columns) {
+    return (bf16 || f32) && J % columns == 0 && reinterpret_cast<uintptr_t>(x) % (columns * (f32 ? 4 : 2)) == 0;
+  };
+  if (fits(4)) {
+    const dim3 grid(C, ceil_div(J, 4 * RING_THREADS));
+    auto kernel = f32 ? kmeans_update_ring_kernel<4> : kmeans_update_ring_kernel<2>;
+    kernel<<<grid, RING_THREADS, 0, stream>>>(x, S, J, labels, centers, planes, stored);
+  } else {
+    const bool pairs = fits(2);
+    const dim3 grid(C, ceil_div(J, pairs ? 512 : 256));
+    auto kernel = !pairs ? kmeans_update_kernel<Single> : (f32 ? kmeans_update_kernel<PairF32> : kmeans_update_kernel<PairBf16>);
+    kernel<<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers, planes, stored);
+  }
   NKV_LAUNCH_CHECK("kmeans_update_kernel");
   return NKV_OK;
 }

@@ -3,8 +3,8 @@
 // (||x||^2 + ||c||^2) - 2 x.c in fp32 and keeps the first minimum.
 //
 // Given centres are bf16.  The C-means' fp32 means come as three bf16 planes side by side along K (hi, mid, lo:
-// every product is exact in the fp32 accumulator) with their norms in `cnorm`; the token rows are walked once per
-// plane.  K is never cut: every sum runs in the order of K, so what is stored does not depend on how a call is tiled.
+// every product is exact in the fp32 accumulator); the token rows are walked once per plane, and the warps that sum
+// norms square the fp32 rows themselves while the second and third plane are multiplied.  K is never cut: every sum runs in the order of K, so what is stored does not depend on how a call is tiled.
 //
 // A thread block owns `rows` tokens and C / parts centres; the `parts` blocks of one token tile are a cluster,
 // whose first block collects the others' minima through its shared memory; the parts share out the norms of the
@@ -65,7 +65,8 @@ struct Params {
   int tmem_columns;
   void* ids_out; int id_bytes;
   int32_t* labels_out;                     // optional 32-bit copy of the ids (the C-means update reads it)
-  const float* cnorm;                      // squared norms of fp32 centres, or NULL: bf16 centres
+  const float* centers;                    // fp32 centres (their planes are the operand), or NULL: bf16 centres
+  int J;
 };
 
 // sums of the eight squares of two pieces, each one chain of fused multiply-adds in the order of its elements
@@ -80,6 +81,35 @@ __device__ __forceinline__ void sumsq8_pair(const uint4& u, const uint4& v, floa
     sum = fma_f32x2(odd, odd, sum);
   }
   split_f32(sum, su, sv);
+}
+
+// Squared norm of an fp32 row of J columns (a multiple of 64), by one warp (lane 0 has it): partial sum t of 256 runs
+// over the columns t, t + 256, ... in turn, and the partial sums are added in halves, 128 and 128, 64 and 64 and so on.
+// A lane keeps the partial sums 4 lane .. 4 lane + 3 of either half.
+__device__ __forceinline__ float row_norm(const float* row, int J, int lane) {
+  float part[2][4] = {};
+  auto square = [&](int half, const float4& v) {
+    part[half][0] = fmaf(v.x, v.x, part[half][0]);
+    part[half][1] = fmaf(v.y, v.y, part[half][1]);
+    part[half][2] = fmaf(v.z, v.z, part[half][2]);
+    part[half][3] = fmaf(v.w, v.w, part[half][3]);
+  };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int k = 4 * lane; k < J; k += 256) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(row + k));
+    const float4 b = k + 128 < J ? __ldg(reinterpret_cast<const float4*>(row + k + 128)) : zero;
+    square(0, a);
+    square(1, b);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float sum = part[0][e] + part[1][e];
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+    part[0][e] = sum;
+  }
+  return (part[0][0] + part[0][2]) + (part[0][1] + part[0][3]);
 }
 
 template <int KC>
@@ -191,13 +221,10 @@ assign_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     // The blocks of a cluster share the work: the parts of a tile its tokens, two tiles their centres.
     const uint32_t me = p.team > 1 ? cluster_ctarank() : 0;
     const int x_share = p.parts > 1 ? (p.rows_pad + p.parts - 1) / p.parts : p.rows_pad, x_first = p.parts > 1 ? part * x_share : 0;
-    const int c_share = p.cnorm != nullptr ? 0 : (p.parts == 1 ? columns / p.team : columns);
+    const int c_share = p.centers != nullptr ? 0 : (p.parts == 1 ? columns / p.team : columns);
     const int c_first = p.parts == 1 ? static_cast<int>(me) * c_share : 0;
     const int x_items = 2 * max(0, min(x_share, p.rows_pad - x_first)), items = x_items + 2 * c_share;
-    // fp32 centres bring their norms; columns past the last centre are infinitely far
-    for (int c = tid; c < MAX_CENTRES; c += COMPUTE_THREADS)
-      if (c >= columns) meta.norm_c[c] = INFINITY;
-      else if (p.cnorm != nullptr) meta.norm_c[c] = __ldg(p.cnorm + n_base + c);
+    for (int c = columns + tid; c < MAX_CENTRES; c += COMPUTE_THREADS) meta.norm_c[c] = INFINITY;   // infinitely far
     const int rot = (tid >> 1) & 3;
     uint32_t at_stage[MAX_ITEMS];         // an item's place in a stage's first chunk; the further chunks follow a tile apart
 #pragma unroll
@@ -245,6 +272,11 @@ assign_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars[NORMS_FREE + s]);
     }
+    if (p.centers != nullptr && ok)
+      for (int c = warp; c < columns; c += WARPS) {
+        const float norm = row_norm(p.centers + static_cast<size_t>(n_base + c) * p.J, p.J, lane);
+        if (lane == 0) meta.norm_c[c] = norm;
+      }
     if (p.team > 1) cluster_wait();
     joined = true;
     if (ok) {
@@ -386,7 +418,7 @@ int launch_assign(const void* x, const void* centers, int S, int J, int C, int p
     if (smem_bytes(rows_pad, columns, cut.kc, cut.stages) <= SMEM_LIMIT) break;
   const size_t smem = smem_bytes(rows_pad, columns, cut.kc, cut.stages);
   NKV_REQUIRE(smem <= SMEM_LIMIT, NKV_ERR_UNSUPPORTED, "assign: %zu bytes of shared memory", smem);
-  p.S = S; p.C = C;
+  p.S = S; p.J = J; p.C = C;
   p.rows = cut.rows; p.rows_pad = rows_pad; p.parts = cut.parts;
   const int tiles = ceil_div(S, p.rows);
   // two tiles share the norms of many centres (bf16 ones: the fp32 ones' are known)
@@ -447,58 +479,16 @@ int tc_assign(const void* x_bf16, const void* centers_bf16, int S, int J, int C,
   return launch_assign(x_bf16, centers_bf16, S, J, C, 1, p, stream);
 }
 
-namespace {
-
-// fp32 centre rows -> three bf16 planes side by side ([C, 3 J]: c = hi + mid + lo exactly, up to the
-// last bit of the third term) and the rows' squared norms in fp32
-__global__ void __launch_bounds__(256)
-split_centers_kernel(const float* centers, int J, uint16_t* planes, float* cnorm) {
-  __shared__ float part[256];
-  const int c = blockIdx.x;
-  const float* row = centers + static_cast<size_t>(c) * J;
-  uint16_t* out = planes + static_cast<size_t>(c) * 3 * J;
-  float sum = 0.f;
-  for (int j = threadIdx.x; j < J; j += 256) {
-    const float v = row[j];
-    sum = fmaf(v, v, sum);
-    const uint16_t hi = float_to_bf16_bits(v);
-    const float r1 = __fsub_rn(v, bf16_bits_to_float(hi));
-    const uint16_t mid = float_to_bf16_bits(r1);
-    const float r2 = __fsub_rn(r1, bf16_bits_to_float(mid));
-    out[j] = hi;
-    out[J + j] = mid;
-    out[2 * J + j] = float_to_bf16_bits(r2);
-  }
-  part[threadIdx.x] = sum;
-  __syncthreads();
-  for (int width = 128; width >= 1; width >>= 1) {
-    if (threadIdx.x < width) part[threadIdx.x] += part[threadIdx.x + width];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) cnorm[c] = part[0];
-}
-
-}  // namespace
-
-size_t tc_assign_f32_workspace_bytes(int J, int C) {
-  return static_cast<size_t>(C) * 3 * J * 2 + static_cast<size_t>(C) * 4 + 256;
-}
-
 // Nearest centre against fp32 centres on the tensor cores: every bf16 x bf16 product is exact in the
 // fp32 accumulator, and the three planes restore the centres' 24 mantissa bits, so the distances
-// carry fp32 accuracy (the accumulation order is the tensor core's).  Writes 32-bit labels.
-int tc_assign_f32(const void* x_bf16, const float* centers_f32, int S, int J, int C, int32_t* labels,
-                  void* workspace, cudaStream_t stream) {
+// carry fp32 accuracy (the accumulation order is the tensor core's).  Writes 32-bit labels, and ids where asked.
+int tc_assign_f32(const void* x_bf16, const float* centers_f32, const uint16_t* planes, int S, int J, int C,
+                  int32_t* labels, void* ids, int id_bytes, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
-  NKV_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, NKV_ERR_INVALID,
-              "assign: plane workspace must be 256-byte aligned");
-  uint16_t* planes = static_cast<uint16_t*>(workspace);
-  float* cnorm = reinterpret_cast<float*>(planes + static_cast<size_t>(C) * 3 * J);
-  split_centers_kernel<<<C, 256, 0, stream>>>(centers_f32, J, planes, cnorm);
-  NKV_LAUNCH_CHECK("split_centers_kernel");
   Params p{};
-  p.labels_out = labels; p.id_bytes = 1;
-  p.cnorm = cnorm;
+  p.labels_out = labels;
+  p.ids_out = ids; p.id_bytes = id_bytes;
+  p.centers = centers_f32;
   return launch_assign(x_bf16, planes, S, J, C, 3, p, stream);
 }
 

@@ -67,3 +67,26 @@ def test_rows_that_are_not_finite_leave_their_neighbours_alone():
         codes, scales = ops.project_quant(bad, centers, ids, mean, encoder, group=group)
         assert torch.equal(codes[keep], want[0][keep]) and torch.equal(scales[keep], want[1][keep])
         assert bool(((codes & 15) <= 14).all() and ((codes >> 4) <= 14).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("S,J", [(40, 64), (1000, 320), (9000, 66)])
+@pytest.mark.parametrize("iters", [0, 1])
+def test_means_of_separated_clusters(S, J, iters, dtype):
+    """Rows within 0.3 sqrt(J) of one of eight centres; the second eight start rows double the first, so their clusters
+    stay empty and keep them.  One fp32 addition per row in token order, one rounding to bf16."""
+    gen = torch.Generator().manual_seed(S + J)
+    base = 4.0 * torch.randn(8, J, generator=gen)
+    pick = torch.cat([torch.arange(8), torch.randint(0, 8, (S - 8,), generator=gen)])
+    rows = (base[pick] + 0.3 * torch.randn(S, J, generator=gen)).to(dtype)
+    init = torch.cat([torch.arange(8), torch.arange(8)])
+    centers, ids = ops.kmeans(rows.cuda(), 16, iters, init)
+    assert torch.equal(ids.cpu().long(), pick if iters else torch.zeros(S, dtype=torch.long))
+    for c in range(16):
+        want = rows[init[c]].float()
+        if iters and c < 8:
+            want = torch.zeros(J)
+            for row in rows[pick == c].float():
+                want += row
+            want /= int((pick == c).sum())
+        assert torch.equal(centers[c].cpu(), want.to(torch.bfloat16))
