@@ -350,8 +350,19 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       };
       uint4 cen[4];
       float4 bias[POS ? 1 : 8];
+      float bias_lane[POS ? 4 : 1];
       load_centers(0, cen);
-      if constexpr (!POS) load_bias(0, bias);
+      if constexpr (POS) {
+        // the registers hold rotation entries instead: a lane keeps one column of every round, rounded once, and the
+        // lanes share theirs through the staging area
+#pragma unroll
+        for (int sub = 0; sub < 4; ++sub) {
+          bias_lane[sub] = sub < rounds ? __ldg(t.bias + nt * TN + wg * 128 + sub * 32 + lane) : 0.f;
+          if (p.round_bias) bias_lane[sub] = round_to_bf16(bias_lane[sub]);
+        }
+      } else {
+        load_bias(0, bias);
+      }
       // positional restore: table rows and frame of the four tokens this lane stores a piece of
       const bool rotate = ROPE && t.rope.cos_sin != nullptr;
       const bool transform = CAM && t.cam.matrices != nullptr;
@@ -385,7 +396,8 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
       // The restore works on the 16-byte pieces a lane stores -- four pairs, or one camera block, of one
       // token -- because four lanes then read 128 contiguous bytes of a token's table row; a lane that
       // kept a whole row of the accumulator would gather from 32 rows at a time.  26,917 rotated tokens x
-      // 5,120 columns, rank 640 (K and V): 627 us, 1,328 with the gather per row.
+      // 5,120 columns, rank 640 (K and V): 570 us; 655 with the entries requested in the round that uses them and every
+      // lane loading and rounding a round's 32 bias columns; 1,328 with the gather per row as well.
       auto load_rotation = [&](int head, int dcol, float2* rot) {
         const int local = dcol / 2 + (lane & 3) * 4;
         const float2* table = reinterpret_cast<const float2*>(t.rope.cos_sin);
@@ -443,40 +455,53 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
         }
         v = make_uint4(word[0], word[1], word[2], word[3]);
       };
+      // rotation entries of the pieces this lane stores, requested behind the round before like the centres
+      float2 rot[ROPE ? 16 : 1];
+      auto fetch_rotation = [&](int sub) {
+        if (!rotate || sub >= rounds) return;
+        const int col0 = nt * TN + wg * 128 + sub * 32, head = col0 / p.D;
+        load_rotation(head, col0 - head * p.D, rot);
+      };
+      fetch_rotation(0);
       ok = wait_all(&bars[ACC_FULL + b], use & 1, abort_flag, 740 + b, p.wait_budget);
       if (!ok) return;
       tc_fence_after();
       auto round = [&](int sub) {
         const int col0 = nt * TN + wg * 128 + sub * 32;
         const int head = col0 / p.D, dcol = col0 - head * p.D;
-        // rotation entries of the pieces this lane stores, in flight under the rebuild
-        float2 rot[ROPE ? 16 : 1];
-        if (rotate) load_rotation(head, dcol, rot);
-        if (POS) asm volatile("prefetch.global.L1 [%0];" ::"l"(t.bias + col0 + (lane & 1) * 16));
         uint32_t acc_raw[32];
         tmem_ld32_issue(tmem_base + lane_sel + b * TN + wg * 128 + sub * 32, acc_raw);
-        tmem_ld32_wait(acc_raw);
         uint32_t packed[16];
+        if constexpr (POS) {
+          reinterpret_cast<float*>(stage)[lane] = sub == 0 ? bias_lane[0] : (sub == 1 ? bias_lane[1] : (sub == 2 ? bias_lane[2] : bias_lane[3]));
+          __syncwarp();
+          ulonglong2 add[8];
 #pragma unroll
-        for (int j4 = 0; j4 < 4; ++j4) {
-          float4 lo, hi;
-          if constexpr (POS) {     // the registers hold rotation entries instead: from the first-level cache
-            lo = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8));
-            hi = __ldg(reinterpret_cast<const float4*>(t.bias + col0 + j4 * 8 + 4));
-          } else {
-            lo = bias[2 * j4];
-            hi = bias[2 * j4 + 1];
+          for (int j = 0; j < 8; ++j) add[j] = reinterpret_cast<const ulonglong2*>(stage)[j];
+          tmem_ld32_wait(acc_raw);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            float lo, hi;
+            split_f32(add_f32x2(pair_bits(acc_raw[2 * j], acc_raw[2 * j + 1]), (j & 1) ? add[j >> 1].y : add[j >> 1].x), lo, hi);
+            packed[j] = pack_bf16x2(lo, hi);
           }
-          float add[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-          if (p.round_bias) {
+          __syncwarp();        // the bias has been read
+        } else {
+          tmem_ld32_wait(acc_raw);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) add[j] = round_to_bf16(add[j]);
-          }
+          for (int j4 = 0; j4 < 4; ++j4) {
+            const float4 lo = bias[2 * j4], hi = bias[2 * j4 + 1];
+            float add[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            if (p.round_bias) {
 #pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            const int j = j4 * 8 + w * 2;
-            packed[j4 * 4 + w] = pack_bf16x2(__uint_as_float(acc_raw[j]) + add[2 * w],
-                                             __uint_as_float(acc_raw[j + 1]) + add[2 * w + 1]);
+              for (int j = 0; j < 8; ++j) add[j] = round_to_bf16(add[j]);
+            }
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              const int j = j4 * 8 + w * 2;
+              packed[j4 * 4 + w] = pack_bf16x2(__uint_as_float(acc_raw[j]) + add[2 * w],
+                                               __uint_as_float(acc_raw[j + 1]) + add[2 * w + 1]);
+            }
           }
         }
         if constexpr (!POS) load_bias(sub + 1, bias);
@@ -498,6 +523,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap map_0, const __grid_const
           if (crow_of[i] >= 0) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(m0 + rloc) * t.row_stride) = v;
         }
         load_centers(sub + 1, cen);
+        fetch_rotation(sub + 1);
         __syncwarp();
       };
 #pragma unroll 1
