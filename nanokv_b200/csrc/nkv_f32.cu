@@ -6,7 +6,7 @@
 // reproduce the rounding points of the bf16 path, which the test-suite uses to cross-check the
 // tensor-core kernels at full size.
 //
-// Two forms of the GEMM, both with packed multiply-adds and the next step's operands in registers while one is
+// Two forms of the GEMM, both with packed multiply-adds and the operands of the next steps in registers while one is
 // multiplied.  Assignment and projection (gemm_ordered): every sum is one chain of fused multiply-adds in the
 // order of K, because what they give is stored -- ids, and codes that another order would move now and then.
 // Row decode (gemm64): 64 x 64 of the product per block; its four groups of 64 threads take a quarter of K each,
@@ -119,10 +119,13 @@ __device__ __forceinline__ float4 tile_sum(const float* sm, int row, int c) {
 
 // ------------------------------------------------------- sums in the order of K
 // TM x 64 of A B^T per block: thread (ty, tx) owns TM / 16 rows x 4 columns, each sum one chain over K.  A step takes
-// 32 columns of K through one of two buffers; load_a(k) / load_b(k) give elements k .. k + 3 of row threadIdx.x % TM
-// resp. % 64.  Bound: 4,096 multiply-adds per column of K and 64 x 64 tile, 32 cycles of an SM.  us, 1,536 columns,
-// projection to 192 / assignment to 16 centres, against K cut in four as in gemm64: 300 tokens 109 / 90 (102 / 83),
-// 2,048 142 / 94 (103 / 84), 4,096 178 / 95 (160 / 84).
+// 32 columns of K through one of two buffers; a.load(k) / b.load(k) give elements k .. k + 3 of row threadIdx.x % TM
+// resp. % 64 as they come from memory, a.value / b.value what is multiplied: the operands of two steps are in flight
+// while one is multiplied.  Bound: 4,096 multiply-adds per column of K and 64 x 64 tile, 32 cycles of an SM (a step of
+// 1,024 cycles, of which about half is reached).  us, 1,536 columns, projection to 192 / assignment to 16 centres, now
+// and with one step in flight whose loads stood in branches on type and range (a branch's result is merged into a
+// register, which waits for the load: no step overlapped its loads): 300 tokens 66 / 56 (84 / 70), 2,048 82 / 55
+// (131 / 90), 4,096 156 / 55 (167 / 89).
 constexpr int STEP = 32;
 template <int TM>
 constexpr int ORDERED_FLOATS = 2 * STEP * (TM + TILE);
@@ -130,40 +133,41 @@ constexpr int ORDERED_FLOATS = 2 * STEP * (TM + TILE);
 // NORMS: threads 0 .. TM - 1 / 128 .. 191 also square row threadIdx.x of A / threadIdx.x - 128 of B, elements
 // j, j + 4, j + 8 ... in chain j.
 template <int TM, bool NORMS, class LA, class LB>
-__device__ __forceinline__ void gemm_ordered(float* sm, int K, LA load_a, LB load_b, float (&sums)[TM / 16][4],
-                                             float (&norm)[4]) {
+__device__ __forceinline__ void gemm_ordered(float* sm, int K, const LA& operand_a, const LB& operand_b,
+                                             float (&sums)[TM / 16][4], float (&norm)[4]) {
   constexpr int ROWS = TM / 16, NA = TM * STEP / 4 / THREADS, NB = TILE * STEP / 4 / THREADS;
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
   const int ra = t % TM, ka = t / TM * 4, rb = t % TILE, kb = t / TILE * 4;   // first piece loaded; the others further along K
   uint64_t acc[ROWS][2];
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) acc[i][0] = acc[i][1] = 0ull;
-  float4 va[NA], vb[NB];
-  auto fetch = [&](int k0) {
+  decltype(operand_a.load(0)) va[2][NA];
+  decltype(operand_b.load(0)) vb[2][NB];
+  auto fetch = [&](int buffer, int k0) {
 #pragma unroll
-    for (int i = 0; i < NA; ++i) va[i] = load_a(k0 + ka + i * (STEP / NA));
+    for (int i = 0; i < NA; ++i) va[buffer][i] = operand_a.load(k0 + ka + i * (STEP / NA));
 #pragma unroll
-    for (int i = 0; i < NB; ++i) vb[i] = load_b(k0 + kb + i * (STEP / NB));
+    for (int i = 0; i < NB; ++i) vb[buffer][i] = operand_b.load(k0 + kb + i * (STEP / NB));
   };
-  fetch(0);
-  int buffer = 0;
-  for (int k0 = 0; k0 < K; k0 += STEP, buffer ^= 1) {
+  auto step = [&](int buffer, int k0) {
     float* as = sm + buffer * STEP * (TM + TILE);
     float* bs = as + STEP * TM;
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
-      const float v[4] = {va[i].x, va[i].y, va[i].z, va[i].w};
+      const float4 f = operand_a.value(va[buffer][i]);
+      const float v[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) as[(ka + i * (STEP / NA) + j) * TM + ra] = v[j];
     }
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
-      const float v[4] = {vb[i].x, vb[i].y, vb[i].z, vb[i].w};
+      const float4 f = operand_b.value(vb[buffer][i]);
+      const float v[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) bs[(kb + i * (STEP / NB) + j) * TILE + rb] = v[j];
     }
     __syncthreads();      // one per step: whoever fills this buffer next is behind the barrier of the step between
-    if (k0 + STEP < K) fetch(k0 + STEP);
+    if (k0 + 2 * STEP < K) fetch(buffer, k0 + 2 * STEP);
 #pragma unroll
     for (int k = 0; k < STEP; ++k) {
       float a[ROWS];
@@ -188,6 +192,13 @@ __device__ __forceinline__ void gemm_ordered(float* sm, int K, LA load_a, LB loa
 #pragma unroll
       for (int k = 0; k < STEP; ++k) norm[k & 3] = fmaf(row[k * pitch], row[k * pitch], norm[k & 3]);
     }
+  };
+  fetch(0, 0);
+  if (STEP < K) fetch(1, STEP);
+#pragma unroll 1
+  for (int k0 = 0; k0 < K; k0 += 2 * STEP) {
+    step(0, k0);
+    if (k0 + STEP < K) step(1, k0 + STEP);
   }
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
@@ -196,8 +207,45 @@ __device__ __forceinline__ void gemm_ordered(float* sm, int K, LA load_a, LB loa
   }
 }
 
+// A row of either operand.  ANY: any type and alignment, rows past the last one zero.  F32 / BF16: rows that are read as
+// vectors, K a multiple of STEP, and no condition on a load -- one merges two values, and the merge waits for the load.
+// Their rows past the last one are another row's (what comes of them is stored nowhere).
+enum Form { ANY = 0, F32_ROWS = 1, BF16_ROWS = 2 };
+template <Form FORM>
+struct RowOperand {
+  const void* base; int dtype; size_t row; int K; bool vector, in;
+  __device__ __forceinline__ float4 load(int k) const {
+    return in ? load4(base, dtype, row, k, K, vector) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  __device__ __forceinline__ float4 value(const float4& v) const { return v; }
+};
+template <>
+struct RowOperand<F32_ROWS> {
+  const void* base; int dtype; size_t row; int K; bool vector, in;
+  __device__ __forceinline__ float4 load(int k) const {
+    return __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + row + k));
+  }
+  __device__ __forceinline__ float4 value(const float4& v) const { return v; }
+};
+template <>
+struct RowOperand<BF16_ROWS> {
+  const void* base; int dtype; size_t row; int K; bool vector, in;
+  __device__ __forceinline__ uint2 load(int k) const {
+    return __ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + row + k));
+  }
+  __device__ __forceinline__ float4 value(const uint2& w) const {
+    return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xFFFF0000u), __uint_as_float(w.y << 16),
+                       __uint_as_float(w.y & 0xFFFF0000u));
+  }
+};
+
+// whether rows can be read as `form`
+bool has_form(Form form, const void* base, int dtype, int K) {
+  return form == ANY || (dtype == (form == F32_ROWS ? NKV_F32 : NKV_BF16) && K % STEP == 0 && vector_rows(base, dtype, K));
+}
+
 // ---------------------------------------------------------------- assignment
-template <int TM>
+template <int TM, Form X, Form C_>
 __global__ void __launch_bounds__(THREADS, 2)
 assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c_dtype, bool c_vec, int S, int J, int C,
               void* ids, int id_bytes, int32_t* labels32) {
@@ -208,7 +256,6 @@ assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c
   const int m0 = blockIdx.x * TM;
   const bool in_a = m0 + t % TM < S;
   const size_t a_row = static_cast<size_t>(in_a ? m0 + t % TM : 0) * J;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   float best[ROWS];
   int best_i[ROWS];
 #pragma unroll
@@ -218,8 +265,8 @@ assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c
     const size_t b_row = static_cast<size_t>(in_b ? n0 + t % TILE : 0) * J;
     float dots[ROWS][4], norm[4] = {0.f, 0.f, 0.f, 0.f};
     __syncthreads();        // the previous tile's operands and norms have been read
-    gemm_ordered<TM, true>(sm, J, [&](int k) { return in_a ? load4(x, x_dtype, a_row, k, J, x_vec) : zero; },
-                           [&](int k) { return in_b ? load4(centers, c_dtype, b_row, k, J, c_vec) : zero; }, dots, norm);
+    gemm_ordered<TM, true>(sm, J, RowOperand<X>{x, x_dtype, a_row, J, x_vec, in_a},
+                           RowOperand<C_>{centers, c_dtype, b_row, J, c_vec, in_b}, dots, norm);
     const float square = (norm[0] + norm[1]) + (norm[2] + norm[3]);
     if (t < TM) xn[t] = square;
     else if (t >= 128 && t < 128 + TILE) cn[t - 128] = square;
@@ -260,7 +307,26 @@ assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c
 }
 
 // ---------------------------------------------------------------- projection
-template <bool BF16, int TM>
+template <bool BF16, Form X, Form C_, Form M>
+struct Residual {      // (x - centre) - mean, rounded to bf16 where the operators are
+  RowOperand<X> x; RowOperand<C_> centre; RowOperand<M> mean;
+  struct Raw {
+    decltype(RowOperand<X>{}.load(0)) x;
+    decltype(RowOperand<C_>{}.load(0)) centre;
+    float4 mean;
+  };
+  __device__ __forceinline__ Raw load(int k) const { return Raw{x.load(k), centre.load(k), mean.load(k)}; }
+  __device__ __forceinline__ float4 value(const Raw& raw) const {
+    const float4 v = x.value(raw.x), c = centre.value(raw.centre), m = raw.mean;
+    float4 res = make_float4(__fsub_rn(__fsub_rn(v.x, c.x), m.x), __fsub_rn(__fsub_rn(v.y, c.y), m.y),
+                             __fsub_rn(__fsub_rn(v.z, c.z), m.z), __fsub_rn(__fsub_rn(v.w, c.w), m.w));
+    if (BF16) res = make_float4(round_to_bf16(res.x), round_to_bf16(res.y), round_to_bf16(res.z), round_to_bf16(res.w));
+    return res;
+  }
+};
+
+// FAST: fp32 rows, operators and mean as vectors; otherwise anything
+template <bool BF16, int TM, bool FAST>
 __global__ void __launch_bounds__(THREADS, 2)
 project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, bool c_vec, const void* ids, int id_bytes,
                const float* mean, const void* encoder, bool e_vec, int S, int J, int r, void* coeff) {
@@ -271,20 +337,11 @@ project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, 
   const bool in_a = m0 + t % TM < S, in_b = n0 + t % TILE < r;
   const size_t a_row = static_cast<size_t>(in_a ? m0 + t % TM : 0) * J, b_row = static_cast<size_t>(in_b ? n0 + t % TILE : 0) * J;
   const size_t c_row = static_cast<size_t>(in_a ? load_id(ids, id_bytes, m0 + t % TM) : 0) * J;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto residual = [&](int k) {
-    if (!in_a) return zero;
-    const float4 v = load4(x, x_dtype, a_row, k, J, x_vec), c = load4(centers, NKV_BF16, c_row, k, J, c_vec);
-    const float4 m = load4(mean, NKV_F32, 0, k, J, e_vec);
-    float4 res = make_float4(__fsub_rn(__fsub_rn(v.x, c.x), m.x), __fsub_rn(__fsub_rn(v.y, c.y), m.y),
-                             __fsub_rn(__fsub_rn(v.z, c.z), m.z), __fsub_rn(__fsub_rn(v.w, c.w), m.w));
-    if (BF16) res = make_float4(round_to_bf16(res.x), round_to_bf16(res.y), round_to_bf16(res.z), round_to_bf16(res.w));
-    return res;
-  };
+  constexpr Form F = FAST ? F32_ROWS : ANY, C_ = FAST ? BF16_ROWS : ANY;
+  const Residual<BF16, F, C_, F> residual{{x, x_dtype, a_row, J, x_vec, in_a}, {centers, NKV_BF16, c_row, J, c_vec, in_a},
+                                          {mean, NKV_F32, 0, J, e_vec, in_a}};
   float sums[ROWS][4], unused[4];
-  gemm_ordered<TM, false>(sm, J, residual,
-                          [&](int k) { return in_b ? load4(encoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, J, e_vec) : zero; },
-                          sums, unused);
+  gemm_ordered<TM, false>(sm, J, residual, RowOperand<F>{encoder, BF16 ? NKV_BF16 : NKV_F32, b_row, J, e_vec, in_b}, sums, unused);
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
     const int token = m0 + ty * ROWS + i;
@@ -547,7 +604,7 @@ int allow_smem(K kernel) {
 }  // namespace
 
 // Rows of a tile in gemm_ordered: 32 while that still gives every block an SM of its own, else 64.  A tile of
-// half the rows takes three quarters of the time (K = 1,536: 109 against 142 us), so two on one SM would lose.
+// half the rows takes four fifths of the time (K = 1,536: 66 against 82 us), so two on one SM would lose.
 static int ordered_rows(int S, int column_tiles) {
   return static_cast<long long>(ceil_div(S, 32)) * column_tiles <= sm_count() ? 32 : 64;
 }
@@ -556,7 +613,12 @@ int simt_assign(const void* x, int x_dtype, const void* centers, int c_dtype, in
                 int C, void* ids, int id_bytes, int32_t* labels32, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
   const int rows = ordered_rows(S, 1);
-  auto kernel = rows == 32 ? assign_kernel<32> : assign_kernel<64>;
+  const bool x_rows = has_form(F32_ROWS, x, x_dtype, J);
+  auto kernel = x_rows && has_form(BF16_ROWS, centers, c_dtype, J)
+                    ? (rows == 32 ? assign_kernel<32, F32_ROWS, BF16_ROWS> : assign_kernel<64, F32_ROWS, BF16_ROWS>)
+                : x_rows && has_form(F32_ROWS, centers, c_dtype, J)
+                    ? (rows == 32 ? assign_kernel<32, F32_ROWS, F32_ROWS> : assign_kernel<64, F32_ROWS, F32_ROWS>)
+                    : (rows == 32 ? assign_kernel<32, ANY, ANY> : assign_kernel<64, ANY, ANY>);
   kernel<<<ceil_div(S, rows), THREADS, 0, stream>>>(
       x, x_dtype, vector_rows(x, x_dtype, J), centers, c_dtype, vector_rows(centers, c_dtype, J), S, J, C, ids,
       id_bytes, labels32);
@@ -571,8 +633,11 @@ int simt_project(const void* x, int x_dtype, const void* centers_bf16, const voi
   const int rows = ordered_rows(S, ceil_div(r, TILE));
   const dim3 grid(ceil_div(S, rows), ceil_div(r, TILE));
   const bool e_vec = vector_rows(encoder, enc_dtype, J) && vector_rows(mean, NKV_F32, J);
-  auto kernel = enc_dtype == NKV_BF16 ? (rows == 32 ? project_kernel<true, 32> : project_kernel<true, 64>)
-                                      : (rows == 32 ? project_kernel<false, 32> : project_kernel<false, 64>);
+  const bool fast = has_form(F32_ROWS, x, x_dtype, J) && has_form(BF16_ROWS, centers_bf16, NKV_BF16, J) &&
+                    has_form(F32_ROWS, encoder, enc_dtype, J) && has_form(F32_ROWS, mean, NKV_F32, J);
+  auto kernel = fast ? (rows == 32 ? project_kernel<false, 32, true> : project_kernel<false, 64, true>)
+                : enc_dtype == NKV_BF16 ? (rows == 32 ? project_kernel<true, 32, false> : project_kernel<true, 64, false>)
+                                        : (rows == 32 ? project_kernel<false, 32, false> : project_kernel<false, 64, false>);
   kernel<<<grid, THREADS, 0, stream>>>(
       x, x_dtype, vector_rows(x, x_dtype, J), static_cast<const uint16_t*>(centers_bf16),
       vector_rows(centers_bf16, NKV_BF16, J), ids, id_bytes, mean, encoder, e_vec, S, J, r, coeff);
