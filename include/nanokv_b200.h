@@ -259,6 +259,25 @@ int nkv_decode_rows_status(const nkv_history* hist, const int32_t* rows_index, i
 int nkv_segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int center_row,
                        void* stream);
 
+/*
+ * Puts `count` segments behind one another into the arrays of a history, in one launch per sixteen of them: codes,
+ * scales, ids and centre rows are copied from the parts (a NULL source: that array is filled by somebody else), and
+ * the segment table gets the parts from segment `first_segment` on, token `first_token`, centre row
+ * `first_center_row`.  code / scale / id / center_bytes: bytes of a token resp. of a centre row.  The stacking that
+ * the reference does by concatenation before it decodes (LB/lingbot_v2_kv_codec.py:404-437).
+ */
+typedef struct nkv_payload {
+  const void* codes;
+  const void* scales;
+  const void* ids;
+  const void* centers;
+  int32_t tokens;
+  int32_t clusters;
+} nkv_payload;
+int nkv_history_stack(const nkv_payload* parts, int count, int first_segment, int first_token, int first_center_row,
+                      int code_bytes, int scale_bytes, int id_bytes, int center_bytes, void* codes, void* scales,
+                      void* ids, void* centers, int32_t* seg_start, int32_t* seg_center_row, void* stream);
+
 /* ---------------------------------------------------------------- attention */
 
 /*

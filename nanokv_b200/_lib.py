@@ -42,6 +42,12 @@ class History(ctypes.Structure):
     ]
 
 
+class Payload(ctypes.Structure):
+    """struct nkv_payload"""
+    _fields_ = [("codes", c_void_p), ("scales", c_void_p), ("ids", c_void_p), ("centers", c_void_p),
+                ("tokens", c_int32), ("clusters", c_int32)]
+
+
 # name -> (restype, argtypes); every symbol the header declares
 SIGNATURES = {
     "nkv_status_string": (c_char_p, [c_int]),
@@ -66,6 +72,8 @@ SIGNATURES = {
                                          c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
                                          c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "nkv_segment_append": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
+    "nkv_history_stack": (c_int, [POINTER(Payload), c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                  c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "nkv_decode_rows": (c_int, [POINTER(History), c_void_p, c_int, c_void_p, c_int, c_void_p,
                                 c_int, c_void_p, c_int, c_void_p]),
     "nkv_decode_rows_status": (c_int, [POINTER(History), c_void_p, c_int, c_void_p, c_int, c_void_p,

@@ -22,7 +22,7 @@ class CompressedHistory:
     def __init__(self, *, joint: int, rank: int, capacity: int, max_segments: int,
                  centers_per_segment: int, group: int | None = None,
                  scale_dtype: torch.dtype = torch.bfloat16, device="cuda",
-                 center_width: int | None = None, shared_centers: bool = False):
+                 center_width: int | None = None, shared_centers: bool = False, zeroed: bool = True):
         if rank % 2:
             raise ValueError("rank must be even")
         self.joint, self.rank = int(joint), int(rank)
@@ -34,18 +34,17 @@ class CompressedHistory:
         device = torch.device(device)
         self.device = device
         width = self.joint if center_width is None else int(center_width)
-        self.codes = torch.zeros(self.capacity, self.rank // 2, dtype=torch.uint8, device=device)
-        self.scales = torch.zeros(self.capacity, self.rank // self.group, dtype=scale_dtype,
-                                  device=device)
-        self.ids = torch.zeros(self.capacity, dtype=ops.id_dtype(self.centers_per_segment),
-                               device=device)
+        # zeroed=False: for a history that is filled to its capacity before anything reads it
+        array = torch.zeros if zeroed else torch.empty
+        self.codes = array(self.capacity, self.rank // 2, dtype=torch.uint8, device=device)
+        self.scales = array(self.capacity, self.rank // self.group, dtype=scale_dtype, device=device)
+        self.ids = array(self.capacity, dtype=ops.id_dtype(self.centers_per_segment), device=device)
         # shared_centers: one externally supplied table serves every segment (fixed-centre form)
         self.shared_centers = bool(shared_centers)
         table_segments = 1 if self.shared_centers else self.max_segments
-        self.centers = torch.zeros(table_segments * self.centers_per_segment, width,
-                                   dtype=torch.bfloat16, device=device)
-        self.seg_start = torch.zeros(self.max_segments + 1, dtype=torch.int32, device=device)
-        self.seg_center_row = torch.zeros(self.max_segments, dtype=torch.int32, device=device)
+        self.centers = array(table_segments * self.centers_per_segment, width, dtype=torch.bfloat16, device=device)
+        self.seg_start = array(self.max_segments + 1, dtype=torch.int32, device=device)
+        self.seg_center_row = array(self.max_segments, dtype=torch.int32, device=device)
         self._starts = [0]
         self._center_rows: list[int] = []
         self._center_used = 0
@@ -59,8 +58,41 @@ class CompressedHistory:
     def segments(self) -> int:
         return len(self._center_rows)
 
-    def reserve_segment(self, count: int, clusters: int):
-        """Claim the next token range and centre rows; returns (offset, centre rows view)."""
+    def _copies(self, codes, scales, ids, centers) -> bool:
+        """Whether a segment's arrays can be copied into this history as they lie in memory."""
+        return (0 < ids.shape[0] == codes.shape[0] == scales.shape[0] and ids.dim() == 1
+                and all(t.shape[1:] == into.shape[1:] and t.device == into.device and t.dtype == into.dtype
+                        and t.is_contiguous()
+                        for t, into in ((codes, self.codes), (scales, self.scales), (ids, self.ids), (centers, self.centers))))
+
+    @classmethod
+    def stacked(cls, parts, *, joint: int, rank: int, device) -> "CompressedHistory":
+        """A history of the given segments, each (codes u8 [S,r/2], scales [S,1], ids [S], centres [C,J]): one launch per
+        sixteen of them, or copies where types or places differ."""
+        total, clusters = sum(p[2].shape[0] for p in parts), max(p[3].shape[0] for p in parts)
+        hist = cls(joint=joint, rank=rank, capacity=total, max_segments=len(parts), centers_per_segment=clusters,
+                   device=device, zeroed=False)
+        if hist.seg_start.is_cuda and all(hist._copies(*p) for p in parts):
+            with torch.cuda.device(hist.codes.device):
+                ops.history_stack(hist, [(*p, p[2].shape[0], p[3].shape[0]) for p in parts], 0, 0, 0)
+            for _, _, ids, centers in parts:
+                hist._starts.append(hist.tokens + ids.shape[0])
+                hist._center_rows.append(hist._center_used)
+                hist._center_used += centers.shape[0]
+            return hist
+        hist.seg_start.zero_()
+        for codes, scales, ids, centers in parts:
+            offset, rows = hist.reserve_segment(ids.shape[0], centers.shape[0])
+            rows.copy_(centers)
+            stop = offset + ids.shape[0]
+            hist.codes[offset:stop].copy_(codes)
+            hist.scales[offset:stop].copy_(scales)
+            hist.ids[offset:stop].copy_(ids)
+        return hist
+
+    def reserve_segment(self, count: int, clusters: int, centers: torch.Tensor | None = None):
+        """Claim the next token range and centre rows; returns (offset, centre rows view).  ``centers``: rows to be
+        copied there, in the same launch where they lie ready."""
         if count <= 0:
             raise ValueError("a segment needs at least one token")
         if self.tokens + count > self.capacity:
@@ -80,13 +112,21 @@ class CompressedHistory:
         self._starts.append(offset + count)
         self._center_rows.append(row)
         index = self.segments - 1
+        into = self.centers[row:row + clusters]
+        ready = (centers is not None and self.seg_start.is_cuda and centers.device == self.centers.device
+                 and centers.dtype == self.centers.dtype and centers.is_contiguous() and centers.shape == into.shape)
         if self.seg_start.is_cuda:
             with torch.cuda.device(self.seg_start.device):
-                ops.segment_append(self.seg_start, self.seg_center_row, index, offset + count, row)
+                if ready:
+                    ops.history_stack(self, [(None, None, None, centers, count, clusters)], index, offset, row)
+                else:
+                    ops.segment_append(self.seg_start, self.seg_center_row, index, offset + count, row)
         else:
             self.seg_start[index + 1] = offset + count
             self.seg_center_row[index] = row
-        return offset, self.centers[row:row + clusters]
+        if centers is not None and not ready:
+            into.copy_(centers.to(torch.bfloat16))
+        return offset, into
 
     def view(self, start_segment: int = 0, stop_segment: int | None = None) -> HistoryView:
         """ABI view of a run of whole segments (default: everything)."""

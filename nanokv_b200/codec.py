@@ -99,7 +99,7 @@ def encode_append(hist: CompressedHistory, rows: torch.Tensor, op: Operator,
         clusters = int(centers.shape[0]) if centers is not None else int(clusters)
     if clusters > hist.centers_per_segment:
         raise ValueError("more centres than the cache reserves per segment")
-    offset, center_rows = hist.reserve_segment(S, clusters)
+    offset, center_rows = hist.reserve_segment(S, clusters, None if resident else centers)
     if centers is None:
         ids = hist.ids[offset:offset + S]
         codes = hist.codes[offset:offset + S]
@@ -110,8 +110,6 @@ def encode_append(hist: CompressedHistory, rows: torch.Tensor, op: Operator,
                           in_coeff_dtype=quant.in_coeff_dtype and op.dtype == torch.bfloat16,
                           codes=codes, scales=scales)
         return offset
-    if not resident:
-        center_rows.copy_(centers.to(torch.bfloat16))
     workspace = torch.empty(S, op.rank, dtype=op.dtype, device=rows.device)
     lib = _lib.library()
     in_bf16 = quant.in_coeff_dtype and op.dtype == torch.bfloat16

@@ -268,6 +268,22 @@ int nkv_segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, i
   return segment_append(seg_start, seg_center_row, index, stop, center_row, static_cast<cudaStream_t>(stream));
 }
 
+int nkv_history_stack(const nkv_payload* parts, int count, int first_segment, int first_token, int first_center_row,
+                      int code_bytes, int scale_bytes, int id_bytes, int center_bytes, void* codes, void* scales,
+                      void* ids, void* centers, int32_t* seg_start, int32_t* seg_center_row, void* stream) {
+  NKV_REQUIRE(count >= 0 && (count == 0 || parts) && first_segment >= 0 && first_token >= 0 && first_center_row >= 0 &&
+                  code_bytes >= 0 && scale_bytes >= 0 && id_bytes >= 0 && center_bytes >= 0 && seg_start && seg_center_row,
+              NKV_ERR_INVALID, "history_stack: count=%d first segment %d token %d row %d", count, first_segment, first_token,
+              first_center_row);
+  for (int i = 0; i < count; ++i)
+    NKV_REQUIRE(parts[i].tokens > 0 && parts[i].clusters >= 0 && (!parts[i].codes || codes) && (!parts[i].scales || scales) &&
+                    (!parts[i].ids || ids) && (!parts[i].centers || centers),
+                NKV_ERR_INVALID, "history_stack: part %d of %d tokens and %d centres", i, parts[i].tokens, parts[i].clusters);
+  return history_stack(parts, count, first_segment, first_token, first_center_row, code_bytes, scale_bytes, id_bytes,
+                       center_bytes, codes, scales, ids, centers, seg_start, seg_center_row,
+                       static_cast<cudaStream_t>(stream));
+}
+
 static int check_selftest(long long budget_cycles, const int32_t* status_word) {
   NKV_REQUIRE(budget_cycles > 0 && budget_cycles <= (1ll << 28) && status_word, NKV_ERR_INVALID,
               "wait self-test: budget=%lld", budget_cycles);

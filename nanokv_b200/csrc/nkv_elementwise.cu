@@ -1015,6 +1015,78 @@ int head_linear(const void* x, int dtype, int64_t stride_row, int64_t stride_hea
   return NKV_OK;
 }
 
+// ---- segments stacked into a history ----------------------------------------------------------------
+// Row y of the grid copies part y: its four arrays one after the other, as wide as source and destination allow, and
+// its entry of the segment table.  Bound: a launch (13 MB of six 4,680-token parts at rank 640 with 64 centres: about
+// 6 us); array by array and part by part the same is 24 copies of 2.8 us and 6 table launches.
+constexpr int STACK_PARTS = 16;
+struct StackRegion { const void* src; void* dst; long long bytes; };
+struct StackArgs {
+  StackRegion region[STACK_PARTS][4];
+  int stop[STACK_PARTS], row[STACK_PARTS];
+  int segment, begin;           // of the first part
+  int32_t* seg_start;
+  int32_t* seg_center_row;
+};
+
+template <class T>
+__device__ __forceinline__ void copy_as(const StackRegion& r) {
+  const long long n = r.bytes / static_cast<long long>(sizeof(T)), step = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += step)
+    static_cast<T*>(r.dst)[i] = __ldg(static_cast<const T*>(r.src) + i);
+}
+
+__global__ void __launch_bounds__(256)
+history_stack_kernel(const __grid_constant__ StackArgs a) {
+  const int part = blockIdx.y;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const StackRegion r = a.region[part][k];
+    if (r.src == nullptr) continue;
+    const uintptr_t low = reinterpret_cast<uintptr_t>(r.src) | reinterpret_cast<uintptr_t>(r.dst) | static_cast<uintptr_t>(r.bytes);
+    if ((low & 15) == 0) copy_as<uint4>(r);
+    else if ((low & 7) == 0) copy_as<uint2>(r);
+    else if ((low & 3) == 0) copy_as<uint32_t>(r);
+    else copy_as<uint8_t>(r);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (part == 0) a.seg_start[a.segment] = a.begin;
+    a.seg_start[a.segment + part + 1] = a.stop[part];
+    a.seg_center_row[a.segment + part] = a.row[part];
+  }
+}
+
+int history_stack(const nkv_payload* parts, int count, int first_segment, int first_token, int first_center_row,
+                  int code_bytes, int scale_bytes, int id_bytes, int center_bytes, void* codes, void* scales, void* ids,
+                  void* centers, int32_t* seg_start, int32_t* seg_center_row, cudaStream_t stream) {
+  int token = first_token, row = first_center_row;
+  for (int first = 0; first < count; first += STACK_PARTS) {
+    StackArgs a{};
+    const int n = count - first < STACK_PARTS ? count - first : STACK_PARTS;
+    a.segment = first_segment + first;
+    a.begin = token;
+    a.seg_start = seg_start;
+    a.seg_center_row = seg_center_row;
+    for (int i = 0; i < n; ++i) {
+      const nkv_payload& p = parts[first + i];
+      auto region = [](const void* src, void* dst, long long at, long long items, int bytes) {
+        return StackRegion{src, static_cast<uint8_t*>(dst) + at * bytes, items * bytes};
+      };
+      a.region[i][0] = region(p.codes, codes, token, p.tokens, code_bytes);
+      a.region[i][1] = region(p.centers, centers, row, p.clusters, center_bytes);
+      a.region[i][2] = region(p.scales, scales, token, p.tokens, scale_bytes);
+      a.region[i][3] = region(p.ids, ids, token, p.tokens, id_bytes);
+      a.row[i] = row;
+      token += p.tokens;
+      row += p.clusters;
+      a.stop[i] = token;
+    }
+    history_stack_kernel<<<dim3(n > 6 ? 48 : 296 / n, n), 256, 0, stream>>>(a);
+    NKV_LAUNCH_CHECK("history_stack_kernel");
+  }
+  return NKV_OK;
+}
+
 __global__ void segment_append_kernel(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int row) {
   seg_start[index + 1] = stop;
   seg_center_row[index] = row;

@@ -54,6 +54,9 @@ int fast_finish(const void* native, const float* native_lse, const void* lifted,
 int head_linear(const void* x, int dtype, int64_t stride_row, int64_t stride_head, const int32_t* heads,
                 const void* w, int64_t rows, int group_heads, int din, int dout, int dout_pad, void* out,
                 cudaStream_t stream);
+int history_stack(const nkv_payload* parts, int count, int first_segment, int first_token, int first_center_row,
+                  int code_bytes, int scale_bytes, int id_bytes, int center_bytes, void* codes, void* scales, void* ids,
+                  void* centers, int32_t* seg_start, int32_t* seg_center_row, cudaStream_t stream);
 int segment_append(int32_t* seg_start, int32_t* seg_center_row, int index, int stop, int row, cudaStream_t stream);
 size_t history_moments_workspace_bytes(int tokens, int rank);
 int history_moments(const nkv_history& h, float* latent_sum, int32_t* center_counts, void* workspace,

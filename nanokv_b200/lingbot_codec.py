@@ -197,18 +197,13 @@ def history_from_payloads(parts: list[dict], *, device) -> CompressedHistory:
     cached = first.get("_nkv_history")
     if cached is not None and cached[0] == key:
         return cached[1]
-    total = sum(int(part["shape"][1]) for part in parts)
-    clusters = max(int(part["centers"].shape[1]) for part in parts)
-    hist = CompressedHistory(joint=joint, rank=rank, capacity=total, max_segments=len(parts),
-                             centers_per_segment=clusters, device=device)
+    segments = []
     for part in parts:
         count = int(part["shape"][1])
-        offset, rows = hist.reserve_segment(count, int(part["centers"].shape[1]))
-        rows.copy_(part["centers"][0].to(device=device, dtype=torch.bfloat16))
-        hist.codes[offset:offset + count].copy_(part["latent_packed"].to(device).reshape(count, -1))
-        hist.scales[offset:offset + count].copy_(
-            part["latent_scale"].to(device=device, dtype=torch.bfloat16).reshape(count, -1))
-        hist.ids[offset:offset + count].copy_(part["ids"].to(device).reshape(-1))
+        segments.append((part["latent_packed"].to(device).reshape(count, -1),
+                         part["latent_scale"].to(device=device, dtype=torch.bfloat16).reshape(count, -1),
+                         part["ids"].to(device).reshape(-1), part["centers"][0].to(device=device, dtype=torch.bfloat16)))
+    hist = CompressedHistory.stacked(segments, joint=joint, rank=rank, device=device)
     first["_nkv_history"] = (key, hist)
     return hist
 

@@ -266,18 +266,12 @@ def history_from_payloads(parts: list[dict], *, device) -> CompressedHistory:
             raise ValueError("incompatible WorldPlay method segments")
     if batch != 1:
         raise ValueError("only batch 1 payloads are supported")
-    total = sum(int(part["shape"][1]) for part in parts)
-    clusters = max(int(part["centers"].shape[1]) for part in parts)
-    hist = CompressedHistory(joint=dim, rank=rank, capacity=total, max_segments=len(parts),
-                             centers_per_segment=clusters, device=device)
+    segments = []
     for part in parts:
         count = int(part["shape"][1])
-        offset, rows = hist.reserve_segment(count, int(part["centers"].shape[1]))
-        rows.copy_(part["centers"][0].to(device=device, dtype=torch.bfloat16))
-        hist.codes[offset:offset + count].copy_(part["packed_codes"].to(device).reshape(count, -1))
-        hist.scales[offset:offset + count].copy_(part["scale"].to(device).reshape(count, -1))
-        hist.ids[offset:offset + count].copy_(part["ids"].to(device).reshape(-1))
-    return hist
+        segments.append((part["packed_codes"].to(device).reshape(count, -1), part["scale"].to(device).reshape(count, -1),
+                         part["ids"].to(device).reshape(-1), part["centers"][0].to(device=device, dtype=torch.bfloat16)))
+    return CompressedHistory.stacked(segments, joint=dim, rank=rank, device=device)
 
 
 @torch.no_grad()

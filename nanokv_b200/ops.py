@@ -180,6 +180,20 @@ def segment_append(seg_start: torch.Tensor, seg_center_row: torch.Tensor, index:
                                                  _stream(seg_start.device)))
 
 
+def history_stack(hist, parts, first_segment: int, first_token: int, first_center_row: int) -> None:
+    """Segments ``parts`` put behind one another into the arrays of ``hist`` on the current stream, with their entries of
+    the segment table (nkv_history_stack): (codes, scales, ids, centres, tokens, clusters) each, contiguous device
+    tensors in the history's types, or None for an array that somebody else fills."""
+    entries = (_lib.Payload * len(parts))(*[
+        _lib.Payload(*(None if t is None else t.data_ptr() for t in tensors), tokens, clusters)
+        for *tensors, tokens, clusters in parts])
+    _lib.check(_lib.library().nkv_history_stack(
+        entries, len(parts), first_segment, first_token, first_center_row, hist.codes.shape[1],
+        hist.scales.shape[1] * hist.scales.element_size(), hist.ids.element_size(), hist.centers.shape[1] * 2,
+        _ptr(hist.codes), _ptr(hist.scales), _ptr(hist.ids), _ptr(hist.centers), _ptr(hist.seg_start),
+        _ptr(hist.seg_center_row), _stream(hist.codes.device)))
+
+
 def gather_view(view: HistoryView, index: torch.Tensor) -> HistoryView:
     """The history restricted to the tokens listed in ``index`` (increasing, device i64): codes,
     scales and ids are gathered, every segment keeps its centre rows and shrinks to its listed
