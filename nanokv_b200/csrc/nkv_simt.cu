@@ -686,6 +686,54 @@ rope_rows_kernel(const void* x, int dtype, long long stride_row, long long strid
   }
 }
 
+// The same for bf16 rows whose heads share their rotation (no pair index) and start on 16 bytes: a thread keeps the four
+// entries of its pairs and takes ROPE_HEADS heads, all loads ahead of the arithmetic.  Bound: memory; with one
+// thread per head and piece the coordinates, divisions and table loads were the time.  4,680 x 40 x 128: 48 us, now 26.
+constexpr int ROPE_HEADS = 8;
+__global__ void __launch_bounds__(256)
+rope_rows_heads_kernel(const uint16_t* x, long long stride_row, long long stride_head, int S, int heads, int d,
+                       nkv_rope rope, uint16_t* out) {
+  const int quads = d / 8, index = blockIdx.x * 256 + threadIdx.x;
+  const int row = index / quads, pl0 = (index - row * quads) * 4;
+  if (row >= S) return;
+  const int th = rope.table_half, third = th / 3, band_a = th - 2 * third, band_b = band_a + third;
+  const int pos = max(__ldg(rope.positions + row), 0);
+  int frame = pos, prow = pos, pcol = pos;   // frame_seqlen 0: one table row per token
+  if (rope.frame_seqlen > 0) {
+    frame = pos / rope.frame_seqlen;
+    const int spatial = pos - frame * rope.frame_seqlen;
+    prow = spatial / rope.width;
+    pcol = spatial - prow * rope.width;
+  }
+  float2 cs[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int pg = pl0 + k;
+    const int coord = min(pg < band_a ? frame : (pg < band_b ? prow : pcol), rope.table_rows - 1);
+    cs[k] = __ldg(reinterpret_cast<const float2*>(rope.cos_sin) + static_cast<size_t>(coord) * th + pg);
+  }
+  const int first = blockIdx.y * ROPE_HEADS;
+  const uint16_t* src = x + static_cast<size_t>(row) * stride_row + static_cast<size_t>(first) * stride_head + 2 * pl0;
+  uint16_t* dst = out + (static_cast<size_t>(row) * heads + first) * d + 2 * pl0;
+  uint4 raw[ROPE_HEADS];
+#pragma unroll
+  for (int h = 0; h < ROPE_HEADS; ++h)
+    if (first + h < heads) raw[h] = __ldg(reinterpret_cast<const uint4*>(src + h * stride_head));
+#pragma unroll
+  for (int h = 0; h < ROPE_HEADS; ++h) {
+    if (first + h >= heads) break;
+    const uint32_t w[4] = {raw[h].x, raw[h].y, raw[h].z, raw[h].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float x0 = __uint_as_float(w[k] << 16), x1 = __uint_as_float(w[k] & 0xFFFF0000u);
+      const __nv_bfloat162 both = __floats2bfloat162_rn(fmaf(x0, cs[k].x, -(x1 * cs[k].y)), fmaf(x0, cs[k].y, x1 * cs[k].x));
+      o[k] = *reinterpret_cast<const uint32_t*>(&both);
+    }
+    *reinterpret_cast<uint4*>(dst + static_cast<size_t>(h) * d) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 int rope_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head, int S, int heads,
               int d, const nkv_rope& rope, void* out, cudaStream_t stream) {
   const int half = d / 2, quads = half / 4 + (half % 4 ? 1 : 0);
@@ -694,6 +742,13 @@ int rope_rows(const void* x, int dtype, int64_t stride_row, int64_t stride_head,
   // 16-byte path: whole groups of 8 elements, every row and head start 16-byte aligned
   const int vector = d % 8 == 0 && stride_row % 8 == 0 && stride_head % 8 == 0 &&
                      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  if (vector && dtype == NKV_BF16 && rope.pair_index == nullptr && (reinterpret_cast<uintptr_t>(rope.cos_sin) & 7) == 0 &&
+      static_cast<long long>(S) * quads < (1ll << 31) - 256) {
+    rope_rows_heads_kernel<<<dim3(ceil_div(S * quads, 256), ceil_div(heads, ROPE_HEADS)), 256, 0, stream>>>(
+        static_cast<const uint16_t*>(x), stride_row, stride_head, S, heads, d, rope, static_cast<uint16_t*>(out));
+    NKV_LAUNCH_CHECK("rope_rows_heads_kernel");
+    return NKV_OK;
+  }
   rope_rows_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(
       x, dtype, stride_row, stride_head, S, heads, d, rope, out, vector);
   NKV_LAUNCH_CHECK("rope_rows_kernel");

@@ -268,3 +268,18 @@ def test_per_token_multipliers_matrix_game_form():
     want, want_lse = oracle.attention_lse(q.permute(1, 0, 2)[None], keys, values, scale=width ** -0.5)
     assert rel_err(out.cpu(), want[0].permute(1, 0, 2)) <= BF16_REL_TOL
     assert float((lse.cpu() - want_lse[0].t()).abs().max()) <= BF16_REL_TOL
+
+
+@pytest.mark.parametrize("heads", [1, 7, 8, 9, 40])
+@pytest.mark.parametrize("S,d,frame_seqlen", [(1, 8, 0), (37, 64, 12), (300, 128, 1560)])
+def test_rows_whose_heads_share_their_rotation(heads, S, d, frame_seqlen):
+    """The kernel that takes eight heads per thread gives the bits of the general one (an identity pair index)."""
+    gen = torch.Generator(device="cuda").manual_seed(heads * S)
+    angles = torch.rand(64, d // 2, generator=gen, device="cuda", dtype=torch.float64).cpu() * 6.0
+    table = attention.RopeTable(torch.polar(torch.ones_like(angles), angles), frame_seqlen=frame_seqlen,
+                                width=0 if frame_seqlen == 0 else 4)
+    positions = torch.randint(0, 100, (S,), generator=gen, device="cuda", dtype=torch.int32)
+    pairs = torch.arange(d // 2, dtype=torch.int32, device="cuda").expand(heads, d // 2).contiguous()
+    rows = torch.randn(S, 2, heads, d, generator=gen, device="cuda").to(torch.bfloat16)
+    for x in (rows[:, 0].contiguous(), rows[:, 1], rows[:, 1].flip(0)):
+        assert torch.equal(table.rotate(x, positions).view(torch.int16), table.rotate(x, positions, pairs).view(torch.int16))
