@@ -206,12 +206,14 @@ class CompressedHistory:
         self._starts, self._center_rows = starts, rows
         if not self.shared_centers:
             self._center_used = row_cursor
-        table = torch.zeros(self.max_segments + 1, dtype=torch.int32)
+        # both tables in one upload
+        table = torch.zeros(2 * self.max_segments + 1, dtype=torch.int32)
         table[:len(starts)] = torch.tensor(starts, dtype=torch.int32)
-        self.seg_start.copy_(table.to(self.device), non_blocking=True)
-        row_table = torch.zeros(self.max_segments, dtype=torch.int32)
-        row_table[:len(rows)] = torch.tensor(rows, dtype=torch.int32) if rows else row_table[:0]
-        self.seg_center_row.copy_(row_table.to(self.device), non_blocking=True)
+        if rows:
+            table[self.max_segments + 1:self.max_segments + 1 + len(rows)] = torch.tensor(rows, dtype=torch.int32)
+        table = ops.upload(table, self.device)
+        self.seg_start.copy_(table[:self.max_segments + 1], non_blocking=True)
+        self.seg_center_row.copy_(table[self.max_segments + 1:], non_blocking=True)
 
     def resident_bytes(self) -> int:
         """Bytes of payload actually in use (codes, scales, ids, centre tables)."""

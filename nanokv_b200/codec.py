@@ -104,7 +104,7 @@ def encode_append(hist: CompressedHistory, rows: torch.Tensor, op: Operator,
         ids = hist.ids[offset:offset + S]
         codes = hist.codes[offset:offset + S]
         scales = hist.scales[offset:offset + S]
-        init = kmeans_init_rows(S, clusters, seed).to(rows.device)
+        init = kmeans_init_rows(S, clusters, seed)
         ops.kmeans(rows, clusters, iters, init, centers=center_rows, ids=ids)
         ops.project_quant(rows, center_rows, ids, op.mean, op.encoder, group=hist.group, eps=quant.eps,
                           in_coeff_dtype=quant.in_coeff_dtype and op.dtype == torch.bfloat16,

@@ -187,7 +187,7 @@ def global_pca_compress_v(x: torch.Tensor, layer_idx: int, tensor_name: str = "v
         raise ValueError(f"semantic clusters must be in [1,min(S,256)], got {clusters}")
     scale_dtype = _scale_storage_dtype()
     rows = x.permute(0, 2, 1, 3).reshape(sequence, JOINT).contiguous()
-    init = kmeans_init_rows(sequence, clusters, 20260804 + int(layer_idx)).to(x.device)
+    init = kmeans_init_rows(sequence, clusters, 20260804 + int(layer_idx))
     centers, ids = ops.kmeans(rows, clusters, iters, init)
     # the residual against the STORED (bf16) centres, rounded to the input dtype as the reference
     # hands it on (:190-208); the projection then takes the mean off in fp32

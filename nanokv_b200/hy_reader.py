@@ -289,7 +289,7 @@ def _compress_one(x: torch.Tensor, layer_idx: int, target: str, runtime: dict) -
     if clusters <= 0 or clusters > sequence or clusters > 256:
         raise ValueError(f"semantic clusters must be in [1,min(S,256)], got {clusters}")
     rows = x.permute(0, 2, 1, 3).reshape(sequence, heads * dim).contiguous()
-    init = kmeans_init_rows(sequence, clusters, 20260804 + int(layer_idx)).to(x.device)
+    init = kmeans_init_rows(sequence, clusters, 20260804 + int(layer_idx))
     centers, ids = ops.kmeans(rows, clusters, iters, init)
     residual = (rows.float() - centers.float().index_select(0, ids.long())).to(x.dtype)
     zero_center = torch.zeros(1, heads * dim, dtype=torch.bfloat16, device=x.device)

@@ -157,7 +157,7 @@ def encode_tensor(value: torch.Tensor, *, target: str, layer: int, sp_rank: int,
     op = _load_operator(basis_root, target=target, sp_rank=sp_rank, layer=layer, joint_dim=joint_dim,
                         rank=rank, device=value.device, linear_root=linear_root)
     rows = value.reshape(sequence, joint_dim).contiguous()
-    init = kmeans_init_rows(sequence, clusters, _seed(layer, sp_rank, target)).to(value.device)
+    init = kmeans_init_rows(sequence, clusters, _seed(layer, sp_rank, target))
     centers, ids = ops.kmeans(rows, clusters, iters, init)
     packed, scale = ops.project_quant(rows, centers, ids, op.mean, op.encoder, eps=LINGBOT_QUANT.eps,
                                       in_coeff_dtype=False)

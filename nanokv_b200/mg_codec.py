@@ -154,7 +154,7 @@ def encode_tensor(kind: str, layer: int, value: torch.Tensor) -> dict:
         raise ValueError(f"C64 clusters must be in [1,min(S,256)], got {clusters}")
     op = _operator(kind, layer, value.device)
     rows = value[0].contiguous()
-    init = kmeans_init_rows(sequence, clusters, 20260804 + int(layer)).to(value.device)
+    init = kmeans_init_rows(sequence, clusters, 20260804 + int(layer))
     centers, ids = ops.kmeans(rows, clusters, _iterations(), init)
     packed, scale = ops.project_quant(rows, centers, ids, op.mean, op.encoder, eps=F32_EPS,
                                       in_coeff_dtype=op.dtype == torch.bfloat16)

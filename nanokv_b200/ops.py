@@ -51,6 +51,15 @@ def id_dtype(clusters: int) -> torch.dtype:
 
 
 # --------------------------------------------------------------------------- encode
+def upload(values: torch.Tensor, device) -> torch.Tensor:
+    """A small host tensor on ``device``, in order on the current stream and without waiting for what is on it: a copy from
+    pageable memory (``values.to(device)``) ends with a synchronisation.  Inside a stream capture it is that copy, which
+    the capture refuses: a graph must not read host memory that is reused."""
+    if torch.device(device).type != "cuda" or values.is_cuda or torch.cuda.is_current_stream_capturing():
+        return values.to(device)
+    return values.pin_memory().to(device, non_blocking=True)
+
+
 def assign(x: torch.Tensor, centers: torch.Tensor, ids: torch.Tensor | None = None) -> torch.Tensor:
     """Nearest-centre ids of rows x [S,J] against centers [C,J]."""
     device = _require_cuda(x, centers, ids)
@@ -78,7 +87,7 @@ def kmeans(x: torch.Tensor, clusters: int, iters: int, init_rows: torch.Tensor, 
         ids = torch.empty(S, dtype=id_dtype(clusters), device=device)
     nbytes = lib.nkv_kmeans_workspace_bytes(S, J, clusters)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    init_rows = init_rows.to(device=device, dtype=torch.int32).contiguous()
+    init_rows = upload(init_rows.to(torch.int32).contiguous(), device)
     _lib.check(lib.nkv_kmeans(
         _ptr(x), dtype_code(x.dtype), S, J, clusters, iters, _ptr(init_rows), _ptr(centers),
         _ptr(ids), ids.element_size(), _ptr(workspace), nbytes, _stream(device)))
