@@ -17,9 +17,10 @@ namespace nkv {
 namespace {
 
 constexpr int TILE = 64, BK = 16, GROUPS = 4, GROUP_THREADS = 64, THREADS = GROUPS * GROUP_THREADS;
-constexpr int OPERAND = BK * TILE;                       // floats of one operand tile
+constexpr int PITCH = TILE + 4;                          // of a column of K in gemm64's operand tiles
+constexpr int OPERAND = BK * PITCH;                      // floats of one operand tile
 constexpr int SMEM_FLOATS = GROUPS * 2 * 2 * OPERAND;    // two buffers of two operands per group
-static_assert(SMEM_FLOATS == GROUPS * TILE * TILE, "the partial sums reuse the operand tiles");
+static_assert(SMEM_FLOATS >= GROUPS * TILE * TILE, "the partial sums reuse the operand tiles");
 
 // elements k .. k + 3 of a row (0 past K); `vector`: rows start on 16 (fp32) or 8 (16-bit) bytes, K % 4 == 0
 __device__ __forceinline__ float4 load4(const void* base, int dtype, size_t row_start, int k, int K, bool vector) {
@@ -41,13 +42,13 @@ bool vector_rows(const void* base, int dtype, int K) {
   return K % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & (dtype == NKV_F32 ? 15 : 7)) == 0;
 }
 
-// The block's 64 x 64 tile of A B^T over K: load_a(k) / load_b(k) give elements k .. k + 3 of row
-// (thread number in its group) of either operand.  Afterwards sums(row, column) of the tile lie in `sm` as
-// GROUPS partial tiles.
-template <class LA, class LB>
-__device__ __forceinline__ void gemm64(float* sm, int K, LA load_a, LB load_b) {
+// The block's 64 x 64 tile of A B^T over K: op.fetch(c) requests the operands' chunk c of BK columns for the thread's
+// group, op.stage(as, bs) puts them into shared memory, column k of K at k * PITCH.  Afterwards the tile's sums lie in
+// `sm` as GROUPS partial tiles; the caller's barrier comes before tile_sum.
+template <class Operands>
+__device__ __forceinline__ void gemm64(float* sm, int K, Operands& op) {
   const int g = threadIdx.x / GROUP_THREADS, t = threadIdx.x % GROUP_THREADS;
-  const int tx = t & 7, ty = t >> 3;
+  const int tx = t & 7, ty = t >> 3;          // rows ty * 8 .. + 7, columns tx * 4 .. + 3 and 32 + tx * 4 .. + 3
   const int chunks = (K + BK - 1) / BK;
   const int first = chunks * g / GROUPS, last = chunks * (g + 1) / GROUPS;
   float* mine = sm + g * 4 * OPERAND;
@@ -56,35 +57,20 @@ __device__ __forceinline__ void gemm64(float* sm, int K, LA load_a, LB load_b) {
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-  float4 ra[4], rb[4];
-  auto fetch = [&](int c) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      ra[j] = load_a(c * BK + 4 * j);
-      rb[j] = load_b(c * BK + 4 * j);
-    }
-  };
-  if (first < last) fetch(first);
+  if (first < last) op.fetch(first);
+#pragma unroll 1
   for (int c = first; c < last; ++c) {
     float* as = mine + (c & 1) * 2 * OPERAND;
     float* bs = as + OPERAND;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float av[4] = {ra[j].x, ra[j].y, ra[j].z, ra[j].w}, bv[4] = {rb[j].x, rb[j].y, rb[j].z, rb[j].w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        as[(4 * j + i) * TILE + t] = av[i];
-        bs[(4 * j + i) * TILE + t] = bv[i];
-      }
-    }
+    op.stage(as, bs);
     asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(GROUP_THREADS) : "memory");
-    if (c + 1 < last) fetch(c + 1);
+    if (c + 1 < last) op.fetch(c + 1);
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
-      const float4 a0 = *reinterpret_cast<const float4*>(as + k * TILE + ty * 8);
-      const float4 a1 = *reinterpret_cast<const float4*>(as + k * TILE + ty * 8 + 4);
-      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(bs + k * TILE + tx * 8);
-      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(bs + k * TILE + tx * 8 + 4);
+      const float4 a0 = *reinterpret_cast<const float4*>(as + k * PITCH + ty * 8);
+      const float4 a1 = *reinterpret_cast<const float4*>(as + k * PITCH + ty * 8 + 4);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(bs + k * PITCH + tx * 4);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(bs + k * PITCH + 32 + tx * 4);
       const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
       const uint64_t b[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
@@ -99,11 +85,10 @@ __device__ __forceinline__ void gemm64(float* sm, int K, LA load_a, LB load_b) {
   float* part = sm + g * TILE * TILE;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    ulonglong2* dst = reinterpret_cast<ulonglong2*>(part + (ty * 8 + i) * TILE + tx * 8);
-    dst[0] = make_ulonglong2(acc[i][0], acc[i][1]);
-    dst[1] = make_ulonglong2(acc[i][2], acc[i][3]);
+    float* dst = part + (ty * 8 + i) * TILE + tx * 4;
+    *reinterpret_cast<ulonglong2*>(dst) = make_ulonglong2(acc[i][0], acc[i][1]);
+    *reinterpret_cast<ulonglong2*>(dst + 32) = make_ulonglong2(acc[i][2], acc[i][3]);
   }
-  __syncthreads();
 }
 
 // columns c .. c + 3 of a finished row: the groups' partial sums in the order of K
@@ -355,75 +340,181 @@ project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, 
 }
 
 // -------------------------------------------------------------------- decode
-// decoder rows, bias and centre columns of `J` columns; out has rows of out_stride elements
+// Operands of gemm64: codes x scales of 64 tokens, 64 decoder rows.
+struct DecodeSource {
+  const nkv_history& h; int token; const void* decoder; int j0, J; bool d_vec;   // token: of row t, -1 for none
+};
+
 template <bool BF16>
-__global__ void __launch_bounds__(THREADS, 2)
-decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* decoder, bool d_vec,
-                   const float* mean, int J, void* out, int out_dtype, long long out_stride) {
-  extern __shared__ float sm[];
-  __shared__ int tok[TILE], crow[TILE];
-  const int t = threadIdx.x % GROUP_THREADS;
-  const int m0 = blockIdx.x * TILE, n0 = blockIdx.y * TILE;
-  if (threadIdx.x < TILE) {
-    int token = -1, row = 0;
-    if (m0 + t < n) {
-      token = rows_index ? rows_index[m0 + t] : m0 + t;
-      if (token < 0 || token >= h.tokens) token = -1; else row = center_row_of(h, token);
-    }
-    tok[t] = token;
-    crow[t] = row;
-  }
-  __syncthreads();
-  const int token = tok[t];
-  const bool in_b = n0 + t < J;
-  const size_t b_row = static_cast<size_t>(in_b ? n0 + t : 0) * h.rank;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int ngroups = h.rank / h.group;
-  const bool quads = h.group % 4 == 0;      // four coefficients share a scale and two whole bytes
-  auto latent = [&](int k) {
+struct AnyDecode {          // any type, group and alignment: thread t takes row t of either operand
+  const DecodeSource& src;
+  float4 a[4], b[4];
+  __device__ __forceinline__ float4 latent(int k) const {
+    const nkv_history& h = src.h;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (token >= 0 && quads && k < h.rank) {
-      const uint8_t* code = h.codes + static_cast<size_t>(token) * (h.rank >> 1) + (k >> 1);
+    if (src.token >= 0 && h.group % 4 == 0 && k < h.rank) {      // four coefficients share a scale and two whole bytes
+      const uint8_t* code = h.codes + static_cast<size_t>(src.token) * (h.rank >> 1) + (k >> 1);
       const int b0 = __ldg(code), b1 = __ldg(code + 1);
       const float scale = load_float(h.scales, h.scale_dtype,
-                                     static_cast<size_t>(token) * ngroups + (ngroups == 1 ? 0 : k / h.group));
+                                     static_cast<size_t>(src.token) * (h.rank / h.group) + (h.group == h.rank ? 0 : k / h.group));
       v[0] = static_cast<float>((b0 & 15) - 7) * scale;
       v[1] = static_cast<float>((b0 >> 4) - 7) * scale;
       v[2] = static_cast<float>((b1 & 15) - 7) * scale;
       v[3] = static_cast<float>((b1 >> 4) - 7) * scale;
-    } else if (token >= 0) {
+    } else if (src.token >= 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (k + i < h.rank) v[i] = latent_value(h, token, k + i);
+        if (k + i < h.rank) v[i] = latent_value(h, src.token, k + i);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (BF16) v[i] = round_to_bf16(v[i]);
     return make_float4(v[0], v[1], v[2], v[3]);
-  };
-  gemm64(sm, h.rank, latent,
-         [&](int k) { return in_b ? load4(decoder, BF16 ? NKV_BF16 : NKV_F32, b_row, k, h.rank, d_vec) : zero; });
-  const uint16_t* centers = static_cast<const uint16_t*>(h.centers);
-  const int row = threadIdx.x >> 2;
-  if (m0 + row >= n || tok[row] < 0) return;
+  }
+  __device__ __forceinline__ void fetch(int c) {
+    const int row = src.j0 + threadIdx.x % GROUP_THREADS, K = src.h.rank;
 #pragma unroll
-  for (int j = 0; j < 16; j += 4) {
-    const int c0 = (threadIdx.x & 3) * 4 + j * 4;
-    const float4 s = tile_sum(sm, row, c0);
-    const float sums[4] = {s.x, s.y, s.z, s.w};
+    for (int j = 0; j < 4; ++j) {
+      a[j] = latent(c * BK + 4 * j);
+      b[j] = row < src.J ? load4(src.decoder, BF16 ? NKV_BF16 : NKV_F32, static_cast<size_t>(row) * K, c * BK + 4 * j, K, src.d_vec)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  __device__ __forceinline__ void stage(float* as, float* bs) const {
+    const int t = threadIdx.x % GROUP_THREADS;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = n0 + c0 + i;
-      if (c >= J) continue;
-      const float center = bf16_bits_to_float(centers[static_cast<size_t>(crow[row]) * h.center_width + c]);
-      float v;
-      if (BF16) {
-        v = round_to_bf16(__fadd_rn(sums[i], round_to_bf16(mean[c])));
-        v = round_to_bf16(__fadd_rn(v, center));
-      } else {
-        v = __fadd_rn(__fadd_rn(sums[i], mean[c]), center);
+    for (int j = 0; j < 4; ++j) {
+      const float av[4] = {a[j].x, a[j].y, a[j].z, a[j].w}, bv[4] = {b[j].x, b[j].y, b[j].z, b[j].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        as[(4 * j + i) * PITCH + t] = av[i];
+        bs[(4 * j + i) * PITCH + t] = bv[i];
       }
-      store_float(out, out_dtype, static_cast<size_t>(m0 + row) * out_stride + c, v);
+    }
+  }
+};
+
+// fp32 decoder rows read as vectors, BK dividing rank and group, the codes of a chunk as one word of 8 bytes: thread t
+// takes the codes and the scale of row t; of the decoder two threads take 32 bytes of a row, which PITCH puts into
+// different banks.  No load has a condition on it, so a chunk's are in flight while the one before is multiplied.
+// Bound: multiply-adds, 128 a cycle and SM, of which 45 to 58% is reached; AnyDecode is bound by its loads, each of
+// which touches a line per lane.  us of a decode, VectorDecode / AnyDecode, x 1,536 columns of rank 192: 300 tokens
+// 8.7 / 14.1, 2,048 37.6 / 64.0; x 3,072 columns of rank 384: 4,096 229 / 404.
+struct VectorDecode {
+  const uint2* codes; const uint16_t* scales; const float* rows; int K, group; bool one, f16;
+  long long half;         // elements to the decoder row 32 further on
+  uint2 a; uint16_t scale; float4 b[4];
+  __device__ __forceinline__ explicit VectorDecode(const DecodeSource& src) {
+    const int t = threadIdx.x % GROUP_THREADS, row = src.j0 + (t >> 1);     // rows and tokens past the last: the first
+    const size_t token = src.token < 0 ? 0 : src.token;
+    K = src.h.rank;
+    group = src.h.group;
+    one = group == K;
+    f16 = src.h.scale_dtype == NKV_F16;
+    codes = reinterpret_cast<const uint2*>(src.h.codes + token * (K >> 1));
+    scales = static_cast<const uint16_t*>(src.h.scales) + token * (one ? 1 : K / group);
+    const long long low = row < src.J ? row : 0, high = row + 32 < src.J ? row + 32 : 0;
+    rows = static_cast<const float*>(src.decoder) + low * K + (t & 1) * 4;
+    half = (high - low) * K;
+  }
+  __device__ __forceinline__ void fetch(int c) {
+    a = __ldg(codes + c);
+    scale = __ldg(scales + (one ? 0 : c * BK / group));
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      b[j] = __ldg(reinterpret_cast<const float4*>(rows + (c * BK + (j & 1) * 8 + (j >> 1) * half)));
+  }
+  __device__ __forceinline__ void stage(float* as, float* bs) const {
+    const int t = threadIdx.x % GROUP_THREADS;
+    const float s = f16 ? __half2float(__ushort_as_half(scale)) : bf16_bits_to_float(scale);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      const int code = (k < 8 ? a.x : a.y) >> (4 * (k & 7)) & 15;
+      as[k * PITCH + t] = static_cast<float>(code - 7) * s;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float v[4] = {b[j].x, b[j].y, b[j].z, b[j].w};
+      const int row = (t >> 1) + (j >> 1) * 32, k = (j & 1) * 8 + (t & 1) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bs[(k + i) * PITCH + row] = v[i];
+    }
+  }
+};
+
+// decoder rows, bias and centre columns of `J` columns; out has rows of out_stride elements.  VECTOR: operands as
+// VectorDecode takes them; mean, centres and out in pieces of four columns.
+template <bool BF16, bool VECTOR>
+__global__ void __launch_bounds__(THREADS, 2)
+decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* decoder, bool d_vec,
+                   const float* mean, int J, void* out, int out_dtype, long long out_stride) {
+  static_assert(!(BF16 && VECTOR), "the bf16 operators' decode of aligned rows is on the tensor cores");
+  extern __shared__ float sm[];
+  __shared__ int tok[TILE], crow[TILE];
+  const int t = threadIdx.x % GROUP_THREADS;
+  const int m0 = blockIdx.x * TILE, n0 = blockIdx.y * TILE;
+  int token = -1;
+  if (m0 + t < n) {
+    token = rows_index ? rows_index[m0 + t] : m0 + t;
+    if (token < 0 || token >= h.tokens) token = -1;
+  }
+  if (threadIdx.x < TILE) {
+    tok[t] = token;
+    crow[t] = token < 0 ? 0 : center_row_of(h, token);
+  }
+  const DecodeSource source{h, token, decoder, n0, J, d_vec};
+  if constexpr (VECTOR) {
+    VectorDecode operands(source);
+    gemm64(sm, h.rank, operands);
+  } else {
+    AnyDecode<BF16> operands{source};
+    gemm64(sm, h.rank, operands);
+  }
+  const uint16_t* centers = static_cast<const uint16_t*>(h.centers);
+  constexpr int PASSES = TILE * TILE / 4 / THREADS;
+  const int row0 = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 4;       // rows row0, row0 + 16 ...
+  if constexpr (VECTOR) {
+    const int col = n0 + c0 < J ? n0 + c0 : 0;
+    uint2 centre[PASSES];
+    const float4 m = __ldg(reinterpret_cast<const float4*>(mean + col));
+    // tok and crow are another thread's: the barrier that gemm64 has in front of its partial sums lies between
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i)
+      centre[i] = __ldg(reinterpret_cast<const uint2*>(centers + static_cast<size_t>(crow[row0 + i * 16]) * h.center_width + col));
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PASSES; ++i) {
+      const int row = row0 + i * 16;
+      if (m0 + row >= n || tok[row] < 0 || n0 + c0 >= J) continue;
+      const float4 s = tile_sum(sm, row, c0);
+      const uint2 c = centre[i];
+      *reinterpret_cast<float4*>(static_cast<float*>(out) + static_cast<size_t>(m0 + row) * out_stride + n0 + c0) =
+          make_float4(__fadd_rn(__fadd_rn(s.x, m.x), __uint_as_float(c.x << 16)),
+                      __fadd_rn(__fadd_rn(s.y, m.y), __uint_as_float(c.x & 0xFFFF0000u)),
+                      __fadd_rn(__fadd_rn(s.z, m.z), __uint_as_float(c.y << 16)),
+                      __fadd_rn(__fadd_rn(s.w, m.w), __uint_as_float(c.y & 0xFFFF0000u)));
+    }
+  } else {
+    __syncthreads();
+#pragma unroll 1
+    for (int row = row0; row < TILE; row += 16) {
+      if (m0 + row >= n || tok[row] < 0) continue;
+      const float4 s = tile_sum(sm, row, c0);
+      const float sums[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = n0 + c0 + i;
+        if (c >= J) continue;
+        const float center = bf16_bits_to_float(centers[static_cast<size_t>(crow[row]) * h.center_width + c]);
+        float v;
+        if (BF16) {
+          v = round_to_bf16(__fadd_rn(sums[i], round_to_bf16(mean[c])));
+          v = round_to_bf16(__fadd_rn(v, center));
+        } else {
+          v = __fadd_rn(__fadd_rn(sums[i], mean[c]), center);
+        }
+        store_float(out, out_dtype, static_cast<size_t>(m0 + row) * out_stride + c, v);
+      }
     }
   }
 }
@@ -650,7 +741,13 @@ int simt_decode_rows(const nkv_history& hist, const int32_t* rows_index, int n,
                      int out_dtype, int64_t out_stride, cudaStream_t stream) {
   if (n == 0) return NKV_OK;
   const dim3 grid(ceil_div(n, TILE), ceil_div(J, TILE));
-  auto kernel = dec_dtype == NKV_BF16 ? decode_rows_kernel<true> : decode_rows_kernel<false>;
+  const auto aligned = [](const void* at, int bytes) { return reinterpret_cast<uintptr_t>(at) % bytes == 0; };
+  const bool vector = dec_dtype == NKV_F32 && out_dtype == NKV_F32 && hist.tokens > 0 && hist.rank % BK == 0 &&
+                      hist.group % BK == 0 && J % 4 == 0 && out_stride % 4 == 0 && hist.center_width % 4 == 0 &&
+                      aligned(decoder, 16) && aligned(mean, 16) && aligned(out, 16) && aligned(hist.codes, 8) &&
+                      aligned(hist.scales, 2) && aligned(hist.centers, 8);
+  auto kernel = dec_dtype == NKV_BF16 ? decode_rows_kernel<true, false>
+                : vector ? decode_rows_kernel<false, true> : decode_rows_kernel<false, false>;
   int rc = allow_smem(kernel);
   if (rc != NKV_OK) return rc;
   kernel<<<grid, THREADS, SMEM_FLOATS * 4, stream>>>(hist, rows_index, n, decoder,

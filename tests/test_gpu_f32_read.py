@@ -67,3 +67,23 @@ def test_assignment_and_projection(S, J, C, dtype):
     want = residual @ encoder.double().T
     bound = (J + 4) * 2.0 ** -24 * (residual.abs() @ encoder.double().abs().T) + 2.0 ** -22 * 16
     assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("tokens", [1, 31, 64, 65, 193])
+@pytest.mark.parametrize("joint,rank,group", [(4, 16, None), (64, 48, 16), (100, 64, 32), (132, 80, 80), (196, 192, 48)])
+@pytest.mark.parametrize("scale_dtype", [torch.bfloat16, torch.float16])
+def test_vector_form_gives_the_general_forms_bits(tokens, joint, rank, group, scale_dtype):
+    """A decoder four bytes off a vector's start is read element by element; both sum in the same order."""
+    hist = random_history(tokens, joint, rank, group=group, scale_dtype=scale_dtype, segments=min(3, tokens))
+    decoder = torch.randn(joint, rank, device="cuda") / rank ** 0.5
+    shifted = torch.empty(joint * rank + 1, device="cuda")[1:].view(joint, rank).copy_(decoder)
+    mean = torch.randn(joint, device="cuda")
+    listed = torch.tensor([tokens - 1, 0, tokens // 2] * 25, dtype=torch.int32, device="cuda")
+    for rows in (None, listed):
+        got, want = (ops.decode_rows(hist.view(), d, mean, rows=rows) for d in (decoder, shifted))
+        assert torch.equal(got, want)
+    listed[1], listed[2] = -1, tokens           # rows that are not there leave the others alone
+    got = ops.decode_rows(hist.view(), decoder, mean, rows=listed)
+    keep = torch.ones(75, dtype=torch.bool, device="cuda")
+    keep[1:3] = False
+    assert torch.equal(got[keep], want[keep])
