@@ -522,7 +522,10 @@ decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* 
 // ----------------------------------------------------------------- attention
 // Block = 64 queries of one head over one run of history tokens, 64 at a time: K and V tiles in shared
 // memory, online softmax in fp32, two blocks per SM.  A thread owns 4 x 4 scores and 4 queries x D / 16
-// columns of O; multiply-adds are packed pairs.
+// columns of O; multiply-adds are packed pairs.  K of the next tile waits in registers while the weights meet V, and V
+// arrives while the scores are made.  Bound: what shared memory gives to registers, 128 bytes a cycle, twice the
+// multiply-adds' time at these 4 x 4 pieces.  us of a read with rank 32, now / with K and V fetched between the tiles:
+// 2,048 tokens, 12 heads of 64 and 256 queries 85 / 91; heads of 128, 4,096 tokens and 512 queries 451 / 457.
 struct RowAttn {
   const float* q; const float* k; const float* v;
   long long q_stride_token, q_stride_head, kv_stride_token, kv_stride_head;
@@ -560,19 +563,30 @@ attn_rows_f32_kernel(RowAttn a) {
 #pragma unroll
     for (int c = 0; c < OP; ++c) o[i][c] = 0ull;
   }
+  constexpr int PIECES = 64 * (D / 4) / 256;       // of four values, per thread and tile
+  float4 kr[PIECES];
+  auto fetch_k = [&](int t0) {                     // tokens past the last: the last one's, whose weight is zero
+    const float* row = a.k + static_cast<size_t>(min(t0 + tid % 64, t_end - 1)) * a.kv_stride_token +
+                       static_cast<size_t>(head) * a.kv_stride_head + tid / 64 * 4;
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) kr[p] = *reinterpret_cast<const float4*>(row + p * 16);
+  };
+  fetch_k(t_begin);
   for (int t0 = t_begin; t0 < t_end; t0 += 64) {
     __syncthreads();                 // previous tile fully consumed
-    for (int idx = tid; idx < 64 * (D / 4); idx += 256) {
-      const int i = idx % 64, d = idx / 64 * 4;
-      const float4 v = t0 + i < t_end ? *reinterpret_cast<const float4*>(a.k + static_cast<size_t>(t0 + i) * a.kv_stride_token +
-                                                                        static_cast<size_t>(head) * a.kv_stride_head + d) : zero;
-      Ks[d * 64 + i] = v.x; Ks[(d + 1) * 64 + i] = v.y; Ks[(d + 2) * 64 + i] = v.z; Ks[(d + 3) * 64 + i] = v.w;
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {             // V: straight to shared memory while the scores are made
+      const int idx = tid + p * 256, i = idx / (D / 4), d = idx % (D / 4) * 4;
+      const int token = min(t0 + i, t_end - 1), bytes = t0 + i < t_end ? 16 : 0;      // past the last: zeros
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(Vs + i * D + d))),
+                   "l"(a.v + static_cast<size_t>(token) * a.kv_stride_token + static_cast<size_t>(head) * a.kv_stride_head + d),
+                   "r"(bytes) : "memory");
     }
-    for (int idx = tid; idx < 64 * (D / 4); idx += 256) {
-      const int i = idx / (D / 4), d = idx % (D / 4) * 4;
-      *reinterpret_cast<float4*>(Vs + i * D + d) =
-          t0 + i < t_end ? *reinterpret_cast<const float4*>(a.v + static_cast<size_t>(t0 + i) * a.kv_stride_token +
-                                                           static_cast<size_t>(head) * a.kv_stride_head + d) : zero;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      float* at = Ks + (tid / 64 * 4 + p * 16) * 64 + tid % 64;
+      at[0] = kr[p].x; at[64] = kr[p].y; at[128] = kr[p].z; at[192] = kr[p].w;
     }
     __syncthreads();
     uint64_t s2[4][2] = {};
@@ -622,6 +636,8 @@ attn_rows_f32_kernel(RowAttn a) {
     for (int j = 0; j < 4; ++j)
       *reinterpret_cast<float4*>(Ps + (tx * 4 + j) * 64 + ty * 4) =
           make_float4(weight[0][j], weight[1][j], weight[2][j], weight[3][j]);
+    if (t0 + 64 < t_end) fetch_k(t0 + 64);         // in flight while the weights meet V
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 #pragma unroll 4
     for (int t = 0; t < 64; ++t) {
