@@ -291,6 +291,157 @@ assign_kernel(const void* x, int x_dtype, bool x_vec, const void* centers, int c
   }
 }
 
+// Few centres: block = 16 rows of x against all TN of them (16, 32 or 64 columns, C used), so that 2,048 rows are 128
+// blocks, and no column of a 64-wide tile is multiplied for nothing.  64 columns of K per stage come by cp.async as they
+// lie in memory, six stages in flight; the multiplying warps (8 rows x 16 centres each, a thread 2 x 2) read four columns
+// of a row at a time, and the norms are other warps' work.  Sums in the order of K and norms in four chains, as in
+// gemm_ordered: the same ids.  Bound: what shared memory gives to registers, 128 bytes a cycle (64 columns of K, 16 bf16
+// centres: 448 cycles, about half of the step's time).  us, 1,536 columns, 16 / 32 / 64 bf16 centres, now (gemm_ordered):
+// 2,048 rows 14 / 18 / 28 (56 / 60 / 67), 9,000 rows 29 / 45 / 85 (71 / 75 / 84), 40,000 rows 107 / 166 / 345
+// (330 / 350 / 385).
+constexpr int FEW_ROWS = 16, FEW_STEP = 64, FEW_STAGES = 6;
+
+template <int TN, Form C_>
+struct Few {
+  static constexpr int MULTIPLY_WARPS = TN / 8, NORM_WARPS = 1 + (TN + 31) / 32;   // x, centres
+  static constexpr int THREADS = (MULTIPLY_WARPS + NORM_WARPS) * 32;
+  static constexpr int X_PITCH = FEW_STEP + 4;                                          // floats
+  static constexpr int C_PITCH = C_ == BF16_ROWS ? FEW_STEP * 2 + 16 : FEW_STEP * 4 + 16;      // bytes
+  static constexpr int X_BYTES = FEW_ROWS * X_PITCH * 4, STAGE = X_BYTES + TN * C_PITCH;
+  static __device__ __forceinline__ float4 centre(const uint8_t* row, int k) {
+    if constexpr (C_ == BF16_ROWS) return RowOperand<BF16_ROWS>{}.value(*reinterpret_cast<const uint2*>(row + k * 2));
+    else return *reinterpret_cast<const float4*>(row + k * 4);
+  }
+};
+
+__device__ __forceinline__ void copy_async(void* smem, const void* global) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
+               "l"(global) : "memory");
+}
+
+template <int TN, Form C_>
+__global__ void __launch_bounds__(Few<TN, C_>::THREADS)
+assign_few_kernel(const float* x, const void* centers, int S, int J, int C, void* ids, int id_bytes, int32_t* labels32) {
+  using F = Few<TN, C_>;
+  extern __shared__ __align__(16) uint8_t stages[];
+  __shared__ float norms[FEW_ROWS + TN];
+  __shared__ float row_d[TN / 16][FEW_ROWS];
+  __shared__ int row_i[TN / 16][FEW_ROWS];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int m0 = blockIdx.x * FEW_ROWS, steps = J / FEW_STEP;
+  constexpr int C_SIZE = C_ == BF16_ROWS ? 2 : 4, C_PIECES = FEW_STEP * C_SIZE / 16, PIECES = FEW_ROWS * 16 + TN * C_PIECES;
+  constexpr int LOADERS = F::NORM_WARPS * 32, LOADS = (PIECES + LOADERS - 1) / LOADERS;
+  const uint8_t* from[LOADS];            // the loader's pieces of 16 bytes, where they come from and go to
+  int to[LOADS];
+  const int loader = t - F::MULTIPLY_WARPS * 32;
+#pragma unroll
+  for (int l = 0; l < LOADS; ++l) {      // rows past the last: another one (of centres not one row for all of them)
+    const int i = loader + l * LOADERS, j = i - FEW_ROWS * 16;
+    if (i < FEW_ROWS * 16) {
+      from[l] = reinterpret_cast<const uint8_t*>(x + static_cast<size_t>(min(m0 + (i >> 4), S - 1)) * J) + (i & 15) * 16;
+      to[l] = (i >> 4) * F::X_PITCH * 4 + (i & 15) * 16;
+    } else {
+      from[l] = static_cast<const uint8_t*>(centers) + static_cast<size_t>(j / C_PIECES % C) * J * C_SIZE + j % C_PIECES * 16;
+      to[l] = F::X_BYTES + j / C_PIECES * F::C_PITCH + j % C_PIECES * 16;
+    }
+  }
+  auto request = [&](int step) {
+    if (step < steps) {
+      uint8_t* at = stages + step % FEW_STAGES * F::STAGE;
+#pragma unroll
+      for (int l = 0; l < LOADS; ++l) {
+        const bool rows_of_x = l * LOADERS + LOADERS <= FEW_ROWS * 16 || loader + l * LOADERS < FEW_ROWS * 16;
+        if (PIECES % LOADERS == 0 || loader + l * LOADERS < PIECES)
+          copy_async(at + to[l], from[l] + step * (FEW_STEP * (rows_of_x ? 4 : C_SIZE)));
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");      // an empty one past the last step keeps the count
+  };
+  const bool multiplies = warp < F::MULTIPLY_WARPS;
+  const int row = (warp & 1) * 8 + (lane >> 3) * 2, column = (warp >> 1) * 16 + (lane & 7);    // and row + 1, column + 8
+  // squared: a row of x by the first of the other warps, a centre by the rest (two types in one warp would merge loads)
+  const bool of_x = warp == F::MULTIPLY_WARPS;
+  const int squared = of_x ? lane : loader - 32;
+  const bool squares = !multiplies && squared < (of_x ? FEW_ROWS : TN);
+  float dot[2][2] = {}, norm[4] = {0.f, 0.f, 0.f, 0.f};
+  if (!multiplies)
+    for (int step = 0; step < FEW_STAGES - 1; ++step) request(step);
+  for (int step = 0; step < steps; ++step) {
+    if (!multiplies) asm volatile("cp.async.wait_group %0;" ::"n"(FEW_STAGES - 2) : "memory");
+    __syncthreads();                      // all copies of this step; the stage before it has been read
+    if (!multiplies) request(step + FEW_STAGES - 1);
+    const uint8_t* at = stages + step % FEW_STAGES * F::STAGE;
+    const float* xs = reinterpret_cast<const float*>(at);
+    const uint8_t* cs = at + F::X_BYTES;
+    if (multiplies) {
+#pragma unroll
+      for (int k = 0; k < FEW_STEP; k += 4) {
+        const float4 a[2] = {*reinterpret_cast<const float4*>(xs + row * F::X_PITCH + k),
+                             *reinterpret_cast<const float4*>(xs + (row + 1) * F::X_PITCH + k)};
+        const float4 b[2] = {F::centre(cs + column * F::C_PITCH, k), F::centre(cs + (column + 8) * F::C_PITCH, k)};
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            dot[i][j] = fmaf(a[i].x, b[j].x, dot[i][j]);
+            dot[i][j] = fmaf(a[i].y, b[j].y, dot[i][j]);
+            dot[i][j] = fmaf(a[i].z, b[j].z, dot[i][j]);
+            dot[i][j] = fmaf(a[i].w, b[j].w, dot[i][j]);
+          }
+      }
+    } else if (squares) {
+      auto square = [&](const float4& v) {
+        norm[0] = fmaf(v.x, v.x, norm[0]);
+        norm[1] = fmaf(v.y, v.y, norm[1]);
+        norm[2] = fmaf(v.z, v.z, norm[2]);
+        norm[3] = fmaf(v.w, v.w, norm[3]);
+      };
+      if (of_x) {
+#pragma unroll 8
+        for (int k = 0; k < FEW_STEP; k += 4) square(*reinterpret_cast<const float4*>(xs + squared * F::X_PITCH + k));
+      } else {
+#pragma unroll 8
+        for (int k = 0; k < FEW_STEP; k += 4) square(F::centre(cs + squared * F::C_PITCH, k));
+      }
+    }
+  }
+  if (squares) norms[(of_x ? 0 : FEW_ROWS) + squared] = (norm[0] + norm[1]) + (norm[2] + norm[3]);
+  __syncthreads();
+  if (multiplies) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float d = INFINITY;
+      int idx = 0x7fffffff;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int c = column + j * 8;
+        // (||x||^2 + ||c||^2) - 2 x.c, in that association, in fp32
+        const float dist = __fsub_rn(__fadd_rn(norms[row + i], norms[FEW_ROWS + c]), __fmul_rn(2.0f, dot[i][j]));
+        if (c < C && dist < d) { d = dist; idx = c; }
+      }
+#pragma unroll
+      for (int off = 1; off < 8; off <<= 1) {
+        const float od = __shfl_xor_sync(0xffffffffu, d, off);
+        const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
+        if (od < d || (od == d && oi < idx)) { d = od; idx = oi; }
+      }
+      if ((lane & 7) == 0) { row_d[warp >> 1][row + i] = d; row_i[warp >> 1][row + i] = idx; }
+    }
+  }
+  __syncthreads();
+  if (t >= FEW_ROWS || m0 + t >= S) return;
+  float best = INFINITY;                  // no distance below it (NaN, infinities): centre 0
+  int best_i = 0;
+#pragma unroll
+  for (int g = 0; g < TN / 16; ++g)
+    if (row_d[g][t] < best) { best = row_d[g][t]; best_i = row_i[g][t]; }
+  if (ids) {
+    if (id_bytes == 1) static_cast<uint8_t*>(ids)[m0 + t] = static_cast<uint8_t>(best_i);
+    else static_cast<uint16_t*>(ids)[m0 + t] = static_cast<uint16_t>(best_i);
+  }
+  if (labels32) labels32[m0 + t] = best_i;
+}
+
 // ---------------------------------------------------------------- projection
 template <bool BF16, Form X, Form C_, Form M>
 struct Residual {      // (x - centre) - mean, rounded to bf16 where the operators are
@@ -716,11 +867,32 @@ static int ordered_rows(int S, int column_tiles) {
   return static_cast<long long>(ceil_div(S, 32)) * column_tiles <= sm_count() ? 32 : 64;
 }
 
+template <int TN>
+static int assign_few(const float* x, const void* centers, int c_dtype, int S, int J, int C, void* ids, int id_bytes,
+                      int32_t* labels32, cudaStream_t stream) {
+  const bool bf16 = c_dtype == NKV_BF16;
+  auto kernel = bf16 ? assign_few_kernel<TN, BF16_ROWS> : assign_few_kernel<TN, F32_ROWS>;
+  const int smem = FEW_STAGES * (bf16 ? Few<TN, BF16_ROWS>::STAGE : Few<TN, F32_ROWS>::STAGE);
+  NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kernel<<<ceil_div(S, FEW_ROWS), Few<TN, BF16_ROWS>::THREADS, smem, stream>>>(x, centers, S, J, C, ids, id_bytes, labels32);
+  NKV_LAUNCH_CHECK("assign_few_kernel");
+  return NKV_OK;
+}
+
 int simt_assign(const void* x, int x_dtype, const void* centers, int c_dtype, int S, int J,
                 int C, void* ids, int id_bytes, int32_t* labels32, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
-  const int rows = ordered_rows(S, 1);
   const bool x_rows = has_form(F32_ROWS, x, x_dtype, J);
+  // 33 to 64 centres in fp32 are twice the bytes of bf16 through shared memory: beyond two blocks per SM gemm_ordered's
+  // tile, whose values are reused more, is ahead (4,096 rows 65 / 69 us, 9,000 rows 129 / 84)
+  const bool few = C >= 1 && (C <= 32 || (C <= 64 && (c_dtype == NKV_BF16 || ceil_div(S, FEW_ROWS) <= 2 * sm_count())));
+  if (few && x_rows && J % FEW_STEP == 0 && (reinterpret_cast<uintptr_t>(centers) & 15) == 0) {
+    const float* rows = static_cast<const float*>(x);
+    return C <= 16   ? assign_few<16>(rows, centers, c_dtype, S, J, C, ids, id_bytes, labels32, stream)
+           : C <= 32 ? assign_few<32>(rows, centers, c_dtype, S, J, C, ids, id_bytes, labels32, stream)
+                     : assign_few<64>(rows, centers, c_dtype, S, J, C, ids, id_bytes, labels32, stream);
+  }
+  const int rows = ordered_rows(S, 1);
   auto kernel = x_rows && has_form(BF16_ROWS, centers, c_dtype, J)
                     ? (rows == 32 ? assign_kernel<32, F32_ROWS, BF16_ROWS> : assign_kernel<64, F32_ROWS, BF16_ROWS>)
                 : x_rows && has_form(F32_ROWS, centers, c_dtype, J)

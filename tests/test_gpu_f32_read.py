@@ -87,3 +87,20 @@ def test_vector_form_gives_the_general_forms_bits(tokens, joint, rank, group, sc
     keep = torch.ones(75, dtype=torch.bool, device="cuda")
     keep[1:3] = False
     assert torch.equal(got[keep], want[keep])
+
+
+@pytest.mark.parametrize("S", [1, 15, 16, 17, 333])
+@pytest.mark.parametrize("C", [1, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("J", [64, 320, 448])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_few_centres_give_the_ids_of_the_general_form(S, C, J, dtype):
+    """Rows four bytes off a vector's start take the general form; both sum in the same order, ties and non-finite rows
+    included."""
+    x = torch.randn(S, J, device="cuda")
+    centers = torch.randn(C, J, device="cuda").to(dtype)
+    centers[C // 2] = centers[C - 1]                          # equal distances: the lower index
+    x[S // 2] = centers[C - 1].float()
+    if S > 4:
+        x[1, 3], x[2, J - 1], x[3] = float("nan"), float("inf"), 3e38
+    shifted = torch.empty(S * J + 1, device="cuda")[1:].view(S, J).copy_(x)
+    assert torch.equal(ops.assign(x, centers), ops.assign(shifted, centers))
