@@ -6,9 +6,9 @@
 // reproduce the rounding points of the bf16 path, which the test-suite uses to cross-check the
 // tensor-core kernels at full size.
 //
-// Two forms of the GEMM, both with packed multiply-adds and the operands of the next steps in registers while one is
-// multiplied.  Assignment and projection (gemm_ordered): every sum is one chain of fused multiply-adds in the
-// order of K, because what they give is stored -- ids, and codes that another order would move now and then.
+// Assignment and projection: every sum is one chain of fused multiply-adds in the order of K, because what they give is
+// stored -- ids, and codes that another order would move now and then.  assign_few_kernel and project_rows_kernel take
+// aligned fp32 rows; gemm_ordered takes the rest, with packed multiply-adds and two steps' operands in registers.
 // Row decode (gemm64): 64 x 64 of the product per block; its four groups of 64 threads take a quarter of K each,
 // with operand tiles and barriers of their own, and add their sums in order at the end.
 #include "nkv_internal.h"
@@ -107,10 +107,10 @@ __device__ __forceinline__ float4 tile_sum(const float* sm, int row, int c) {
 // 32 columns of K through one of two buffers; a.load(k) / b.load(k) give elements k .. k + 3 of row threadIdx.x % TM
 // resp. % 64 as they come from memory, a.value / b.value what is multiplied: the operands of two steps are in flight
 // while one is multiplied.  Bound: 4,096 multiply-adds per column of K and 64 x 64 tile, 32 cycles of an SM (a step of
-// 1,024 cycles, of which about half is reached).  us, 1,536 columns, projection to 192 / assignment to 16 centres, now
-// and with one step in flight whose loads stood in branches on type and range (a branch's result is merged into a
-// register, which waits for the load: no step overlapped its loads): 300 tokens 66 / 56 (84 / 70), 2,048 82 / 55
-// (131 / 90), 4,096 156 / 55 (167 / 89).
+// 1,024 cycles); reached is what shared memory gives to registers, 128 bytes a cycle, twice that time at pieces of
+// 4 x 4.  us, 1,536 columns, assignment to 256 bf16 centres, now and with one step in flight whose loads stood in
+// branches on type and range (a branch's result is merged into a register, which waits for the load: no step
+// overlapped its loads): 2,048 tokens 262 (316), 9,000 322 (399).
 constexpr int STEP = 32;
 template <int TM>
 constexpr int ORDERED_FLOATS = 2 * STEP * (TM + TILE);
@@ -443,26 +443,24 @@ assign_few_kernel(const float* x, const void* centers, int S, int J, int C, void
 }
 
 // ---------------------------------------------------------------- projection
-template <bool BF16, Form X, Form C_, Form M>
+__device__ __forceinline__ float4 residual_of(const float4& x, const float4& c, const float4& m) {
+  return make_float4(__fsub_rn(__fsub_rn(x.x, c.x), m.x), __fsub_rn(__fsub_rn(x.y, c.y), m.y),
+                     __fsub_rn(__fsub_rn(x.z, c.z), m.z), __fsub_rn(__fsub_rn(x.w, c.w), m.w));
+}
+
+template <bool BF16>
 struct Residual {      // (x - centre) - mean, rounded to bf16 where the operators are
-  RowOperand<X> x; RowOperand<C_> centre; RowOperand<M> mean;
-  struct Raw {
-    decltype(RowOperand<X>{}.load(0)) x;
-    decltype(RowOperand<C_>{}.load(0)) centre;
-    float4 mean;
-  };
+  RowOperand<ANY> x, centre, mean;
+  struct Raw { float4 x, centre, mean; };
   __device__ __forceinline__ Raw load(int k) const { return Raw{x.load(k), centre.load(k), mean.load(k)}; }
   __device__ __forceinline__ float4 value(const Raw& raw) const {
-    const float4 v = x.value(raw.x), c = centre.value(raw.centre), m = raw.mean;
-    float4 res = make_float4(__fsub_rn(__fsub_rn(v.x, c.x), m.x), __fsub_rn(__fsub_rn(v.y, c.y), m.y),
-                             __fsub_rn(__fsub_rn(v.z, c.z), m.z), __fsub_rn(__fsub_rn(v.w, c.w), m.w));
+    float4 res = residual_of(raw.x, raw.centre, raw.mean);
     if (BF16) res = make_float4(round_to_bf16(res.x), round_to_bf16(res.y), round_to_bf16(res.z), round_to_bf16(res.w));
     return res;
   }
 };
 
-// FAST: fp32 rows, operators and mean as vectors; otherwise anything
-template <bool BF16, int TM, bool FAST>
+template <bool BF16, int TM>
 __global__ void __launch_bounds__(THREADS, 2)
 project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, bool c_vec, const void* ids, int id_bytes,
                const float* mean, const void* encoder, bool e_vec, int S, int J, int r, void* coeff) {
@@ -473,11 +471,10 @@ project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, 
   const bool in_a = m0 + t % TM < S, in_b = n0 + t % TILE < r;
   const size_t a_row = static_cast<size_t>(in_a ? m0 + t % TM : 0) * J, b_row = static_cast<size_t>(in_b ? n0 + t % TILE : 0) * J;
   const size_t c_row = static_cast<size_t>(in_a ? load_id(ids, id_bytes, m0 + t % TM) : 0) * J;
-  constexpr Form F = FAST ? F32_ROWS : ANY, C_ = FAST ? BF16_ROWS : ANY;
-  const Residual<BF16, F, C_, F> residual{{x, x_dtype, a_row, J, x_vec, in_a}, {centers, NKV_BF16, c_row, J, c_vec, in_a},
-                                          {mean, NKV_F32, 0, J, e_vec, in_a}};
+  const Residual<BF16> residual{{x, x_dtype, a_row, J, x_vec, in_a}, {centers, NKV_BF16, c_row, J, c_vec, in_a},
+                                {mean, NKV_F32, 0, J, e_vec, in_a}};
   float sums[ROWS][4], unused[4];
-  gemm_ordered<TM, false>(sm, J, residual, RowOperand<F>{encoder, BF16 ? NKV_BF16 : NKV_F32, b_row, J, e_vec, in_b}, sums, unused);
+  gemm_ordered<TM, false>(sm, J, residual, RowOperand<ANY>{encoder, BF16 ? NKV_BF16 : NKV_F32, b_row, J, e_vec, in_b}, sums, unused);
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
     const int token = m0 + ty * ROWS + i;
@@ -486,6 +483,108 @@ project_kernel(const void* x, int x_dtype, bool x_vec, const uint16_t* centers, 
     for (int j = 0; j < 4; ++j) {
       const int c = n0 + tx * 4 + j;
       if (c < r) store_float(coeff, BF16 ? NKV_BF16 : NKV_F32, static_cast<size_t>(token) * r + c, sums[i][j]);
+    }
+  }
+}
+
+// fp32 rows, operators and mean as vectors: block = TM rows x 64 columns of the encoder, thread = TM / 8 x 4 sums, each one
+// chain in the order of K as above.  Bound: what shared memory gives to registers, 128 bytes a cycle -- (TM / 8 + 4) * 4
+// cycles per column of K, where gemm_ordered's 4 x 4 pieces take 64 for 64 rows -- and the lines that loads touch: eight
+// threads read a line of a row of x here, one row per thread there.  Operand tiles lie as in memory, 32 columns of K and
+// four words of padding a row, which the reads of eight rows need; a thread takes four columns of K at a time.  The
+// encoder's come by cp.async, three steps ahead; x, centre and mean wait in registers, two steps ahead.  us, 1,536
+// columns to 192, now (gemm_ordered): 300 tokens 25 (67), 2,048 44 (83), 4,096 77 (162), 20,000 300 (551).
+constexpr int ROW_THREADS = 128, ROW_PITCH = STEP + 4, ROW_STAGES = 4;
+template <int TM>
+constexpr int ROW_SMEM = (ROW_STAGES * TILE + 2 * TM) * ROW_PITCH * 4;
+
+template <int TM>
+__global__ void __launch_bounds__(ROW_THREADS, 2)
+project_rows_kernel(const float* x, const uint16_t* centers, const void* ids, int id_bytes, const float* mean,
+                    const float* encoder, int S, int J, int r, float* coeff) {
+  extern __shared__ float sm[];
+  constexpr int PIECES = TM / 16, ROWS = TM / 8;
+  const int t = threadIdx.x, m0 = blockIdx.x * TM, n0 = blockIdx.y * TILE, steps = J / STEP;
+  const int piece = (t & 7) * 4, first = t >> 3;         // loads: columns piece .. + 3 of rows first, first + 16 ...
+  const float* x_at[PIECES];
+  const uint16_t* c_at[PIECES];
+  const float* e_at[TILE / 16];
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {                      // rows past the last: another one's, stored nowhere
+    const int token = min(m0 + first + p * 16, S - 1);
+    x_at[p] = x + static_cast<size_t>(token) * J + piece;
+    c_at[p] = centers + static_cast<size_t>(load_id(ids, id_bytes, token)) * J + piece;
+  }
+#pragma unroll
+  for (int p = 0; p < TILE / 16; ++p) {
+    const int row = n0 + first + p * 16;
+    e_at[p] = encoder + static_cast<size_t>(row < r ? row : row % r) * J + piece;
+  }
+  float4 xv[2][PIECES], mv[2];
+  uint2 cv[2][PIECES];
+  auto fetch = [&](int buffer, int step) {
+    mv[buffer] = __ldg(reinterpret_cast<const float4*>(mean + step * STEP + piece));
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      xv[buffer][p] = __ldg(reinterpret_cast<const float4*>(x_at[p] + step * STEP));
+      cv[buffer][p] = __ldg(reinterpret_cast<const uint2*>(c_at[p] + step * STEP));
+    }
+  };
+  auto request = [&](int step) {
+    if (step < steps) {
+      float* at = sm + step % ROW_STAGES * TILE * ROW_PITCH + first * ROW_PITCH + piece;
+#pragma unroll
+      for (int p = 0; p < TILE / 16; ++p) copy_async(at + p * 16 * ROW_PITCH, e_at[p] + step * STEP);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");      // an empty one past the last step keeps the count
+  };
+  const int tx = t & 15, ty = t >> 4;                     // sums: rows ty + 8 i, columns tx + 16 j
+  float sums[ROWS][4] = {};
+  auto step = [&](int buffer, int s) {
+    float* as = sm + (ROW_STAGES * TILE + buffer * TM) * ROW_PITCH;
+    const float* bs = sm + s % ROW_STAGES * TILE * ROW_PITCH;
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p)
+      *reinterpret_cast<float4*>(as + (first + p * 16) * ROW_PITCH + piece) =
+          residual_of(xv[buffer][p], RowOperand<BF16_ROWS>{}.value(cv[buffer][p]), mv[buffer]);
+    asm volatile("cp.async.wait_group %0;" ::"n"(ROW_STAGES - 2) : "memory");
+    __syncthreads();        // this step's tiles; what they lie on next time has been read behind the barrier before
+    if (s + 2 < steps) fetch(buffer, s + 2);
+    request(s + ROW_STAGES - 1);
+#pragma unroll
+    for (int k = 0; k < STEP; k += 4) {
+      float4 a[ROWS], b[4];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) a[i] = *reinterpret_cast<const float4*>(as + (ty + i * 8) * ROW_PITCH + k);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(bs + (tx + j * 16) * ROW_PITCH + k);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sums[i][j] = fmaf(a[i].x, b[j].x, sums[i][j]);
+          sums[i][j] = fmaf(a[i].y, b[j].y, sums[i][j]);
+          sums[i][j] = fmaf(a[i].z, b[j].z, sums[i][j]);
+          sums[i][j] = fmaf(a[i].w, b[j].w, sums[i][j]);
+        }
+    }
+  };
+  fetch(0, 0);
+  if (1 < steps) fetch(1, 1);
+  for (int s = 0; s < ROW_STAGES - 1; ++s) request(s);
+#pragma unroll 1
+  for (int s = 0; s < steps; s += 2) {
+    step(0, s);
+    if (s + 1 < steps) step(1, s + 1);
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const int token = m0 + ty + i * 8;
+    if (token >= S) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = n0 + tx + j * 16;
+      if (c < r) coeff[static_cast<size_t>(token) * r + c] = sums[i][j];
     }
   }
 }
@@ -905,18 +1004,46 @@ int simt_assign(const void* x, int x_dtype, const void* centers, int c_dtype, in
   return NKV_OK;
 }
 
+template <int TM>
+static int project_rows(const float* x, const uint16_t* centers, const void* ids, int id_bytes, const float* mean,
+                        const float* encoder, int S, int J, int r, float* coeff, cudaStream_t stream) {
+  NKV_CUDA(cudaFuncSetAttribute(project_rows_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROW_SMEM<TM>));
+  project_rows_kernel<TM><<<dim3(ceil_div(S, TM), ceil_div(r, TILE)), ROW_THREADS, ROW_SMEM<TM>, stream>>>(
+      x, centers, ids, id_bytes, mean, encoder, S, J, r, coeff);
+  NKV_LAUNCH_CHECK("project_rows_kernel");
+  return NKV_OK;
+}
+
+// Rows of a tile of project_rows_kernel: the least blocks on the fullest SM times what one takes (TM / 8 + 4 reads of
+// shared memory; one block alone, K = 1,536: 16 rows 25 us, 32 rows 34, 48 rows 44); of equal ones the largest, which
+// reads the encoder least often.  64 rows take 220 registers and 91 us, more than two blocks of 48 (77).
+static int project_tile(int S, int r) {
+  int best = 48;
+  long long least = 0;
+  for (int rows = 48; rows >= 16; rows -= 16) {
+    const long long blocks = static_cast<long long>(ceil_div(S, rows)) * ceil_div(r, TILE);
+    const long long cost = (blocks + sm_count() - 1) / sm_count() * (rows / 8 + 4);
+    if (rows == 48 || cost < least) { best = rows; least = cost; }
+  }
+  return best;
+}
+
 int simt_project(const void* x, int x_dtype, const void* centers_bf16, const void* ids,
                  int id_bytes, const float* mean, const void* encoder, int enc_dtype, int S,
                  int J, int r, void* coeff, cudaStream_t stream) {
   if (S == 0) return NKV_OK;
+  if (has_form(F32_ROWS, x, x_dtype, J) && has_form(BF16_ROWS, centers_bf16, NKV_BF16, J) &&
+      has_form(F32_ROWS, encoder, enc_dtype, J) && has_form(F32_ROWS, mean, NKV_F32, J)) {
+    const int tile = project_tile(S, r);
+    auto run = tile == 16 ? project_rows<16> : tile == 32 ? project_rows<32> : project_rows<48>;
+    return run(static_cast<const float*>(x), static_cast<const uint16_t*>(centers_bf16), ids, id_bytes, mean,
+               static_cast<const float*>(encoder), S, J, r, static_cast<float*>(coeff), stream);
+  }
   const int rows = ordered_rows(S, ceil_div(r, TILE));
   const dim3 grid(ceil_div(S, rows), ceil_div(r, TILE));
   const bool e_vec = vector_rows(encoder, enc_dtype, J) && vector_rows(mean, NKV_F32, J);
-  const bool fast = has_form(F32_ROWS, x, x_dtype, J) && has_form(BF16_ROWS, centers_bf16, NKV_BF16, J) &&
-                    has_form(F32_ROWS, encoder, enc_dtype, J) && has_form(F32_ROWS, mean, NKV_F32, J);
-  auto kernel = fast ? (rows == 32 ? project_kernel<false, 32, true> : project_kernel<false, 64, true>)
-                : enc_dtype == NKV_BF16 ? (rows == 32 ? project_kernel<true, 32, false> : project_kernel<true, 64, false>)
-                                        : (rows == 32 ? project_kernel<false, 32, false> : project_kernel<false, 64, false>);
+  auto kernel = enc_dtype == NKV_BF16 ? (rows == 32 ? project_kernel<true, 32> : project_kernel<true, 64>)
+                                      : (rows == 32 ? project_kernel<false, 32> : project_kernel<false, 64>);
   kernel<<<grid, THREADS, 0, stream>>>(
       x, x_dtype, vector_rows(x, x_dtype, J), static_cast<const uint16_t*>(centers_bf16),
       vector_rows(centers_bf16, NKV_BF16, J), ids, id_bytes, mean, encoder, e_vec, S, J, r, coeff);

@@ -104,3 +104,16 @@ def test_few_centres_give_the_ids_of_the_general_form(S, C, J, dtype):
         x[1, 3], x[2, J - 1], x[3] = float("nan"), float("inf"), 3e38
     shifted = torch.empty(S * J + 1, device="cuda")[1:].view(S, J).copy_(x)
     assert torch.equal(ops.assign(x, centers), ops.assign(shifted, centers))
+
+
+@pytest.mark.parametrize("S", [1, 15, 17, 48, 49, 700, 3000])
+@pytest.mark.parametrize("J,r", [(32, 2), (64, 64), (96, 66), (224, 192)])
+def test_projection_of_aligned_rows_gives_the_general_forms_bits(S, J, r):
+    """Rows four bytes off a vector's start take the general form; both sum in the same order."""
+    x = torch.randn(S, J, device="cuda")
+    centers = torch.randn(16, J, device="cuda").bfloat16()
+    ids = torch.randint(0, 16, (S,), device="cuda").to(torch.uint8)
+    mean, encoder = torch.randn(J, device="cuda"), torch.randn(r, J, device="cuda")
+    shifted = torch.empty(S * J + 1, device="cuda")[1:].view(S, J).copy_(x)
+    got, want = (ops.project(rows, centers, ids, mean, encoder) for rows in (x, shifted))
+    assert torch.equal(got, want)
