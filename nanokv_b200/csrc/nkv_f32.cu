@@ -771,11 +771,12 @@ decode_rows_kernel(nkv_history h, const int32_t* rows_index, int n, const void* 
 
 // ----------------------------------------------------------------- attention
 // Block = 64 queries of one head over one run of history tokens, 64 at a time: K and V tiles in shared
-// memory, online softmax in fp32, two blocks per SM.  A thread owns 4 x 4 scores and 4 queries x D / 16
-// columns of O; multiply-adds are packed pairs.  K of the next tile waits in registers while the weights meet V, and V
-// arrives while the scores are made.  Bound: what shared memory gives to registers, 128 bytes a cycle, twice the
-// multiply-adds' time at these 4 x 4 pieces.  us of a read with rank 32, now / with K and V fetched between the tiles:
-// 2,048 tokens, 12 heads of 64 and 256 queries 85 / 91; heads of 128, 4,096 tokens and 512 queries 451 / 457.
+// memory, online softmax in fp32, two blocks per SM.  A thread owns 8 x 4 scores and 8 queries x D / 16
+// columns of O.  K of the next tile arrives while the weights meet V, and V while the scores are made.
+// Bound: what shared memory gives to registers, 128 bytes a cycle: 48 cycles per column of K and 64 (heads of 64: 48) per
+// token of V, against 32 and 64 (32) of multiply-adds; pieces of 4 x 4 took 64 and 96.  us of a read with rank 32, now /
+// with 4 x 4: 2,048 tokens, 12 heads of 128 and 256 queries 127 / 146, 4,096 tokens and 512 queries 382 / 452; heads of
+// 64, 2,048 tokens and 256 queries 76 / 85.
 struct RowAttn {
   const float* q; const float* k; const float* v;
   long long q_stride_token, q_stride_head, kv_stride_token, kv_stride_head;
@@ -784,85 +785,76 @@ struct RowAttn {
   float* out; float* lse;      // partial z at z * Q * out_heads rows
 };
 
+constexpr int ATTN_THREADS = 128;
+
 template <int D>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(ATTN_THREADS, 2)
 attn_rows_f32_kernel(RowAttn a) {
-  extern __shared__ float smem[];
-  float* Qs = smem;                  // [D][64]
-  float* Ks = Qs + D * 64;           // [D][64]
-  float* Vs = Ks + D * 64;           // [64][D]
-  float* Ps = Vs + 64 * D;           // [64 tokens][64 queries]
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  extern __shared__ __align__(16) float smem[];
+  float* Qs = smem;                  // [64][D], as in memory but for the order of a row's pieces of four
+  float* Ks = Qs + 64 * D;           // [64][D], the same
+  float* Vs = Ks + 64 * D;           // [64][D]
+  float* Ps = Vs + 64 * D;           // [64 tokens][64 queries], pieces of four queries in another order too
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;       // queries ty * 8 .. + 7, tokens tx * 4 .. + 3
   const int q0 = blockIdx.x * 64, head = blockIdx.y, z = blockIdx.z;
   const int t_begin = z * a.tokens_per_split, t_end = min(a.N, t_begin + a.tokens_per_split);
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  // lane -> row, so that the transposed stores are consecutive
-  for (int idx = tid; idx < 64 * (D / 4); idx += 256) {
-    const int i = idx % 64, d = idx / 64 * 4;
-    const float4 v = q0 + i < a.Q ? *reinterpret_cast<const float4*>(a.q + static_cast<size_t>(q0 + i) * a.q_stride_token +
-                                                                    static_cast<size_t>(head) * a.q_stride_head + d) : zero;
-    Qs[d * 64 + i] = v.x; Qs[(d + 1) * 64 + i] = v.y; Qs[(d + 2) * 64 + i] = v.z; Qs[(d + 3) * 64 + i] = v.w;
-  }
-  constexpr int OP = D / 32;         // pairs of O columns per thread
-  uint64_t o[4][OP];
-  float m_run[4], l_run[4];
+  // piece p of row r lies at p ^ (r / 4 % 8): eight threads read one piece of rows four apart from different banks
+  auto copy_tile = [&](float* tile, const float* base, long long stride, int row0, int rows, bool permuted) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+    for (int n = 0; n < 64 * (D / 4) / ATTN_THREADS; ++n) {
+      const int idx = tid + n * ATTN_THREADS, i = idx / (D / 4), piece = idx % (D / 4);
+      const int row = min(row0 + i, rows - 1), bytes = row0 + i < rows ? 16 : 0;      // past the last: zeros
+      const float* at = tile + i * D + (permuted ? piece ^ (i >> 2 & 7) : piece) * 4;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(at))),
+                   "l"(base + static_cast<size_t>(row) * stride + piece * 4), "r"(bytes) : "memory");
+    }
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  const float* k_head = a.k + static_cast<size_t>(head) * a.kv_stride_head;
+  const float* v_head = a.v + static_cast<size_t>(head) * a.kv_stride_head;
+  copy_tile(Qs, a.q + static_cast<size_t>(head) * a.q_stride_head, a.q_stride_token, q0, a.Q, true);
+  copy_tile(Ks, k_head, a.kv_stride_token, t_begin, t_end, true);
+  commit();
+  constexpr int OC = D / 64;         // pieces of four O columns per thread: c * 64 + tx * 4
+  float o[8][OC][4] = {};
+  float m_run[8], l_run[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
     m_run[i] = -INFINITY;
     l_run[i] = 0.f;
-#pragma unroll
-    for (int c = 0; c < OP; ++c) o[i][c] = 0ull;
   }
-  constexpr int PIECES = 64 * (D / 4) / 256;       // of four values, per thread and tile
-  float4 kr[PIECES];
-  auto fetch_k = [&](int t0) {                     // tokens past the last: the last one's, whose weight is zero
-    const float* row = a.k + static_cast<size_t>(min(t0 + tid % 64, t_end - 1)) * a.kv_stride_token +
-                       static_cast<size_t>(head) * a.kv_stride_head + tid / 64 * 4;
-#pragma unroll
-    for (int p = 0; p < PIECES; ++p) kr[p] = *reinterpret_cast<const float4*>(row + p * 16);
-  };
-  fetch_k(t_begin);
+#pragma unroll 1
   for (int t0 = t_begin; t0 < t_end; t0 += 64) {
-    __syncthreads();                 // previous tile fully consumed
-#pragma unroll
-    for (int p = 0; p < PIECES; ++p) {             // V: straight to shared memory while the scores are made
-      const int idx = tid + p * 256, i = idx / (D / 4), d = idx % (D / 4) * 4;
-      const int token = min(t0 + i, t_end - 1), bytes = t0 + i < t_end ? 16 : 0;      // past the last: zeros
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(Vs + i * D + d))),
-                   "l"(a.v + static_cast<size_t>(token) * a.kv_stride_token + static_cast<size_t>(head) * a.kv_stride_head + d),
-                   "r"(bytes) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-#pragma unroll
-    for (int p = 0; p < PIECES; ++p) {
-      float* at = Ks + (tid / 64 * 4 + p * 16) * 64 + tid % 64;
-      at[0] = kr[p].x; at[64] = kr[p].y; at[128] = kr[p].z; at[192] = kr[p].w;
-    }
+    copy_tile(Vs, v_head, a.kv_stride_token, t0, t_end, false);
+    commit();
+    asm volatile("cp.async.wait_group 1;" ::: "memory");        // K, and Q
     __syncthreads();
-    uint64_t s2[4][2] = {};
-#pragma unroll 8
-    for (int d = 0; d < D; ++d) {
-      const float4 qa = *reinterpret_cast<const float4*>(Qs + d * 64 + ty * 4);
-      const ulonglong2 kb = *reinterpret_cast<const ulonglong2*>(Ks + d * 64 + tx * 4);
-      const float qv[4] = {qa.x, qa.y, qa.z, qa.w};
+    float s[8][4] = {};
+#pragma unroll 4
+    for (int piece = 0; piece < D / 4; ++piece) {
+      float4 q[8], k[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint64_t q2 = pair_f32(qv[i], qv[i]);
-        s2[i][0] = fma_f32x2(q2, kb.x, s2[i][0]);
-        s2[i][1] = fma_f32x2(q2, kb.y, s2[i][1]);
-      }
+      for (int i = 0; i < 8; ++i)
+        q[i] = *reinterpret_cast<const float4*>(Qs + (ty * 8 + i) * D + (piece ^ ((ty * 2 + i / 4) & 7)) * 4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4*>(Ks + (tx * 4 + j) * D + (piece ^ (tx & 7)) * 4);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(q[i].x, k[j].x, s[i][j]);
+          s[i][j] = fmaf(q[i].y, k[j].y, s[i][j]);
+          s[i][j] = fmaf(q[i].z, k[j].z, s[i][j]);
+          s[i][j] = fmaf(q[i].w, k[j].w, s[i][j]);
+        }
     }
-    float weight[4][4];              // [query][token]
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float s[4];
-      split_f32(s2[i][0], s[0], s[1]);
-      split_f32(s2[i][1], s[2], s[3]);
+    for (int i = 0; i < 8; ++i) {
       float mx = -INFINITY;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        s[j] = t0 + tx * 4 + j < t_end ? s[j] * a.scale : -INFINITY;
-        mx = fmaxf(mx, s[j]);
+        s[i][j] = t0 + tx * 4 + j < t_end ? s[i][j] * a.scale : -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
       }
 #pragma unroll
       for (int off = 8; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
@@ -871,51 +863,58 @@ attn_rows_f32_kernel(RowAttn a) {
       float sum = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        weight[i][j] = expf(s[j] - m_new);
-        sum += weight[i][j];
+        s[i][j] = expf(s[i][j] - m_new);
+        sum += s[i][j];
       }
 #pragma unroll
       for (int off = 8; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
       l_run[i] = l_run[i] * alpha + sum;
       m_run[i] = m_new;
-      const uint64_t alpha2 = pair_f32(alpha, alpha);
 #pragma unroll
-      for (int c = 0; c < OP; ++c) o[i][c] = fma_f32x2(o[i][c], alpha2, 0ull);
+      for (int c = 0; c < OC; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][c][e] = fmaf(o[i][c][e], alpha, 0.f);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      *reinterpret_cast<float4*>(Ps + (tx * 4 + j) * 64 + ty * 4) =
-          make_float4(weight[0][j], weight[1][j], weight[2][j], weight[3][j]);
-    if (t0 + 64 < t_end) fetch_k(t0 + 64);         // in flight while the weights meet V
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+        *reinterpret_cast<float4*>(Ps + (tx * 4 + j) * 64 + ((ty * 2 + half) ^ (tx & 7)) * 4) =
+            make_float4(s[half * 4][j], s[half * 4 + 1][j], s[half * 4 + 2][j], s[half * 4 + 3][j]);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");        // V
+    __syncthreads();                 // and everyone has read K
+    if (t0 + 64 < t_end) copy_tile(Ks, k_head, a.kv_stride_token, t0 + 64, t_end, true);
+    commit();
 #pragma unroll 4
     for (int t = 0; t < 64; ++t) {
-      const float4 p4 = *reinterpret_cast<const float4*>(Ps + t * 64 + ty * 4);
-      const float pv[4] = {p4.x, p4.y, p4.z, p4.w};
-      uint64_t vv[OP];
+      const float4 p0 = *reinterpret_cast<const float4*>(Ps + t * 64 + ((ty * 2) ^ (t >> 2 & 7)) * 4);
+      const float4 p1 = *reinterpret_cast<const float4*>(Ps + t * 64 + ((ty * 2 + 1) ^ (t >> 2 & 7)) * 4);
+      const float p[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
-      for (int c = 0; c < OP; ++c) vv[c] = *reinterpret_cast<const uint64_t*>(Vs + t * D + c * 32 + tx * 2);
+      for (int c = 0; c < OC; ++c) {
+        const float4 v = *reinterpret_cast<const float4*>(Vs + t * D + c * 64 + tx * 4);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint64_t p2 = pair_f32(pv[i], pv[i]);
-#pragma unroll
-        for (int c = 0; c < OP; ++c) o[i][c] = fma_f32x2(p2, vv[c], o[i][c]);
+        for (int i = 0; i < 8; ++i) {
+          o[i][c][0] = fmaf(p[i], v.x, o[i][c][0]);
+          o[i][c][1] = fmaf(p[i], v.y, o[i][c][1]);
+          o[i][c][2] = fmaf(p[i], v.z, o[i][c][2]);
+          o[i][c][3] = fmaf(p[i], v.w, o[i][c][3]);
+        }
       }
     }
+    __syncthreads();                 // V and the weights have been read
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int qi = q0 + ty * 4 + i;
+  for (int i = 0; i < 8; ++i) {
+    const int qi = q0 + ty * 8 + i;
     if (qi >= a.Q) continue;
     const float inv = l_run[i] > 0.f ? 1.0f / l_run[i] : 0.f;
     const size_t row = (static_cast<size_t>(z) * a.Q + qi) * a.out_heads + head;
 #pragma unroll
-    for (int c = 0; c < OP; ++c) {
-      float lo, hi;
-      split_f32(o[i][c], lo, hi);
-      *reinterpret_cast<float2*>(a.out + row * D + c * 32 + tx * 2) = make_float2(lo * inv, hi * inv);
-    }
+    for (int c = 0; c < OC; ++c)
+      *reinterpret_cast<float4*>(a.out + row * D + c * 64 + tx * 4) =
+          make_float4(o[i][c][0] * inv, o[i][c][1] * inv, o[i][c][2] * inv, o[i][c][3] * inv);
     if (tx == 0) a.lse[row] = l_run[i] > 0.f ? m_run[i] + logf(l_run[i]) : -INFINITY;
   }
 }
@@ -1106,7 +1105,7 @@ template <int D>
 int launch_rows(const RowAttn& a, int heads, int splits, cudaStream_t stream) {
   const size_t smem = sizeof(float) * (3 * D * 64 + 64 * 64);
   NKV_CUDA(cudaFuncSetAttribute(attn_rows_f32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  attn_rows_f32_kernel<D><<<dim3(ceil_div(a.Q, 64), heads, splits), 256, smem, stream>>>(a);
+  attn_rows_f32_kernel<D><<<dim3(ceil_div(a.Q, 64), heads, splits), ATTN_THREADS, smem, stream>>>(a);
   NKV_LAUNCH_CHECK("attn_rows_f32_kernel");
   return NKV_OK;
 }
