@@ -34,7 +34,7 @@ class CompressedHistory:
         device = torch.device(device)
         self.device = device
         width = self.joint if center_width is None else int(center_width)
-        # zeroed=False: for a history that is filled to its capacity before anything reads it
+        # zeroed=False: for a caller that fills every array to its end before anything reads it
         array = torch.zeros if zeroed else torch.empty
         self.codes = array(self.capacity, self.rank // 2, dtype=torch.uint8, device=device)
         self.scales = array(self.capacity, self.rank // self.group, dtype=scale_dtype, device=device)
@@ -79,6 +79,7 @@ class CompressedHistory:
                 hist._starts.append(hist.tokens + ids.shape[0])
                 hist._center_rows.append(hist._center_used)
                 hist._center_used += centers.shape[0]
+            hist._clear_unused_centers()
             return hist
         hist.seg_start.zero_()
         for codes, scales, ids, centers in parts:
@@ -88,7 +89,14 @@ class CompressedHistory:
             hist.codes[offset:stop].copy_(codes)
             hist.scales[offset:stop].copy_(scales)
             hist.ids[offset:stop].copy_(ids)
+        hist._clear_unused_centers()
         return hist
+
+    def _clear_unused_centers(self) -> None:
+        """Zeroes the table's rows behind the last segment's.  There are some where segments have different numbers of
+        centres, no token has their ids, but sums over the table (counts @ centres) read them: 0 times what lay there."""
+        if self._center_used < self.centers.shape[0]:
+            self.centers[self._center_used:].zero_()
 
     def reserve_segment(self, count: int, clusters: int, centers: torch.Tensor | None = None):
         """Claim the next token range and centre rows; returns (offset, centre rows view).  ``centers``: rows to be
