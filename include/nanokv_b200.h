@@ -136,7 +136,7 @@ int nkv_assign(const void* x, int x_dtype, const void* centers, int centers_dtyp
  * Reference: semantic_residual, MGM/nanokv_codec.py:302-330,
  * LB/lingbot_v2_kv_codec.py:210-239 (the seeded randperm that picks
  * init_rows stays on the host, as it does there).
- * workspace: nkv_kmeans_workspace_bytes(S, J, C) bytes of device scratch.
+ * workspace: nkv_kmeans_workspace_bytes(S, J, C) bytes of device scratch, at any address.
  */
 size_t nkv_kmeans_workspace_bytes(int S, int J, int C);
 int nkv_kmeans(const void* x, int x_dtype, int S, int J, int C, int iters,

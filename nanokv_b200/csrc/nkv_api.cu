@@ -154,15 +154,16 @@ int nkv_kmeans(const void* x, int x_dtype, int S, int J, int C, int iters,
   NKV_REQUIRE(workspace && workspace_bytes >= nkv_kmeans_workspace_bytes(S, J, C), NKV_ERR_INVALID,
               "kmeans: workspace of %zu bytes is too small", workspace_bytes);
   auto s = static_cast<cudaStream_t>(stream);
-  float* centers = static_cast<float*>(workspace);
+  // the workspace may start anywhere, the centres are read four at a time and their planes by TMA: the 256 spare bytes
+  uint8_t* space = static_cast<uint8_t*>(workspace);
+  space += (256 - (reinterpret_cast<uintptr_t>(space) & 255)) & 255;
+  float* centers = reinterpret_cast<float*>(space);
   int32_t* labels = reinterpret_cast<int32_t*>(centers + static_cast<size_t>(C) * J);
   // bf16 rows: the assignment runs on the tensor cores against the fp32 centres split into bf16
   // planes (fp32-accurate distances); anything else on the fp32 CUDA-core kernel
   const bool tensor = x_dtype == NKV_BF16 && !simt_forced() && tc_assign_supported(J, C) &&
                       (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  uint8_t* plane_space = static_cast<uint8_t*>(workspace) + kmeans_planes_offset(S, J, C);
-  plane_space += (256 - (reinterpret_cast<uintptr_t>(plane_space) & 255)) & 255;
-  uint16_t* planes = tensor ? reinterpret_cast<uint16_t*>(plane_space) : nullptr;
+  uint16_t* planes = tensor ? reinterpret_cast<uint16_t*>(space + kmeans_planes_offset(S, J, C)) : nullptr;
   int rc = kmeans_gather_init(x, x_dtype, J, C, init_rows, centers, planes, s);
   if (rc != NKV_OK) return rc;
   if (iters == 0) {
