@@ -4,7 +4,10 @@
 //
 // Given centres are bf16.  The C-means' fp32 means come as three bf16 planes side by side along K (hi, mid, lo:
 // every product is exact in the fp32 accumulator); the token rows are walked once per plane, and the warps that sum
-// norms square the fp32 rows themselves while the second and third plane are multiplied.  K is never cut: every sum runs in the order of K, so what is stored does not depend on how a call is tiled.
+// norms square the fp32 rows themselves while the second and third plane are multiplied.  K is never cut, every sum
+// runs in the order of K, and every tile starts at a multiple of eight tokens (a row's place modulo eight is part of
+// its norm's order): what is stored does not depend on how a call is tiled, nor on where a history is cut into calls
+// as long as the calls start at multiples of eight tokens of it.
 //
 // A thread block owns `rows` tokens and C / parts centres; the `parts` blocks of one token tile are a cluster,
 // whose first block collects the others' minima through its shared memory; the parts share out the norms of the
@@ -216,8 +219,8 @@ assign_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const uint32_t lane_sel = static_cast<uint32_t>(32 * (warp & 3)) << 16;
     // ---- squared norms from the resident tiles: half-rows of 32 columns, tokens first, then centres.  The order
     // of a half-row's sums (four pieces of eight columns, in the order they have in the swizzled tile) is part of
-    // what the stored ids were made with: a row's place modulo 8 in its tile decides it, so tiles start at
-    // multiples of 8 tokens wherever a call may be cut at will.
+    // what the stored ids were made with: a row's place modulo 8 in its tile decides it, so every
+    // tile starts at a multiple of 8 tokens.
     // The blocks of a cluster share the work: the parts of a tile its tokens, two tiles their centres.
     const uint32_t me = p.team > 1 ? cluster_ctarank() : 0;
     const int x_share = p.parts > 1 ? (p.rows_pad + p.parts - 1) / p.parts : p.rows_pad, x_first = p.parts > 1 ? part * x_share : 0;
@@ -379,13 +382,13 @@ struct Cut { int rows, parts, kc, stages; };
 
 // Tokens per tile and parts of the centres.  Estimate in SM cycles: a 64-column chunk takes its bytes from L2 at 48
 // per clock, at least 130 cycles of hand-offs; a block has about 6,000 cycles of prologue and epilogue.  Calls that
-// one round of 64-row tiles covers take tiles of 16, 32 or 64 rows, longer ones the rows that fill whole rounds
-// (the squares of a row are summed in an order that its place in the tile decides, see the kernel).  Measured against
+// one round of 64-row tiles covers take tiles of 16, 32 or 64 rows, longer ones the rows that fill whole rounds, up
+// to the next multiple of eight (a row's place modulo eight decides the order of its norm's sum, see the kernel).  Measured against
 // the alternatives, us: 4,680 x 5,120, 64 centres, 64 rows x 2 parts 22, 64 x 1 24, 32 x 1 25; 256 centres, 64 x 2 34,
 // 64 x 1 51; 1,560 x 5,120, 512 centres, 64 x 4 32, 64 x 8 45, 64 x 2 50.
 Cut plan_assign(int S, int C, int a_chunks, int planes) {
   const int sms = sm_count();
-  const int whole = pick_rows(S, 1);
+  const int whole = (pick_rows(S, 1) + 7) / 8 * 8;
   Cut best{whole, 1, 1, 2};
   double best_cost = -1;
   for (int rows = whole; rows >= 16; rows /= 2) {
