@@ -112,9 +112,11 @@ __device__ __noinline__ uint32_t quant_word_any(uint4 v, float scale, float inv,
   return out;
 }
 
-// packed codes of 32 coefficients; `finite`: none of them is a NaN or an infinity
+// packed codes of 32 coefficients; `finite`: none of them is a NaN or an infinity.  A scale below 2^-128 (a caller's
+// small eps) has no finite reciprocal, and quant_word takes every quotient through it.
 __device__ __forceinline__ uint4 pack_codes(const uint32_t (&w)[16], float scale, bool in_bf16, bool finite) {
   const float inv = __frcp_rn(scale);
+  finite = finite && inv < INFINITY;
   uint32_t words[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
