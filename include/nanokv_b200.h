@@ -176,12 +176,15 @@ int nkv_quant_pack(const void* coeff, int coeff_dtype, int S, int r, int group, 
  * nkv_assign): coeff = ((x - centre[id]) - mean) @ encoder^T rounded once to the encoder dtype, then
  * nkv_quant_pack of those coefficients, written to codes [S,r/2] and scales [S,r/group].
  * Reference: the second half of encode_tensor, MGM/nanokv_codec.py:345-351, LB/lingbot_v2_kv_codec.py:280-287.
- * With bf16 operands and one scale per token (group == r, r a multiple of 64 that tiles over at most
- * two column parts of at most 512) one kernel does all of it: the coefficients stay in tensor memory, the
- * per-token maximum crosses the thread blocks of a token tile (up to eight) through their shared memory, and `workspace`
- * is not touched.  Otherwise it runs nkv_project into `workspace` (S * r elements of the encoder
- * dtype) followed by nkv_quant_pack.  Same bytes either way.
+ * With bf16 operands, J a multiple of 64, codes on 16 bytes and either one scale per token (group == r, r a multiple of
+ * 64 that tiles over at most two column parts of at most 512) or one per 32 coefficients (r above 32, tiled over at most
+ * sixteen parts) one kernel does all of it: the coefficients stay in tensor memory, a token's maximum crosses the thread
+ * blocks of its tile (up to eight) through their shared memory, and `workspace` is not touched.  Otherwise it runs
+ * nkv_project into `workspace` (S * r elements of the encoder dtype) followed by nkv_quant_pack.  Same bytes either way.
+ * nkv_project_quant_workspace_bytes says what a call takes: 0 where the one kernel does it.
  */
+size_t nkv_project_quant_workspace_bytes(int x_dtype, int encoder_dtype, int S, int J, int r, int group,
+                                         const uint8_t* codes);
 int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
                       const float* mean, const void* encoder, int encoder_dtype, int S, int J, int r,
                       int group, float eps, int quant_mode, int scale_dtype, uint8_t* codes,

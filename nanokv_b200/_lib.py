@@ -62,6 +62,7 @@ SIGNATURES = {
                             c_int, c_int, c_int, c_void_p, c_void_p]),
     "nkv_quant_pack": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
                                c_void_p, c_void_p, c_void_p]),
+    "nkv_project_quant_workspace_bytes": (c_size_t, [c_int] * 6 + [c_void_p]),
     "nkv_project_quant": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                   c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p,
                                   c_void_p, c_size_t, c_void_p]),

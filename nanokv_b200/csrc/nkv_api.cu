@@ -213,6 +213,19 @@ int nkv_quant_pack(const void* coeff, int coeff_dtype, int S, int r, int group, 
                     static_cast<cudaStream_t>(stream));
 }
 
+// bf16 operands with one scale per token or per 32 coefficients: projection, quantiser and packing in one kernel, the
+// coefficients stay on chip
+static bool project_quant_in_one(int x_dtype, int encoder_dtype, int J, int r, int group, const uint8_t* codes) {
+  return encoder_dtype == NKV_BF16 && x_dtype == NKV_BF16 && !simt_forced() && tc_project_quant_supported(J, r, group) &&
+         (reinterpret_cast<uintptr_t>(codes) & 15) == 0;
+}
+
+size_t nkv_project_quant_workspace_bytes(int x_dtype, int encoder_dtype, int S, int J, int r, int group,
+                                         const uint8_t* codes) {
+  if (S <= 0 || J <= 0 || r <= 0 || project_quant_in_one(x_dtype, encoder_dtype, J, r, group, codes)) return 0;
+  return static_cast<size_t>(S) * r * dtype_bytes(encoder_dtype);
+}
+
 int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, const void* ids, int id_bytes,
                       const float* mean, const void* encoder, int encoder_dtype, int S, int J, int r,
                       int group, float eps, int quant_mode, int scale_dtype, uint8_t* codes,
@@ -227,10 +240,7 @@ int nkv_project_quant(const void* x, int x_dtype, const void* centers_bf16, cons
               "project_quant: quant_mode=%d", quant_mode);
   NKV_REQUIRE(quant_mode != NKV_QUANT_IN_BF16 || encoder_dtype == NKV_BF16, NKV_ERR_INVALID,
               "project_quant: NKV_QUANT_IN_BF16 needs bf16 coefficients");
-  // bf16 operands with one scale per token: projection, quantiser and packing in one kernel, the
-  // coefficients stay on chip
-  if (encoder_dtype == NKV_BF16 && x_dtype == NKV_BF16 && !simt_forced() &&
-      tc_project_quant_supported(J, r, group) && (reinterpret_cast<uintptr_t>(codes) & 15) == 0)
+  if (project_quant_in_one(x_dtype, encoder_dtype, J, r, group, codes))
     return tc_project_quant(x, centers_bf16, ids, id_bytes, mean, encoder, S, J, r, group, eps, quant_mode,
                             scale_dtype, codes, scales, static_cast<cudaStream_t>(stream));
   NKV_REQUIRE(workspace && workspace_bytes >= static_cast<size_t>(S) * r * dtype_bytes(encoder_dtype),
