@@ -69,23 +69,24 @@ class CompressedHistory:
     def stacked(cls, parts, *, joint: int, rank: int, device) -> "CompressedHistory":
         """A history of the given segments, each (codes u8 [S,r/2], scales [S,1], ids [S], centres [C,J]): one launch per
         sixteen of them, or copies where types or places differ."""
-        total, clusters = sum(p[2].shape[0] for p in parts), max(p[3].shape[0] for p in parts)
+        # a segment has as many tokens as rows of codes: ids or scales of another number are no segment of that many
+        total, clusters = sum(p[0].shape[0] for p in parts), max(p[3].shape[0] for p in parts)
         hist = cls(joint=joint, rank=rank, capacity=total, max_segments=len(parts), centers_per_segment=clusters,
                    device=device, zeroed=False)
         if hist.seg_start.is_cuda and all(hist._copies(*p) for p in parts):
             with torch.cuda.device(hist.codes.device):
-                ops.history_stack(hist, [(*p, p[2].shape[0], p[3].shape[0]) for p in parts], 0, 0, 0)
-            for _, _, ids, centers in parts:
-                hist._starts.append(hist.tokens + ids.shape[0])
+                ops.history_stack(hist, [(*p, p[0].shape[0], p[3].shape[0]) for p in parts], 0, 0, 0)
+            for codes, _, _, centers in parts:
+                hist._starts.append(hist.tokens + codes.shape[0])
                 hist._center_rows.append(hist._center_used)
                 hist._center_used += centers.shape[0]
             hist._clear_unused_centers()
             return hist
         hist.seg_start.zero_()
         for codes, scales, ids, centers in parts:
-            offset, rows = hist.reserve_segment(ids.shape[0], centers.shape[0])
+            offset, rows = hist.reserve_segment(codes.shape[0], centers.shape[0])
             rows.copy_(centers)
-            stop = offset + ids.shape[0]
+            stop = offset + codes.shape[0]
             hist.codes[offset:stop].copy_(codes)
             hist.scales[offset:stop].copy_(scales)
             hist.ids[offset:stop].copy_(ids)
