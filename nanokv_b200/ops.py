@@ -53,11 +53,15 @@ def id_dtype(clusters: int) -> torch.dtype:
 # --------------------------------------------------------------------------- encode
 def upload(values: torch.Tensor, device) -> torch.Tensor:
     """A small host tensor on ``device``, in order on the current stream and without waiting for what is on it: a copy from
-    pageable memory (``values.to(device)``) ends with a synchronisation.  Inside a stream capture it is that copy, which
-    the capture refuses: a graph must not read host memory that is reused."""
+    pageable memory (``values.to(device)``) ends with a synchronisation.  The copy reads pinned memory of its own, also
+    where ``values`` are pinned already: the caller may write to them as soon as this returns.  Inside a stream capture it
+    is ``values.to(device)``, which the capture refuses: a graph must not read host memory that is reused."""
     if torch.device(device).type != "cuda" or values.is_cuda or torch.cuda.is_current_stream_capturing():
         return values.to(device)
-    return values.pin_memory().to(device, non_blocking=True)
+    pinned = values.pin_memory()
+    if pinned.data_ptr() == values.data_ptr():          # the caller's own memory
+        pinned = torch.empty(values.shape, dtype=values.dtype, pin_memory=True).copy_(values)
+    return pinned.to(device, non_blocking=True)
 
 
 def assign(x: torch.Tensor, centers: torch.Tensor, ids: torch.Tensor | None = None) -> torch.Tensor:
