@@ -410,37 +410,39 @@ __device__ __forceinline__ void store_centre(const float (&sum)[COLS], int count
   }
 }
 
-// Rows of bf16 or fp32, four columns per thread.  Bound: the chain of row loads of the largest cluster -- start rows
+// bf16 rows, four columns per thread.  Bound: the chain of row loads of the largest cluster -- start rows
 // drawn from one true cluster leave others to be shared, so a cluster can hold several times the mean.  The members'
 // pieces run through a ring in shared memory that every thread fills for itself: registers filled in
 // turn share a handful of scoreboards, and waiting for one waits for the ones filled after it.
 // us per call, 64 centres, 4,680 x 5,120 / 880 x 3,072 / 8,000 x 1,536: 41 / 9 / 52 with two columns per thread, 32 row
 // loads at a time and a thread's labels side by side (32 lines per load of a warp); 35 / 9 / 42 with this ring in groups
 // of four rows and labels in whole lines; 22 / 6 / 25 with groups of eight whose places come in one load.
-constexpr int RING_THREADS = 128, RING_GROUP = 8;
-template <int BYTES>     // of an element
+// Threads past the last column copy nothing: copies of column 0 in their place cost 20,000 x 128 to 16 centres 214 us
+// instead of 73, more than two columns per thread (132).  fp32 rows go two columns per thread: a ring for them
+// holds 16 rows of 16 bytes a thread and was slower at every size (3,000 x 1,536 to 16 centres 21 us against 16, 9,500
+// x 128 73 against 34).
+constexpr int RING_THREADS = 128, RING_GROUP = 8, RING_GROUPS = 3;
 __global__ void __launch_bounds__(RING_THREADS)
-kmeans_update_ring_kernel(const void* x, int S, int J, const int32_t* labels, float* centers, uint16_t* planes,
+kmeans_update_ring_kernel(const uint16_t* x, int S, int J, const int32_t* labels, float* centers, uint16_t* planes,
                           uint16_t* stored) {
-  constexpr int PIECE = 4 * BYTES, GROUPS = BYTES == 2 ? 3 : 2;   // 24 rows of bf16, 16 of fp32
-  constexpr int SPAN = BYTES == 2 ? UPDATE_SPAN : UPDATE_SPAN / 2;
-  __shared__ __align__(16) uint16_t list[SPAN];
+  constexpr int PIECE = 8;
+  __shared__ __align__(16) uint16_t list[UPDATE_SPAN];
   __shared__ int warp_total[RING_THREADS / 32];
-  __shared__ __align__(16) uint8_t ring[GROUPS * RING_GROUP][RING_THREADS * PIECE];
+  __shared__ __align__(16) uint8_t ring[RING_GROUPS * RING_GROUP][RING_THREADS * PIECE];
   const int c = blockIdx.x, j = (blockIdx.y * RING_THREADS + threadIdx.x) * 4;
   const bool in = j < J;
-  const uint8_t* column = static_cast<const uint8_t*>(x) + static_cast<size_t>(in ? j : 0) * BYTES;
-  const uint32_t pitch = static_cast<uint32_t>(J) * BYTES;
+  const uint8_t* column = reinterpret_cast<const uint8_t*>(x + (in ? j : 0));
+  const uint32_t pitch = static_cast<uint32_t>(J) * 2;
   const uint32_t my_ring = static_cast<uint32_t>(__cvta_generic_to_shared(&ring[0][threadIdx.x * PIECE]));
   float sum[4] = {};
   int count = 0;
-  for (int s0 = 0; s0 < S; s0 += SPAN) {
-    const int total = list_members<RING_THREADS>(labels, s0, min(SPAN, S - s0), c, list, warp_total);
+  for (int s0 = 0; s0 < S; s0 += UPDATE_SPAN) {
+    const int total = list_members<RING_THREADS>(labels, s0, min(UPDATE_SPAN, S - s0), c, list, warp_total);
     count += total;
+    if (!in) continue;
     auto copy = [&](uint32_t dst, uint32_t member) {
-      const uint8_t* src = column + static_cast<uint64_t>(member) * pitch;
-      if constexpr (BYTES == 2) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-      else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(column + static_cast<uint64_t>(member) * pitch)
+                   : "memory");
     };
     auto fetch = [&](int first, int slot) {       // members first .. first + RING_GROUP - 1, a group always
       const uint32_t dst = my_ring + slot * RING_GROUP * RING_THREADS * PIECE;
@@ -456,23 +458,17 @@ kmeans_update_ring_kernel(const void* x, int S, int J, const int32_t* labels, fl
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto add = [&](const uint8_t* piece) {
-      float v[4];
-      if constexpr (BYTES == 2) {
-        const uint2 w = *reinterpret_cast<const uint2*>(piece);
-        v[0] = __uint_as_float(w.x << 16); v[1] = __uint_as_float(w.x & 0xFFFF0000u);
-        v[2] = __uint_as_float(w.y << 16); v[3] = __uint_as_float(w.y & 0xFFFF0000u);
-      } else {
-        const float4 w = *reinterpret_cast<const float4*>(piece);
-        v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) sum[q] = __fadd_rn(sum[q], v[q]);
+      const uint2 w = *reinterpret_cast<const uint2*>(piece);
+      sum[0] = __fadd_rn(sum[0], __uint_as_float(w.x << 16));
+      sum[1] = __fadd_rn(sum[1], __uint_as_float(w.x & 0xFFFF0000u));
+      sum[2] = __fadd_rn(sum[2], __uint_as_float(w.y << 16));
+      sum[3] = __fadd_rn(sum[3], __uint_as_float(w.y & 0xFFFF0000u));
     };
 #pragma unroll
-    for (int g = 0; g < GROUPS; ++g) fetch(g * RING_GROUP, g);
+    for (int g = 0; g < RING_GROUPS; ++g) fetch(g * RING_GROUP, g);
     int slot = 0;
     for (int i = 0; i < total; i += RING_GROUP) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(GROUPS - 1) : "memory");
+      asm volatile("cp.async.wait_group %0;" ::"n"(RING_GROUPS - 1) : "memory");
       const uint8_t* piece = &ring[slot * RING_GROUP][threadIdx.x * PIECE];
       if (i + RING_GROUP <= total) {
 #pragma unroll
@@ -480,8 +476,8 @@ kmeans_update_ring_kernel(const void* x, int S, int J, const int32_t* labels, fl
       } else {
         for (int k = 0; i + k < total; ++k) add(piece + k * RING_THREADS * PIECE);
       }
-      fetch(i + GROUPS * RING_GROUP, slot);
-      if (++slot == GROUPS) slot = 0;
+      fetch(i + RING_GROUPS * RING_GROUP, slot);
+      if (++slot == RING_GROUPS) slot = 0;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
@@ -764,18 +760,15 @@ int kmeans_gather_init(const void* x, int x_dtype, int J, int C, const int32_t* 
 
 int kmeans_update(const void* x, int x_dtype, int S, int J, int C, const int32_t* labels,
                   float* centers, uint16_t* planes, uint16_t* stored, cudaStream_t stream) {
-  // four or two columns per thread for bf16 and fp32 rows that start on a multiple of that many; every other
-  // form (fp16 rows among them) one column, converted by load_float
+  // four columns per thread for bf16 rows that start on a multiple of that many, two for the others and for fp32; every
+  // other form (fp16 rows among them) one column, converted by load_float
   const bool bf16 = x_dtype == NKV_BF16, f32 = x_dtype == NKV_F32;
-  auto fits = [&](int columns) {
-    return (bf16 || f32) && J % columns == 0 && reinterpret_cast<uintptr_t>(x) % (columns * (f32 ? 4 : 2)) == 0;
-  };
-  if (fits(4)) {
-    const dim3 grid(C, ceil_div(J, 4 * RING_THREADS));
-    auto kernel = f32 ? kmeans_update_ring_kernel<4> : kmeans_update_ring_kernel<2>;
-    kernel<<<grid, RING_THREADS, 0, stream>>>(x, S, J, labels, centers, planes, stored);
+  auto fits = [&](int columns) { return J % columns == 0 && reinterpret_cast<uintptr_t>(x) % (columns * (f32 ? 4 : 2)) == 0; };
+  if (bf16 && fits(4)) {
+    kmeans_update_ring_kernel<<<dim3(C, ceil_div(J, 4 * RING_THREADS)), RING_THREADS, 0, stream>>>(
+        static_cast<const uint16_t*>(x), S, J, labels, centers, planes, stored);
   } else {
-    const bool pairs = fits(2);
+    const bool pairs = (bf16 || f32) && fits(2);
     const dim3 grid(C, ceil_div(J, pairs ? 512 : 256));
     auto kernel = !pairs ? kmeans_update_kernel<Single> : (f32 ? kmeans_update_kernel<PairF32> : kmeans_update_kernel<PairBf16>);
     kernel<<<grid, 256, 0, stream>>>(x, x_dtype, S, J, labels, centers, planes, stored);
