@@ -43,7 +43,7 @@ constexpr int THREADS = COMPUTE_THREADS + 64;
 constexpr int MAX_STAGES = 8;
 constexpr int MAX_PARTS = 8;            // thread blocks of one token tile that form a cluster
 constexpr int MAX_MEAN = 8192;          // widest row whose mean is kept in shared memory
-enum Bar { FULL = 0, FORMED = 8, FREE = 16, ACC_DONE = 24, SIDE_READY = 25, PEER_READY = 26, NUM_BARS = 27 };
+enum Bar { FULL = 0, FORMED = 8, FREE = 16, B_FULL = 24, ACC_DONE = 32, SIDE_READY = 33, PEER_READY = 34, NUM_BARS = 35 };
 
 struct Meta {
   uint64_t bars[NUM_BARS];
@@ -56,7 +56,8 @@ struct Meta {
 struct Params {
   int S, J, rows, rows_pad, NB, NACC, n_total;          // n_total = r
   int parts, kc;            // column parts of a tile; 64-column chunks of a stage
-  int nstages, nchunks, tmem_columns, mean_bytes;       // mean_bytes 0: the mean is read where it lies
+  int nstages, units;       // stages of the ring; SPLIT: stages of token rows, and units of encoder rows
+  int nchunks, tmem_columns, mean_bytes;                // mean_bytes 0: the mean is read where it lies
   const uint16_t* centers; const void* ids; int id_bytes;
   const float* mean; uint16_t* coeff;
   // project + quantise: codes u8 [S, r/2] and scales [S, r/group] at the history's token offset
@@ -127,8 +128,13 @@ __device__ __forceinline__ uint4 pack_codes(const uint32_t (&w)[16], float scale
   return make_uint4(words[0], words[1], words[2], words[3]);
 }
 
-// SLOTS: rows of a stage's residual of which a thread forms 16 bytes, their centres fetched DEPTH stages ahead
-template <bool QUANT, int SLOTS, int DEPTH>
+// SLOTS: rows of a stage's residual of which a thread forms 16 bytes, their centres fetched DEPTH stages ahead.
+// SPLIT: token rows and encoder rows have rings of their own, the encoder's in units of one accumulator's columns, each
+// free as soon as its MMAs are done.  For tiles so wide that two whole stages is all that fits: with two, a stage is
+// loaded, formed and multiplied with only one other under way.  us, two whole stages / SPLIT: 12,480 x 2,048 x 512 43 / 35,
+// 12,480 x 3,072 x 1,024 122 / 98, 9,500 x 5,120 x 512 109 / 76.  With three whole stages and more one barrier for both
+// operands is as fast or faster (20,000 x 2,048 x 256 47, SPLIT 49; 4,680 x 5,120 x 640 59, SPLIT 62).
+template <bool QUANT, bool SPLIT, int SLOTS, int DEPTH>
 __global__ void __launch_bounds__(THREADS, 1)
 project_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ Params p) {
@@ -138,7 +144,9 @@ project_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   uint8_t* ring = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(mean_smem) + p.mean_bytes + 1023) & ~static_cast<uintptr_t>(1023));
   const int a_tile = p.rows_pad * 128, b_tile = p.NB * 128;       // one 64-column chunk; of one accumulator
-  const int kc = p.kc, a_bytes = kc * a_tile, stage_bytes = a_bytes + kc * p.NACC * b_tile;
+  const int kc = p.kc, a_bytes = kc * a_tile, stage_bytes = SPLIT ? a_bytes : a_bytes + kc * p.NACC * b_tile;
+  uint8_t* units = ring + p.nstages * a_bytes;                    // SPLIT: the encoder's ring
+  const int unit_bytes = kc * b_tile;
   const int nst = p.nstages, nchunks = p.nchunks, steps = (nchunks + kc - 1) / kc;
   uint64_t* bars = meta.bars;
   volatile int* abort_flag = &meta.abort_flag;
@@ -152,7 +160,8 @@ project_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     for (int s = 0; s < MAX_STAGES; ++s) {
       mbar_init(&bars[FULL + s], 1);
       mbar_init(&bars[FORMED + s], WARPS);
-      mbar_init(&bars[FREE + s], 1);
+      mbar_init(&bars[FREE + s], 1);                       // SPLIT: of a unit
+      mbar_init(&bars[B_FULL + s], 1);
     }
     mbar_init(&bars[ACC_DONE], 1);
     mbar_init(&bars[SIDE_READY], COMPUTE_THREADS);
@@ -190,7 +199,40 @@ project_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       prefetch_tensormap(&map_x);
       prefetch_tensormap(&map_b);
       Ring at;
-      for (int i = 0; i < steps && ok; ++i, at.advance(nst)) {
+      if constexpr (SPLIT) {
+        // chunks past the row's end arrive as zeros and are not used
+        const int all = steps * p.NACC;
+        int rows = 0, loaded = 0, row_place = 0, place = 0, column = 0, chunk = 0;
+        auto load_rows = [&] {
+          mbar_arrive_expect_tx(&bars[FULL + row_place], a_bytes);
+          tma_load_3d(ring + row_place * a_bytes, &map_x, 0, m0, rows++ * kc, &bars[FULL + row_place]);
+          if (++row_place == nst) row_place = 0;
+        };
+        auto load_unit = [&] {
+          mbar_arrive_expect_tx(&bars[B_FULL + place], unit_bytes);
+          tma_load_3d(units + place * unit_bytes, &map_b, 0, n_base + column, chunk, &bars[B_FULL + place]);
+          ++loaded;
+          if (++place == p.units) place = 0;
+          column += p.NB;
+          if (column == columns) { column = 0; chunk += kc; }
+        };
+        while (rows < min(nst, steps) || loaded < min(p.units, all)) {
+          if (rows < min(nst, steps)) load_rows();
+          if (loaded < min(p.units, all)) load_unit();
+        }
+        // a unit's MMAs done free its place, those of a stage's last unit the token rows' too
+        int acc = 0;
+        for (; ok && (rows < steps || loaded < all); at.advance(p.units)) {
+          ok = mbar_wait(&bars[FREE + at.stage], at.phase, abort_flag, 400 + at.stage);
+          if (!ok) break;
+          if (++acc == p.NACC) {
+            acc = 0;
+            if (rows < steps) load_rows();
+          }
+          if (loaded < all) load_unit();
+        }
+      }
+      for (int i = 0; !SPLIT && i < steps && ok; ++i, at.advance(nst)) {
         const int s = at.stage;
         if (i >= nst) ok = mbar_wait(&bars[FREE + s], at.phase ^ 1, abort_flag, 400 + s);
         if (!ok) break;
@@ -211,8 +253,33 @@ project_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const bool leader = elect_one();
     const uint32_t idesc = make_idesc_bf16(TM, p.NB);
     const uint32_t ring_base = smem_u32(ring);
+    if constexpr (SPLIT) {
+      const uint32_t unit_base = smem_u32(units);
+      Ring at, at_unit;
+      for (int i = 0; i < steps && ok; ++i, at.advance(nst)) {
+        ok = wait_all(&bars[FORMED + at.stage], at.phase, abort_flag, 410 + at.stage);
+        const uint32_t rows = ring_base + at.stage * a_bytes;
+        const int last = min(kc, nchunks - i * kc);
+        for (int a = 0; a < p.NACC && ok; ++a, at_unit.advance(p.units)) {
+          ok = wait_all(&bars[B_FULL + at_unit.stage], at_unit.phase, abort_flag, 420 + at_unit.stage);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t unit = unit_base + at_unit.stage * unit_bytes;
+          if (leader) {
+            for (int q = 0; q < last; ++q) {
+              const uint64_t a_desc = make_smem_desc_sw128(rows + q * a_tile);
+              const uint64_t b_desc = make_smem_desc_sw128(unit + q * b_tile);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) mma_bf16(tmem_base + a * 256, a_desc + 2 * k, b_desc + 2 * k, idesc, (i | q | k) != 0);
+            }
+            mma_commit(&bars[FREE + at_unit.stage]);
+          }
+          __syncwarp();
+        }
+      }
+    }
     Ring at;
-    for (int i = 0; i < steps && ok; ++i, at.advance(nst)) {
+    for (int i = 0; !SPLIT && i < steps && ok; ++i, at.advance(nst)) {
       const int s = at.stage;
       ok = wait_all(&bars[FORMED + s], at.phase, abort_flag, 410 + s);
       if (!ok) break;
@@ -421,6 +488,12 @@ size_t smem_bytes(int J, int rows_pad, int columns, int kc, int stages) {
   const size_t reach = last_a + TM * 128;
   return sizeof(Meta) + 16 + mean_bytes(J) + 1024 + (reach > end ? reach : end);
 }
+// the same for rings of their own
+size_t split_bytes(int J, int rows_pad, int nb, int kc, int stages, int units) {
+  const size_t tile = static_cast<size_t>(rows_pad) * 128, tiles = static_cast<size_t>(stages) * kc;
+  const size_t end = tiles * tile + static_cast<size_t>(units) * kc * nb * 128, reach = (tiles - 1) * tile + TM * 128;
+  return sizeof(Meta) + 16 + mean_bytes(J) + 1024 + (reach > end ? reach : end);
+}
 
 // Tokens per tile, column parts and chunks of a stage.  The estimate counts SM cycles.  A 64-column chunk costs the
 // longer of its bytes from L2 (encoder rows, x and centre rows) at 45 per clock and its MMAs (four in a chain of 86
@@ -454,9 +527,9 @@ Cut plan_project(int S, int J, int r, int first_parts, bool cluster) {
   return best;
 }
 
-template <bool QUANT, int SLOTS, int DEPTH>
+template <bool QUANT, bool SPLIT, int SLOTS, int DEPTH>
 int launch_slots(const CUtensorMap (&maps)[2], const Params& p, size_t smem, cudaStream_t stream) {
-  auto kernel = project_gemm_kernel<QUANT, SLOTS, DEPTH>;
+  auto kernel = project_gemm_kernel<QUANT, SPLIT, SLOTS, DEPTH>;
   NKV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(static_cast<unsigned>(ceil_div(p.S, p.rows)) * p.parts);
@@ -495,7 +568,18 @@ int launch_project(const void* x, const void* centers, const void* encoder, Para
   p.nchunks = p.J / 64;
   p.mean_bytes = static_cast<int>(mean_bytes(p.J));
   p.centers = static_cast<const uint16_t*>(centers);
-  const size_t smem = smem_bytes(p.J, p.rows_pad, columns, p.kc, p.nstages);
+  // two accumulators with room for two whole stages only (512 columns): as many units as fit beside their token rows,
+  // five or four, and token rows in the rest
+  const bool split = p.NACC == 2 && p.nstages == 2;
+  size_t smem = smem_bytes(p.J, p.rows_pad, columns, p.kc, p.nstages);
+  if (split) {
+    auto bytes = [&](int stages, int units) { return split_bytes(p.J, p.rows_pad, p.NB, p.kc, stages, units); };
+    p.units = MAX_STAGES;
+    while (p.units > 4 && bytes((p.units + 1) / 2, p.units) > SMEM_LIMIT) --p.units;
+    p.nstages = MAX_STAGES;
+    while (p.nstages > 2 && bytes(p.nstages, p.units) > SMEM_LIMIT) --p.nstages;
+    smem = bytes(p.nstages, p.units);
+  }
   NKV_REQUIRE(smem <= SMEM_LIMIT, NKV_ERR_UNSUPPORTED, "projection: %zu bytes of shared memory", smem);
   CUtensorMap maps[2];     // rows, encoder
   const uint64_t chunk_strides[2] = {static_cast<uint64_t>(p.J) * 2, 128};
@@ -512,9 +596,10 @@ int launch_project(const void* x, const void* centers, const void* encoder, Para
     if (rc != NKV_OK) return rc;
   }
   const int slots = ceil_div(p.rows_pad, COMPUTE_THREADS / 8 / p.kc);
-  if (slots <= 1) return launch_slots<QUANT, 1, 6>(maps, p, smem, stream);
-  if (slots <= 2) return launch_slots<QUANT, 2, 4>(maps, p, smem, stream);
-  return launch_slots<QUANT, 4, 3>(maps, p, smem, stream);
+  auto launch = slots <= 1   ? (split ? launch_slots<QUANT, true, 1, 6> : launch_slots<QUANT, false, 1, 6>)
+                : slots <= 2 ? (split ? launch_slots<QUANT, true, 2, 4> : launch_slots<QUANT, false, 2, 4>)
+                             : (split ? launch_slots<QUANT, true, 4, 3> : launch_slots<QUANT, false, 4, 3>);
+  return launch(maps, p, smem, stream);
 }
 
 }  // namespace
